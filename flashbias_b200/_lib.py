@@ -18,6 +18,7 @@ FB_FLAG_FORCE_GENERAL = 1
 FB_FLAG_BWD_QUERY_MAJOR = 2
 FB_FLAG_BWD_ONE_ITEM = 4
 FB_FLAG_BWD_PERSISTENT = 8
+FB_FLAG_BWD_FUSED_DELTA = 16
 
 I64x3 = C.c_int64 * 3
 

@@ -246,5 +246,6 @@ extern "C" int fb_bwd(const fb_params* p, void* cuda_stream) {
     return launch_bwd_sm100(p, plan, st);
   }
   if ((rc = check_workspace(p, bwd_general_workspace(p)))) return rc;
+  if (fused_delta(p) && (rc = launch_bwd_preprocess(p, st))) return rc;
   return launch_bwd_general(p, st);
 }

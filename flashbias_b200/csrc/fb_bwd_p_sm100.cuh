@@ -18,17 +18,6 @@
 
 namespace fb {
 
-// n / d for 0 <= n < 2^31 with (m, s) from fast_div_magic(d): one multiply-high, one add, one shift
-__device__ __forceinline__ int fast_div(int n, const uint32_t (&ms)[2]) {
-  return (int)((__umulhi((uint32_t)n, ms[0]) + (uint32_t)n) >> ms[1]);
-}
-inline void fast_div_magic(int d, uint32_t (&ms)[2]) {
-  uint32_t s = 0;
-  while ((1u << s) < (uint32_t)d) ++s;  // ceil(log2 d)
-  ms[0] = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << s) - (uint64_t)d)) / (uint64_t)d + 1);
-  ms[1] = s;
-}
-
 // one work item of the backward: a tile of 128 keys of one (batch, head) and the query tiles that see it
 struct BwdItem {
   int kt, bh, b, h, k0, i_begin, n_it;
@@ -40,7 +29,7 @@ struct BwdItem {
 struct BwdPArgs {
   int total_items;   // (key tile, batch, head) work items = nk_tiles * B * H
   int active_items;  // the first so many have query tiles to visit (all of them unless causal with Sq < Sk)
-  uint32_t div_bh[2], div_nk[2], div_h[2];  // (multiplier, shift) of the divisions by B*H, nk_tiles and H
+  Div div_bh, div_nk, div_h;  // divisions by B*H, nk_tiles and H
 };
 
 template <typename T, int D, int RP, int NQ, int MODE>
@@ -84,13 +73,13 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int idx = w * G + ((w & 1) ? G - 1 - c : c);
     x.valid = idx < limit;
     if (a.causal) {
-      x.kt = fast_div(idx, pa.div_bh);
+      x.kt = (int)pa.div_bh.quot(idx);
       x.bh = idx - x.kt * BH;
     } else {
-      x.bh = fast_div(idx, pa.div_nk);
+      x.bh = (int)pa.div_nk.quot(idx);
       x.kt = idx - x.bh * a.nk_tiles;
     }
-    x.b = fast_div(x.bh, pa.div_h);
+    x.b = (int)pa.div_h.quot(x.bh);
     x.h = x.bh - x.b * a.H;
     x.k0 = x.kt * 128;
     x.i_begin = a.causal ? x.kt : 0;    // first query tile with a row >= k0
@@ -174,6 +163,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                                            // different times
       }
       mbar_fence_init();
+      grid_dep_wait();
       // the first loads start before the rest of the CTA has finished its set-up
       lx = next_active(lw);
       if (lx.valid) {
@@ -186,6 +176,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dep_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -799,9 +790,9 @@ int launch_bwd_p(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     BwdPArgs pa;
     pa.total_items = (int)((int64_t)a.nk_tiles * p->B * p->H);
     pa.active_items = (p->causal && a.nq_tiles < a.nk_tiles ? a.nq_tiles : a.nk_tiles) * p->B * p->H;
-    fast_div_magic(p->B * p->H, pa.div_bh);
-    fast_div_magic(a.nk_tiles, pa.div_nk);
-    fast_div_magic(p->H, pa.div_h);
+    pa.div_bh = Div(p->B * p->H);
+    pa.div_nk = Div(a.nk_tiles);
+    pa.div_h = Div(p->H);
     CUtensorMap tDK, tDV;  // dK and dV leave through tile stores
     if ((rc = make_tmap_4d(&tDK, p->dk, D, p->Sk, p->H, p->B, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], D, 128)))
       return rc;
@@ -826,10 +817,9 @@ int launch_bwd_p(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     // one CTA per SM (or fewer, if there are fewer work items)
     const unsigned grid = (unsigned)(pa.total_items < sms ? pa.total_items : sms);
     prof_before(KC_BWD_MAIN, st);
-    kern<<<grid, 512, Cfg::SMEM, st>>>(L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, L.tKs, tDK, tDV, a, pa);
+    rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, L.tKs, tDK, tDV, a, pa);
     prof_after(KC_BWD_MAIN, st);
-    note_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+    if (rc) return rc;
     return bwd_finish<T, D, RP, NQ>(p, L, st);
   }
 }

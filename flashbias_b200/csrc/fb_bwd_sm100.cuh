@@ -155,13 +155,6 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Byte offset of 16-byte chunk `ch` of row `r` in a staged [128][D] fp32 dQ tile: 128-byte lines, chunks XOR-swizzled
-// by row so that one row per thread writes without bank conflicts.  The fp32 dQ accumulator in global memory keeps
-// this arrangement per (batch, head, query tile) when the tile is reduced in bulk.
-__host__ __device__ __forceinline__ int dq_stage_off(int r, int ch) {
-  return (ch >> 3) * (128 * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
-}
-
 // dq_bias of one query tile, one thread per query row: dq_bias = dS . k_bias, evaluated per group of 32 keys as
 // dS16 . (k_bias - c) + c * rowsum_fp32(dS) with c the k_bias of the group's middle key (rows of dS sum to ~0, so
 // rounding dS to 16 bits against a large, slowly varying factor -- ALiBi positions -- would otherwise dominate the
@@ -280,6 +273,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                            // different times
       }
       mbar_fence_init();
+      grid_dep_wait();
       if (n_it > 0) {
         // the first loads start before the rest of the CTA has finished its set-up
         const int hk = a.hk_bcast ? 0 : h, bk = a.bk_bcast ? 0 : b;
@@ -300,6 +294,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dep_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -808,37 +803,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-// dq = T(scale * acc).  acc is fp32, laid out (B, Sq, H, D), or -- `tiled` -- per (batch, head, query tile) as the
-// staged [128][D] tile of dq_stage_off.
-template <typename T>
-__global__ void __launch_bounds__(256) dq_store_kernel(const float* __restrict__ acc, T* __restrict__ dq, int B, int Sq,
-                                                       int H, int D, int64_t sb, int64_t sh, int64_t ss, float scale,
-                                                       int tiled) {
-  const int64_t idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;  // 8 consecutive d
-  const int64_t total = (int64_t)B * Sq * H * D;
-  if (idx >= total) return;
-  const int d = (int)(idx % D);
-  const int h = (int)((idx / D) % H);
-  const int s = (int)((idx / ((int64_t)D * H)) % Sq);
-  const int b = (int)(idx / ((int64_t)D * H * Sq));
-  float4 x, y;
-  if (tiled) {
-    const int nq_tiles = (Sq + 127) / 128;
-    const char* tile = reinterpret_cast<const char*>(acc + (((int64_t)b * H + h) * nq_tiles + s / 128) * (128 * D));
-    x = *reinterpret_cast<const float4*>(tile + dq_stage_off(s % 128, d / 4));
-    y = *reinterpret_cast<const float4*>(tile + dq_stage_off(s % 128, d / 4 + 1));
-  } else {
-    x = *reinterpret_cast<const float4*>(acc + idx);
-    y = *reinterpret_cast<const float4*>(acc + idx + 4);
-  }
-  uint4 w;
-  w.x = Pack2<T>::pack(x.x * scale, x.y * scale);
-  w.y = Pack2<T>::pack(x.z * scale, x.w * scale);
-  w.z = Pack2<T>::pack(y.x * scale, y.y * scale);
-  w.w = Pack2<T>::pack(y.z * scale, y.w * scale);
-  *reinterpret_cast<uint4*>(dq + b * sb + h * sh + s * ss + d) = w;
-}
-
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
@@ -964,10 +928,8 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
   a.mask_batch_period = p->mask_batch_period;
   a.alibi_slopes = p->alibi_slopes;
   // launches last: the tensor maps and arguments above are ready when the main kernel's turn comes
-  if ((rc = launch_pack_operands(p, plan, qpack, kpack, kcenter, true, ws + w.off_qs, st))) return rc;
-  cudaError_t e = cudaMemsetAsync(ws + w.off_dq, 0, w.zero_bytes, st);
-  if (e != cudaSuccess) return (int)e;
-  return 0;
+  return launch_prepare(p, plan, {qpack, kpack, kcenter, ws + w.off_qs, true, fused_delta(p), ws + w.off_dq, w.zero_bytes},
+                        st);
 }
 
 // Host work after the main kernel: dq and the factor gradients leave their fp32 accumulators.
@@ -975,18 +937,10 @@ template <typename T, int D, int RP, int NQ>
 int bwd_finish(const fb_params* p, const BwdLaunch& L, cudaStream_t st) {
   using Cfg = BwdCfg<D, RP, NQ>;
   const BwdArgs& a = L.a;
-  cudaError_t e;
-  const int64_t n8 = ((int64_t)p->B * p->Sq * p->H * D) / 8;
-  dq_store_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(
-      a.dq_acc, reinterpret_cast<T*>(p->dq), p->B, p->Sq, p->H, D, p->dq_stride[0], p->dq_stride[1], p->dq_stride[2],
-      p->softmax_scale, Cfg::STAGED ? 1 : 0);
-  note_launch();
-  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-  if (p->R > 0)
-    return store_factor_grads_from(p, a.dqb_acc, a.dkb_acc, st,
-                                   {(int64_t)a.nq_tiles * 128, a.dqb_slots, a.dqb_slot_stride},
-                                   {(int64_t)a.nk_tiles * 128, a.dkb_slots, a.dkb_slot_stride});
-  return 0;
+  return launch_store_grads(p, {a.dq_acc, Cfg::STAGED ? 1 : 0, a.dqb_acc, a.dkb_acc,
+                                {(int64_t)a.nq_tiles * 128, a.dqb_slots, a.dqb_slot_stride},
+                                {(int64_t)a.nk_tiles * 128, a.dkb_slots, a.dkb_slot_stride}},
+                            st);
 }
 
 template <typename T, int D, int RP, int NQ, int MODE>
@@ -1016,10 +970,9 @@ int launch_bwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   }
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);
   prof_before(KC_BWD_MAIN, st);
-  kern<<<grid, 512, Cfg::SMEM, st>>>(L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, L.tKs, a);
+  rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, L.tKs, a);
   prof_after(KC_BWD_MAIN, st);
-  note_launch();
-  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+  if (rc) return rc;
   return bwd_finish<T, D, RP, NQ>(p, L, st);
   }
 }

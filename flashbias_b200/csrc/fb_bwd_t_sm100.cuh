@@ -119,6 +119,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_init(pds_ready + 8 * i, 8);   // the compute warps; alternating by query tile
       }
       mbar_fence_init();
+      grid_dep_wait();
       if (n_it > 0) {
         mbar_expect_tx(kv_full, Cfg::KV_BYTES);
         tma_tile_bwd<D>(sK, &tmK, kv_full, k0, h, b);
@@ -130,6 +131,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
+  grid_dep_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -515,8 +517,6 @@ int launch_bwd_t_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   int rc;
   const BwdWs w = bwd_layout(p, plan);
   uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
-  cudaError_t e = cudaMemsetAsync(ws + w.off_dq, 0, w.zero_bytes, st);
-  if (e != cudaSuccess) return (int)e;
   CUtensorMap tQ, tK, tV, tDO;
   if ((rc = make_tmap_4d(&tQ, p->q, D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, 128)))
     return rc;
@@ -561,23 +561,19 @@ int launch_bwd_t_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!attr_done[dev & 63]) {
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
       if (e != cudaSuccess) return (int)e;
       attr_done[dev & 63] = true;
     }
   }
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);
+  if ((rc = launch_prepare(p, plan, {nullptr, nullptr, nullptr, nullptr, true, fused_delta(p), ws + w.off_dq, w.zero_bytes}, st)))
+    return rc;
   prof_before(KC_BWD_MAIN, st);
-  kern<<<grid, 512, Cfg::SMEM, st>>>(tQ, tK, tV, tDO, a);
+  rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, tQ, tK, tV, tDO, a);
   prof_after(KC_BWD_MAIN, st);
-  note_launch();
-  if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-  const int64_t n8 = ((int64_t)p->B * p->Sq * p->H * D) / 8;
-  dq_store_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(
-      a.dq_acc, reinterpret_cast<T*>(p->dq), p->B, p->Sq, p->H, D, p->dq_stride[0], p->dq_stride[1], p->dq_stride[2],
-      p->softmax_scale, 1);
-  note_launch();
-  return (int)cudaGetLastError();
+  if (rc) return rc;
+  return launch_store_grads(p, {a.dq_acc, 1, nullptr, nullptr, {}, {}}, st);
 }
 
 }  // namespace fb

@@ -99,6 +99,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // ---------------------------------------------------------------------------------------------
+// Programmatic dependent launch
+// ---------------------------------------------------------------------------------------------
+// Waits until the grids this one depends on have completed and their writes are visible.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The dependent grid may be scheduled once every CTA of this one has got here (or exited).
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------------------------
 // Fences
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -465,6 +473,13 @@ __device__ __forceinline__ uint32_t tile_chunk_offset(int row, int col) {
   // 128B swizzle XORs the chunk index with row%8; 64B with (row/2)%4; 32B with (row/4)%2.
   const int x = SWB == 128 ? (row & 7) : SWB == 64 ? ((row >> 1) & 3) : SWB == 32 ? ((row >> 2) & 1) : 0;
   return blk * (128 * SWB) + row * SWB + (((chunk ^ x) & (CHUNKS - 1)) << 4);
+}
+
+// Byte offset of 16-byte chunk `ch` of row `r` in a staged [128][D] fp32 dQ tile: 128-byte lines, chunks XOR-swizzled
+// by row so that one row per thread writes without bank conflicts.  The fp32 dQ accumulator in global memory keeps
+// this arrangement per (batch, head, query tile) when the tile is reduced in bulk.
+__host__ __device__ __forceinline__ int dq_stage_off(int r, int ch) {
+  return (ch >> 3) * (128 * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
 }
 
 }  // namespace fb

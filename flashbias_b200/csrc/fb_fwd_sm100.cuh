@@ -171,6 +171,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tmem_alloc(smem_u32(tmem_slot), Cfg::TMEM_COLS);
     tmem_relinquish();
   }
+  grid_dep_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -538,7 +539,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     a.alibi_slopes = p->alibi_slopes;
     // (the tensor maps above are encoded first: the host then has the main kernel's launch ready while the operand
     // preparation runs)
-    if ((rc = launch_pack_operands(p, plan, qpack, kpack, nullptr, false, qs, st))) return rc;
+    if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, qs, false, nullptr, nullptr, 0}, st))) return rc;
     auto kern = fwd_sm100_kernel<T, D, RP, NQ, ALIBI>;
     // per kernel instantiation and device: raise the dynamic shared-memory limit once
     static std::mutex mu;
@@ -560,10 +561,9 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     const int slots = sm_count[dev & 63] * Cfg::MINB;
     const unsigned grid = (unsigned)(a.total_items < slots ? a.total_items : slots);
     prof_before(KC_FWD_MAIN, st);
-    kern<<<grid, 256, Cfg::SMEM, st>>>(tQ, tK, tV, tQb, tKb, a);
+    rc = launch_pdl(kern, grid, 256, Cfg::SMEM, st, tQ, tK, tV, tQb, tKb, a);
     prof_after(KC_FWD_MAIN, st);
-    note_launch();
-    return (int)cudaGetLastError();
+    return rc;
   }
 }
 

@@ -107,34 +107,6 @@ __global__ void __launch_bounds__(kWarps * 32) fwd_general_kernel(const fb_param
   if (lane == 0) p.lse[(int64_t)bh * p.lse_stride_bh + i] = l > 0.f ? m + logf(l) : -INFINITY;
 }
 
-// delta[bh, i] = sum_d o[i, d] * dout[i, d]
-template <typename T>
-__global__ void __launch_bounds__(256) bwd_preprocess_kernel(const fb_params p) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // (b, i, h), h fastest
-  const int64_t total = (int64_t)p.B * p.Sq * p.H;
-  if (idx >= total) return;
-  const int h = (int)(idx % p.H);
-  const int i = (int)((idx / p.H) % p.Sq);
-  const int b = (int)(idx / ((int64_t)p.H * p.Sq));
-  const T* orow = row_ptr<T>(p.o, p.o_stride, b, h, i);
-  const T* drow = row_ptr<T>(p.dout, p.dout_stride, b, h, i);
-  float acc = 0.f;
-  const bool vec = (p.D % 8 == 0) && ((reinterpret_cast<uintptr_t>(orow) | reinterpret_cast<uintptr_t>(drow)) & 15) == 0;
-  if (vec) {
-    for (int d = 0; d < p.D; d += 8) {
-      const uint4 a = *reinterpret_cast<const uint4*>(orow + d);
-      const uint4 c = *reinterpret_cast<const uint4*>(drow + d);
-      const T* pa = reinterpret_cast<const T*>(&a);
-      const T* pc = reinterpret_cast<const T*>(&c);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc += to_f32(pa[e]) * to_f32(pc[e]);
-    }
-  } else {
-    for (int d = 0; d < p.D; ++d) acc += to_f32(orow[d]) * to_f32(drow[d]);
-  }
-  p.delta[((int64_t)b * p.H + h) * p.lse_stride_bh + i] = acc;
-}
-
 // fp32 accumulators of the factor gradients live in the workspace, un-expanded (broadcast dims of
 // size 1), contiguous (Bx, S, Hx, R).
 struct FactorAcc {
@@ -327,79 +299,12 @@ __global__ void __launch_bounds__(kWarps * 32) bwd_dkv_general_kernel(const fb_p
   }
 }
 
-// fp32 accumulator -> 16-bit gradient tensor with the factor's own strides.  The accumulator is addressed
-// (b, h, s, r) through element strides (ab, ah, as, ar): (Bx, S, Hx, R), or -- `tiled` -- head-major in tiles of
-// 128 rows stored rank-major, [r][row in tile] (the tensor-core backward stages its tiles that way: consecutive
-// rows are consecutive floats, which keeps the threads' shared-memory stores free of bank conflicts); `slots`
-// copies at distance `slot_stride` are summed.
-template <typename T>
-struct FactorStoreJob {
-  const float* acc;
-  int64_t ab, ah, as;
-  int tiled, slots;
-  int64_t slot_stride;
-  T* out;
-  int Bx, S, Hx;
-  int64_t sb, sh, ss;
-};
-
-// One launch for both factors: blocks [0, nbq) store dq_bias, the rest dk_bias.
-template <typename T>
-__global__ void __launch_bounds__(256) factor_grad_store_kernel(FactorStoreJob<T> jq, FactorStoreJob<T> jk, unsigned nbq,
-                                                                int R) {
-  const bool is_q = blockIdx.x < nbq;
-  const FactorStoreJob<T>& j = is_q ? jq : jk;
-  const int64_t idx = (int64_t)(is_q ? blockIdx.x : blockIdx.x - nbq) * blockDim.x + threadIdx.x;
-  const int64_t total = (int64_t)j.Bx * j.S * j.Hx * R;
-  if (idx >= total) return;
-  const int r = (int)(idx % R);
-  const int h = (int)((idx / R) % j.Hx);
-  const int s = (int)((idx / ((int64_t)R * j.Hx)) % j.S);
-  const int b = (int)(idx / ((int64_t)R * j.Hx * j.S));
-  const float* src = j.tiled ? j.acc + b * j.ab + h * j.ah + (int64_t)(s / 128) * (128 * R) + r * 128 + (s % 128)
-                             : j.acc + b * j.ab + h * j.ah + s * j.as + r;
-  float v = 0.f;
-  for (int e = 0; e < j.slots; ++e) v += src[e * j.slot_stride];
-  j.out[b * j.sb + h * j.sh + s * j.ss + r] = from_f32<T>(v);
-}
-
 size_t bwd_general_workspace(const fb_params* p) {
   if (p->R <= 0) return 0;
   const FactorAcc fa = factor_acc(*p);
   const size_t nq = (((size_t)fa.Bq * p->Sq * fa.Hq * p->R) + 63) & ~size_t(63);
   const size_t nk = (((size_t)fa.Bk * p->Sk * fa.Hk * p->R) + 63) & ~size_t(63);
   return round256((nq + nk) * sizeof(float));
-}
-
-template <typename T>
-static FactorStoreJob<T> factor_store_job(const float* acc, FactorAccLayout l, T* out, int Bx, int S, int Hx, int R,
-                                          const int64_t* stride) {
-  if (l.rows > 0)  // (slots, Bx, Hx, rows, R)
-    return {acc, Hx * l.rows * R, l.rows * R, R, 1, l.slots, l.slot_stride, out, Bx, S, Hx, stride[0], stride[1], stride[2]};
-  // (Bx, S, Hx, R)
-  return {acc, (int64_t)S * Hx * R, R, (int64_t)Hx * R, 0, 1, 0, out, Bx, S, Hx, stride[0], stride[1], stride[2]};
-}
-
-template <typename T>
-static int launch_store_factor_grads(const fb_params* p, float* dqb, float* dkb, cudaStream_t st,
-                                     FactorAccLayout ql, FactorAccLayout kl) {
-  const FactorAcc fa = factor_acc(*p);
-  const FactorStoreJob<T> jq = factor_store_job<T>(dqb, ql, reinterpret_cast<T*>(p->dq_bias), fa.Bq, p->Sq, fa.Hq, p->R,
-                                                   p->dq_bias_stride);
-  const FactorStoreJob<T> jk = factor_store_job<T>(dkb, kl, reinterpret_cast<T*>(p->dk_bias), fa.Bk, p->Sk, fa.Hk, p->R,
-                                                   p->dk_bias_stride);
-  const unsigned nbq = (unsigned)(((int64_t)fa.Bq * p->Sq * fa.Hq * p->R + 255) / 256);
-  const unsigned nbk = (unsigned)(((int64_t)fa.Bk * p->Sk * fa.Hk * p->R + 255) / 256);
-  factor_grad_store_kernel<T><<<nbq + nbk, 256, 0, st>>>(jq, jk, nbq, p->R);
-  note_launch();
-  return (int)cudaGetLastError();
-}
-
-// Round the fp32 factor-gradient accumulators into dq_bias / dk_bias.
-int store_factor_grads_from(const fb_params* p, float* dqb, float* dkb, cudaStream_t st, FactorAccLayout q_layout,
-                            FactorAccLayout k_layout) {
-  return p->dtype == FB_DTYPE_F16 ? launch_store_factor_grads<__half>(p, dqb, dkb, st, q_layout, k_layout)
-                                  : launch_store_factor_grads<__nv_bfloat16>(p, dqb, dkb, st, q_layout, k_layout);
 }
 
 int launch_fwd_general(const fb_params* p, cudaStream_t st) {
@@ -411,19 +316,6 @@ int launch_fwd_general(const fb_params* p, cudaStream_t st) {
   else
     fwd_general_kernel<__nv_bfloat16><<<blocks, kWarps * 32, 0, st>>>(*p);
   prof_after(KC_FWD_MAIN, st);
-  note_launch();
-  return (int)cudaGetLastError();
-}
-
-int launch_bwd_preprocess(const fb_params* p, cudaStream_t st) {
-  const int64_t rows = (int64_t)p->B * p->H * p->Sq;
-  const unsigned blocks = (unsigned)((rows + 255) / 256);
-  prof_before(KC_BWD_PREPROCESS, st);
-  if (p->dtype == FB_DTYPE_F16)
-    bwd_preprocess_kernel<__half><<<blocks, 256, 0, st>>>(*p);
-  else
-    bwd_preprocess_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(*p);
-  prof_after(KC_BWD_PREPROCESS, st);
   note_launch();
   return (int)cudaGetLastError();
 }
@@ -449,7 +341,7 @@ int launch_bwd_general(const fb_params* p, cudaStream_t st) {
   if (e != cudaSuccess) return (int)e;
   if (p->R <= 0) return 0;
   const FactorAcc fa = factor_acc(*p);
-  return store_factor_grads_from(p, fa.dqb, fa.dkb, st);
+  return launch_store_grads(p, {nullptr, 0, fa.dqb, fa.dkb, {0, 1, 0}, {0, 1, 0}}, st);
 }
 
 }  // namespace fb

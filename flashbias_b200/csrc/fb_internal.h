@@ -10,6 +10,24 @@
 
 namespace fb {
 
+// Division by a launch constant: multiply-high, add and shift while the dividend is below 2^31 (every index of the
+// sizes that occur; four 64-bit divisions per thread cost the elementwise passes more than their memory traffic), the
+// 64-bit division beyond.
+struct Div {
+  uint32_t d, m, s;
+  Div() = default;
+  explicit Div(int d_) : d((uint32_t)d_), m(0), s(0) {
+    while ((1u << s) < d) ++s;  // ceil(log2 d)
+    m = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << s) - d)) / d + 1);
+  }
+#ifdef __CUDACC__
+  __device__ __forceinline__ int64_t quot(int64_t n) const {
+    if (n < 0x80000000LL) return (int64_t)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s);
+    return n / d;
+  }
+#endif
+};
+
 // ---- tensor maps (fb_tmap.cu) ---------------------------------------------------------------
 // Tiled tensor map over a 16-bit tensor addressed (col, row, head, batch); strides in elements.
 // Box = (box_cols x box_rows x 1 x 1), swizzle chosen from box_cols (32/64/128 bytes).
@@ -39,11 +57,20 @@ struct PackPlan {
 };
 // false if the rank does not fit the tensor path; for_bwd reserves room for the centred (hi, lo) k-side copy
 bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd = false);
-// One launch prepares every operand of a call: packed q/k factors, kcenter (optional, rows of plan.RC columns:
-// k_bias minus the k_bias of the middle key of each group of 32 keys) and, when plan.nq == 2, the (hi, lo) split
-// of q*scale (forward) or k*scale (backward; scaled_is_key), laid out (B, H, S, 2D).
-int launch_pack_operands(const fb_params* p, const PackPlan& plan, void* qpack, void* kpack, void* kcenter,
-                         bool scaled_is_key, void* scaled, cudaStream_t st);
+// What one launch prepares for a call: packed q/k factors, kcenter (optional, rows of plan.RC columns: k_bias minus the
+// k_bias of the middle key of each group of 32 keys), when plan.nq == 2 the (hi, lo) split of q*scale (forward) or
+// k*scale (backward; scaled_is_key), laid out (B, H, S, 2D), and for the backward delta (optional) and the zeroed
+// accumulators.
+struct PrepBuffers {
+  void *qpack, *kpack, *kcenter, *scaled;
+  bool scaled_is_key;
+  float* delta;
+  void* zero;
+  size_t zero_bytes;
+};
+int launch_prepare(const fb_params* p, const PackPlan& plan, const PrepBuffers& buf, cudaStream_t st);
+// where fb_bwd takes delta itself (null: the caller has run fb_bwd_preprocess)
+inline float* fused_delta(const fb_params* p) { return (p->flags & FB_FLAG_BWD_FUSED_DELTA) ? p->delta : nullptr; }
 
 // ---- kernels ------------------------------------------------------------------------------------
 int launch_fwd_general(const fb_params* p, cudaStream_t st);
@@ -68,8 +95,15 @@ struct FactorAccLayout {
   int slots;            // copies to sum
   int64_t slot_stride;  // floats between copies
 };
-int store_factor_grads_from(const fb_params* p, float* dqb, float* dkb, cudaStream_t st,
-                            FactorAccLayout q_layout = {0, 1, 0}, FactorAccLayout k_layout = {0, 1, 0});
+// The fp32 accumulators of a backward; launch_store_grads rounds them into p->dq (unless dq is null: the main kernel
+// has stored it), p->dq_bias and p->dk_bias.
+struct GradAccs {
+  const float* dq;
+  int dq_tiled;  // per (batch, head, query tile) as dq_stage_off arranges it, else (B, Sq, H, D)
+  const float *dqb, *dkb;
+  FactorAccLayout dqb_layout, dkb_layout;
+};
+int launch_store_grads(const fb_params* p, const GradAccs& g, cudaStream_t st);
 
 // ---- instrumentation (fb_api.cu) ----------------------------------------------------------------
 // Every kernel launch of the library is counted; while profiling is armed for a kernel class, a pair
@@ -80,5 +114,24 @@ void note_launch(int n = 1);
 int device_sm_count(int dev);
 void prof_before(int kernel_class, cudaStream_t st);
 void prof_after(int kernel_class, cudaStream_t st);
+
+// Launch with programmatic stream serialization: the grid may be set up while the kernel before it in the stream
+// drains.  Every kernel launched this way executes grid_dep_wait() before it touches global memory.
+template <typename... P, typename... A>
+int launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  if (e == cudaSuccess) note_launch();
+  return (int)e;
+}
 
 }  // namespace fb

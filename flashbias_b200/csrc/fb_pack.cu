@@ -62,99 +62,111 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   return true;
 }
 
-// One factor: (Bx, Hx, S, R) with strides -> packed rows (and the centred copy for the k side of the backward).
+// One factor: (Bx, Hx, S, R) with strides -> rows of W packed columns.
 template <typename T>
 struct FactorJob {
   const T* src;
   int64_t sb, sh, ss;
-  int Bx, Hx, S;
+  int S, W;
   float mult;
+  bool vec;       // rows are whole, 16-byte aligned groups of 8 elements
+  bool centered;  // the centred (hi, lo) copy instead of the factor itself
   T* dst;
-  T* dst_centered;
+  Div div_w8, div_s, div_h;  // divisions by W/8 (threads per row), S and Hx
+  int64_t units;             // threads: rows x W/8
 };
 // One tensor scaled and split: (B, H, S, D) with strides -> (B, H, S, 2D) = [hi | lo] of x * scale.
 template <typename T>
 struct ScaledJob {
   const T* src;
   int64_t sb, sh, ss;
-  int S;
-  T* dst;  // nullptr: no such job
+  int S, D;
+  T* dst;
+  Div div_d8, div_s, div_h;
+  int64_t units;  // rows x D/8
+};
+// delta[bh, i] = sum_d o[i, d] * dout[i, d]: G threads per row
+template <typename T>
+struct DeltaJob {
+  const T *o, *dout;
+  int64_t o_st[3], do_st[3];
+  int D, G, H;
+  bool vec;
+  float* delta;
+  int64_t stride_bh;
+  Div div_g, div_h, div_s;
+  int64_t units;  // rows x G, head fastest
 };
 
-// One thread per (b, h, s) row; the packed row is built 8 columns (one 16-byte store) at a time.
+// One thread per 8 packed columns (one 16-byte store): consecutive threads write consecutive chunks of a row and read
+// its elements side by side, so both sides coalesce whatever the rank (a thread per row took 26 us for the 3 x 1536 x 16
+// rows of rank 32, all of it in serial, strided requests; this form 4).
 template <typename T>
-__device__ __forceinline__ void pack_factor_row(const FactorJob<T>& j, int64_t idx, int R, int RP, int RC, int* status) {
-  const T* __restrict__ src = j.src;
-  const int64_t sb = j.sb, sh = j.sh, ss = j.ss;
-  const int Hx = j.Hx, S = j.S;
-  const float mult = j.mult;
-  T* __restrict__ dst = j.dst;
-  T* __restrict__ dst_centered = j.dst_centered;
-  const int64_t total = (int64_t)j.Bx * Hx * S;
-  if (idx >= total) return;
-  const int s = (int)(idx % S);
-  const int h = (int)((idx / S) % Hx);
-  const int b = (int)(idx / ((int64_t)S * Hx));
-  const T* in = src + b * sb + h * sh + s * ss;
-  bool overflow = false;
-  for (int c0 = 0; c0 < RP; c0 += 8) {
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    T* y = reinterpret_cast<T*>(&w);
+__device__ __forceinline__ void pack_factor_chunk(const FactorJob<T>& j, int64_t idx, int R, int* status) {
+  if (idx >= j.units) return;
+  const int64_t row = j.div_w8.quot(idx);
+  const int c0 = (int)(idx - row * j.div_w8.d) * 8;
+  const int64_t bh = j.div_s.quot(row);
+  const int s = (int)(row - bh * j.S);
+  const int64_t b = j.div_h.quot(bh);
+  const int h = (int)(bh - b * j.div_h.d);
+  const T* base = j.src + b * j.sb + h * j.sh;
+  const T* in = base + (int64_t)s * j.ss;
+  uint4 w = make_uint4(0u, 0u, 0u, 0u);
+  T* y = reinterpret_cast<T*>(&w);
+  if (!j.centered) {
+    bool overflow = false;
+    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+    T* e = reinterpret_cast<T*>(&raw);
+    if (j.vec) {
+      if (c0 < R) raw = *reinterpret_cast<const uint4*>(in + c0);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + i < R) e[i] = in[c0 + i];
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int c = c0 + i;
-      if (c < R) {
-        const float x = to_f32(in[c]);
-        y[i] = from_f32<T>(x * mult);  // mult is 1 or a power of two: exact unless it overflows
+      if (c0 + i < R) {
+        const float x = to_f32(e[i]);
+        y[i] = from_f32<T>(x * j.mult);  // mult is 1 or a power of two: exact unless it overflows
         overflow |= !isfinite(to_f32(y[i])) && isfinite(x);
       }
     }
-    *reinterpret_cast<uint4*>(dst + idx * RP + c0) = w;
-  }
-  if (overflow && status) atomicExch(status, FB_DEV_FACTOR_OVERFLOW);
-  if (dst_centered) {
+    if (overflow && status) atomicExch(status, FB_DEV_FACTOR_OVERFLOW);
+  } else {
     // k-side factor minus the factor of the middle key of its group of 32 keys: small-magnitude copy used
     // for dq_bias = dS.k_bias (the removed constant is re-applied in fp32 through the row sum of dS);
-    // two-term split: columns [0,R) hi, [RC/2, RC/2 + R) lo, zero elsewhere
-    int s0 = (s & ~31) + 16;
-    if (s0 > S - 1) s0 = S - 1;
-    const T* in0 = src + b * sb + h * sh + (int64_t)s0 * ss;
-    for (int c0 = 0; c0 < RC; c0 += 8) {
-      uint4 w = make_uint4(0u, 0u, 0u, 0u);
-      T* y = reinterpret_cast<T*>(&w);
+    // two-term split: columns [0,R) hi, [W/2, W/2 + R) lo, zero elsewhere
+    const T* in0 = base + (int64_t)min((s & ~31) + 16, j.S - 1) * j.ss;
+    const bool lo = c0 >= j.W / 2;
+    const int cc0 = lo ? c0 - j.W / 2 : c0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = c0 + i;
-        const bool lo = c >= RC / 2;
-        const int cc = lo ? c - RC / 2 : c;
-        if (cc < R) {
-          const float x = to_f32(in[cc]) - to_f32(in0[cc]);
-          const T hi = from_f32<T>(x);
-          y[i] = lo ? from_f32<T>(x - to_f32(hi)) : hi;
-        }
+    for (int i = 0; i < 8; ++i) {
+      const int cc = cc0 + i;
+      if (cc < R) {
+        const float x = to_f32(in[cc]) - to_f32(in0[cc]);
+        const T hi = from_f32<T>(x);
+        y[i] = lo ? from_f32<T>(x - to_f32(hi)) : hi;
       }
-      *reinterpret_cast<uint4*>(dst_centered + idx * RC + c0) = w;
     }
   }
+  *reinterpret_cast<uint4*>(j.dst + row * j.W + c0) = w;
 }
 
 // qs[b][h][s][0:D] = T(x * scale), qs[b][h][s][D:2D] = T(x * scale - hi): the scaled query (or key) as two 16-bit
 // terms.
 // One thread converts 8 consecutive elements (16-byte load, two 16-byte stores).
 template <typename T>
-__device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t idx, int B, int H, int D, float scale) {
-  const T* __restrict__ q = j.src;
-  const int64_t sb = j.sb, sh = j.sh, ss = j.ss;
-  const int S = j.S;
-  T* __restrict__ qs = j.dst;
-  const int d8 = D / 8;  // idx = (b, h, s, d/8)
-  const int64_t total = (int64_t)B * H * S * d8;
-  if (idx >= total) return;
-  const int c = (int)(idx % d8);
-  const int s = (int)((idx / d8) % S);
-  const int h = (int)((idx / ((int64_t)d8 * S)) % H);
-  const int b = (int)(idx / ((int64_t)d8 * S * H));
-  const uint4 raw = *reinterpret_cast<const uint4*>(q + b * sb + h * sh + s * ss + c * 8);
+__device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t idx, float scale) {
+  if (idx >= j.units) return;
+  const int64_t row = j.div_d8.quot(idx);
+  const int c = (int)(idx - row * j.div_d8.d) * 8;
+  const int64_t bh = j.div_s.quot(row);
+  const int s = (int)(row - bh * j.S);
+  const int64_t b = j.div_h.quot(bh);
+  const int h = (int)(bh - b * j.div_h.d);
+  const uint4 raw = *reinterpret_cast<const uint4*>(j.src + b * j.sb + h * j.sh + s * j.ss + c);
   const T* x = reinterpret_cast<const T*>(&raw);
   uint4 hi4, lo4;
   T* hi = reinterpret_cast<T*>(&hi4);
@@ -165,60 +177,166 @@ __device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t
     hi[e] = from_f32<T>(v);
     lo[e] = from_f32<T>(v - to_f32(hi[e]));
   }
-  T* row = qs + (((int64_t)b * H + h) * S + s) * (2 * D);
-  *reinterpret_cast<uint4*>(row + c * 8) = hi4;
-  *reinterpret_cast<uint4*>(row + D + c * 8) = lo4;
+  T* out = j.dst + row * (2 * j.D);
+  *reinterpret_cast<uint4*>(out + c) = hi4;
+  *reinterpret_cast<uint4*>(out + j.D + c) = lo4;
 }
 
-// All operand preparation of one call in one launch: blocks [0, nbq) pack the q-side factor, [nbq, nbq + nbk) the
-// k-side factor (and its centred copy), the rest split the scaled query (forward) or key (backward).
 template <typename T>
-__global__ void __launch_bounds__(256) pack_operands_kernel(FactorJob<T> fq, FactorJob<T> fk, ScaledJob<T> sc,
-                                                            unsigned nbq, unsigned nbk, int B, int H, int D, int R,
-                                                            int RP, int RC, float scale, int* status) {
+__device__ __forceinline__ void delta_chunk(const DeltaJob<T>& j, int64_t idx) {
+  const bool live = idx < j.units;
+  float acc = 0.f;
+  int64_t out = 0;
+  int part = 0;
+  if (live) {
+    const int64_t row = j.div_g.quot(idx);  // (b, i, h), h fastest
+    part = (int)(idx - row * j.G);
+    const int64_t bi = j.div_h.quot(row);
+    const int h = (int)(row - bi * j.H);
+    const int64_t b = j.div_s.quot(bi);
+    const int i = (int)(bi - b * j.div_s.d);
+    const T* orow = j.o + b * j.o_st[0] + h * j.o_st[1] + i * j.o_st[2];
+    const T* drow = j.dout + b * j.do_st[0] + h * j.do_st[1] + i * j.do_st[2];
+    if (j.vec) {
+      for (int d = part * 8; d < j.D; d += j.G * 8) {
+        const uint4 a = *reinterpret_cast<const uint4*>(orow + d);
+        const uint4 c = *reinterpret_cast<const uint4*>(drow + d);
+        const T* pa = reinterpret_cast<const T*>(&a);
+        const T* pc = reinterpret_cast<const T*>(&c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc += to_f32(pa[e]) * to_f32(pc[e]);
+      }
+    } else {
+      for (int d = part; d < j.D; d += j.G) acc += to_f32(orow[d]) * to_f32(drow[d]);
+    }
+    out = (b * j.H + h) * j.stride_bh + i;
+  }
+  for (int o = j.G >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);  // G: a power of two
+  if (live && part == 0) j.delta[out] = acc;
+}
+
+// Everything a call needs before its main kernel, in one launch: block ranges pack the q-side factor, the k-side
+// factor and its centred copy, split the scaled query (forward) or key (backward), take delta = rowsum(o * dout) and
+// zero the fp32 accumulators (backward).  Three launches and a memset before; at small sizes each of them costs more in
+// launch and drain than in work.
+template <typename T>
+struct PrepJobs {
+  FactorJob<T> fq, fk, fc;
+  ScaledJob<T> sc;
+  DeltaJob<T> dl;
+  uint4* zero;
+  int64_t zero_vecs;                      // 16-byte units to clear
+  unsigned end_q, end_k, end_c, end_s, end_d;  // exclusive block ranges, in this order; then the zeroing blocks
+};
+constexpr int kZeroPerThread = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(256) prepare_operands_kernel(const __grid_constant__ PrepJobs<T> j, int R, float scale,
+                                                               int* status) {
+  grid_dep_launch();  // the main kernel may set itself up; it waits for this grid before it reads anything
+  grid_dep_wait();    // (whatever produced the inputs)
   const unsigned blk = blockIdx.x;
-  if (blk < nbq) {
-    pack_factor_row<T>(fq, (int64_t)blk * 256 + threadIdx.x, R, RP, RC, status);
-  } else if (blk < nbq + nbk) {
-    pack_factor_row<T>(fk, (int64_t)(blk - nbq) * 256 + threadIdx.x, R, RP, RC, status);
-  } else {
-    pack_scaled_chunk<T>(sc, (int64_t)(blk - nbq - nbk) * 256 + threadIdx.x, B, H, D, scale);
+  const int tid = threadIdx.x;
+  if (blk < j.end_q) pack_factor_chunk<T>(j.fq, (int64_t)blk * 256 + tid, R, status);
+  else if (blk < j.end_k) pack_factor_chunk<T>(j.fk, (int64_t)(blk - j.end_q) * 256 + tid, R, status);
+  else if (blk < j.end_c) pack_factor_chunk<T>(j.fc, (int64_t)(blk - j.end_k) * 256 + tid, R, status);
+  else if (blk < j.end_s) pack_scaled_chunk<T>(j.sc, (int64_t)(blk - j.end_c) * 256 + tid, scale);
+  else if (blk < j.end_d) delta_chunk<T>(j.dl, (int64_t)(blk - j.end_s) * 256 + tid);
+  else {
+    const int64_t base = (int64_t)(blk - j.end_d) * (256 * kZeroPerThread) + tid;
+#pragma unroll
+    for (int i = 0; i < kZeroPerThread; ++i)
+      if (base + i * 256 < j.zero_vecs) j.zero[base + i * 256] = make_uint4(0u, 0u, 0u, 0u);
   }
+}
+
+static unsigned blocks_for(int64_t units, int per_block = 256) { return (unsigned)((units + per_block - 1) / per_block); }
+
+template <typename T>
+static FactorJob<T> factor_job(const void* src, const int64_t* st, int Bx, int Hx, int S, int R, int W, float mult,
+                               bool centered, void* dst) {
+  FactorJob<T> j;
+  j.src = reinterpret_cast<const T*>(src);
+  j.sb = st[0]; j.sh = st[1]; j.ss = st[2];
+  j.S = S; j.W = W;
+  j.mult = mult;
+  j.centered = centered;
+  j.vec = R % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && !((st[0] | st[1] | st[2]) & 7);
+  j.dst = reinterpret_cast<T*>(dst);
+  j.div_w8 = Div(W / 8); j.div_s = Div(S); j.div_h = Div(Hx);
+  j.units = (int64_t)Bx * Hx * S * (W / 8);
+  return j;
 }
 
 template <typename T>
-static int launch_pack_operands_t(const fb_params* p, const PackPlan& plan, void* qpack, void* kpack, void* kcenter,
-                                  bool scaled_is_key, void* scaled, cudaStream_t st) {
-  FactorJob<T> fq{}, fk{};
-  ScaledJob<T> sc{};
-  unsigned nbq = 0, nbk = 0, nbs = 0;
+static int launch_prepare_t(const fb_params* p, const PackPlan& plan, const PrepBuffers& buf, cudaStream_t st) {
+  PrepJobs<T> j{};
+  unsigned n = 0;
   if (plan.RP) {
-    fq = {reinterpret_cast<const T*>(p->q_bias), p->q_bias_stride[0], p->q_bias_stride[1], p->q_bias_stride[2],
-          plan.Bq, plan.Hq, p->Sq, plan.qb_mult, reinterpret_cast<T*>(qpack), nullptr};
-    fk = {reinterpret_cast<const T*>(p->k_bias), p->k_bias_stride[0], p->k_bias_stride[1], p->k_bias_stride[2],
-          plan.Bk, plan.Hk, p->Sk, 1.f, reinterpret_cast<T*>(kpack), reinterpret_cast<T*>(kcenter)};
-    nbq = (unsigned)(((int64_t)plan.Bq * plan.Hq * p->Sq + 255) / 256);
-    nbk = (unsigned)(((int64_t)plan.Bk * plan.Hk * p->Sk + 255) / 256);
+    j.fq = factor_job<T>(p->q_bias, p->q_bias_stride, plan.Bq, plan.Hq, p->Sq, p->R, plan.RP, plan.qb_mult, false, buf.qpack);
+    j.fk = factor_job<T>(p->k_bias, p->k_bias_stride, plan.Bk, plan.Hk, p->Sk, p->R, plan.RP, 1.f, false, buf.kpack);
+    if (buf.kcenter)
+      j.fc = factor_job<T>(p->k_bias, p->k_bias_stride, plan.Bk, plan.Hk, p->Sk, p->R, plan.RC, 1.f, true, buf.kcenter);
   }
+  j.end_q = n += blocks_for(j.fq.units);
+  j.end_k = n += blocks_for(j.fk.units);
+  j.end_c = n += blocks_for(j.fc.units);
   if (plan.nq == 2) {
-    const int S = scaled_is_key ? p->Sk : p->Sq;
-    const int64_t* stv = scaled_is_key ? p->k_stride : p->q_stride;
-    sc = {reinterpret_cast<const T*>(scaled_is_key ? p->k : p->q), stv[0], stv[1], stv[2], S,
-          reinterpret_cast<T*>(scaled)};
-    nbs = (unsigned)(((int64_t)p->B * p->H * S * (p->D / 8) + 255) / 256);
+    ScaledJob<T>& s = j.sc;
+    const int64_t* stv = buf.scaled_is_key ? p->k_stride : p->q_stride;
+    s.src = reinterpret_cast<const T*>(buf.scaled_is_key ? p->k : p->q);
+    s.sb = stv[0]; s.sh = stv[1]; s.ss = stv[2];
+    s.S = buf.scaled_is_key ? p->Sk : p->Sq;
+    s.D = p->D;
+    s.dst = reinterpret_cast<T*>(buf.scaled);
+    s.div_d8 = Div(p->D / 8); s.div_s = Div(s.S); s.div_h = Div(p->H);
+    s.units = (int64_t)p->B * p->H * s.S * (p->D / 8);
   }
-  if (nbq + nbk + nbs == 0) return 0;
-  pack_operands_kernel<T><<<nbq + nbk + nbs, 256, 0, st>>>(fq, fk, sc, nbq, nbk, p->B, p->H, p->D, p->R, plan.RP,
-                                                           plan.RC, p->softmax_scale, p->status);
-  note_launch();
-  return (int)cudaGetLastError();
+  j.end_s = n += blocks_for(j.sc.units);
+  if (buf.delta) {
+    DeltaJob<T>& d = j.dl;
+    d.o = reinterpret_cast<const T*>(p->o);
+    d.dout = reinterpret_cast<const T*>(p->dout);
+    uintptr_t bits = reinterpret_cast<uintptr_t>(p->o) | reinterpret_cast<uintptr_t>(p->dout);
+    for (int i = 0; i < 3; ++i) {
+      d.o_st[i] = p->o_stride[i];
+      d.do_st[i] = p->dout_stride[i];
+      bits |= (uintptr_t)(p->o_stride[i] | p->dout_stride[i]) * 2;
+    }
+    d.D = p->D; d.H = p->H;
+    d.vec = p->D % 8 == 0 && (bits & 15) == 0;
+    // as many threads per row as it has 16-byte chunks, as far as that is a power of two (shuffle groups)
+    d.G = 1;
+    if (d.vec)
+      while (d.G < 16 && (p->D / 8) % (2 * d.G) == 0) d.G *= 2;
+    d.delta = buf.delta;
+    d.stride_bh = p->lse_stride_bh;
+    d.div_g = Div(d.G); d.div_h = Div(p->H); d.div_s = Div(p->Sq);
+    d.units = (int64_t)p->B * p->Sq * p->H * d.G;
+  }
+  j.end_d = n += blocks_for(j.dl.units);
+  j.zero = reinterpret_cast<uint4*>(buf.zero);
+  j.zero_vecs = (int64_t)(buf.zero_bytes / 16);
+  n += blocks_for(j.zero_vecs, 256 * kZeroPerThread);
+  if (n == 0) return 0;
+  return launch_pdl(prepare_operands_kernel<T>, n, 256, 0, st, j, (int)p->R, (float)p->softmax_scale, p->status);
 }
 
-int launch_pack_operands(const fb_params* p, const PackPlan& plan, void* qpack, void* kpack, void* kcenter,
-                         bool scaled_is_key, void* scaled, cudaStream_t st) {
-  return p->dtype == FB_DTYPE_F16
-             ? launch_pack_operands_t<__half>(p, plan, qpack, kpack, kcenter, scaled_is_key, scaled, st)
-             : launch_pack_operands_t<__nv_bfloat16>(p, plan, qpack, kpack, kcenter, scaled_is_key, scaled, st);
+int launch_prepare(const fb_params* p, const PackPlan& plan, const PrepBuffers& buf, cudaStream_t st) {
+  return p->dtype == FB_DTYPE_F16 ? launch_prepare_t<__half>(p, plan, buf, st)
+                                  : launch_prepare_t<__nv_bfloat16>(p, plan, buf, st);
+}
+
+// delta alone (the separate pre-pass of the C ABI)
+int launch_bwd_preprocess(const fb_params* p, cudaStream_t st) {
+  PackPlan none{};
+  none.nq = 1;
+  PrepBuffers buf{};
+  buf.delta = p->delta;
+  prof_before(KC_BWD_PREPROCESS, st);
+  const int rc = launch_prepare(p, none, buf, st);
+  prof_after(KC_BWD_PREPROCESS, st);
+  return rc;
 }
 
 }  // namespace fb

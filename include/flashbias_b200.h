@@ -45,6 +45,8 @@ extern "C" {
                                      head)) per CTA, whatever the shape */
 #define FB_FLAG_BWD_PERSISTENT 8 /* ... one persistent CTA per SM walking the work items, whatever the shape (by
                                      default: chosen when a work item has few query tiles) */
+#define FB_FLAG_BWD_FUSED_DELTA 16 /* fb_bwd takes delta itself, in the launch that prepares its operands: no
+                                      fb_bwd_preprocess call is needed before it (p->delta is written either way) */
 
 /* error codes (negative); positive return values are cudaError_t */
 #define FB_OK 0
