@@ -201,7 +201,8 @@ extern "C" int fb_bwd_uses_tensor_path(const fb_params* p) {
   int rc = validate_common(p);
   if (rc) return rc;
   PackPlan plan;
-  return bwd_sm100_supported(p, &plan) ? 1 : 0;
+  // (what this has always answered: head_dim 128 has a tensor-core backward without factor operands, but is not counted)
+  return bwd_sm100_supported(p, &plan) && plan.TD <= 64 ? 1 : 0;
 }
 
 extern "C" size_t fb_fwd_workspace_bytes(const fb_params* p) {

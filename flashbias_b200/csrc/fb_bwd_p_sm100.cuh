@@ -548,7 +548,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         T* dvrow = reinterpret_cast<T*>(a.dv) + b * a.dv_stride[0] + h * a.dv_stride[1] + (int64_t)krow * a.dv_stride[2];
         T* dkrow = reinterpret_cast<T*>(a.dk) + b * a.dk_stride[0] + h * a.dk_stride[1] + (int64_t)krow * a.dk_stride[2];
         const uint4 z = make_uint4(0, 0, 0, 0);
-        for (int c0 = wg * (D / 2); c0 < wg * (D / 2) + D / 2; c0 += 8) {
+        for (int c0 = wg * (D / 2); c0 < min(wg * (D / 2) + D / 2, a.D); c0 += 8) {
           *reinterpret_cast<uint4*>(dvrow + c0) = z;
           *reinterpret_cast<uint4*>(dkrow + c0) = z;
         }
@@ -794,9 +794,9 @@ int launch_bwd_p(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     pa.div_nk = Div(a.nk_tiles);
     pa.div_h = Div(p->H);
     CUtensorMap tDK, tDV;  // dK and dV leave through tile stores
-    if ((rc = make_tmap_4d(&tDK, p->dk, D, p->Sk, p->H, p->B, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], D, 128)))
+    if ((rc = make_tmap_4d(&tDK, p->dk, p->D, p->Sk, p->H, p->B, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], D, 128)))
       return rc;
-    if ((rc = make_tmap_4d(&tDV, p->dv, D, p->Sk, p->H, p->B, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], D, 128)))
+    if ((rc = make_tmap_4d(&tDV, p->dv, p->D, p->Sk, p->H, p->B, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], D, 128)))
       return rc;
     auto kern = bwd_p_sm100_kernel<T, D, RP, NQ, MODE>;
     // per kernel instantiation and device: raise the dynamic shared-memory limit once

@@ -18,16 +18,17 @@ bool bwd_cfg_fits(int D, int RP, int nq) {
   FB_FIT(32, 0) FB_FIT(32, 16) FB_FIT(32, 32) FB_FIT(32, 64)
   FB_FIT(64, 0) FB_FIT(64, 16) FB_FIT(64, 32)
 #undef FB_FIT
+  if (D == 128 && RP == 0) return true;  // key-major kernel only
   return false;
 }
 
 bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->flags & FB_FLAG_FORCE_GENERAL) return false;
   if (p->alibi_slopes && p->mask_kind != FB_MASK_NONE) return false;  // both at once: shape-generic kernels
-  if (!(p->D == 32 || p->D == 64)) return false;
+  if (p->D % 8 != 0) return false;  // other multiples of 8 run in the next wider tile, zero-filled by the loads
   if (!(p->softmax_scale > 0.f) || !isfinite(p->softmax_scale)) return false;
   if (!plan_pack(p, plan, true)) return false;
-  if (!bwd_cfg_fits(p->D, plan->RP, plan->nq)) return false;  // shared or tensor memory of an SM exceeded
+  if (!bwd_cfg_fits(plan->TD, plan->RP, plan->nq)) return false;  // shared or tensor memory of an SM exceeded
   if (!tma_compatible(p->q, p->q_stride[2], p->q_stride[1], p->q_stride[0], p->H, p->B)) return false;
   if (!tma_compatible(p->k, p->k_stride[2], p->k_stride[1], p->k_stride[0], p->H, p->B)) return false;
   if (!tma_compatible(p->v, p->v_stride[2], p->v_stride[1], p->v_stride[0], p->H, p->B)) return false;
@@ -55,12 +56,17 @@ static bool bwd_prefers_persistent(const fb_params* p) {
 
 int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   // (the persistent form writes dK and dV with tile stores: their layout must be one a tensor map can describe)
-  if (p->D == 32 && plan.RP > 0 && !p->alibi_slopes && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
+  if (plan.TD == 32 && plan.RP > 0 && !p->alibi_slopes && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
       ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p)) &&
       tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B) &&
       tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B))
     return dispatch_bwd_d32p(p, plan, st);
-  return p->D == 32 ? dispatch_bwd_d32(p, plan, st) : p->D == 64 ? dispatch_bwd_d64(p, plan, st) : FB_ENOTBUILT;
+  switch (plan.TD) {
+    case 32: return dispatch_bwd_d32(p, plan, st);
+    case 64: return dispatch_bwd_d64(p, plan, st);
+    case 128: return dispatch_bwd_d128(p, plan, st);
+  }
+  return FB_ENOTBUILT;
 }
 
 }  // namespace fb

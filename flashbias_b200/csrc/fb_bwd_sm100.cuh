@@ -33,7 +33,7 @@
 namespace fb {
 
 struct BwdArgs {
-  int B, H, Sq, Sk, nq_tiles, nk_tiles, causal, R;
+  int B, H, Sq, Sk, D, nq_tiles, nk_tiles, causal, R;  // D <= the tile's head_dim (columns beyond it are zeros)
   int hq_bcast, bq_bcast, hk_bcast, bk_bcast;
   int Hq, Hk;  // head extents of the un-expanded factors
   float dk_scale;    // applied to dK on store
@@ -129,13 +129,13 @@ struct BwdCfg {
   static constexpr bool FITS = SMEM <= 227 * 1024 && T_END <= 512;
 };
 
-template <int C>
+template <int C, int ROWS = 128>
 __device__ __forceinline__ void tma_tile_bwd(uint32_t dst, const CUtensorMap* m, uint32_t bar, int row0, int h,
                                              int b, int col0 = 0) {
   constexpr int SWB = swizzle_bytes(C);
   constexpr int NB = C * 2 / SWB;
 #pragma unroll
-  for (int blk = 0; blk < NB; ++blk) tma_load_4d(dst + blk * 128 * SWB, m, bar, col0 + blk * (SWB / 2), row0, h, b);
+  for (int blk = 0; blk < NB; ++blk) tma_load_4d(dst + blk * ROWS * SWB, m, bar, col0 + blk * (SWB / 2), row0, h, b);
 }
 
 __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
@@ -740,6 +740,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (krow < a.Sk) {
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
+            if (c0 + g * 8 >= a.D) break;
             uint4 wv, wk;
             wv.x = Pack2<T>::pack(__uint_as_float(rv[g * 8 + 0]), __uint_as_float(rv[g * 8 + 1]));
             wv.y = Pack2<T>::pack(__uint_as_float(rv[g * 8 + 2]), __uint_as_float(rv[g * 8 + 3]));
@@ -789,7 +790,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       T* dvrow = reinterpret_cast<T*>(a.dv) + b * a.dv_stride[0] + h * a.dv_stride[1] + (int64_t)krow * a.dv_stride[2];
       T* dkrow = reinterpret_cast<T*>(a.dk) + b * a.dk_stride[0] + h * a.dk_stride[1] + (int64_t)krow * a.dk_stride[2];
       const uint4 z = make_uint4(0, 0, 0, 0);
-      for (int c0 = wg * (D / 2); c0 < wg * (D / 2) + D / 2; c0 += 8) {
+      for (int c0 = wg * (D / 2); c0 < min(wg * (D / 2) + D / 2, a.D); c0 += 8) {
         *reinterpret_cast<uint4*>(dvrow + c0) = z;
         *reinterpret_cast<uint4*>(dkrow + c0) = z;
       }
@@ -819,7 +820,7 @@ inline BwdWs bwd_layout(const fb_params* p, const PackPlan& plan) {
   w.off_qs = w.off_kcenter + plan.kc_bytes;
   w.off_dq = w.off_qs + plan.qs_bytes;
   // query rows padded to whole tiles: the bulk reductions of the backward write whole [128][D] tiles
-  const size_t dq = round256((size_t)p->B * ((p->Sq + 127) / 128) * 128 * p->H * p->D * 4);
+  const size_t dq = round256((size_t)p->B * ((p->Sq + 127) / 128) * 128 * p->H * plan.TD * 4);
   // (Bq, Hq, query rows padded to whole tiles, R): a query tile's rows are contiguous for the bulk reduction.
   // When the factor is shared by several (batch, head) pairs they would all add into the same addresses; up to
   // 64 copies spread them, the final store sums the copies.
@@ -856,7 +857,7 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
   void* kpack = ws + w.off_kpack;
   void* kcenter = ws + w.off_kcenter;
   CUtensorMap &tQ = L.tQ, &tK = L.tK, &tV = L.tV, &tDO = L.tDO, &tQb = L.tQb, &tKb = L.tKb, &tKc = L.tKc, &tKs = L.tKs;
-  if ((rc = make_tmap_4d(&tQ, p->q, D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, 128)))
     return rc;
   if (NQ == 2) {
     // key operand of S = (hi, lo) of k*scale, laid out (B, H, Sk, 2D) in the workspace
@@ -865,12 +866,12 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
                            (int64_t)2 * D * p->Sk * p->H, D, 128)))
       return rc;
   }
-  if ((rc = make_tmap_4d(&tK, p->k, D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], D, 128)))
     return rc;
   if (NQ != 2) tKs = tK;
-  if ((rc = make_tmap_4d(&tV, p->v, D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], D, 128)))
     return rc;
-  if ((rc = make_tmap_4d(&tDO, p->dout, D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1],
+  if ((rc = make_tmap_4d(&tDO, p->dout, p->D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1],
                          p->dout_stride[0], D, 128)))
     return rc;
   if (RP) {
@@ -890,7 +891,7 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
     tKc = tK;
   }
   BwdArgs& a = L.a;
-  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk;
+  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
   a.nq_tiles = (p->Sq + 127) / 128;
   a.nk_tiles = (p->Sk + 127) / 128;
   a.causal = p->causal;
@@ -937,7 +938,7 @@ template <typename T, int D, int RP, int NQ>
 int bwd_finish(const fb_params* p, const BwdLaunch& L, cudaStream_t st) {
   using Cfg = BwdCfg<D, RP, NQ>;
   const BwdArgs& a = L.a;
-  return launch_store_grads(p, {a.dq_acc, Cfg::STAGED ? 1 : 0, a.dqb_acc, a.dkb_acc,
+  return launch_store_grads(p, {a.dq_acc, Cfg::STAGED ? DQ_SWIZZLED : DQ_ROWS, D, a.dqb_acc, a.dkb_acc,
                                 {(int64_t)a.nq_tiles * 128, a.dqb_slots, a.dqb_slot_stride},
                                 {(int64_t)a.nk_tiles * 128, a.dkb_slots, a.dkb_slot_stride}},
                             st);
@@ -980,6 +981,7 @@ int launch_bwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
 bool bwd_cfg_fits(int D, int RP, int nq);
 int dispatch_bwd_d32(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_bwd_d64(const fb_params* p, const PackPlan& plan, cudaStream_t st);
+int dispatch_bwd_d128(const fb_params* p, const PackPlan& plan, cudaStream_t st);  // without factor operands
 // persistent form (head_dim 32 with factor operands, plain or masked logits)
 int dispatch_bwd_d32p(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 

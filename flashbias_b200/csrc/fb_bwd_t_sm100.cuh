@@ -1,5 +1,5 @@
 // Backward FlashBias attention for sm_100a, key-major ("transposed") form, for problems without factor operands
-// (no bias, an additive mask tensor, or the fused ALiBi producer) at head_dim 32.
+// (no bias, an additive mask tensor, or the fused ALiBi producer) at head_dim 32 and 128.
 //
 // At head_dim 32 the backward is bound by shared-memory bandwidth (128 bytes per clock feed both the tensor
 // core's operand fetches and the threads' stores): in the query-major kernel of fb_bwd_sm100.cuh every query
@@ -23,6 +23,12 @@
 //               memory with one bulk reduction per query tile (thread = query row)
 //   warp 12     TMA producer (Q, dO tiles through a 3-stage ring) and issuer of the dQ chain
 //   warps 13-15 MMA issuers: S^T and dP^T; dV; dK
+//
+// At head_dim 128 the dV and dK accumulators take half of the tensor memory, so a query tile has QT = 64 rows there, and
+// dQ is taken transposed as well (dQ^T = K^T.dS^T: 128 lanes x 64 columns instead of a 64-row product, which would use
+// half of the lanes); 3 stages of 64-row tiles then just fit beside the resident tiles.  What bounds it: ~270 KB of
+// shared-memory traffic per 128 x 64 tile (2100 clk).  B2 H16 S2048 causal, forward + backward: 130 ms when head_dim 128
+// ran on the CUDA-core kernels.
 #pragma once
 
 #include "fb_bwd_sm100.cuh"
@@ -31,26 +37,30 @@ namespace fb {
 
 template <int D>
 struct BwdTCfg {
+  static constexpr int QT = D == 128 ? 64 : 128;  // query rows of a tile
+  static constexpr bool DQ_T = D == 128;          // dQ accumulated transposed: lane = column of dQ
   static constexpr int D_BYTES = tile_bytes(D);
   static constexpr int AUX_BYTES = tile_bytes(16);  // [128][16] tiles of the extra contraction step
   // resident: K, V and the two constant key-side tiles of the extra step (ones in columns 0-2 / 3-5)
   static constexpr int OFF_K = 0, OFF_V = D_BYTES, OFF_ES = 2 * D_BYTES, OFF_ED = OFF_ES + AUX_BYTES;
   static constexpr int KV_BYTES = 2 * D_BYTES;  // bytes that arrive by TMA
   // one stage: Q, dO (TMA) and the query-side tile of the extra step (written by threads)
-  static constexpr int OFF_DO = D_BYTES, OFF_AUX = 2 * D_BYTES, TMA_STAGE_BYTES = 2 * D_BYTES;
-  static constexpr int STAGE_BYTES = TMA_STAGE_BYTES + AUX_BYTES;
+  static constexpr int Q_BYTES = tile_bytes(D, QT);
+  static constexpr int OFF_DO = Q_BYTES, OFF_AUX = 2 * Q_BYTES, TMA_STAGE_BYTES = 2 * Q_BYTES;
+  static constexpr int STAGE_BYTES = TMA_STAGE_BYTES + tile_bytes(16, QT);
   static constexpr int NSTAGE = 3;
   static constexpr int OFF_STAGE = OFF_ED + AUX_BYTES;
-  static constexpr int TILE128 = tile_bytes(128);
-  static constexpr int OFF_DS = OFF_STAGE + NSTAGE * STAGE_BYTES;  // dS^T tile, [128 keys][128 queries]
-  static constexpr int OFF_STG = OFF_DS + TILE128;                 // fp32 dQ staging tile
-  static constexpr int OFF_BAR = OFF_STG + 128 * D * 4;
+  static constexpr int OFF_DS = OFF_STAGE + NSTAGE * STAGE_BYTES;  // dS^T tile, [128 keys][QT queries]
+  static constexpr int OFF_STG = OFF_DS + tile_bytes(QT);          // fp32 dQ staging tile
+  static constexpr int OFF_BAR = OFF_STG + QT * D * 4;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  // tensor memory: S^T fp32 [0,128), dP^T fp32 [128,256), P^T 16-bit pairs [256,320), dS^T pairs [320,384),
-  // dV [384, 384+D), dK, then two dQ accumulators
-  static constexpr int T_ST = 0, T_DPT = 128, T_PT = 256, T_DST = 320, T_DV = 384, T_DK = T_DV + D, T_DQ = T_DK + D;
-  static constexpr int NDQ = (T_DQ + 2 * D <= 512) ? 2 : 1;
-  static constexpr bool FITS = SMEM <= 227 * 1024 && T_DQ + D <= 512;
+  // tensor memory: S^T fp32, dP^T fp32 (QT columns each), P^T 16-bit pairs, dS^T pairs (QT / 2 each), dV, dK (D each),
+  // then one or two dQ accumulators
+  static constexpr int T_ST = 0, T_DPT = QT, T_PT = 2 * QT, T_DST = T_PT + QT / 2, T_DV = 3 * QT, T_DK = T_DV + D,
+                       T_DQ = T_DK + D;
+  static constexpr int DQ_COLS = DQ_T ? QT : D;
+  static constexpr int NDQ = (T_DQ + 2 * DQ_COLS <= 512) ? 2 : 1;
+  static constexpr bool FITS = SMEM <= 227 * 1024 && T_DQ + DQ_COLS <= 512;
 };
 
 template <typename T, int D, int MODE>
@@ -59,6 +69,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                    const BwdArgs a) {
   using Cfg = BwdTCfg<D>;
+  constexpr int QT = Cfg::QT;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   constexpr float kLog2e = 1.4426950408889634f;
 
@@ -87,17 +98,17 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   const int b = bh / a.H, h = bh % a.H;
   const int k0 = kt * 128;
-  const int i_begin = a.causal ? kt : 0;  // first query tile with a row >= k0
-  const int n_it = a.nq_tiles - i_begin;  // may be <= 0 when Sq < Sk under causal masking
+  const int i_begin = a.causal ? k0 / QT : 0;  // first query tile with a row >= k0
+  const int n_it = (a.Sq + QT - 1) / QT - i_begin;  // may be <= 0 when Sq < Sk under causal masking
 
   // producer thread only: one stage of the query-tile ring
   auto load_tile = [&](int it) {
     const int st = it % Cfg::NSTAGE;
     const uint32_t base = sStage + st * Cfg::STAGE_BYTES;
     mbar_expect_tx(qdo_full + 8 * st, Cfg::TMA_STAGE_BYTES);
-    const int q0 = (i_begin + it) * 128;
-    tma_tile_bwd<D>(base, &tmQ, qdo_full + 8 * st, q0, h, b);
-    tma_tile_bwd<D>(base + Cfg::OFF_DO, &tmDO, qdo_full + 8 * st, q0, h, b);
+    const int q0 = (i_begin + it) * QT;
+    tma_tile_bwd<D, QT>(base, &tmQ, qdo_full + 8 * st, q0, h, b);
+    tma_tile_bwd<D, QT>(base + Cfg::OFF_DO, &tmDO, qdo_full + 8 * st, q0, h, b);
   };
 
   if (warp == 12) {
@@ -141,14 +152,15 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     setmaxnreg_dec<64>();
     if (lane == 0 && n_it > 0) {
       // B operands read transposed (MN-major: rows are the contraction index), A of dQ likewise
-      constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, 128);  // S^T, dP^T: both operands K-major
+      constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, QT);   // S^T, dP^T: both operands K-major
       constexpr uint32_t idTS = instr_desc(kBf16, false, true, 128, D);    // dV, dK: A in TMEM, B MN-major
-      constexpr uint32_t idQ = instr_desc(kBf16, true, true, 128, D);      // dQ: A = dS (transposed tile), B = K
+      // dQ: A = dS (transposed tile), B = K; dQ^T: A = K^T, B = dS^T
+      constexpr uint32_t idQ = instr_desc(kBf16, true, true, 128, Cfg::DQ_COLS);
       mbar_wait(kv_full, 0, abort_flag, a.status);
       tc_fence_after_sync();
       if (warp == 12) {
         // ------------------------------------------------------------------ TMA producer, dQ chain
-        const DescBase mDS = mnmajor_base<128>(sDS), mK = mnmajor_base<D>(sK);
+        const DescBase mDS = mnmajor_base<QT>(sDS), mK = mnmajor_base<D>(sK);
 #pragma unroll 1
         for (int it = 0; it < n_it; ++it) {
           const int qb = it % Cfg::NDQ;
@@ -157,9 +169,10 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag, a.status);
           tc_fence_after_sync();
 #pragma unroll
-          for (int s = 0; s < 8; ++s)  // contraction over the 128 keys
-            umma_ss(tmem + Cfg::T_DQ + qb * D, desc_at(mDS, mnmajor_step<128>(s)), desc_at(mK, mnmajor_step<D>(s)),
-                    idQ, s > 0);
+          for (int s = 0; s < 8; ++s) {  // contraction over the 128 keys
+            const uint64_t ds = desc_at(mDS, mnmajor_step<QT>(s)), k = desc_at(mK, mnmajor_step<D>(s));
+            umma_ss(tmem + Cfg::T_DQ + qb * Cfg::DQ_COLS, Cfg::DQ_T ? k : ds, Cfg::DQ_T ? ds : k, idQ, s > 0);
+          }
           umma_commit(dq_full + 8 * qb);
           umma_commit(pds_free);
           if (it + Cfg::NSTAGE < n_it) {  // the S^T|dP^T, dV and dK chains have finished reading the stage of tile it
@@ -169,9 +182,9 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       } else if (warp == 13) {
         // ------------------------------------------------------------------ S^T = K.Q^T, dP^T = V.dO^T
-        const DescBase kK = kmajor_base<D>(sK), kV = kmajor_base<D>(sV), kQ = kmajor_base<D>(sStage),
-                       kDO = kmajor_base<D>(sStage + Cfg::OFF_DO), kES = kmajor_base<16>(sES),
-                       kED = kmajor_base<16>(sED), kAux = kmajor_base<16>(sStage + Cfg::OFF_AUX);
+        const DescBase kK = kmajor_base<D>(sK), kV = kmajor_base<D>(sV), kQ = kmajor_base<D, QT>(sStage),
+                       kDO = kmajor_base<D, QT>(sStage + Cfg::OFF_DO), kES = kmajor_base<16>(sES),
+                       kED = kmajor_base<16>(sED), kAux = kmajor_base<16, QT>(sStage + Cfg::OFF_AUX);
 #pragma unroll 1
         for (int it = 0; it < n_it; ++it) {
           const int st = it % Cfg::NSTAGE;
@@ -185,11 +198,11 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < D / 16; ++s)
-            umma_ss(tmem + Cfg::T_ST, desc_at(kK, kmajor_step<D>(s)), desc_at(kQ, so + kmajor_step<D>(s)), idS, s > 0);
+            umma_ss(tmem + Cfg::T_ST, desc_at(kK, kmajor_step<D>(s)), desc_at(kQ, so + kmajor_step<D, QT>(s)), idS, s > 0);
           umma_ss(tmem + Cfg::T_ST, desc_at(kES, 0), desc_at(kAux, so), idS, 1u);  // + (-lse2_i / c) per column
 #pragma unroll
           for (int s = 0; s < D / 16; ++s)
-            umma_ss(tmem + Cfg::T_DPT, desc_at(kV, kmajor_step<D>(s)), desc_at(kDO, so + kmajor_step<D>(s)), idS,
+            umma_ss(tmem + Cfg::T_DPT, desc_at(kV, kmajor_step<D>(s)), desc_at(kDO, so + kmajor_step<D, QT>(s)), idS,
                     s > 0);
           umma_ss(tmem + Cfg::T_DPT, desc_at(kED, 0), desc_at(kAux, so), idS, 1u);  // + (-delta_i) per column
           umma_commit(dp_full);
@@ -197,7 +210,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       } else {
         // ------------------------------------------------------------------ dV += P^T.dO (14), dK += dS^T.Q (15)
-        const DescBase mB = mnmajor_base<D>(warp == 14 ? sStage + Cfg::OFF_DO : sStage);
+        const DescBase mB = mnmajor_base<D, QT>(warp == 14 ? sStage + Cfg::OFF_DO : sStage);
         const uint32_t tA = tmem + (warp == 14 ? Cfg::T_PT : Cfg::T_DST);
         const uint32_t tD = tmem + (warp == 14 ? Cfg::T_DV : Cfg::T_DK);
 #pragma unroll 1
@@ -208,7 +221,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
           tc_fence_after_sync();
 #pragma unroll
-          for (int s = 0; s < 8; ++s)  // contraction over the 128 query rows; A: 8 TMEM columns per 16 rows
+          for (int s = 0; s < QT / 16; ++s)  // contraction over the query rows; A: 8 TMEM columns per 16 rows
             umma_ts(tD, tA + s * 8, desc_at(mB, so + mnmajor_step<D>(s)), idTS, (it > 0 || s > 0) ? 1u : 0u);
           umma_commit(qdo_free + 8 * st);
           umma_commit(pds_free);
@@ -218,14 +231,14 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   } else if (warp >= 8) {
     setmaxnreg_dec<64>();
-    // ------------------------------------------------------------------ drain warpgroup (thread = query row)
+    // ------------------------------------------------------------------ drain warpgroup (thread = query row, or column)
     if (n_it > 0) {
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
 #pragma unroll 1
       for (int it = 0; it < n_it; ++it) {
         const int qb = it % Cfg::NDQ;
-        const uint32_t tq = tmem + Cfg::T_DQ + qb * D + lane_off;
+        const uint32_t tq = tmem + Cfg::T_DQ + qb * Cfg::DQ_COLS + lane_off;
         mbar_wait(dq_full + 8 * qb, (it / Cfg::NDQ) & 1, abort_flag, a.status);
         tc_fence_after_sync();
         // The first columns are fetched into registers while the copy engine may still be reading the previous
@@ -238,13 +251,23 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         __syncwarp();
         asm volatile("bar.sync 3, 128;" ::: "memory");  // the drain warpgroup only
 #pragma unroll 1
-        for (int c0 = 0; c0 < D; c0 += 32) {
+        for (int c0 = 0; c0 < Cfg::DQ_COLS; c0 += 32) {
           if (c0 > 0) {
             tmem_ld16(tq + c0, r0);
             tmem_ld16(tq + c0 + 16, r1);
           }
           tmem_wait_ld(r0);
           tmem_wait_ld(r1);
+          if (Cfg::DQ_T) {
+            // [query][column of dQ]: the 32 lanes of a warp store 32 consecutive floats of a query row
+            float* stg = reinterpret_cast<float*>(smem + Cfg::OFF_STG) + c0 * D + row;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              stg[i * D] = __uint_as_float(r0[i]);
+              stg[(16 + i) * D] = __uint_as_float(r1[i]);
+            }
+            continue;
+          }
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             st_shared_v4(sStg + dq_stage_off(row, c0 / 4 + g), r0[g * 4], r0[g * 4 + 1], r0[g * 4 + 2], r0[g * 4 + 3]);
@@ -257,7 +280,9 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         fence_proxy_async_smem();               // the staged tile becomes visible to the copy engine
         asm volatile("bar.sync 3, 128;" ::: "memory");
         if (warp == 8 && lane == 0) {
-          bulk_reduce_add_f32(a.dq_acc + ((int64_t)bh * a.nq_tiles + (i_begin + it)) * (128 * D), sStg, 128 * D * 4);
+          // (nq_tiles counts tiles of 128 rows)
+          bulk_reduce_add_f32(a.dq_acc + (int64_t)bh * a.nq_tiles * (128 * D) + (int64_t)(i_begin + it) * (QT * D), sStg,
+                              QT * D * 4);
           bulk_commit_group();
         }
       }
@@ -286,13 +311,13 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mcol = reinterpret_cast<const char*>(a.mask) +
              (mb * a.mask_stride[0] + h * a.mask_stride[1] + min(key, a.Sk - 1)) * msize;
     }
-    // Row statistics of query tile `it`: threads 0..127 each fetch one query row (raw loads; consumed one tile later,
+    // Row statistics of query tile `it`: threads 0..QT-1 each fetch one query row (raw loads; consumed one tile later,
     // so the latency hides under the arithmetic in between) ...
     auto load_row_stats = [&](int it, float& lse_raw, float& dlt) {
-      const int g = (i_begin + it) * 128 + (int)threadIdx.x;
+      const int g = (i_begin + it) * QT + (int)threadIdx.x;
       lse_raw = -INFINITY;  // rows beyond Sq and rows that saw no key: probabilities exactly zero
       dlt = 0.f;
-      if (threadIdx.x < 128 && it < n_it && g < a.Sq) {
+      if (threadIdx.x < QT && it < n_it && g < a.Sq) {
         asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(lse_raw) : "l"(a.lse + (int64_t)bh * a.lse_stride_bh + g));
         asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(dlt) : "l"(a.delta + (int64_t)bh * a.lse_stride_bh + g));
       }
@@ -308,8 +333,8 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       lo = from_f32<T>(r1 - to_f32(mid));
     };
     auto store_row_stats = [&](int it, float lse_raw, float dlt) {
-      if (threadIdx.x < 128) {
-        const int g = (i_begin + it) * 128 + (int)threadIdx.x;
+      if (threadIdx.x < QT) {
+        const int g = (i_begin + it) * QT + (int)threadIdx.x;
         const float kMostNeg = kBf16 ? -1e30f : -6e4f;
         float x = kMostNeg;
         if (lse_raw != -INFINITY) {
@@ -322,8 +347,8 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         split3(x, e[0], e[1], e[2]);
         split3(-dlt, e[3], e[4], e[5]);
         const uint32_t base = sStage + (it % Cfg::NSTAGE) * Cfg::STAGE_BYTES + Cfg::OFF_AUX;
-        st_shared_v4(base + tile_chunk_offset<16>((int)threadIdx.x, 0), w.x, w.y, w.z, w.w);
-        st_shared_v4(base + tile_chunk_offset<16>((int)threadIdx.x, 8), 0u, 0u, 0u, 0u);
+        st_shared_v4(base + tile_chunk_offset<16, QT>((int)threadIdx.x, 0), w.x, w.y, w.z, w.w);
+        st_shared_v4(base + tile_chunk_offset<16, QT>((int)threadIdx.x, 8), 0u, 0u, 0u, 0u);
       }
       if (wg == 0) {
         fence_proxy_async_smem();
@@ -349,31 +374,36 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     store_row_stats(0, lse_raw, dlt);
     load_row_stats(1, lse_raw, dlt);
     uint32_t rs0[32], rd0[32], rs1[32], rd1[32];
-    const uint32_t tSl = tmem + Cfg::T_ST + lane_off + wg * 64, tDl = tmem + Cfg::T_DPT + lane_off + wg * 64;
+    const uint32_t tSl = tmem + Cfg::T_ST + lane_off + wg * (QT / 2),
+                   tDl = tmem + Cfg::T_DPT + lane_off + wg * (QT / 2);
     mbar_wait(dp_full, 0, abort_flag, a.status);  // committed after the S^T and the dP^T products: covers both
     tc_fence_after_sync();
     tmem_ld32(tSl, rs0);
     tmem_ld32(tDl, rd0);
 #pragma unroll 1
     for (int it = 0; it < n_it; ++it) {
-      const int q0 = (i_begin + it) * 128;
+      const int q0 = (i_begin + it) * QT;
       const bool need_mask = (a.causal && k0 + 127 > q0) || (k0 + 128 > a.Sk);
       // the next tile's statistics tile (its stage was last read two tiles ago); the S^T|dP^T products of that tile
       // wait for it
       if (it + 1 < n_it) store_row_stats(it + 1, lse_raw, dlt);
       load_row_stats(it + 2, lse_raw, dlt);
-      tmem_ld32(tSl + 32, rs1);
-      tmem_ld32(tDl + 32, rd1);
+      if (QT == 128) {
+        tmem_ld32(tSl + 32, rs1);
+        tmem_ld32(tDl + 32, rd1);
+      }
       tmem_wait_ld(rs0);
       tmem_wait_ld(rd0);
-      tmem_wait_ld(rs1);
-      tmem_wait_ld(rd1);
+      if (QT == 128) {
+        tmem_wait_ld(rs1);
+        tmem_wait_ld(rd1);
+      }
       tc_fence_before_sync();
       mbar_arrive_warp(sdp_read);
       // P^T and dS^T of the tile stay in registers as packed 16-bit pairs until both chunks are done: the tensor
       // memory and shared-memory tiles are still being read by the products of the previous tile
       auto chunk = [&](uint32_t (&rs)[32], uint32_t (&rd)[32], uint32_t (&pk)[16], uint32_t (&dk)[16], int c) {
-        const int col0 = wg * 64 + c * 32;  // first query column of the chunk
+        const int col0 = wg * (QT / 2) + c * 32;  // first query column of the chunk
         const uint64_t sl2p = f2(sl2, sl2), akp = f2(akey, akey);
         float mv[32];
         if (MODE == BWD_MASK) {
@@ -414,7 +444,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       };
       uint32_t pk0[16], pk1[16], dk0[16], dk1[16];
       chunk(rs0, rd0, pk0, dk0, 0);
-      chunk(rs1, rd1, pk1, dk1, 1);
+      if (QT == 128) chunk(rs1, rd1, pk1, dk1, 1);
       // Chunk 0 of the next tile is fetched under the stores below if its S^T and dP^T are already there.
       bool prefetched = false;
       if (it + 1 < n_it) {
@@ -429,17 +459,18 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (it >= 1) mbar_wait(pds_free, (it - 1) & 1, abort_flag, a.status);
       tc_fence_after_sync();
       // P^T and dS^T into tensor memory (A operands of dV and dK) ...
-      tmem_st16(tmem + Cfg::T_PT + lane_off + wg * 32, pk0);
-      tmem_st16(tmem + Cfg::T_PT + lane_off + wg * 32 + 16, pk1);
-      tmem_st16(tmem + Cfg::T_DST + lane_off + wg * 32, dk0);
-      tmem_st16(tmem + Cfg::T_DST + lane_off + wg * 32 + 16, dk1);
+      tmem_st16(tmem + Cfg::T_PT + lane_off + wg * (QT / 4), pk0);
+      if (QT == 128) tmem_st16(tmem + Cfg::T_PT + lane_off + wg * (QT / 4) + 16, pk1);
+      tmem_st16(tmem + Cfg::T_DST + lane_off + wg * (QT / 4), dk0);
+      if (QT == 128) tmem_st16(tmem + Cfg::T_DST + lane_off + wg * (QT / 4) + 16, dk1);
       // ... and dS^T into shared memory as well (A operand of dQ, read transposed)
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        st_shared_v4(sDS + tile_chunk_offset<128>(row, wg * 64 + g * 8), dk0[g * 4], dk0[g * 4 + 1], dk0[g * 4 + 2],
+        st_shared_v4(sDS + tile_chunk_offset<QT>(row, wg * (QT / 2) + g * 8), dk0[g * 4], dk0[g * 4 + 1], dk0[g * 4 + 2],
                      dk0[g * 4 + 3]);
-        st_shared_v4(sDS + tile_chunk_offset<128>(row, wg * 64 + 32 + g * 8), dk1[g * 4], dk1[g * 4 + 1],
-                     dk1[g * 4 + 2], dk1[g * 4 + 3]);
+        if (QT == 128)
+          st_shared_v4(sDS + tile_chunk_offset<QT>(row, wg * (QT / 2) + 32 + g * 8), dk1[g * 4], dk1[g * 4 + 1],
+                       dk1[g * 4 + 2], dk1[g * 4 + 3]);
       }
       tmem_wait_st();
       fence_proxy_async_smem();
@@ -470,6 +501,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (key < a.Sk) {
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
+            if (c0 + g * 8 >= a.D) break;  // D is a multiple of 8
             uint4 wv, wk;
             wv.x = Pack2<T>::pack(__uint_as_float(rv[g * 8 + 0]), __uint_as_float(rv[g * 8 + 1]));
             wv.y = Pack2<T>::pack(__uint_as_float(rv[g * 8 + 2]), __uint_as_float(rv[g * 8 + 3]));
@@ -493,7 +525,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       T* dvrow = reinterpret_cast<T*>(a.dv) + b * a.dv_stride[0] + h * a.dv_stride[1] + (int64_t)krow * a.dv_stride[2];
       T* dkrow = reinterpret_cast<T*>(a.dk) + b * a.dk_stride[0] + h * a.dk_stride[1] + (int64_t)krow * a.dk_stride[2];
       const uint4 z = make_uint4(0, 0, 0, 0);
-      for (int c0 = wg * (D / 2); c0 < wg * (D / 2) + D / 2; c0 += 8) {
+      for (int c0 = wg * (D / 2); c0 < min(wg * (D / 2) + D / 2, a.D); c0 += 8) {
         *reinterpret_cast<uint4*>(dvrow + c0) = z;
         *reinterpret_cast<uint4*>(dkrow + c0) = z;
       }
@@ -517,18 +549,19 @@ int launch_bwd_t_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   int rc;
   const BwdWs w = bwd_layout(p, plan);
   uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
+  constexpr int QT = Cfg::QT, BOX = D > 64 ? 64 : D;
   CUtensorMap tQ, tK, tV, tDO;
-  if ((rc = make_tmap_4d(&tQ, p->q, D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], BOX, QT)))
     return rc;
-  if ((rc = make_tmap_4d(&tK, p->k, D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], BOX, 128)))
     return rc;
-  if ((rc = make_tmap_4d(&tV, p->v, D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], BOX, 128)))
     return rc;
-  if ((rc = make_tmap_4d(&tDO, p->dout, D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1],
-                         p->dout_stride[0], D, 128)))
+  if ((rc = make_tmap_4d(&tDO, p->dout, p->D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1],
+                         p->dout_stride[0], BOX, QT)))
     return rc;
   BwdArgs a = {};
-  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk;
+  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
   a.nq_tiles = (p->Sq + 127) / 128;
   a.nk_tiles = (p->Sk + 127) / 128;
   a.causal = p->causal;
@@ -573,7 +606,7 @@ int launch_bwd_t_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, tQ, tK, tV, tDO, a);
   prof_after(KC_BWD_MAIN, st);
   if (rc) return rc;
-  return launch_store_grads(p, {a.dq_acc, 1, nullptr, nullptr, {}, {}}, st);
+  return launch_store_grads(p, {a.dq_acc, Cfg::DQ_T ? DQ_HEAD_ROWS : DQ_SWIZZLED, D, nullptr, nullptr, {}, {}}, st);
 }
 
 }  // namespace fb

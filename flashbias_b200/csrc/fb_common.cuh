@@ -166,14 +166,14 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // ---------------------------------------------------------------------------------------------
 // Descriptors
 // ---------------------------------------------------------------------------------------------
-// Shared-memory operand tiles are always [128 rows][C columns] of a 16-bit type, stored the way a
-// TMA box of (min(C,64) columns x 128 rows) with the matching swizzle writes them: `nblk` column
-// blocks, each 128 rows of SWB = min(2C,128) bytes, 16-byte chunks XOR-swizzled within each
+// Shared-memory operand tiles are always [ROWS (128, or 64) rows][C columns] of a 16-bit type, stored the way a
+// TMA box of (min(C,64) columns x ROWS rows) with the matching swizzle writes them: `nblk` column
+// blocks, each ROWS rows of SWB = min(2C,128) bytes, 16-byte chunks XOR-swizzled within each
 // 8-row group.  The same bytes can be read by the tensor core
 //   * K-major  : rows are the M/N index, columns the contraction index, or
 //   * MN-major : columns are the M/N index, rows the contraction index.
 constexpr __host__ __device__ int swizzle_bytes(int cols) { return cols * 2 >= 128 ? 128 : cols * 2; }
-constexpr __host__ __device__ int tile_bytes(int cols) { return 128 * cols * 2; }
+constexpr __host__ __device__ int tile_bytes(int cols, int rows = 128) { return rows * cols * 2; }
 
 // sm_100 shared-memory matrix descriptor: start address [0,14), leading byte offset [16,30),
 // stride byte offset [32,46) (all in 16-byte units), version 1 at [46,48), layout type at [61,64).
@@ -183,22 +183,22 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes,
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) | (layout << 61);
 }
 
-// K-major view, contraction columns [col0, col0+16) of a [128][C] tile at `base`.
-template <int C>
+// K-major view, contraction columns [col0, col0+16) of a [ROWS][C] tile at `base`.
+template <int C, int ROWS = 128>
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int col0) {
   constexpr int SWB = swizzle_bytes(C);
   const int byte0 = col0 * 2;
-  const uint32_t addr = base + (byte0 / SWB) * (128 * SWB) + (byte0 % SWB);
+  const uint32_t addr = base + (byte0 / SWB) * (ROWS * SWB) + (byte0 % SWB);
   return smem_desc(addr, 16, 8 * SWB, SWB);
 }
 
-// MN-major view, contraction rows [row0, row0+16) of a [128][C] tile at `base`; the M/N extent
+// MN-major view, contraction rows [row0, row0+16) of a [ROWS][C] tile at `base`; the M/N extent
 // starts at column `col0` (a multiple of the swizzle atom width, SWB/2 columns).
-template <int C>
+template <int C, int ROWS = 128>
 __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int row0, int col0 = 0) {
   constexpr int SWB = swizzle_bytes(C);
-  const uint32_t addr = base + ((col0 * 2) / SWB) * (128 * SWB) + row0 * SWB;
-  return smem_desc(addr, 128 * SWB, 8 * SWB, SWB);
+  const uint32_t addr = base + ((col0 * 2) / SWB) * (ROWS * SWB) + row0 * SWB;
+  return smem_desc(addr, ROWS * SWB, 8 * SWB, SWB);
 }
 
 // Descriptors whose base address is only known at run time: everything but the start-address field is
@@ -206,20 +206,20 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int row0, int co
 struct DescBase {
   uint32_t lo, hi;
 };
-template <int C>
+template <int C, int ROWS = 128>
 __device__ __forceinline__ DescBase kmajor_base(uint32_t base) {
-  const uint64_t d = desc_kmajor<C>(base, 0);
+  const uint64_t d = desc_kmajor<C, ROWS>(base, 0);
   return DescBase{(uint32_t)d, (uint32_t)(d >> 32)};
 }
-template <int C>
+template <int C, int ROWS = 128>
 __device__ __forceinline__ DescBase mnmajor_base(uint32_t base) {
-  const uint64_t d = desc_mnmajor<C>(base, 0, 0);
+  const uint64_t d = desc_mnmajor<C, ROWS>(base, 0, 0);
   return DescBase{(uint32_t)d, (uint32_t)(d >> 32)};
 }
-// byte offset of K-step s (16 contraction elements) inside a [128][C] tile
-template <int C>
+// byte offset of K-step s (16 contraction elements) inside a [ROWS][C] tile
+template <int C, int ROWS = 128>
 __host__ __device__ constexpr uint32_t kmajor_step(int s) {
-  return ((s * 32) / swizzle_bytes(C)) * (128 * swizzle_bytes(C)) + (s * 32) % swizzle_bytes(C);
+  return ((s * 32) / swizzle_bytes(C)) * (ROWS * swizzle_bytes(C)) + (s * 32) % swizzle_bytes(C);
 }
 template <int C>
 __host__ __device__ constexpr uint32_t mnmajor_step(int s) {
@@ -461,9 +461,9 @@ __device__ __forceinline__ void load_mask_chunk(const MT* __restrict__ p, int n,
   }
 }
 
-// Byte offset of the 16-byte chunk holding columns [col, col+8) of `row` inside a [128][C] tile
+// Byte offset of the 16-byte chunk holding columns [col, col+8) of `row` inside a [ROWS][C] tile
 // (the layout described above); `col` is a multiple of 8.
-template <int C>
+template <int C, int ROWS = 128>
 __device__ __forceinline__ uint32_t tile_chunk_offset(int row, int col) {
   constexpr int SWB = swizzle_bytes(C);
   constexpr int CHUNKS = SWB / 16;  // chunks per row of one block
@@ -472,7 +472,7 @@ __device__ __forceinline__ uint32_t tile_chunk_offset(int row, int col) {
   const int chunk = (byte0 % SWB) >> 4;
   // 128B swizzle XORs the chunk index with row%8; 64B with (row/2)%4; 32B with (row/4)%2.
   const int x = SWB == 128 ? (row & 7) : SWB == 64 ? ((row >> 1) & 3) : SWB == 32 ? ((row >> 2) & 1) : 0;
-  return blk * (128 * SWB) + row * SWB + (((chunk ^ x) & (CHUNKS - 1)) << 4);
+  return blk * (ROWS * SWB) + row * SWB + (((chunk ^ x) & (CHUNKS - 1)) << 4);
 }
 
 // Byte offset of 16-byte chunk `ch` of row `r` in a staged [128][D] fp32 dQ tile: 128-byte lines, chunks XOR-swizzled

@@ -5,13 +5,12 @@
 
 namespace fb {
 
-// dq = T(scale * acc), 8 consecutive d per thread.  acc is fp32, laid out (B, Sq, H, D), or -- `tiled` -- per (batch,
-// head, query tile) as the staged [128][D] tile of dq_stage_off.
+// dq = T(scale * acc), 8 consecutive d per thread; arrangements of the accumulator: see DQ_*.
 template <typename T>
 struct DqStoreJob {
   const float* acc;
   T* dq;
-  int D, H, Sq, tiled;
+  int cols, H, Sq, layout;
   int64_t sb, sh, ss;
   float scale;
   Div div_d8, div_h, div_s;
@@ -78,14 +77,16 @@ __global__ void __launch_bounds__(256) store_grads_kernel(const __grid_constant_
   const int64_t b = dq.div_s.quot(bs);
   const int s = (int)(bs - b * dq.Sq);
   float4 x, y;
-  if (dq.tiled) {
-    const int nq_tiles = (dq.Sq + 127) / 128;
-    const char* tile = reinterpret_cast<const char*>(dq.acc + ((b * dq.H + h) * nq_tiles + s / 128) * (128 * dq.D));
+  const int nq_tiles = (dq.Sq + 127) / 128;
+  if (dq.layout == DQ_SWIZZLED) {
+    const char* tile = reinterpret_cast<const char*>(dq.acc + ((b * dq.H + h) * nq_tiles + s / 128) * (128 * dq.cols));
     x = *reinterpret_cast<const float4*>(tile + dq_stage_off(s % 128, d / 4));
     y = *reinterpret_cast<const float4*>(tile + dq_stage_off(s % 128, d / 4 + 1));
   } else {
-    x = *reinterpret_cast<const float4*>(dq.acc + idx * 8);
-    y = *reinterpret_cast<const float4*>(dq.acc + idx * 8 + 4);
+    const int64_t row = dq.layout == DQ_HEAD_ROWS ? (b * dq.H + h) * (nq_tiles * 128) + s : rowh;
+    const float* src = dq.acc + row * dq.cols + d;
+    x = *reinterpret_cast<const float4*>(src);
+    y = *reinterpret_cast<const float4*>(src + 4);
   }
   uint4 w;
   w.x = Pack2<T>::pack(x.x * dq.scale, x.y * dq.scale);
@@ -117,7 +118,7 @@ static int launch_store_t(const fb_params* p, const GradAccs& g, cudaStream_t st
   if (g.dq) {
     dq.acc = g.dq;
     dq.dq = reinterpret_cast<T*>(p->dq);
-    dq.D = p->D; dq.H = p->H; dq.Sq = p->Sq; dq.tiled = g.dq_tiled;
+    dq.cols = g.dq_cols; dq.H = p->H; dq.Sq = p->Sq; dq.layout = g.dq_layout;
     dq.sb = p->dq_stride[0]; dq.sh = p->dq_stride[1]; dq.ss = p->dq_stride[2];
     dq.scale = p->softmax_scale;
     dq.div_d8 = Div(p->D / 8); dq.div_h = Div(p->H); dq.div_s = Div(p->Sq);

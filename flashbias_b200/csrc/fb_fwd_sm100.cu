@@ -24,7 +24,7 @@ bool fwd_cfg_fits(int D, int RP, int nq) {
 bool fwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->flags & FB_FLAG_FORCE_GENERAL) return false;
   if (p->alibi_slopes && p->mask_kind != FB_MASK_NONE) return false;  // both at once: shape-generic kernels
-  if (!(p->D == 32 || p->D == 64 || p->D == 128)) return false;
+  if (p->D % 8 != 0) return false;  // other multiples of 8 run in the next wider tile, zero-filled by the loads
   if (!(p->softmax_scale > 0.f) || !isfinite(p->softmax_scale)) return false;
   if (!tma_compatible(p->q, p->q_stride[2], p->q_stride[1], p->q_stride[0], p->H, p->B)) return false;
   if (!tma_compatible(p->k, p->k_stride[2], p->k_stride[1], p->k_stride[0], p->H, p->B)) return false;
@@ -32,11 +32,11 @@ bool fwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (!o_store_ok(p)) return false;
   if ((int64_t)p->B * p->H * ((p->Sq + 127) / 128) > 0x7fffffffLL) return false;
   if (!plan_pack(p, plan)) return false;
-  return fwd_cfg_fits(p->D, plan->RP, plan->nq);  // shared or tensor memory of an SM exceeded: generic kernels
+  return fwd_cfg_fits(plan->TD, plan->RP, plan->nq);  // shared or tensor memory of an SM exceeded: generic kernels
 }
 
 int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
-  switch (p->D) {
+  switch (plan.TD) {
     case 32: return dispatch_fwd_d32(p, plan, st);
     case 64: return dispatch_fwd_d64(p, plan, st);
     case 128: return dispatch_fwd_d128(p, plan, st);

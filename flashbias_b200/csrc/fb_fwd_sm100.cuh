@@ -38,7 +38,7 @@
 namespace fb {
 
 struct FwdArgs {
-  int B, H, Sq, Sk, nq_tiles, causal;
+  int B, H, Sq, Sk, D, nq_tiles, causal;  // D <= the tile's head_dim: columns beyond it are zero-filled by the loads
   int total_items;  // query tiles x batch x heads: the CTAs walk them with a stride of the grid size
   int hq_bcast, bq_bcast, hk_bcast, bk_bcast;  // 1 = the packed factor has extent 1 on that dim
   float scale, scale_log2;
@@ -446,6 +446,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (grow < a.Sq) {
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
+          if (c * 32 + g * 8 >= a.D) break;  // D is a multiple of 8
           uint4 w;
           w.x = Pack2<T>::pack(__uint_as_float(r[g * 8 + 0]) * inv, __uint_as_float(r[g * 8 + 1]) * inv);
           w.y = Pack2<T>::pack(__uint_as_float(r[g * 8 + 2]) * inv, __uint_as_float(r[g * 8 + 3]) * inv);
@@ -495,14 +496,14 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       if ((rc = make_tmap_4d(&tQ, qs, 2 * D, p->Sq, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sq,
                              (int64_t)2 * D * p->Sq * p->H, BOXD, 128)))
         return rc;
-    } else if ((rc = make_tmap_4d(&tQ, p->q, D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0],
+    } else if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0],
                                   BOXD, 128))) {
       return rc;
     }
-    if ((rc = make_tmap_4d(&tK, p->k, D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], BOXD,
+    if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], BOXD,
                            128)))
       return rc;
-    if ((rc = make_tmap_4d(&tV, p->v, D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], BOXD,
+    if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], BOXD,
                            128)))
       return rc;
     if (RP) {
@@ -517,7 +518,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       tKb = tK;
     }
     FwdArgs a;
-    a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk;
+    a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
     a.nq_tiles = (p->Sq + 127) / 128;
     a.total_items = (int)((int64_t)a.nq_tiles * p->B * p->H);
     a.causal = p->causal;

@@ -341,7 +341,7 @@ int launch_bwd_general(const fb_params* p, cudaStream_t st) {
   if (e != cudaSuccess) return (int)e;
   if (p->R <= 0) return 0;
   const FactorAcc fa = factor_acc(*p);
-  return launch_store_grads(p, {nullptr, 0, fa.dqb, fa.dkb, {0, 1, 0}, {0, 1, 0}}, st);
+  return launch_store_grads(p, {nullptr, 0, 0, fa.dqb, fa.dkb, {0, 1, 0}, {0, 1, 0}}, st);
 }
 
 }  // namespace fb

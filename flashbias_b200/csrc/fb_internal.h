@@ -42,13 +42,14 @@ bool tma_compatible(const void* ptr, int64_t stride_row, int64_t stride_head, in
 // The tensor-core kernels contract over [scaled query terms | packed rank] in one fp32 accumulator.
 //   nq == 1 (softmax_scale an exact power of two): the query operand is the caller's q, the q-side factor is
 //           q_bias / scale (exact), logits = scale * S.
-//   nq == 2: the query operand is q*scale as a (hi, lo) pair of 16-bit terms, laid out (B, H, Sq, 2D); factors
+//   nq == 2: the query operand is q*scale as a (hi, lo) pair of 16-bit terms, laid out (B, H, Sq, 2 TD); factors
 //           are used as given, logits = S.  (The backward splits k*scale instead: its key tile is the resident
 //           one.)
 // Packed factors: (Bb, Hb, S, RP) contiguous, Bb/Hb = 1 on broadcast dims, zero-padded to RP columns.
 struct PackPlan {
   int nq;          // 1 or 2 query terms
   float qb_mult;   // multiplier applied to q_bias when packing (1/scale when nq == 1)
+  int TD;          // head_dim padded to the tile width: 32, 64 or 128 (missing columns are read as zero)
   int RP;          // packed factor width: 0 (no bias), 16, 32 or 64
   int RC;          // width of the centred k-side copy of the backward (>= RP; 32 beside a head_dim-32 K tile)
   int Bq, Hq, Bk, Hk;
@@ -59,7 +60,7 @@ struct PackPlan {
 bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd = false);
 // What one launch prepares for a call: packed q/k factors, kcenter (optional, rows of plan.RC columns: k_bias minus the
 // k_bias of the middle key of each group of 32 keys), when plan.nq == 2 the (hi, lo) split of q*scale (forward) or
-// k*scale (backward; scaled_is_key), laid out (B, H, S, 2D), and for the backward delta (optional) and the zeroed
+// k*scale (backward; scaled_is_key), laid out (B, H, S, 2 TD), and for the backward delta (optional) and the zeroed
 // accumulators.
 struct PrepBuffers {
   void *qpack, *kpack, *kcenter, *scaled;
@@ -95,11 +96,15 @@ struct FactorAccLayout {
   int slots;            // copies to sum
   int64_t slot_stride;  // floats between copies
 };
+// Arrangement of the fp32 dq accumulator: (B, Sq, H, cols); per (batch, head, tile of 128 rows) as dq_stage_off has it;
+// (B, H, rows padded to 128, cols)
+enum { DQ_ROWS = 0, DQ_SWIZZLED = 1, DQ_HEAD_ROWS = 2 };
 // The fp32 accumulators of a backward; launch_store_grads rounds them into p->dq (unless dq is null: the main kernel
 // has stored it), p->dq_bias and p->dk_bias.
 struct GradAccs {
   const float* dq;
-  int dq_tiled;  // per (batch, head, query tile) as dq_stage_off arranges it, else (B, Sq, H, D)
+  int dq_layout;  // DQ_*
+  int dq_cols;    // columns of an accumulator row (>= D)
   const float *dqb, *dkb;
   FactorAccLayout dqb_layout, dkb_layout;
 };

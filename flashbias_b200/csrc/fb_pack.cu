@@ -29,6 +29,7 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   plan->Hq = p->q_bias_stride[1] == 0 ? 1 : p->H;
   plan->Bk = p->k_bias_stride[0] == 0 ? 1 : p->B;
   plan->Hk = p->k_bias_stride[1] == 0 ? 1 : p->H;
+  plan->TD = p->D <= 32 ? 32 : p->D <= 64 ? 64 : 128;
   int e;
   bool pow2 = frexpf(p->softmax_scale, &e) == 0.5f;
   // fp16 factors divided by a scale below one could leave the range of the type: take the split form instead
@@ -38,7 +39,7 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   plan->nq = pow2 ? 1 : 2;
   plan->qb_mult = (pow2 && p->R > 0) ? (float)(1.0 / (double)p->softmax_scale) : 1.f;
   // forward: scaled-query copy; backward: scaled-key copy
-  plan->qs_bytes = pow2 ? 0 : round256((size_t)p->B * p->H * (for_bwd ? p->Sk : p->Sq) * 2 * p->D * 2);
+  plan->qs_bytes = pow2 ? 0 : round256((size_t)p->B * p->H * (for_bwd ? p->Sk : p->Sq) * 2 * plan->TD * 2);
   plan->RC = 0;
   plan->kc_bytes = 0;
   if (p->R <= 0) {
@@ -50,13 +51,13 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   plan->RP = pad_pow2_16(for_bwd ? 2 * p->R : p->R);
   // backward at head_dim 32: factor tiles as wide as the Q/K tiles, so that [Q | Qb] and [K | Kc] are read as one
   // MMA operand each (one product instead of two per 16 query rows / keys)
-  if (for_bwd && p->D == 32 && plan->RP < 32) plan->RP = 32;
+  if (for_bwd && plan->TD == 32 && plan->RP < 32) plan->RP = 32;
   if (plan->RP > (for_bwd ? 64 : 128)) return false;
   plan->q_bytes = round256((size_t)plan->Bq * plan->Hq * p->Sq * plan->RP * 2);
   plan->k_bytes = round256((size_t)plan->Bk * plan->Hk * p->Sk * plan->RP * 2);
   if (for_bwd) {
     // beside a head_dim-32 K tile the centred copy is 32 columns wide: [K | Kc] then reads as one MMA operand
-    plan->RC = (p->D == 32 && plan->RP < 32) ? 32 : plan->RP;
+    plan->RC = (plan->TD == 32 && plan->RP < 32) ? 32 : plan->RP;
     plan->kc_bytes = round256((size_t)plan->Bk * plan->Hk * p->Sk * plan->RC * 2);
   }
   return true;
@@ -75,15 +76,15 @@ struct FactorJob {
   Div div_w8, div_s, div_h;  // divisions by W/8 (threads per row), S and Hx
   int64_t units;             // threads: rows x W/8
 };
-// One tensor scaled and split: (B, H, S, D) with strides -> (B, H, S, 2D) = [hi | lo] of x * scale.
+// One tensor scaled and split: (B, H, S, D) with strides -> (B, H, S, 2W) = [hi | lo] of x * scale, W >= D (zeros beyond).
 template <typename T>
 struct ScaledJob {
   const T* src;
   int64_t sb, sh, ss;
-  int S, D;
+  int S, D, W;
   T* dst;
-  Div div_d8, div_s, div_h;
-  int64_t units;  // rows x D/8
+  Div div_w8, div_s, div_h;
+  int64_t units;  // rows x W/8
 };
 // delta[bh, i] = sum_d o[i, d] * dout[i, d]: G threads per row
 template <typename T>
@@ -154,19 +155,20 @@ __device__ __forceinline__ void pack_factor_chunk(const FactorJob<T>& j, int64_t
   *reinterpret_cast<uint4*>(j.dst + row * j.W + c0) = w;
 }
 
-// qs[b][h][s][0:D] = T(x * scale), qs[b][h][s][D:2D] = T(x * scale - hi): the scaled query (or key) as two 16-bit
+// qs[b][h][s][0:W] = T(x * scale), qs[b][h][s][W:2W] = T(x * scale - hi): the scaled query (or key) as two 16-bit
 // terms.
 // One thread converts 8 consecutive elements (16-byte load, two 16-byte stores).
 template <typename T>
 __device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t idx, float scale) {
   if (idx >= j.units) return;
-  const int64_t row = j.div_d8.quot(idx);
-  const int c = (int)(idx - row * j.div_d8.d) * 8;
+  const int64_t row = j.div_w8.quot(idx);
+  const int c = (int)(idx - row * j.div_w8.d) * 8;
   const int64_t bh = j.div_s.quot(row);
   const int s = (int)(row - bh * j.S);
   const int64_t b = j.div_h.quot(bh);
   const int h = (int)(bh - b * j.div_h.d);
-  const uint4 raw = *reinterpret_cast<const uint4*>(j.src + b * j.sb + h * j.sh + s * j.ss + c);
+  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+  if (c < j.D) raw = *reinterpret_cast<const uint4*>(j.src + b * j.sb + h * j.sh + s * j.ss + c);
   const T* x = reinterpret_cast<const T*>(&raw);
   uint4 hi4, lo4;
   T* hi = reinterpret_cast<T*>(&hi4);
@@ -177,9 +179,9 @@ __device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t
     hi[e] = from_f32<T>(v);
     lo[e] = from_f32<T>(v - to_f32(hi[e]));
   }
-  T* out = j.dst + row * (2 * j.D);
+  T* out = j.dst + row * (2 * j.W);
   *reinterpret_cast<uint4*>(out + c) = hi4;
-  *reinterpret_cast<uint4*>(out + j.D + c) = lo4;
+  *reinterpret_cast<uint4*>(out + j.W + c) = lo4;
 }
 
 template <typename T>
@@ -287,10 +289,10 @@ static int launch_prepare_t(const fb_params* p, const PackPlan& plan, const Prep
     s.src = reinterpret_cast<const T*>(buf.scaled_is_key ? p->k : p->q);
     s.sb = stv[0]; s.sh = stv[1]; s.ss = stv[2];
     s.S = buf.scaled_is_key ? p->Sk : p->Sq;
-    s.D = p->D;
+    s.D = p->D; s.W = plan.TD;
     s.dst = reinterpret_cast<T*>(buf.scaled);
-    s.div_d8 = Div(p->D / 8); s.div_s = Div(s.S); s.div_h = Div(p->H);
-    s.units = (int64_t)p->B * p->H * s.S * (p->D / 8);
+    s.div_w8 = Div(plan.TD / 8); s.div_s = Div(s.S); s.div_h = Div(p->H);
+    s.units = (int64_t)p->B * p->H * s.S * (plan.TD / 8);
   }
   j.end_s = n += blocks_for(j.sc.units);
   if (buf.delta) {

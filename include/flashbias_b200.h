@@ -128,7 +128,9 @@ int fb_version(void);
 size_t fb_params_size(void); /* sizeof(fb_params) as compiled, for bindings to check their mirror of the struct */
 const char *fb_strerror(int code);
 
-/* 1 if the tcgen05/TMA kernels handle this problem, 0 if the shape-generic kernels do, <0 on invalid arguments */
+/* 1 if the tcgen05/TMA kernels handle this problem, 0 if the shape-generic kernels do, <0 on invalid arguments.
+ * (fb_bwd_uses_tensor_path answers for head dimensions up to 64; without factor operands the tcgen05 kernels also
+ * take 65..128, for which it keeps answering 0.) */
 int fb_fwd_uses_tensor_path(const fb_params *p);
 int fb_bwd_uses_tensor_path(const fb_params *p);
 
