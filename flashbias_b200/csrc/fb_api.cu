@@ -207,6 +207,7 @@ extern "C" int fb_bwd_uses_tensor_path(const fb_params* p) {
 
 extern "C" size_t fb_fwd_workspace_bytes(const fb_params* p) {
   if (validate_common(p)) return 0;
+  if (decode_supported(p)) return decode_workspace(p);
   PackPlan plan;
   if (fwd_sm100_supported(p, &plan)) return plan.q_bytes + plan.k_bytes + plan.qs_bytes;
   return 0;
@@ -216,6 +217,10 @@ extern "C" int fb_fwd(const fb_params* p, void* cuda_stream) {
   int rc = validate_common(p);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
+  if (decode_supported(p)) {
+    if ((rc = check_workspace(p, decode_workspace(p)))) return rc;
+    return launch_decode(p, st);
+  }
   PackPlan plan;
   if (fwd_sm100_supported(p, &plan)) {
     if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes + plan.qs_bytes))) return rc;

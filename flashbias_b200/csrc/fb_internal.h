@@ -79,6 +79,11 @@ int launch_bwd_preprocess(const fb_params* p, cudaStream_t st);
 int launch_bwd_general(const fb_params* p, cudaStream_t st);
 size_t bwd_general_workspace(const fb_params* p);
 
+// one query row per (batch, head)
+bool decode_supported(const fb_params* p);
+size_t decode_workspace(const fb_params* p);
+int launch_decode(const fb_params* p, cudaStream_t st);
+
 bool fwd_sm100_supported(const fb_params* p, PackPlan* plan);
 int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 
