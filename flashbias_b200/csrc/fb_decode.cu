@@ -7,7 +7,11 @@
 // of a CTA cover neighbouring heads of the same key, so that a (B, S, H, D) cache is read as whole contiguous rows; the
 // keys are split over enough CTAs to fill the GPU once, and a second small kernel merges the splits.  All arithmetic is
 // fp32 on the given 16-bit values (probabilities are not rounded), and no operand is packed.
-// B16 H50 Sk5001 D32 R2: 233 us with the tiled kernel (2.2 TB/s).
+// B16 H50 Sk5001 D32 R2: 233 us with the tiled kernel (2.2 TB/s), 86 us here (5.9 TB/s; 124 us when the rounds in flight
+// were held in registers, 92 us with 3 CTAs and rounds of 2 keys).
+#include <mutex>
+#include <type_traits>
+
 #include "fb_common.cuh"
 #include "fb_internal.h"
 
@@ -30,15 +34,35 @@ struct DecodeArgs {
 };
 
 constexpr int kDecodeThreads = 256;
-constexpr int kDecodeUnroll = 4;  // keys in flight per lane
+constexpr int kDecodeUnroll = 4;  // keys of a round
+constexpr int kDecodeDepth = 3;   // rounds in the ring
+constexpr int kDecodeCtas = 2;    // resident per SM
+constexpr int kDecodeRing = kDecodeDepth * kDecodeUnroll * 2 * kDecodeThreads * 16;
 constexpr float kLog2eD = 1.4426950408889634f;
 constexpr float kLn2D = 0.6931471805599453f;
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4u(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// 8 consecutive 16-bit values as fp32 pairs
 template <typename T>
-__device__ __forceinline__ void unpack8(const uint4& raw, float (&x)[8]) {
-  const T* e = reinterpret_cast<const T*>(&raw);
+__device__ __forceinline__ void unpack8(const uint4& raw, uint64_t (&x)[4]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) x[i] = to_f32(e[i]);
+  for (int i = 0; i < 4; ++i) {
+    if (std::is_same<T, __nv_bfloat16>::value) {
+      x[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+    } else {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+      x[i] = f2(f.x, f.y);
+    }
+  }
 }
 
 template <typename T>
@@ -51,11 +75,9 @@ __device__ __forceinline__ void store_row8(const DecodeArgs& a, int b, int h, in
   *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.o) + b * a.o_st[0] + h * a.o_st[1] + d0) = w;
 }
 
-// G lanes per head, NRS bias columns per lane (rank <= G * NRS)
-template <typename T, int G, int NRS>
-__global__ void __launch_bounds__(kDecodeThreads, 3) decode_kernel(const DecodeArgs a) {
-  __shared__ float s_acc[kDecodeThreads * 8];
-  __shared__ float2 s_ml[kDecodeThreads];
+// G lanes per head, NRS bias columns per lane (rank <= G * NRS); EXTRA: a mask or slopes complete the logits
+template <typename T, int G, int NRS, bool EXTRA>
+__global__ void __launch_bounds__(kDecodeThreads, kDecodeCtas) decode_kernel(const DecodeArgs a) {
   grid_dep_wait();
   const int split = blockIdx.x % a.nsplit, hgi = (blockIdx.x / a.nsplit) % a.nhg, b = blockIdx.x / (a.nsplit * a.nhg);
   const int unit = threadIdx.x / G, part = threadIdx.x % G;
@@ -66,19 +88,21 @@ __global__ void __launch_bounds__(kDecodeThreads, 3) decode_kernel(const DecodeA
 
   float qv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, qb[NRS ? NRS : 1] = {};
   float slope2 = 0.f;
-  const T *kp_ = nullptr, *vp_ = nullptr, *kbp = nullptr;
+  const T *kp_ = reinterpret_cast<const T*>(a.k), *vp_ = reinterpret_cast<const T*>(a.v);
+  const T* kbp = reinterpret_cast<const T*>(a.k_bias);
   const char* mp = nullptr;
   if (live) {
     if (cols) {
-      unpack8<T>(*reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.q) + b * a.q_st[0] + h * a.q_st[1] + part * 8), qv);
+      uint64_t x[4];
+      unpack8<T>(*reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.q) + b * a.q_st[0] + h * a.q_st[1] + part * 8), x);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) qv[i] *= a.scale_log2;
+      for (int i = 0; i < 4; ++i) f2_unpack(f2_mul(x[i], f2(a.scale_log2, a.scale_log2)), qv[2 * i], qv[2 * i + 1]);
     }
-    kp_ = reinterpret_cast<const T*>(a.k) + b * a.k_st[0] + h * a.k_st[1] + part * 8;
-    vp_ = reinterpret_cast<const T*>(a.v) + b * a.v_st[0] + h * a.v_st[1] + part * 8;
+    kp_ += b * a.k_st[0] + h * a.k_st[1] + (cols ? part * 8 : 0);
+    vp_ += b * a.v_st[0] + h * a.v_st[1] + (cols ? part * 8 : 0);
     if (NRS) {
       const T* src = reinterpret_cast<const T*>(a.q_bias) + b * a.qb_st[0] + h * a.qb_st[1];
-      kbp = reinterpret_cast<const T*>(a.k_bias) + b * a.kb_st[0] + h * a.kb_st[1];
+      kbp += b * a.kb_st[0] + h * a.kb_st[1];
 #pragma unroll
       for (int r = 0; r < NRS; ++r)
         if (part + r * G < a.R) qb[r] = to_f32(src[part + r * G]) * kLog2eD;
@@ -91,62 +115,117 @@ __global__ void __launch_bounds__(kDecodeThreads, 3) decode_kernel(const DecodeA
     }
   }
 
-  float m = -INFINITY, l = 0.f, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  // every lane of a warp runs the same number of rounds (the shuffles need all of them)
-  for (int k0 = split * a.per_split; k0 < k_end; k0 += a.kp * kDecodeUnroll) {
-    uint4 kr[kDecodeUnroll], vr[kDecodeUnroll];
-    float s[kDecodeUnroll];
+  // Each lane copies its own 16-byte chunks of K and V into its own slots of a shared-memory ring, a few rounds ahead of
+  // their use: what is in flight is then bounded by shared memory (2 CTAs x 96 KB) and not by registers, and no
+  // synchronisation is needed, since only the lane that copied a chunk reads it.
+  extern __shared__ uint4 ring[];  // [kDecodeDepth][kDecodeUnroll][K, V][thread]
+  const uint32_t slot0 = smem_u32(ring + threadIdx.x);
+  constexpr uint32_t kChunk = kDecodeThreads * 16, kRound = 2 * kDecodeUnroll * kChunk;
+  const int step = a.kp * kDecodeUnroll;
+  const int k_begin = split * a.per_split;
+  const int64_t ks = (int64_t)a.kp * a.k_st[2], vs = (int64_t)a.kp * a.v_st[2], bs = (int64_t)a.kp * a.kb_st[2];
+  const T* kf = kp_ + (int64_t)(k_begin + kl) * a.k_st[2];
+  const T* vf = vp_ + (int64_t)(k_begin + kl) * a.v_st[2];
+  const T* bf = kbp + (NRS ? (int64_t)(k_begin + kl) * a.kb_st[2] + part : 0);
+  int key_f = k_begin + kl;  // key of the first copy of the next round to fetch
+  auto fetch = [&](uint32_t slot) {
 #pragma unroll
     for (int u = 0; u < kDecodeUnroll; ++u) {
-      const int key = k0 + u * a.kp + kl;
-      kr[u] = vr[u] = make_uint4(0u, 0u, 0u, 0u);
-      s[u] = 0.f;
-      if (cols && key < k_end) {
-        kr[u] = __ldg(reinterpret_cast<const uint4*>(kp_ + (int64_t)key * a.k_st[2]));
-        vr[u] = __ldg(reinterpret_cast<const uint4*>(vp_ + (int64_t)key * a.v_st[2]));
-      }
-      if (NRS && live && key < k_end) {
-#pragma unroll
-        for (int r = 0; r < NRS; ++r)
-          if (part + r * G < a.R) s[u] = fmaf(qb[r], to_f32(kbp[(int64_t)key * a.kb_st[2] + part + r * G]), s[u]);
-      }
+      const uint32_t bytes = cols && key_f + u * a.kp < k_end ? 16u : 0u;  // beyond the range: zeros, nothing is read
+      cp_async16(slot + 2 * u * kChunk, bytes ? kf + u * ks : kp_, bytes);
+      cp_async16(slot + (2 * u + 1) * kChunk, bytes ? vf + u * vs : vp_, bytes);
     }
-    float mx = m;
+    key_f += step;
+    kf += kDecodeUnroll * ks;
+    vf += kDecodeUnroll * vs;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  T kb[kDecodeUnroll][NRS ? NRS : 1];
+  int key_b = k_begin + kl;
+  auto fetch_bias = [&] {
+    if constexpr (NRS > 0) {
+#pragma unroll
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+#pragma unroll
+        for (int c = 0; c < NRS; ++c)
+          kb[u][c] = live && key_b + u * a.kp < k_end && part + c * G < a.R ? bf[u * bs + c * G] : from_f32<T>(0.f);
+      }
+      key_b += step;
+      bf += kDecodeUnroll * bs;
+    }
+  };
+  float m = -INFINITY, l = 0.f;
+  uint64_t acc2[4] = {0ull, 0ull, 0ull, 0ull};
+  const uint64_t q2[4] = {f2(qv[0], qv[1]), f2(qv[2], qv[3]), f2(qv[4], qv[5]), f2(qv[6], qv[7])};
+#pragma unroll
+  for (int i = 0; i < kDecodeDepth - 1; ++i) fetch(slot0 + i * kRound);
+  fetch_bias();
+  uint32_t rs = 0, fs = (kDecodeDepth - 1) * kRound;  // ring offsets read and filled next
+  for (int k0 = k_begin; k0 < k_end; k0 += step) {    // (the same number of rounds for every lane: the shuffles need all)
+    fetch(slot0 + fs);
+    fs = fs + kRound == kDecodeDepth * kRound ? 0 : fs + kRound;
+    float s[kDecodeUnroll], mx = m;
+    if constexpr (NRS > 0) {
+#pragma unroll
+      for (int u = 0; u < kDecodeUnroll; ++u) {
+        s[u] = 0.f;
+#pragma unroll
+        for (int c = 0; c < NRS; ++c) s[u] = fmaf(qb[c], to_f32(kb[u][c]), s[u]);
+      }
+      fetch_bias();
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDecodeDepth - 1) : "memory");
 #pragma unroll
     for (int u = 0; u < kDecodeUnroll; ++u) {
-      const int key = k0 + u * a.kp + kl;
-      float x[8];
-      unpack8<T>(kr[u], x);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s[u] = fmaf(qv[i], x[i], s[u]);
+      uint64_t x[4];
+      unpack8<T>(ld_shared_v4u(slot0 + rs + 2 * u * kChunk), x);
+      uint64_t t = f2_mul(q2[0], x[0]), w = f2_mul(q2[1], x[1]);
+      t = f2_fma(q2[2], x[2], t);
+      w = f2_fma(q2[3], x[3], w);
+      float t0, t1;
+      f2_unpack(f2_add(t, w), t0, t1);
+      s[u] = NRS ? s[u] + (t0 + t1) : t0 + t1;
 #pragma unroll
       for (int o = G / 2; o; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-      s[u] = fmaf(slope2, (float)key, s[u]);
-      if (mp && key < k_end)
-        s[u] += kLog2eD * (a.mask_dtype == FB_DTYPE_F32   ? reinterpret_cast<const float*>(mp)[key]
-                           : a.mask_dtype == FB_DTYPE_F16 ? __half2float(reinterpret_cast<const __half*>(mp)[key])
-                                                          : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(mp)[key]));
+      const int key = k0 + u * a.kp + kl;
+      if (EXTRA) {
+        s[u] = fmaf(slope2, (float)key, s[u]);
+        if (mp && key < k_end)
+          s[u] += kLog2eD * (a.mask_dtype == FB_DTYPE_F32   ? reinterpret_cast<const float*>(mp)[key]
+                             : a.mask_dtype == FB_DTYPE_F16 ? __half2float(reinterpret_cast<const __half*>(mp)[key])
+                                                            : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(mp)[key]));
+      }
       if (key >= k_end) s[u] = -INFINITY;
       mx = fmaxf(mx, s[u]);
     }
-    const float msub = mx == -INFINITY ? 0.f : mx;
+    const float msub = fmaxf(mx, -1e38f);  // no visible key yet: every exponential below is zero
     const float alpha = fast_exp2(m - msub);  // 0 while m is still -inf
     m = mx;
     l *= alpha;
+    const uint64_t alpha2 = f2(alpha, alpha);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] *= alpha;
+    for (int i = 0; i < 4; ++i) acc2[i] = f2_mul(acc2[i], alpha2);
 #pragma unroll
     for (int u = 0; u < kDecodeUnroll; ++u) {
       const float p = fast_exp2(s[u] - msub);
-      float x[8];
-      unpack8<T>(vr[u], x);
       l += p;
+      const uint64_t p2 = f2(p, p);
+      uint64_t x[4];
+      unpack8<T>(ld_shared_v4u(slot0 + rs + (2 * u + 1) * kChunk), x);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = fmaf(p, x[i], acc[i]);
+      for (int i = 0; i < 4; ++i) acc2[i] = f2_fma(p2, x[i], acc2[i]);
     }
+    rs = rs + kRound == kDecodeDepth * kRound ? 0 : rs + kRound;
   }
+  float acc[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f2_unpack(acc2[i], acc[2 * i], acc[2 * i + 1]);
 
-  if (a.kp > 1) {  // merge the keys visited side by side
+  if (a.kp > 1) {  // merge the keys visited side by side, in the ring's memory
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float* s_acc = reinterpret_cast<float*>(ring);
+    float2* s_ml = reinterpret_cast<float2*>(s_acc + 8 * kDecodeThreads);
     s_ml[threadIdx.x] = make_float2(m, l);
 #pragma unroll
     for (int i = 0; i < 8; ++i) s_acc[i * kDecodeThreads + threadIdx.x] = acc[i];
@@ -212,10 +291,12 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeArgs a) {
   __syncthreads();
   if (sl > 0) return;
   l = 0.f;
+#pragma unroll 4
   for (int j = 0; j < LANES; ++j) l += s_l[j];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     acc[i] = 0.f;
+#pragma unroll 4
     for (int j = 0; j < LANES; ++j) acc[i] += s_acc[(j * G + part) * 9 + i];
   }
   const int b = (int)(bh / a.H), h = (int)(bh % a.H);
@@ -236,17 +317,17 @@ DecodePlan plan_decode(const fb_params* p) {
   DecodePlan d;
   d.G = p->D <= 8 ? 1 : p->D <= 16 ? 2 : p->D <= 32 ? 4 : p->D <= 64 ? 8 : 16;
   const int need = (p->R + d.G - 1) / d.G;
-  d.NRS = need <= 1 ? need : need <= 4 ? 4 : 16;
+  d.NRS = need <= 1 ? need : 4;
   d.Sk = p->causal ? 1 : p->Sk;
   // all heads in one CTA if they fit, else the smallest number of equal groups
   const int fit = kDecodeThreads / d.G;
   d.nhg = (p->H + fit - 1) / fit;
   d.hg = (p->H + d.nhg - 1) / d.nhg;
   d.kp = fit / d.hg;
-  // as many key ranges as fill the resident CTA slots (3 per SM) once, none shorter than 8 rounds
+  // as many key ranges as fill the resident CTA slots once, none shorter than 8 rounds
   int dev = 0;
   cudaGetDevice(&dev);
-  const int slots = 3 * (device_sm_count(dev) > 0 ? device_sm_count(dev) : 148);
+  const int slots = kDecodeCtas * (device_sm_count(dev) > 0 ? device_sm_count(dev) : 148);
   const int64_t ctas = (int64_t)p->B * d.nhg;
   int64_t ns = slots / ctas;
   const int64_t most = (d.Sk + (int64_t)d.kp * kDecodeUnroll * 8 - 1) / ((int64_t)d.kp * kDecodeUnroll * 8);
@@ -261,16 +342,35 @@ DecodePlan plan_decode(const fb_params* p) {
   return d;
 }
 
+template <typename T, int G, int NRS>
+int launch_decode_n(const DecodeArgs& a, unsigned grid, cudaStream_t st) {
+  auto kern = a.mask || a.alibi_slopes ? decode_kernel<T, G, NRS, true> : decode_kernel<T, G, NRS, false>;
+  static std::mutex mu;
+  static bool attr_done[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!attr_done[dev & 63]) {
+      cudaError_t e = cudaFuncSetAttribute(decode_kernel<T, G, NRS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecodeRing);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(decode_kernel<T, G, NRS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecodeRing);
+      if (e != cudaSuccess) return (int)e;
+      attr_done[dev & 63] = true;
+    }
+  }
+  return launch_pdl(kern, grid, kDecodeThreads, kDecodeRing, st, a);
+}
+
 template <typename T, int G>
 int launch_decode_g(const DecodeArgs& a, const DecodePlan& d, int B, cudaStream_t st) {
   const unsigned grid = (unsigned)((int64_t)B * d.nhg * d.nsplit);
   prof_before(KC_FWD_MAIN, st);
   int rc = FB_ENOTBUILT;
   switch (d.NRS) {
-    case 0: rc = launch_pdl(decode_kernel<T, G, 0>, grid, kDecodeThreads, 0, st, a); break;
-    case 1: rc = launch_pdl(decode_kernel<T, G, 1>, grid, kDecodeThreads, 0, st, a); break;
-    case 4: rc = launch_pdl(decode_kernel<T, G, 4>, grid, kDecodeThreads, 0, st, a); break;
-    case 16: rc = launch_pdl(decode_kernel<T, G, 16>, grid, kDecodeThreads, 0, st, a); break;
+    case 0: rc = launch_decode_n<T, G, 0>(a, grid, st); break;
+    case 1: rc = launch_decode_n<T, G, 1>(a, grid, st); break;
+    case 4: rc = launch_decode_n<T, G, 4>(a, grid, st); break;
   }
   prof_after(KC_FWD_MAIN, st);
   if (rc || d.nsplit == 1) return rc;
@@ -302,7 +402,7 @@ bool decode_supported(const fb_params* p) {
   }
   if (bits & 15) return false;
   const int G = p->D <= 8 ? 1 : p->D <= 16 ? 2 : p->D <= 32 ? 4 : p->D <= 64 ? 8 : 16;
-  return p->R <= 16 * G && (int64_t)p->B * p->H <= 0x7fffffffLL / 1024;
+  return p->R <= 4 * G && (int64_t)p->B * p->H <= 0x7fffffffLL / 1024;
 }
 
 size_t decode_workspace(const fb_params* p) {

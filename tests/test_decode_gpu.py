@@ -19,8 +19,8 @@ CASES = [
     (2, 16, 2049, 32, 0, True, None, False, torch.float16),      # several keys side by side, splits with a remainder
     (1, 50, 5001, 64, 5, False, None, False, torch.float16),     # two head groups, many splits
     (2, 50, 300, 128, 20, True, None, False, torch.bfloat16),    # four head groups, two bias columns per lane
-    (2, 3, 130, 24, 96, True, None, False, torch.bfloat16),      # rows shorter than the lane group, rank that does not fit
-    (2, 3, 130, 48, 96, True, None, False, torch.bfloat16),      # ... and one that does (12 columns per lane)
+    (2, 3, 130, 24, 96, True, None, False, torch.bfloat16),      # rank that does not fit the lane group (tiled kernel)
+    (2, 3, 130, 24, 15, True, None, False, torch.bfloat16),      # rows shorter than the lane group, four columns per lane
     (4, 2, 257, 8, 1, True, "vector", False, torch.bfloat16),    # one lane per head, key-padding mask
     (4, 6, 100, 16, 3, False, "matrix", False, torch.float16),   # periodic 16-bit mask
     (2, 4, 65, 32, 2, True, None, True, torch.bfloat16),         # causal, top-left aligned: the first key only
