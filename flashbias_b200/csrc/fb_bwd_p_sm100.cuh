@@ -148,7 +148,10 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(sdp_done, 1);  // the last S|dP products of an item have completed
       mbar_init(dp_full, 1);
       mbar_init(sdp_read, 8);  // every compute warp has S and dP of the tile in registers
-      mbar_init(all_done, 4);  // one commit per issuing thread, per item
+      // One commit per thread that issues the item's dV, dK, dQ (or dKb) products.  The thread that only issues S and dP
+      // is not one of them: it runs ahead, and when the next item has a single query tile its commit for that item
+      // would arrive before the dK product of this one and complete the phase early.
+      mbar_init(all_done, Cfg::SEP_DKB ? 4 : 3);
       mbar_init(acc_free, 8);  // the compute warps have read the dV / dK | dKb accumulators of an item
       for (int i = 0; i < 2; ++i)  // the dV, dK, dQ (and dKb) chains have read P and dS of a query tile (per buffer pair)
         mbar_init(pds_free + 8 * i, Cfg::SEP_DKB ? 4 : 3);
@@ -339,8 +342,10 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               load_kva(nx);
             }
           }
-          if (Cfg::SEP_DKB) issue_dKb(x.n_it - 1, tn - 1);
-          umma_commit(all_done);  // every MMA of this thread for the item
+          if (Cfg::SEP_DKB) {
+            issue_dKb(x.n_it - 1, tn - 1);
+            umma_commit(all_done);  // every MMA of this thread for the item
+          }
           ++n;
         }
       } else {
