@@ -13,7 +13,7 @@
 //               and V tiles through rings of shared-memory stages.
 //   warp 5      MMA issuer (one thread): S = [Q|Qb].[K|Kb]^T into TMEM, bias products first.
 //   warp 6      MMA issuer (one thread, another warp scheduler): O += P.V with P read from TMEM.
-//   warp 7      idle (completes the second warpgroup, which hands most of its registers to the first).
+//   warp 7      mask tiles through a ring of their own, where there is a mask that TMA can address.
 //   warps 0-3   softmax: one thread per query row (= one TMEM lane).  The thread takes all 128 logits of
 //               its row into registers with one round of TMEM loads and releases S at once, so the tensor
 //               core computes the next key tile's logits under this tile's exponentials.  Row maximum,
@@ -23,7 +23,7 @@
 //               rescale"), which is exact because the row sum carries the same reference maximum.
 // All logit terms share one accumulator: S' = qs.k + qb.k_bias, with qs = q and qb = q_bias/scale when the
 // scale is a power of two (p = exp2((S' - m) * scale * log2 e)), else qs = (hi, lo) of q*scale and qb = q_bias.
-// An additive mask tensor is added in registers (row-contiguous loads, one mask row per thread); the fused
+// An additive mask tensor is added in registers (one mask row per thread, through a TMA ring where the mask's rows are aligned); the fused
 // ALiBi producer adds slope * (col - row) with one FMA per logit and needs no factor operands at all.
 // Two CTAs share an SM when their tiles fit (256 TMEM columns each) so one CTA's softmax overlaps the
 // other's MMAs and loads.
@@ -50,10 +50,11 @@ struct FwdArgs {
   const void* mask;  // additive mask, (batch, head, row) element strides; row stride 0 for a (1, Sk) mask
   int64_t mask_stride[3];
   int mask_kind, mask_dtype, mask_batch_period;
+  int mask_tma, mask_b1, mask_h1;  // mask tiles come by TMA; the mask has extent 1 on batch / heads
   const float* alibi_slopes;
 };
 
-template <int D, int RP, int NQ>
+template <int D, int RP, int NQ, bool MASKED = false>
 struct FwdCfg {
   static constexpr int RPX = RP ? RP : 16;  // keeps templates well-formed when there is no bias
   static constexpr int Q_BYTES = tile_bytes(D);
@@ -73,17 +74,23 @@ struct FwdCfg {
   static constexpr int MINB = TWO ? 2 : 1;
   // as many K|Kb and V stages (up to 4) as fit: the TMA producer runs that many key tiles ahead, which is
   // what hides the L2/HBM latency of the loads
-  static constexpr int KST = smem_for(4, 4) <= LIM ? 4 : smem_for(3, 3) <= LIM ? 3 : smem_for(2, 2) <= LIM ? 2
-                             : smem_for(2, 1) <= LIM ? 2 : 1;
+  // With a mask, stages of it (128 rows of 128 bytes) come before a third stage of K and V.
+  static constexpr int M_STAGE = 128 * 128;
+  static constexpr int MOST = MASKED ? 2 : 4;
+  static constexpr int KST = MOST >= 4 && smem_for(4, 4) <= LIM ? 4 : MOST >= 3 && smem_for(3, 3) <= LIM ? 3
+                             : smem_for(2, 2) <= LIM ? 2 : smem_for(2, 1) <= LIM ? 2 : 1;
   static constexpr int VST = smem_for(KST, KST) <= LIM ? KST : 1;
-  static constexpr int SMEM = smem_for(KST, VST);
+  static constexpr int MST_FIT = MASKED ? (LIM - smem_for(KST, VST)) / M_STAGE : 0;
+  static constexpr int MST = MST_FIT < 0 ? 0 : MST_FIT > 4 ? 4 : MST_FIT;  // 0: masks are read by the softmax threads
+  static constexpr int SMEM = smem_for(KST, VST) + MST * M_STAGE;
   static constexpr bool FITS = SMEM <= LIM;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_QB = OFF_Q + NQ * Q_BYTES;  // NQ query terms (q, or hi and lo of q*scale), then Qb
   static constexpr int OFF_K = OFF_QB + QB_BYTES;
   static constexpr int OFF_KB = OFF_K + KST * Q_BYTES;
   static constexpr int OFF_V = OFF_KB + KST * QB_BYTES;
-  static constexpr int OFF_BAR = OFF_V + VST * Q_BYTES;
+  static constexpr int OFF_M = OFF_V + VST * Q_BYTES;
+  static constexpr int OFF_BAR = OFF_M + MST * M_STAGE;
 };
 
 template <int C>
@@ -97,12 +104,15 @@ __device__ __forceinline__ void tma_tile_4d(uint32_t dst, const CUtensorMap* m, 
 
 enum { FWD_PLAIN = 0, FWD_MASK = 1, FWD_ALIBI = 2 };
 
-template <typename T, int D, int RP, int NQ, bool ALIBI>
-__global__ void __launch_bounds__(256, FwdCfg<D, RP, NQ>::MINB)
+// MODE: how the logits are completed -- as computed, plus an additive mask tensor, plus the fused ALiBi term.  A kernel
+// parameter rather than a run-time branch: the mask ring takes shared memory from the K and V rings.
+template <typename T, int D, int RP, int NQ, int MODE>
+__global__ void __launch_bounds__(256, FwdCfg<D, RP, NQ, MODE == FWD_MASK>::MINB)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQb,
-                 const __grid_constant__ CUtensorMap tmKb, const FwdArgs a) {
-  using Cfg = FwdCfg<D, RP, NQ>;
+                 const __grid_constant__ CUtensorMap tmKb, const __grid_constant__ CUtensorMap tmM, const FwdArgs a) {
+  using Cfg = FwdCfg<D, RP, NQ, MODE == FWD_MASK>;
+  constexpr int MST = Cfg::MST;
   constexpr int KST = Cfg::KST, VST = Cfg::VST;
   constexpr int RPX = Cfg::RPX;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
@@ -111,12 +121,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
   const uint32_t sQ = sbase + Cfg::OFF_Q, sQb = sbase + Cfg::OFF_QB, sK = sbase + Cfg::OFF_K,
-                 sKb = sbase + Cfg::OFF_KB, sV = sbase + Cfg::OFF_V;
+                 sKb = sbase + Cfg::OFF_KB, sV = sbase + Cfg::OFF_V, sM = sbase + Cfg::OFF_M;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   // barrier slots
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t q_full = bar0, s_full = bar0 + 8, p_ready = bar0 + 16, pv_done = bar0 + 24, s_read = bar0 + 176;
   const uint32_t k_full = bar0 + 32, k_free = bar0 + 64, v_full = bar0 + 96, v_free = bar0 + 128;  // 4 slots each
+  const uint32_t m_full = bar0 + 192, m_free = bar0 + 224;  // likewise
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 160);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 168);
 
@@ -163,6 +174,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_init(k_free + 8 * i, 1);
         mbar_init(v_full + 8 * i, 1);
         mbar_init(v_free + 8 * i, 1);
+        mbar_init(m_full + 8 * i, 1);
+        mbar_init(m_free + 8 * i, 4);  // one arrival per softmax warp
       }
       mbar_init(q_free, 1);
       mbar_fence_init();
@@ -273,6 +286,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
     }
+    if constexpr (MST > 0) {
+      if (warp == 7 && lane == 0 && a.mask_tma) {
+        // ---------------------------------------------------------------- mask tiles, 128 bytes of every row at a time
+        const int per = a.mask_dtype == FB_DTYPE_F32 ? 32 : 64;  // columns of a stage
+        int mc = 0;
+        for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w) {
+          const Item it = item_of(idx);
+          const int mb = a.mask_b1 ? 0 : a.mask_batch_period > 0 ? it.b % a.mask_batch_period : it.b;
+          const int mh = a.mask_h1 ? 0 : it.h;
+          for (int col = 0; col < it.n_kv * 128; col += per, ++mc) {
+            const int st = mc % MST;
+            if (mc >= MST) mbar_wait(m_free + 8 * st, ((mc / MST) - 1) & 1, abort_flag, a.status);
+            mbar_expect_tx(m_full + 8 * st, Cfg::M_STAGE);
+            tma_load_4d(sM + st * Cfg::M_STAGE, &tmM, m_full + 8 * st, col, it.q0, mh, mb);
+          }
+        }
+      }
+    }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
     if constexpr (Cfg::MINB == 2) setmaxnreg_inc<208>();
@@ -285,15 +316,43 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     float m_used = -INFINITY, l = 0.f;  // running reference maximum and row sum, in units of log2 (logit * log2 e)
     float slope2 = 0.f;                 // ALiBi slope of this head, times log2 e
     const char* mrow = nullptr;         // additive mask: this thread's row
-    int msize = 4;
     bool mvec = false;
     int t = 0;  // key tiles processed so far by this CTA (barrier phases run across work items)
     uint32_t s[4][32];  // the thread's row of the logit tile
 
-    // One key tile.  MODE: how the logits are completed (plain / + mask tensor / + ALiBi term);
-    // DEAD: the tile has columns beyond Sk or above the causal diagonal.
-    auto tile = [&](int j, auto mode_c, auto dead_c) {
-      constexpr int MODE = decltype(mode_c)::value;
+    // Additive mask, 32 values of the thread's row as fp32, times log2 e.  They come through the ring that warp 7 fills;
+    // rows that TMA cannot address (unaligned, or a (1, Sk) mask) are loaded by the threads.  A row per thread makes every
+    // load of a warp touch 32 lines, and that, not latency, was the cost: B1024 H8 S256 D32 with a shifted window's mask,
+    // 535 us with the loads behind the logits, 520 us with all of a row's loads requested ahead of them, 440 us here.
+    int mc = 0;  // mask stages consumed so far
+    auto mask_chunk = [&](int k0, int c, auto mask_c, float (&mv)[32]) {
+      using MT = decltype(mask_c);
+      if (MST > 0 && a.mask_tma) {
+        constexpr int V = 2 * (int)sizeof(MT);  // 16-byte vectors of a chunk: a stage holds one (fp32) or two of them
+        const int st = mc % (MST > 0 ? MST : 1);
+        if (V == 8 || (c & 1) == 0) mbar_wait(m_full + 8 * st, (mc / (MST > 0 ? MST : 1)) & 1, abort_flag, a.status);
+        const uint32_t base = sM + st * Cfg::M_STAGE + row * 128;
+#pragma unroll
+        for (int g = 0; g < V; ++g) {
+          const int ch = (V == 8 ? 0 : (c & 1) * 4) + g;
+          uint32_t w[4];
+          ld_shared_v4(base + ((ch ^ (row & 7)) << 4), w[0], w[1], w[2], w[3]);
+          const MT* e = reinterpret_cast<const MT*>(w);
+#pragma unroll
+          for (int i = 0; i < 32 / V; ++i) mv[g * (32 / V) + i] = to_f32(e[i]) * kLog2e;
+        }
+        if (V == 8 || (c & 1) == 1) {
+          mbar_arrive_warp(m_free + 8 * st);
+          ++mc;
+        }
+      } else {
+        const int n = min(32, a.Sk - (k0 + c * 32));
+        load_mask_chunk(reinterpret_cast<const MT*>(mrow) + (k0 + c * 32), n, mvec && n == 32, mv);
+      }
+    };
+
+    // One key tile.  DEAD: the tile has columns beyond Sk or above the causal diagonal.
+    auto tile = [&](int j, auto dead_c, auto mask_c) {
       constexpr bool DEAD = decltype(dead_c)::value;
       const int k0 = j * 128;
       // ---- logits from tensor memory (the load of one 32-column chunk overlaps the arithmetic of the previous
@@ -304,14 +363,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t tSl = tS + lane_off;
       auto complete = [&](int c) {
         float mv[32];
-        if (MODE == FWD_MASK) {
-          const int n = min(32, a.Sk - (k0 + c * 32));
-          const char* p = mrow + (int64_t)(k0 + c * 32) * msize;
-          const bool vec = mvec && n == 32;
-          if (a.mask_dtype == FB_DTYPE_F32) load_mask_chunk(reinterpret_cast<const float*>(p), n, vec, mv);
-          else if (a.mask_dtype == FB_DTYPE_F16) load_mask_chunk(reinterpret_cast<const __half*>(p), n, vec, mv);
-          else load_mask_chunk(reinterpret_cast<const __nv_bfloat16*>(p), n, vec, mv);
-        }
+        if constexpr (MODE == FWD_MASK) mask_chunk(k0, c, mask_c, mv);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float v0 = __uint_as_float(s[c][i]), v1 = __uint_as_float(s[c][i + 1]);
@@ -405,9 +457,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     grow = q0 + row;
     m_used = -INFINITY;
     l = 0.f;
-    if (ALIBI) slope2 = __ldg(a.alibi_slopes + h) * kLog2e;
-    if (!ALIBI && a.mask_kind != FB_MASK_NONE) {
-      msize = a.mask_dtype == FB_DTYPE_F32 ? 4 : 2;
+    if (MODE == FWD_ALIBI) slope2 = __ldg(a.alibi_slopes + h) * kLog2e;
+    if (MODE == FWD_MASK) {
+      const int msize = a.mask_dtype == FB_DTYPE_F32 ? 4 : 2;
       const int mb = a.mask_batch_period > 0 ? b % a.mask_batch_period : b;
       const int64_t off = mb * a.mask_stride[0] + h * a.mask_stride[1] +
                           (int64_t)min(grow, a.Sq - 1) * a.mask_stride[2];
@@ -419,16 +471,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_wait(s_full, t & 1, abort_flag, a.status);
       tc_fence_after_sync();
       const bool dead = (a.causal && k0 + 127 > q0) || (k0 + 128 > a.Sk);
-      if constexpr (ALIBI) {
-        if (dead) tile(j, std::integral_constant<int, FWD_ALIBI>{}, std::true_type{});
-        else tile(j, std::integral_constant<int, FWD_ALIBI>{}, std::false_type{});
-      } else if (mrow) {
-        if (dead) tile(j, std::integral_constant<int, FWD_MASK>{}, std::true_type{});
-        else tile(j, std::integral_constant<int, FWD_MASK>{}, std::false_type{});
-      } else {
-        if (dead) tile(j, std::integral_constant<int, FWD_PLAIN>{}, std::true_type{});
-        else tile(j, std::integral_constant<int, FWD_PLAIN>{}, std::false_type{});
-      }
+      auto step = [&](auto mask_c) {
+        if (dead) tile(j, std::true_type{}, mask_c);
+        else tile(j, std::false_type{}, mask_c);
+      };
+      if (MODE == FWD_MASK && a.mask_dtype == FB_DTYPE_F16) step(__half{});
+      else if (MODE == FWD_MASK && a.mask_dtype == FB_DTYPE_BF16) step(__nv_bfloat16{});
+      else step(float{});
       tmem_wait_st();
       tc_fence_before_sync();
       mbar_arrive_warp(p_ready);
@@ -477,9 +526,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-template <typename T, int D, int RP, int NQ, bool ALIBI>
+template <typename T, int D, int RP, int NQ, int MODE>
 int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
-  using Cfg = FwdCfg<D, RP, NQ>;
+  using Cfg = FwdCfg<D, RP, NQ, MODE == FWD_MASK>;
   if constexpr (!Cfg::FITS) {
     return FB_ENOTBUILT;
   } else {
@@ -537,11 +586,15 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     a.mask_kind = p->mask_kind;
     a.mask_dtype = p->mask_dtype;
     a.mask_batch_period = p->mask_batch_period;
+    a.mask_b1 = p->mask_stride[0] == 0;
+    a.mask_h1 = p->mask_stride[1] == 0;
+    CUtensorMap tM = tQ;
+    a.mask_tma = MODE == FWD_MASK && Cfg::MST > 0 && make_tmap_mask(&tM, p);
     a.alibi_slopes = p->alibi_slopes;
     // (the tensor maps above are encoded first: the host then has the main kernel's launch ready while the operand
     // preparation runs)
     if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, qs, false, nullptr, nullptr, 0}, st))) return rc;
-    auto kern = fwd_sm100_kernel<T, D, RP, NQ, ALIBI>;
+    auto kern = fwd_sm100_kernel<T, D, RP, NQ, MODE>;
     // per kernel instantiation and device: raise the dynamic shared-memory limit once
     static std::mutex mu;
     static int sm_count[64] = {};  // 0: not set up on that device yet
@@ -562,7 +615,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     const int slots = sm_count[dev & 63] * Cfg::MINB;
     const unsigned grid = (unsigned)(a.total_items < slots ? a.total_items : slots);
     prof_before(KC_FWD_MAIN, st);
-    rc = launch_pdl(kern, grid, 256, Cfg::SMEM, st, tQ, tK, tV, tQb, tKb, a);
+    rc = launch_pdl(kern, grid, 256, Cfg::SMEM, st, tQ, tK, tV, tQb, tKb, tM, a);
     prof_after(KC_FWD_MAIN, st);
     return rc;
   }
@@ -577,21 +630,26 @@ int dispatch_fwd_d64(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_fwd_d128(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 
 #define FB_FWD_DISPATCH_BODY(DD)                                                                            \
-  template <typename T>                                                                                     \
-  static int dispatch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {                    \
-    if (p->alibi_slopes) return launch_fwd_t<T, DD, 0, 1, true>(p, plan, st);                               \
+  template <typename T, int MODE>                                                                           \
+  static int dispatch_rank(const fb_params* p, const PackPlan& plan, cudaStream_t st) {                     \
     switch (plan.RP) {                                                                                      \
-      case 0: return launch_fwd_t<T, DD, 0, 1, false>(p, plan, st);                                         \
-      case 16: return plan.nq == 2 ? launch_fwd_t<T, DD, 16, 2, false>(p, plan, st)                         \
-                                   : launch_fwd_t<T, DD, 16, 1, false>(p, plan, st);                        \
-      case 32: return plan.nq == 2 ? launch_fwd_t<T, DD, 32, 2, false>(p, plan, st)                         \
-                                   : launch_fwd_t<T, DD, 32, 1, false>(p, plan, st);                        \
-      case 64: return plan.nq == 2 ? launch_fwd_t<T, DD, 64, 2, false>(p, plan, st)                         \
-                                   : launch_fwd_t<T, DD, 64, 1, false>(p, plan, st);                        \
-      case 128: return plan.nq == 2 ? launch_fwd_t<T, DD, 128, 2, false>(p, plan, st)                       \
-                                    : launch_fwd_t<T, DD, 128, 1, false>(p, plan, st);                      \
+      case 0: return launch_fwd_t<T, DD, 0, 1, MODE>(p, plan, st);                                          \
+      case 16: return plan.nq == 2 ? launch_fwd_t<T, DD, 16, 2, MODE>(p, plan, st)                          \
+                                   : launch_fwd_t<T, DD, 16, 1, MODE>(p, plan, st);                         \
+      case 32: return plan.nq == 2 ? launch_fwd_t<T, DD, 32, 2, MODE>(p, plan, st)                          \
+                                   : launch_fwd_t<T, DD, 32, 1, MODE>(p, plan, st);                         \
+      case 64: return plan.nq == 2 ? launch_fwd_t<T, DD, 64, 2, MODE>(p, plan, st)                          \
+                                   : launch_fwd_t<T, DD, 64, 1, MODE>(p, plan, st);                         \
+      case 128: return plan.nq == 2 ? launch_fwd_t<T, DD, 128, 2, MODE>(p, plan, st)                        \
+                                    : launch_fwd_t<T, DD, 128, 1, MODE>(p, plan, st);                       \
     }                                                                                                       \
     return FB_ENOTBUILT;                                                                                    \
+  }                                                                                                         \
+  template <typename T>                                                                                     \
+  static int dispatch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {                    \
+    if (p->alibi_slopes) return launch_fwd_t<T, DD, 0, 1, FWD_ALIBI>(p, plan, st);                          \
+    if (p->mask_kind != FB_MASK_NONE) return dispatch_rank<T, FWD_MASK>(p, plan, st);                       \
+    return dispatch_rank<T, FWD_PLAIN>(p, plan, st);                                                        \
   }
 
 }  // namespace fb

@@ -34,6 +34,9 @@ struct Div {
 // Returns 0 or a negative FB_E* / positive cudaError_t.
 int make_tmap_4d(CUtensorMap* out, const void* ptr, int cols, int64_t rows, int64_t heads, int64_t batch,
                  int64_t stride_row, int64_t stride_head, int64_t stride_batch, int box_cols, int box_rows);
+// Tensor map over a matrix mask of any element type, box = 128 rows of 128 bytes (128-byte swizzle), extents 1 on broadcast
+// dimensions; false if TMA cannot address its rows (base or a stride not a multiple of 16 bytes, a (1, Sk) mask).
+bool make_tmap_mask(CUtensorMap* out, const fb_params* p);
 // True if a (ptr, strides) tensor can be described by make_tmap_4d.
 bool tma_compatible(const void* ptr, int64_t stride_row, int64_t stride_head, int64_t stride_batch, int64_t heads,
                     int64_t batch);

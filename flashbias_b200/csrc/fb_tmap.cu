@@ -66,4 +66,23 @@ int make_tmap_4d(CUtensorMap* out, const void* ptr, int cols, int64_t rows, int6
   return r == CUDA_SUCCESS ? 0 : FB_EINVAL_STRIDE;
 }
 
+bool make_tmap_mask(CUtensorMap* out, const fb_params* p) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc || p->mask_kind != FB_MASK_MATRIX || (reinterpret_cast<uintptr_t>(p->mask) & 15)) return false;
+  const int es = p->mask_dtype == FB_DTYPE_F32 ? 4 : 2;
+  const int64_t row = p->mask_stride[2] * es;
+  int64_t head = p->mask_stride[1] * es, batch = p->mask_stride[0] * es;
+  if (row <= 0 || row % 16 || head % 16 || batch % 16) return false;
+  const int64_t heads = head ? p->H : 1, batches = !batch ? 1 : p->mask_batch_period > 0 ? p->mask_batch_period : p->B;
+  if (!head) head = row * p->Sq;  // a dimension of extent 1 never advances: any legal stride
+  if (!batch) batch = head * heads;
+  cuuint64_t dims[4] = {(cuuint64_t)p->Sk, (cuuint64_t)p->Sq, (cuuint64_t)heads, (cuuint64_t)batches};
+  cuuint64_t strides[3] = {(cuuint64_t)row, (cuuint64_t)head, (cuuint64_t)batch};
+  cuuint32_t box[4] = {(cuuint32_t)(128 / es), 128, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return enc(out, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4,
+             const_cast<void*>(p->mask), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace fb

@@ -1,0 +1,51 @@
+"""Mask tiles through the forward's TMA ring: element types, ragged and causal tiles, broadcast, periodic and per-head
+masks, strided rows, and a mask whose rows TMA cannot address beside one that it can."""
+import math
+
+import pytest
+import torch
+
+from flashbias_b200 import check_device_status
+from flashbias_b200.flash_bias import flash_bias_forward
+from oracle import flashbias_oracle as orc
+from tests.helpers import check_close
+
+pytestmark = pytest.mark.gpu
+
+# (B, H, Sq, Sk, D, R, causal, mask batch, mask heads, mask dtype, dtype)
+CASES = [
+    (40, 8, 256, 256, 32, 16, False, 4, 1, torch.float32, torch.float16),     # many items per CTA, periodic
+    (40, 8, 144, 144, 32, 16, False, 40, 8, torch.float16, torch.float16),    # 16-bit, a mask of its own for every head
+    (2, 3, 200, 328, 32, 0, False, 1, 3, torch.bfloat16, torch.bfloat16),     # ragged in both directions
+    (1, 4, 130, 260, 64, 5, True, 1, 1, torch.float32, torch.bfloat16),       # causal, Sq < Sk: tiles beyond the diagonal
+    (2, 2, 300, 516, 64, 40, False, 2, 1, torch.float32, torch.float16),      # packed rank 64
+    (1, 2, 264, 400, 128, 20, False, 1, 2, torch.bfloat16, torch.bfloat16),   # head_dim 128
+    (2, 2, 256, 384, 32, 70, False, 2, 2, torch.float32, torch.bfloat16),     # packed rank 128
+    (2, 2, 196, 49, 32, 8, False, 2, 1, torch.float32, torch.bfloat16),       # rows of 196 bytes: not addressable by TMA
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "B%dH%dSq%dSk%dD%dR%d%s" % (*c[:6], "c" if c[6] else ""))
+@pytest.mark.parametrize("padded_rows", [False, True])
+def test_masked_forward(case, padded_rows):
+    B, H, Sq, Sk, D, R, causal, mB, mH, mdtype, dtype = case
+    g = torch.Generator().manual_seed(Sq + Sk + D)
+    q = torch.randn(B, Sq, H, D, generator=g).to(dtype)
+    k, v = (torch.randn(B, Sk, H, D, generator=g).to(dtype) for _ in range(2))
+    qb = kb = None
+    if R:
+        qb, kb = ((torch.randn(1, S, H, R, generator=g) * 0.5).to(dtype) for S in (Sq, Sk))
+    mask = torch.randn(mB, mH, Sq, Sk, generator=g)
+    mask = torch.where(torch.rand(mB, mH, Sq, Sk, generator=g) < 0.2, torch.tensor(-100.0), mask).to(mdtype)
+    mask[..., Sq // 2, 1:] = float("-inf")  # a row that sees one key
+    mdev = torch.zeros(mB, mH, Sq, Sk + 24, dtype=mdtype, device="cuda")[..., :Sk] if padded_rows else torch.empty_like(mask, device="cuda")
+    mdev.copy_(mask)
+    dev = [t.cuda() if t is not None else None for t in (q, k, v, qb, kb)]
+    o, lse, _ = flash_bias_forward(*dev, mdev, causal, None)
+    torch.cuda.synchronize()
+    check_device_status()
+    f = [t.float() if t is not None else None for t in (q, k, v, qb, kb)]
+    m = mask.float().repeat(B // mB, 1, 1, 1) if mB > 1 else mask.float()
+    o_ref, lse_ref = orc.attention_forward(*f, m, causal, 1.0 / math.sqrt(D))
+    check_close("mask_ring/B%dSq%dSk%dD%dR%d%s" % (B, Sq, Sk, D, R, "p" if padded_rows else ""), o, o_ref, dtype)
+    assert (lse[:, :, :Sq].float().cpu() - lse_ref).abs().max().item() < 2e-2
