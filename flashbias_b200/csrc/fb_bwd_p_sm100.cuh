@@ -7,7 +7,7 @@
 // item are computed, and the allocation of tensor memory, the barrier set-up and the CTA launch happen once.
 // Between items the resident key tiles are reloaded in two groups, each as soon as its last reader has completed
 // (the S|dP operands one query tile before the item ends), the dV / dK accumulators are handed over through one
-// more barrier (acc_free), and dV, dK and dk_bias leave as staged tiles through the copy engine.
+// more barrier (acc_free), and dV, dK and dk_bias leave as staged tiles through the copy engine (BwdPCfg: by which warps).
 //
 // Short sequences are what this form is for (windowed attention: two query tiles per item), where the set-up
 // and drain of a CTA cost more than its tiles; with many query tiles per item the one-item-per-CTA kernel, whose
@@ -25,6 +25,20 @@ struct BwdItem {
 };
 
 
+// Tensor memory of the persistent form.  Where dK and dkb are one accumulator (packed rank 32) there are two sets of dV and
+// dK | dkb accumulators, used by alternating items, beside one dQ | dQb accumulator: the drain warpgroup then stores an
+// item's dV, dK and dkb while the compute warps are on the next item's tiles.  (With one set the compute warps waited
+// for the item's last products and stored them themselves: 4100 of an item's 12000 clk on the windowed shape.)
+template <int D, int RP, int NQ>
+struct BwdPCfg : BwdCfg<D, RP, NQ> {
+  using Base = BwdCfg<D, RP, NQ>;
+  static constexpr bool ASYNC = Base::MERGE_K && Base::STAGED && RP == 32;
+  static constexpr int ACC_STRIDE = ASYNC ? D + 64 : 0;  // columns between the two accumulator sets
+  static constexpr int NDQ = ASYNC ? 1 : Base::NDQ;
+  static constexpr int T_DQ = ASYNC ? Base::T_DV + 2 * ACC_STRIDE : Base::T_DQ, T_DQB = T_DQ + D;
+  static_assert(!Base::FITS || T_DQB + Base::RC + (NDQ - 1) * Base::DQ_STRIDE <= 512, "tensor memory");
+};
+
 // arguments of the persistent form beyond BwdArgs
 struct BwdPArgs {
   int total_items;   // (key tile, batch, head) work items = nk_tiles * B * H
@@ -40,7 +54,8 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                  const __grid_constant__ CUtensorMap tmKc, const __grid_constant__ CUtensorMap tmKs,
                  const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
                  const BwdArgs a, const BwdPArgs pa) {
-  using Cfg = BwdCfg<D, RP, NQ>;
+  using Cfg = BwdPCfg<D, RP, NQ>;
+  constexpr bool ASYNC = Cfg::ASYNC;
   constexpr int RPX = Cfg::RPX;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   constexpr float kLog2e = 1.4426950408889634f;
@@ -57,6 +72,13 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                  dq_full = bar0 + 32 /*2*/, qdo_full = bar0 + 48 /*3*/, qdo_free = bar0 + 72 /*3*/,
                  all_done = bar0 + 112, pds_free = bar0 + 120, pds_ready = bar0 + 136 /*2*/,
                  dq_drained = bar0 + 152 /*2*/, acc_free = bar0 + 168, sdp_done = bar0 + 176;
+  // per accumulator set (item n uses set n & 1; one set: always the first)
+  auto all_done_of = [&](int n) { return ASYNC && (n & 1) ? bar0 + 184 : all_done; };
+  auto acc_free_of = [&](int n) { return ASYNC && (n & 1) ? bar0 + 192 : acc_free; };
+  // Issuing threads, before an item's first product into the accumulators: the item that used the set last has been read.
+  auto wait_acc_free = [&](int n, volatile int* flag) {
+    if (ASYNC ? n >= 2 : n > 0) mbar_wait(acc_free_of(n), ASYNC ? ((n >> 1) - 1) & 1 : (n - 1) & 1, flag);
+  };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 96);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 104);
 
@@ -73,13 +95,13 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int idx = w * G + ((w & 1) ? G - 1 - c : c);
     x.valid = idx < limit;
     if (a.causal) {
-      x.kt = (int)pa.div_bh.quot(idx);
+      x.kt = pa.div_bh.quot32(idx);
       x.bh = idx - x.kt * BH;
     } else {
-      x.bh = (int)pa.div_nk.quot(idx);
+      x.bh = pa.div_nk.quot32(idx);
       x.kt = idx - x.bh * a.nk_tiles;
     }
-    x.b = (int)pa.div_h.quot(x.bh);
+    x.b = pa.div_h.quot32(x.bh);
     x.h = x.bh - x.b * a.H;
     x.k0 = x.kt * 128;
     x.i_begin = a.causal ? x.kt : 0;    // first query tile with a row >= k0
@@ -151,8 +173,12 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       // One commit per thread that issues the item's dV, dK, dQ (or dKb) products.  The thread that only issues S and dP
       // is not one of them: it runs ahead, and when the next item has a single query tile its commit for that item
       // would arrive before the dK product of this one and complete the phase early.
-      mbar_init(all_done, Cfg::SEP_DKB ? 4 : 3);
-      mbar_init(acc_free, 8);  // the compute warps have read the dV / dK | dKb accumulators of an item
+      // (Two sets: the dV and the dK thread, per set, so that the one that is ahead cannot commit for the other's item.)
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(all_done_of(i), ASYNC ? 2 : Cfg::SEP_DKB ? 4 : 3);
+        mbar_init(acc_free_of(i), ASYNC ? 4 : 8);  // the warps that read an item's dV / dK | dKb accumulators
+        if (!ASYNC) break;
+      }
       for (int i = 0; i < 2; ++i)  // the dV, dK, dQ (and dKb) chains have read P and dS of a query tile (per buffer pair)
         mbar_init(pds_free + 8 * i, Cfg::SEP_DKB ? 4 : 3);
       for (int i = 0; i < 3; ++i) {
@@ -206,9 +232,9 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int qb = (int)(it % Cfg::NDQ);  // dQ|dQb accumulator of this tile
         const uint32_t tq = tmem + qb * Cfg::DQ_STRIDE;
         const uint32_t pb = (it % Cfg::NBUF) * Cfg::PDS_STRIDE;  // P/dS buffer pair of this tile
-        mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+        mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
         if (it >= (uint32_t)Cfg::NDQ)  // the drain warpgroup has read the tile that used this accumulator last
-          mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag, a.status);
+          mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag);
         tc_fence_after_sync();
 #pragma unroll
         for (int s = 0; s < 8; ++s) {  // contraction over the 128 keys
@@ -232,20 +258,20 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int w = 0;; ++w) {
         const BwdItem x = next_active(w);
         if (!x.valid) break;
-        mbar_wait(kvb_full, n & 1, abort_flag, a.status);
+        mbar_wait(kvb_full, n & 1, abort_flag);
 #pragma unroll 1
         for (int it = 0; it < x.n_it; ++it, ++tn) {
           issue_dQ(tn);
           if (lx.valid) {  // the S|dP, dV and dK chains have finished reading the stage of tile tn: tile tn + NSTAGE
-            mbar_wait(qdo_free + 8 * (tn % Cfg::NSTAGE), (tn / Cfg::NSTAGE) & 1, abort_flag, a.status);
+            mbar_wait(qdo_free + 8 * (tn % Cfg::NSTAGE), (tn / Cfg::NSTAGE) & 1, abort_flag);
             load_next();
           }
         }
-        umma_commit(all_done);
+        if (!ASYNC) umma_commit(all_done);
         const BwdItem nx = get_item(w + 1, pa.active_items);
         if (nx.valid) {  // K and Kc are free once the dQ | dQb products of the item's last tile have completed
           const uint32_t tl = tn - 1;
-          mbar_wait(dq_full + 8 * (tl % Cfg::NDQ), (tl / Cfg::NDQ) & 1, abort_flag, a.status);
+          mbar_wait(dq_full + 8 * (tl % Cfg::NDQ), (tl / Cfg::NDQ) & 1, abort_flag);
           load_kvb(nx);
         }
         ++n;
@@ -281,9 +307,8 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         auto issue_dKb = [&](int it, uint32_t t) {  // it: tile of the item, t: running tile count
           const int st = (int)(t % Cfg::NSTAGE);
           const uint32_t so = st * Cfg::STAGE_BYTES;
-          mbar_wait(pds_ready + 8 * (t & 1), (t >> 1) & 1, abort_flag, a.status);
-          if (it == 0 && n > 0)  // the compute warps have read the previous item's accumulator
-            mbar_wait(acc_free, (n - 1) & 1, abort_flag, a.status);
+          mbar_wait(pds_ready + 8 * (t & 1), (t >> 1) & 1, abort_flag);
+          if (it == 0) wait_acc_free(n, abort_flag);
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < 8; ++s)
@@ -296,18 +321,18 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int w = 0;; ++w) {
           const BwdItem x = next_active(w);
           if (!x.valid) break;
-          mbar_wait(kva_full, n & 1, abort_flag, a.status);
-          if (NQ != 2) mbar_wait(kvb_full, n & 1, abort_flag, a.status);  // S reads K itself
+          mbar_wait(kva_full, n & 1, abort_flag);
+          if (NQ != 2) mbar_wait(kvb_full, n & 1, abort_flag);  // S reads K itself
           tc_fence_after_sync();
 #pragma unroll 1
           for (int it = 0; it < x.n_it; ++it, ++tn) {
             const int st = (int)(tn % Cfg::NSTAGE);
             const uint32_t so = st * Cfg::STAGE_BYTES;
             if (tn > 0) {  // the compute warps hold S and dP of the previous tile in registers
-              mbar_wait(sdp_read, (tn - 1) & 1, abort_flag, a.status);
+              mbar_wait(sdp_read, (tn - 1) & 1, abort_flag);
               tc_fence_after_sync();
             }
-            mbar_wait(qdo_full + 8 * st, (tn / Cfg::NSTAGE) & 1, abort_flag, a.status);
+            mbar_wait(qdo_full + 8 * st, (tn / Cfg::NSTAGE) & 1, abort_flag);
             tc_fence_after_sync();
             // bias products first, into the empty accumulator (large factor terms cancel among themselves)
             if (RP) {
@@ -338,7 +363,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           {
             const BwdItem nx = get_item(w + 1, pa.active_items);
             if (nx.valid) {  // group A of the next item, while the compute warps are on this item's last tile
-              mbar_wait(sdp_done, n & 1, abort_flag, a.status);
+              mbar_wait(sdp_done, n & 1, abort_flag);
               load_kva(nx);
             }
           }
@@ -364,31 +389,31 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             const uint32_t so = st * Cfg::STAGE_BYTES;
             const uint32_t acc0 = it > 0 ? 1u : 0u;
             const uint32_t pb = (tn % Cfg::NBUF) * Cfg::PDS_STRIDE;  // P/dS buffer pair of this tile
-            mbar_wait(qdo_full + 8 * st, (tn / Cfg::NSTAGE) & 1, abort_flag, a.status);
-            mbar_wait(pds_ready + 8 * (tn & 1), (tn >> 1) & 1, abort_flag, a.status);
-            if (it == 0 && n > 0)  // the compute warps have read the previous item's accumulators
-              mbar_wait(acc_free, (n - 1) & 1, abort_flag, a.status);
+            mbar_wait(qdo_full + 8 * st, (tn / Cfg::NSTAGE) & 1, abort_flag);
+            mbar_wait(pds_ready + 8 * (tn & 1), (tn >> 1) & 1, abort_flag);
+            if (it == 0) wait_acc_free(n, abort_flag);
             tc_fence_after_sync();
+            const uint32_t acc = tmem + (n & 1) * Cfg::ACC_STRIDE;
             if (role == 1) {
 #pragma unroll
               for (int s = 0; s < 8; ++s)  // contraction over the 128 query rows
-                umma_ss(tmem + Cfg::T_DV, desc_at(mP, pb + mnmajor_step<128>(s)),
+                umma_ss(acc + Cfg::T_DV, desc_at(mP, pb + mnmajor_step<128>(s)),
                         desc_at(mDO, so + mnmajor_step<D>(s)), idTD, (acc0 | (s > 0)) ? 1u : 0u);
             } else {
 #pragma unroll
               for (int s = 0; s < 8; ++s) {
                 if (Cfg::MERGE_K)
-                  umma_ss(tmem + Cfg::T_DK, desc_at(mDS, pb + mnmajor_step<128>(s)),
+                  umma_ss(acc + Cfg::T_DK, desc_at(mDS, pb + mnmajor_step<128>(s)),
                           desc_at(mQQb, so + mnmajor_step<D>(s)), idKM, (acc0 | (s > 0)) ? 1u : 0u);
                 else
-                  umma_ss(tmem + Cfg::T_DK, desc_at(mDS, pb + mnmajor_step<128>(s)),
+                  umma_ss(acc + Cfg::T_DK, desc_at(mDS, pb + mnmajor_step<128>(s)),
                           desc_at(mQ, so + mnmajor_step<D>(s)), idTD, (acc0 | (s > 0)) ? 1u : 0u);
               }
             }
             umma_commit(qdo_free + 8 * st);
             umma_commit(pds_free + 8 * (tn % Cfg::NBUF));  // this chain no longer reads P / dS of the tile
           }
-          umma_commit(all_done);  // every MMA of this thread for the item
+          umma_commit(all_done_of(n));  // every MMA of this thread for the item
           ++n;
         }
       }
@@ -421,6 +446,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (first.valid) fetch_kbc(first);
       }
       uint32_t tn = 0;  // running tile count
+      int n = 0;        // items so far
 #pragma unroll 1
       for (int w = 0;; ++w) {
       const BwdItem x = next_active(w);
@@ -439,7 +465,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int grow = (i_begin + it) * 128 + row;
         const int qb = (int)(tn % Cfg::NDQ);
         const uint32_t tq = tmem + qb * Cfg::DQ_STRIDE + lane_off;
-        mbar_wait(dq_full + 8 * qb, (tn / Cfg::NDQ) & 1, abort_flag, a.status);
+        mbar_wait(dq_full + 8 * qb, (tn / Cfg::NDQ) & 1, abort_flag);
         tc_fence_after_sync();
         if (!Cfg::STAGED) {
           // no staging tile: reduce straight from registers (one row per thread)
@@ -514,6 +540,52 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
         }
       }
+      if (ASYNC) {
+        // dV, dK and dkb of the item: from their accumulators through the staging tile (16-bit [128][D] tiles that TMA
+        // stores, and dkb rank-major), thread = key
+        const uint32_t acc = tmem + (n & 1) * Cfg::ACC_STRIDE + lane_off;
+        mbar_wait(all_done_of(n), (n >> 1) & 1, abort_flag);
+        tc_fence_after_sync();
+        if (warp == 8 && lane == 0) bulk_wait_group_read0();
+        __syncwarp();
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        auto stage = [&](uint32_t from, uint32_t to, float mult) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < D; c0 += 16) {
+            uint32_t v[16];
+            tmem_ld16(from + c0, v);
+            tmem_wait_ld(v);
+            auto p2 = [&](int i) { return Pack2<T>::pack(__uint_as_float(v[i]) * mult, __uint_as_float(v[i + 1]) * mult); };
+            st_shared_v4(to + tile_chunk_offset<D>(row, c0), p2(0), p2(2), p2(4), p2(6));
+            st_shared_v4(to + tile_chunk_offset<D>(row, c0 + 8), p2(8), p2(10), p2(12), p2(14));
+          }
+        };
+        stage(acc + Cfg::T_DV, sStg, 1.f);
+        stage(acc + Cfg::T_DK, sStg + Cfg::D_BYTES, a.dk_scale);
+        {
+          float* stg = reinterpret_cast<float*>(smem + Cfg::OFF_STG + 128 * D * 4) + row;
+          uint32_t v[16];  // rank <= 16 where the packed rank is 32
+          tmem_ld16(acc + Cfg::T_DKB, v);
+          tmem_wait_ld(v);
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (i < a.R) stg[i * 128] = __uint_as_float(v[i]) * a.dkb_scale;
+        }
+        tc_fence_before_sync();
+        mbar_arrive_warp(acc_free_of(n));  // the accumulators may be overwritten
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        if (warp == 8 && lane == 0) {
+          const int bk = a.bk_bcast ? 0 : b, hk = a.hk_bcast ? 0 : h;
+          tma_store_4d(&tmDV, sStg, 0, x.k0, h, b);
+          tma_store_4d(&tmDK, sStg + Cfg::D_BYTES, 0, x.k0, h, b);
+          bulk_reduce_add_f32(a.dkb_acc + (bh % a.dkb_slots) * a.dkb_slot_stride +
+                                  (((int64_t)bk * a.Hk + hk) * a.nk_tiles + x.kt) * (128 * a.R),
+                              sStgB, 128 * a.R * 4);
+          bulk_commit_group();
+        }
+      }
+      ++n;
       }
       // the staging tile must outlive the last reduction's reads; its global side completes with the kernel
       if (Cfg::STAGED && warp == 8 && lane == 0) bulk_wait_group_read0();
@@ -576,7 +648,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // head of the tile, S and dP are released and the tensor core computes the next tile's under this tile's math.
     uint32_t rs0[32], rd0[32], rs1[32], rd1[32];
     const uint32_t tSl = tmem + Cfg::T_S + lane_off + wg * 64, tDl = tmem + Cfg::T_DP + lane_off + wg * 64;
-    mbar_wait(dp_full, tn & 1, abort_flag, a.status);  // committed after the S and the dP products: covers both
+    mbar_wait(dp_full, tn & 1, abort_flag);  // committed after the S and the dP products: covers both
     tc_fence_after_sync();
     tmem_ld32(tSl, rs0);
     tmem_ld32(tDl, rd0);
@@ -616,34 +688,34 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           else load_mask_chunk(reinterpret_cast<const __nv_bfloat16*>(p), n, vec, mv);
         }
         const float abase = slope2 * (float)(k0 + col0 - grow) - lse2_cur;  // ALiBi term of column col0, minus lse
-        // the masked and the unmasked tile get separate straight-line loops: a per-element test of need_mask
-        // becomes a branch per element and the 32 elements then run one after the other
-        auto elems = [&](auto masked) {
+        // Dead columns (beyond Sk, above the diagonal) become -inf logits ahead of the one straight-line loop: their P and
+        // dS are then exactly zero.  (A second copy of the loop for tiles with dead columns doubled the hottest code, and the
+        // roles of this kernel together already overflow the instruction cache.)
+        if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
-            uint64_t arg;
-            if (MODE == BWD_PLAIN) arg = f2_fma(sp, sl2p, nlse);
-            if (MODE == BWD_MASK) arg = f2_fma(sp, sl2p, f2_add(f2(mv[i], mv[i + 1]), nlse));
-            if (MODE == BWD_ALIBI)
-              arg = f2_fma(sp, sl2p, f2(fmaf((float)i, slope2, abase), fmaf((float)(i + 1), slope2, abase)));
-            float a0, a1;
-            f2_unpack(arg, a0, a1);
-            float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-            if (decltype(masked)::value) {
-              const int col = k0 + col0 + i;
-              if (col >= a.Sk || (a.causal && col > grow)) p0 = 0.f;
-              if (col + 1 >= a.Sk || (a.causal && col + 1 > grow)) p1 = 0.f;
-            }
-            const uint64_t ds = f2_mul(f2(p0, p1), f2_add(f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), ndlt));
-            if (RP) sum2 = f2_add(sum2, ds);
-            float d0, d1;
-            f2_unpack(ds, d0, d1);
-            pk[i / 2] = Pack2<T>::pack(p0, p1);
-            dk[i / 2] = Pack2<T>::pack(d0, d1);
+          for (int i = 0; i < 32; ++i) {
+            const int col = k0 + col0 + i;
+            if (col >= a.Sk || (a.causal && col > grow)) rs[i] = __float_as_uint(-INFINITY);
           }
-        };
-        if (need_mask) elems(std::true_type{}); else elems(std::false_type{});
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
+          uint64_t arg;
+          if (MODE == BWD_PLAIN) arg = f2_fma(sp, sl2p, nlse);
+          if (MODE == BWD_MASK) arg = f2_fma(sp, sl2p, f2_add(f2(mv[i], mv[i + 1]), nlse));
+          if (MODE == BWD_ALIBI)
+            arg = f2_fma(sp, sl2p, f2(fmaf((float)i, slope2, abase), fmaf((float)(i + 1), slope2, abase)));
+          float a0, a1;
+          f2_unpack(arg, a0, a1);
+          float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
+          const uint64_t ds = f2_mul(f2(p0, p1), f2_add(f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), ndlt));
+          if (RP) sum2 = f2_add(sum2, ds);
+          float d0, d1;
+          f2_unpack(ds, d0, d1);
+          pk[i / 2] = Pack2<T>::pack(p0, p1);
+          dk[i / 2] = Pack2<T>::pack(d0, d1);
+        }
         float x0, x1;
         f2_unpack(sum2, x0, x1);
         return x0 + x1;
@@ -672,7 +744,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
       // the dV, dK and dQ products of the query tile that used this buffer pair last have read P and dS
       if (tn >= (uint32_t)Cfg::NBUF)
-        mbar_wait(pds_free + 8 * (tn % Cfg::NBUF), (tn / Cfg::NBUF - 1) & 1, abort_flag, a.status);
+        mbar_wait(pds_free + 8 * (tn % Cfg::NBUF), (tn / Cfg::NBUF - 1) & 1, abort_flag);
       if (it == 0 && staged_out) {  // the previous item's epilogue tiles have left the P tile
         if (threadIdx.x == 0) bulk_wait_group_read0();
         __syncwarp();
@@ -698,14 +770,18 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before_sync();
       mbar_arrive_warp(pds_ready + 8 * (tn & 1));
       if (it + 1 < n_it && !prefetched) {
-        mbar_wait(dp_full, (tn + 1) & 1, abort_flag, a.status);
+        mbar_wait(dp_full, (tn + 1) & 1, abort_flag);
         tc_fence_after_sync();
         tmem_ld32(tSl, rs0);
         tmem_ld32(tDl, rd0);
       }
     }
+    if (ASYNC) {  // the drain warpgroup stores the item's dV, dK and dkb
+      ++n;
+      continue;
+    }
     // the dV and dK|dKb accumulators are final once every MMA of the CTA has completed
-    mbar_wait(all_done, n & 1, abort_flag, a.status);
+    mbar_wait(all_done, n & 1, abort_flag);
     tc_fence_after_sync();
 
     // ---- epilogue: dV, dK (x scale), dKb.  The tiles are staged in the (now idle) P tile -- dV, dK as the 16-bit
@@ -774,6 +850,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
+  report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
     __syncwarp();
     tmem_dealloc(tmem, 512);

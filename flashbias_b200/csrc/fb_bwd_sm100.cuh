@@ -317,14 +317,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // [K | Kc]: 32-column blocks of 64-byte-swizzled rows, the second block at the distance between the tiles
       const uint64_t dKKc = smem_desc(sK, Cfg::OFF_KC - Cfg::OFF_K, 8 * 64, 64);
       const DescBase mKKc{(uint32_t)dKKc, (uint32_t)(dKKc >> 32)};
-      mbar_wait(kv_full, 0, abort_flag, a.status);
+      mbar_wait(kv_full, 0, abort_flag);
       auto issue_dQ = [&](int it) {
         const int qb = it % Cfg::NDQ;  // dQ|dQb accumulator of this tile
         const uint32_t tq = tmem + qb * Cfg::DQ_STRIDE;
         const uint32_t pb = (it % Cfg::NBUF) * Cfg::PDS_STRIDE;  // P/dS buffer pair of this tile
-        mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+        mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
         if (it >= Cfg::NDQ)  // the drain warpgroup has read the tile that used this accumulator last
-          mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag, a.status);
+          mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag);
         tc_fence_after_sync();
 #pragma unroll
         for (int s = 0; s < 8; ++s) {  // contraction over the 128 keys
@@ -346,7 +346,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int it = 0; it < n_it; ++it) {
         issue_dQ(it);
         if (it + Cfg::NSTAGE < n_it) {  // the S|dP, dV and dK chains have finished reading the stage of tile it
-          mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
+          mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag);
           load_tile(it + Cfg::NSTAGE);
         }
       }
@@ -368,7 +368,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       constexpr uint32_t idTD = instr_desc(kBf16, true, true, 128, D);     // dV, dK: A^T (MN-major), B MN-major
       constexpr uint32_t idTR = instr_desc(kBf16, true, true, 128, RPX);   // dKb
       constexpr uint32_t idKM = instr_desc(kBf16, true, true, 128, 64);    // dK | dKb merged
-      mbar_wait(kv_full, 0, abort_flag, a.status);
+      mbar_wait(kv_full, 0, abort_flag);
       tc_fence_after_sync();
       if (role == 0) {
         // descriptor views built once (stage 0); each MMA adds a constant to the address field
@@ -382,7 +382,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         auto issue_dKb = [&](int it) {
           const int st = it % Cfg::NSTAGE;
           const uint32_t so = st * Cfg::STAGE_BYTES;
-          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < 8; ++s)
@@ -396,10 +396,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int st = it % Cfg::NSTAGE;
           const uint32_t so = st * Cfg::STAGE_BYTES;
           if (it > 0) {  // the compute warps hold S and dP of the previous tile in registers
-            mbar_wait(sdp_read, (it - 1) & 1, abort_flag, a.status);
+            mbar_wait(sdp_read, (it - 1) & 1, abort_flag);
             tc_fence_after_sync();
           }
-          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
+          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag);
           tc_fence_after_sync();
           // bias products first, into the empty accumulator (large factor terms cancel among themselves)
           if (RP) {
@@ -439,8 +439,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const uint32_t so = st * Cfg::STAGE_BYTES;
           const uint32_t acc0 = it > 0 ? 1u : 0u;
           const uint32_t pb = (it % Cfg::NBUF) * Cfg::PDS_STRIDE;  // P/dS buffer pair of this tile
-          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
-          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag);
+          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
           tc_fence_after_sync();
           if (role == 1) {
 #pragma unroll
@@ -478,7 +478,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int grow = (i_begin + it) * 128 + row;
         const int qb = it % Cfg::NDQ;
         const uint32_t tq = tmem + qb * Cfg::DQ_STRIDE + lane_off;
-        mbar_wait(dq_full + 8 * qb, (it / Cfg::NDQ) & 1, abort_flag, a.status);
+        mbar_wait(dq_full + 8 * qb, (it / Cfg::NDQ) & 1, abort_flag);
         tc_fence_after_sync();
         if (!Cfg::STAGED) {
           // no staging tile: reduce straight from registers (one row per thread)
@@ -604,7 +604,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // head of the tile, S and dP are released and the tensor core computes the next tile's under this tile's math.
     uint32_t rs0[32], rd0[32], rs1[32], rd1[32];
     const uint32_t tSl = tmem + Cfg::T_S + lane_off + wg * 64, tDl = tmem + Cfg::T_DP + lane_off + wg * 64;
-    mbar_wait(dp_full, 0, abort_flag, a.status);  // committed after the S and the dP products: covers both
+    mbar_wait(dp_full, 0, abort_flag);  // committed after the S and the dP products: covers both
     tc_fence_after_sync();
     tmem_ld32(tSl, rs0);
     tmem_ld32(tDl, rd0);
@@ -644,34 +644,34 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           else load_mask_chunk(reinterpret_cast<const __nv_bfloat16*>(p), n, vec, mv);
         }
         const float abase = slope2 * (float)(k0 + col0 - grow) - lse2_cur;  // ALiBi term of column col0, minus lse
-        // the masked and the unmasked tile get separate straight-line loops: a per-element test of need_mask
-        // becomes a branch per element and the 32 elements then run one after the other
-        auto elems = [&](auto masked) {
+        // Dead columns (beyond Sk, above the diagonal) become -inf logits ahead of the one straight-line loop: their P and
+        // dS are then exactly zero.  (A second copy of the loop for tiles with dead columns doubled the hottest code, and the
+        // roles of this kernel together already overflow the instruction cache.)
+        if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
-            uint64_t arg;
-            if (MODE == BWD_PLAIN) arg = f2_fma(sp, sl2p, nlse);
-            if (MODE == BWD_MASK) arg = f2_fma(sp, sl2p, f2_add(f2(mv[i], mv[i + 1]), nlse));
-            if (MODE == BWD_ALIBI)
-              arg = f2_fma(sp, sl2p, f2(fmaf((float)i, slope2, abase), fmaf((float)(i + 1), slope2, abase)));
-            float a0, a1;
-            f2_unpack(arg, a0, a1);
-            float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-            if (decltype(masked)::value) {
-              const int col = k0 + col0 + i;
-              if (col >= a.Sk || (a.causal && col > grow)) p0 = 0.f;
-              if (col + 1 >= a.Sk || (a.causal && col + 1 > grow)) p1 = 0.f;
-            }
-            const uint64_t ds = f2_mul(f2(p0, p1), f2_add(f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), ndlt));
-            if (RP) sum2 = f2_add(sum2, ds);
-            float d0, d1;
-            f2_unpack(ds, d0, d1);
-            pk[i / 2] = Pack2<T>::pack(p0, p1);
-            dk[i / 2] = Pack2<T>::pack(d0, d1);
+          for (int i = 0; i < 32; ++i) {
+            const int col = k0 + col0 + i;
+            if (col >= a.Sk || (a.causal && col > grow)) rs[i] = __float_as_uint(-INFINITY);
           }
-        };
-        if (need_mask) elems(std::true_type{}); else elems(std::false_type{});
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
+          uint64_t arg;
+          if (MODE == BWD_PLAIN) arg = f2_fma(sp, sl2p, nlse);
+          if (MODE == BWD_MASK) arg = f2_fma(sp, sl2p, f2_add(f2(mv[i], mv[i + 1]), nlse));
+          if (MODE == BWD_ALIBI)
+            arg = f2_fma(sp, sl2p, f2(fmaf((float)i, slope2, abase), fmaf((float)(i + 1), slope2, abase)));
+          float a0, a1;
+          f2_unpack(arg, a0, a1);
+          float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
+          const uint64_t ds = f2_mul(f2(p0, p1), f2_add(f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), ndlt));
+          if (RP) sum2 = f2_add(sum2, ds);
+          float d0, d1;
+          f2_unpack(ds, d0, d1);
+          pk[i / 2] = Pack2<T>::pack(p0, p1);
+          dk[i / 2] = Pack2<T>::pack(d0, d1);
+        }
         float x0, x1;
         f2_unpack(sum2, x0, x1);
         return x0 + x1;
@@ -694,7 +694,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // the dV, dK and dQ products of the query tile that used this buffer pair last have read P and dS
       if (it >= Cfg::NBUF)
-        mbar_wait(pds_free + 8 * (it % Cfg::NBUF), (it / Cfg::NBUF - 1) & 1, abort_flag, a.status);
+        mbar_wait(pds_free + 8 * (it % Cfg::NBUF), (it / Cfg::NBUF - 1) & 1, abort_flag);
       const uint32_t pb = (it % Cfg::NBUF) * Cfg::PDS_STRIDE;
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
@@ -715,14 +715,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before_sync();
       mbar_arrive_warp(pds_ready + 8 * (it & 1));
       if (it + 1 < n_it && !prefetched) {
-        mbar_wait(dp_full, (it + 1) & 1, abort_flag, a.status);
+        mbar_wait(dp_full, (it + 1) & 1, abort_flag);
         tc_fence_after_sync();
         tmem_ld32(tSl, rs0);
         tmem_ld32(tDl, rd0);
       }
     }
     // the dV and dK|dKb accumulators are final once every MMA of the CTA has completed
-    mbar_wait(all_done, 0, abort_flag, a.status);
+    mbar_wait(all_done, 0, abort_flag);
     tc_fence_after_sync();
 
     // ---- epilogue: dV, dK (x scale), dKb
@@ -798,6 +798,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   tc_fence_before_sync();
   __syncthreads();
+  report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
     __syncwarp();
     tmem_dealloc(tmem, 512);

@@ -156,7 +156,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       constexpr uint32_t idTS = instr_desc(kBf16, false, true, 128, D);    // dV, dK: A in TMEM, B MN-major
       // dQ: A = dS (transposed tile), B = K; dQ^T: A = K^T, B = dS^T
       constexpr uint32_t idQ = instr_desc(kBf16, true, true, 128, Cfg::DQ_COLS);
-      mbar_wait(kv_full, 0, abort_flag, a.status);
+      mbar_wait(kv_full, 0, abort_flag);
       tc_fence_after_sync();
       if (warp == 12) {
         // ------------------------------------------------------------------ TMA producer, dQ chain
@@ -164,9 +164,9 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll 1
         for (int it = 0; it < n_it; ++it) {
           const int qb = it % Cfg::NDQ;
-          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
           if (it >= Cfg::NDQ)  // the drain warpgroup has read the tile that used this accumulator last
-            mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag, a.status);
+            mbar_wait(dq_drained + 8 * qb, (it / Cfg::NDQ - 1) & 1, abort_flag);
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < 8; ++s) {  // contraction over the 128 keys
@@ -176,7 +176,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           umma_commit(dq_full + 8 * qb);
           umma_commit(pds_free);
           if (it + Cfg::NSTAGE < n_it) {  // the S^T|dP^T, dV and dK chains have finished reading the stage of tile it
-            mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
+            mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag);
             load_tile(it + Cfg::NSTAGE);
           }
         }
@@ -190,11 +190,11 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int st = it % Cfg::NSTAGE;
           const uint32_t so = st * Cfg::STAGE_BYTES;
           if (it > 0) {  // the compute warps hold S^T and dP^T of the previous tile in registers
-            mbar_wait(sdp_read, (it - 1) & 1, abort_flag, a.status);
+            mbar_wait(sdp_read, (it - 1) & 1, abort_flag);
             tc_fence_after_sync();
           }
-          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
-          mbar_wait(aux_ready + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
+          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag);
+          mbar_wait(aux_ready + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag);
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < D / 16; ++s)
@@ -217,8 +217,8 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int it = 0; it < n_it; ++it) {
           const int st = it % Cfg::NSTAGE;
           const uint32_t so = st * Cfg::STAGE_BYTES;
-          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag, a.status);
-          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag, a.status);
+          mbar_wait(qdo_full + 8 * st, (it / Cfg::NSTAGE) & 1, abort_flag);
+          mbar_wait(pds_ready + 8 * (it & 1), (it >> 1) & 1, abort_flag);
           tc_fence_after_sync();
 #pragma unroll
           for (int s = 0; s < QT / 16; ++s)  // contraction over the query rows; A: 8 TMEM columns per 16 rows
@@ -239,7 +239,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int it = 0; it < n_it; ++it) {
         const int qb = it % Cfg::NDQ;
         const uint32_t tq = tmem + Cfg::T_DQ + qb * Cfg::DQ_COLS + lane_off;
-        mbar_wait(dq_full + 8 * qb, (it / Cfg::NDQ) & 1, abort_flag, a.status);
+        mbar_wait(dq_full + 8 * qb, (it / Cfg::NDQ) & 1, abort_flag);
         tc_fence_after_sync();
         // The first columns are fetched into registers while the copy engine may still be reading the previous
         // tile from the staging tile; the thread that issued that reduction then waits for its shared-memory
@@ -376,7 +376,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint32_t rs0[32], rd0[32], rs1[32], rd1[32];
     const uint32_t tSl = tmem + Cfg::T_ST + lane_off + wg * (QT / 2),
                    tDl = tmem + Cfg::T_DPT + lane_off + wg * (QT / 2);
-    mbar_wait(dp_full, 0, abort_flag, a.status);  // committed after the S^T and the dP^T products: covers both
+    mbar_wait(dp_full, 0, abort_flag);  // committed after the S^T and the dP^T products: covers both
     tc_fence_after_sync();
     tmem_ld32(tSl, rs0);
     tmem_ld32(tDl, rd0);
@@ -456,7 +456,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       // the dV, dK and dQ products of the previous query tile have read P^T and dS^T
-      if (it >= 1) mbar_wait(pds_free, (it - 1) & 1, abort_flag, a.status);
+      if (it >= 1) mbar_wait(pds_free, (it - 1) & 1, abort_flag);
       tc_fence_after_sync();
       // P^T and dS^T into tensor memory (A operands of dV and dK) ...
       tmem_st16(tmem + Cfg::T_PT + lane_off + wg * (QT / 4), pk0);
@@ -477,14 +477,14 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before_sync();
       mbar_arrive_warp(pds_ready + 8 * (it & 1));
       if (it + 1 < n_it && !prefetched) {
-        mbar_wait(dp_full, (it + 1) & 1, abort_flag, a.status);
+        mbar_wait(dp_full, (it + 1) & 1, abort_flag);
         tc_fence_after_sync();
         tmem_ld32(tSl, rs0);
         tmem_ld32(tDl, rd0);
       }
     }
     // the dV and dK accumulators are final once every MMA of the CTA has completed
-    mbar_wait(all_done, 0, abort_flag, a.status);
+    mbar_wait(all_done, 0, abort_flag);
     tc_fence_after_sync();
 
     // ---- epilogue: dV, dK (x scale); thread = key row, each warpgroup half of the columns
@@ -533,6 +533,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
+  report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
     __syncwarp();
     tmem_dealloc(tmem, 512);

@@ -84,18 +84,24 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  `abort_flag` lives in shared memory: once any wait of the CTA has expired every
-// later wait returns at once, so a broken pipeline drains in bounded time.  Returns false on expiry.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status) {
-  if (mbar_try_wait(bar, parity)) return true;
-  for (uint32_t it = 0; it < kSpinLimit; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 1023u) == 1023u && *abort_flag) return false;
+// Bounded wait.  `abort_flag` lives in shared memory: once any wait of the CTA has expired every later wait returns at
+// once, so a broken pipeline drains in bounded time; the kernel reports it at its end (report_expired_wait).  Returns
+// false on expiry.  Kept to a handful of instructions: a kernel has some thirty waits, and with the status write and an
+// unrolled poll loop in each of them they were a third of the backward's code, whose roles together overflow the
+// instruction cache (windowed backward: 4.6 of 9 stall cycles per instruction were instruction fetch).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (uint32_t n = kSpinLimit; !mbar_try_wait(bar, parity); --n) {
+    if (n == 0 || *abort_flag) {
+      *abort_flag = 1;
+      return false;
+    }
   }
-  *abort_flag = 1;
-  if (status) atomicExch(status, FB_DEV_WAIT_TIMEOUT);
-  return false;
+  return true;
+}
+// At the end of a kernel, after its last CTA-wide barrier.
+__device__ __forceinline__ void report_expired_wait(volatile int* abort_flag, int* status) {
+  if (threadIdx.x == 0 && *abort_flag && status) atomicExch(status, FB_DEV_WAIT_TIMEOUT);
 }
 
 // ---------------------------------------------------------------------------------------------

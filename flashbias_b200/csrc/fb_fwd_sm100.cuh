@@ -203,18 +203,18 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const Item it = item_of(idx);
           const int hq = a.hq_bcast ? 0 : it.h, bq = a.bq_bcast ? 0 : it.b;
           const int hk = a.hk_bcast ? 0 : it.h, bk = a.bk_bcast ? 0 : it.b;
-          if (n > 0) mbar_wait(q_free, (n - 1) & 1, abort_flag, a.status);
+          if (n > 0) mbar_wait(q_free, (n - 1) & 1, abort_flag);
           mbar_expect_tx(q_full, NQ * Cfg::Q_BYTES + Cfg::QB_BYTES);
 #pragma unroll
           for (int t = 0; t < NQ; ++t) tma_tile_4d<D>(sQ + t * Cfg::Q_BYTES, &tmQ, q_full, it.q0, it.h, it.b, t * D);
           if (RP) tma_tile_4d<RPX>(sQb, &tmQb, q_full, it.q0, hq, bq);
           for (int j = 0; j < it.n_kv; ++j, ++kc, ++vc) {
             const int ks = kc % KST, vs = vc % VST;
-            if (kc >= KST) mbar_wait(k_free + 8 * ks, ((kc / KST) - 1) & 1, abort_flag, a.status);
+            if (kc >= KST) mbar_wait(k_free + 8 * ks, ((kc / KST) - 1) & 1, abort_flag);
             mbar_expect_tx(k_full + 8 * ks, Cfg::Q_BYTES + Cfg::QB_BYTES);
             tma_tile_4d<D>(sK + ks * Cfg::Q_BYTES, &tmK, k_full + 8 * ks, j * 128, it.h, it.b);
             if (RP) tma_tile_4d<RPX>(sKb + ks * Cfg::QB_BYTES, &tmKb, k_full + 8 * ks, j * 128, hk, bk);
-            if (vc >= VST) mbar_wait(v_free + 8 * vs, ((vc / VST) - 1) & 1, abort_flag, a.status);
+            if (vc >= VST) mbar_wait(v_free + 8 * vs, ((vc / VST) - 1) & 1, abort_flag);
             mbar_expect_tx(v_full + 8 * vs, Cfg::Q_BYTES);
             tma_tile_4d<D>(sV + vs * Cfg::Q_BYTES, &tmV, v_full + 8 * vs, j * 128, it.h, it.b);
           }
@@ -230,14 +230,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         int t = 0, n = 0;  // key tiles and items issued so far
         for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w, ++n) {
           const Item it = item_of(idx);
-          mbar_wait(q_full, n & 1, abort_flag, a.status);
+          mbar_wait(q_full, n & 1, abort_flag);
           for (int j = 0; j < it.n_kv; ++j, ++t) {
             if (t > 0) {  // the softmax warps hold the logits of the previous key tile in registers
-              mbar_wait(s_read, (t - 1) & 1, abort_flag, a.status);
+              mbar_wait(s_read, (t - 1) & 1, abort_flag);
               tc_fence_after_sync();
             }
             const int ks = t % KST;
-            mbar_wait(k_full + 8 * ks, (t / KST) & 1, abort_flag, a.status);
+            mbar_wait(k_full + 8 * ks, (t / KST) & 1, abort_flag);
             tc_fence_after_sync();
             const uint32_t ko = ks * Cfg::Q_BYTES, kbo = ks * Cfg::QB_BYTES;
             // The bias products go first, into the empty accumulator: factor terms as large as a sequence
@@ -273,8 +273,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const Item it = item_of(idx);
           for (int j = 0; j < it.n_kv; ++j, ++t) {
             const int vs = t % VST;
-            mbar_wait(v_full + 8 * vs, (t / VST) & 1, abort_flag, a.status);
-            mbar_wait(p_ready, t & 1, abort_flag, a.status);
+            mbar_wait(v_full + 8 * vs, (t / VST) & 1, abort_flag);
+            mbar_wait(p_ready, t & 1, abort_flag);
             tc_fence_after_sync();
             const uint32_t vo = vs * Cfg::Q_BYTES;
 #pragma unroll
@@ -297,7 +297,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int mh = a.mask_h1 ? 0 : it.h;
           for (int col = 0; col < it.n_kv * 128; col += per, ++mc) {
             const int st = mc % MST;
-            if (mc >= MST) mbar_wait(m_free + 8 * st, ((mc / MST) - 1) & 1, abort_flag, a.status);
+            if (mc >= MST) mbar_wait(m_free + 8 * st, ((mc / MST) - 1) & 1, abort_flag);
             mbar_expect_tx(m_full + 8 * st, Cfg::M_STAGE);
             tma_load_4d(sM + st * Cfg::M_STAGE, &tmM, m_full + 8 * st, col, it.q0, mh, mb);
           }
@@ -330,7 +330,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (MST > 0 && a.mask_tma) {
         constexpr int V = 2 * (int)sizeof(MT);  // 16-byte vectors of a chunk: a stage holds one (fp32) or two of them
         const int st = mc % (MST > 0 ? MST : 1);
-        if (V == 8 || (c & 1) == 0) mbar_wait(m_full + 8 * st, (mc / (MST > 0 ? MST : 1)) & 1, abort_flag, a.status);
+        if (V == 8 || (c & 1) == 0) mbar_wait(m_full + 8 * st, (mc / (MST > 0 ? MST : 1)) & 1, abort_flag);
         const uint32_t base = sM + st * Cfg::M_STAGE + row * 128;
 #pragma unroll
         for (int g = 0; g < V; ++g) {
@@ -403,7 +403,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (MODE == FWD_PLAIN) mx *= sl2;  // sl2 > 0
       const float m_new = fmaxf(m_used, mx);
       if (j > 0) {
-        mbar_wait(pv_done, (t - 1) & 1, abort_flag, a.status);  // P buffer free, O stable
+        mbar_wait(pv_done, (t - 1) & 1, abort_flag);  // P buffer free, O stable
         tc_fence_after_sync();
         const bool grow_needed = m_new - m_used > 8.f;
         if (__any_sync(0xffffffffu, grow_needed)) {
@@ -468,7 +468,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     for (int j = 0; j < n_kv; ++j, ++t) {
       const int k0 = j * 128;
-      mbar_wait(s_full, t & 1, abort_flag, a.status);
+      mbar_wait(s_full, t & 1, abort_flag);
       tc_fence_after_sync();
       const bool dead = (a.causal && k0 + 127 > q0) || (k0 + 128 > a.Sk);
       auto step = [&](auto mask_c) {
@@ -483,7 +483,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_arrive_warp(p_ready);
     }
     // ---- epilogue: O / l -> global, lse
-    mbar_wait(pv_done, (t - 1) & 1, abort_flag, a.status);
+    mbar_wait(pv_done, (t - 1) & 1, abort_flag);
     tc_fence_after_sync();
     const float inv = l > 0.f ? 1.f / l : 0.f;
     T* orow = reinterpret_cast<T*>(a.o) + b * a.o_stride[0] + h * a.o_stride[1] + (int64_t)grow * a.o_stride[2];
@@ -517,6 +517,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   tc_fence_before_sync();
   __syncthreads();
+  report_expired_wait(abort_flag, a.status);
   if (warp == 5) {
     __syncwarp();
     tmem_dealloc(tmem, Cfg::TMEM_COLS);

@@ -21,6 +21,7 @@ struct Div {
     m = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << s) - d)) / d + 1);
   }
 #ifdef __CUDACC__
+  __device__ __forceinline__ int quot32(int n) const { return (int)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s); }
   __device__ __forceinline__ int64_t quot(int64_t n) const {
     if (n < 0x80000000LL) return (int64_t)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s);
     return n / d;

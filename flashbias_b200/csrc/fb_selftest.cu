@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
       tma_tile<(C2 ? C2 : 16)>(smem_u32(sA2), &tmA2, bar_tma, C);
       tma_tile<(C2 ? C2 : 16)>(smem_u32(sB2), &tmB2, bar_tma, C);
     }
-    mbar_wait(bar_tma, 0, abort_flag, status);
+    mbar_wait(bar_tma, 0, abort_flag);
     tc_fence_after_sync();
     if (MODE == 0) {
       const uint32_t id = instr_desc(bf16 != 0, false, false, 128, 128);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
     umma_commit(bar_mma);
   }
   __syncwarp();
-  mbar_wait(bar_mma, 0, abort_flag, status);
+  mbar_wait(bar_mma, 0, abort_flag);
   tc_fence_after_sync();
   const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
   for (int c0 = 0; c0 < N; c0 += 16) {
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
   }
   tc_fence_before_sync();
   __syncthreads();
+  report_expired_wait(abort_flag, status);
   if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
