@@ -76,11 +76,11 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   auto all_done_of = [&](int n) { return ASYNC && (n & 1) ? bar0 + 184 : all_done; };
   auto acc_free_of = [&](int n) { return ASYNC && (n & 1) ? bar0 + 192 : acc_free; };
   // Issuing threads, before an item's first product into the accumulators: the item that used the set last has been read.
-  auto wait_acc_free = [&](int n, volatile int* flag) {
+  auto wait_acc_free = [&](int n, uint32_t flag) {
     if (ASYNC ? n >= 2 : n > 0) mbar_wait(acc_free_of(n), ASYNC ? ((n >> 1) - 1) & 1 : (n - 1) & 1, flag);
   };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 96);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 104);
+  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 104;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -164,7 +164,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 12) {
     if (lane == 0) {
-      *abort_flag = 0;
+      st_shared_flag(abort_flag, 0u);
       mbar_init(kva_full, 1);
       mbar_init(kvb_full, 1);
       mbar_init(sdp_done, 1);  // the last S|dP products of an item have completed
@@ -692,11 +692,10 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // dS are then exactly zero.  (A second copy of the loop for tiles with dead columns doubled the hottest code, and the
         // roles of this kernel together already overflow the instruction cache.)
         if (need_mask) {
+          const int last = (a.causal ? min(grow, a.Sk - 1) : a.Sk - 1) - (k0 + col0);  // last live column of the chunk
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int col = k0 + col0 + i;
-            if (col >= a.Sk || (a.causal && col > grow)) rs[i] = __float_as_uint(-INFINITY);
-          }
+          for (int i = 0; i < 32; ++i)
+            if (i > last) rs[i] = __float_as_uint(-INFINITY);
         }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {

@@ -224,7 +224,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  all_done = bar0 + 112, pds_free = bar0 + 120, pds_ready = bar0 + 136 /*2*/,
                  dq_drained = bar0 + 152 /*2*/;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 96);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 104);
+  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 104;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -255,7 +255,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (warp == 12) {
     if (lane == 0) {
-      *abort_flag = 0;
+      st_shared_flag(abort_flag, 0u);
       mbar_init(kv_full, 1);
       mbar_init(dp_full, 1);
       mbar_init(sdp_read, 8);  // every compute warp has S and dP of the tile in registers
@@ -648,11 +648,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // dS are then exactly zero.  (A second copy of the loop for tiles with dead columns doubled the hottest code, and the
         // roles of this kernel together already overflow the instruction cache.)
         if (need_mask) {
+          const int last = (a.causal ? min(grow, a.Sk - 1) : a.Sk - 1) - (k0 + col0);  // last live column of the chunk
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int col = k0 + col0 + i;
-            if (col >= a.Sk || (a.causal && col > grow)) rs[i] = __float_as_uint(-INFINITY);
-          }
+          for (int i = 0; i < 32; ++i)
+            if (i > last) rs[i] = __float_as_uint(-INFINITY);
         }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {

@@ -60,6 +60,9 @@ struct BwdTCfg {
                        T_DQ = T_DK + D;
   static constexpr int DQ_COLS = DQ_T ? QT : D;
   static constexpr int NDQ = (T_DQ + 2 * DQ_COLS <= 512) ? 2 : 1;
+  // registers per thread of the two compute and of the drain and issuer warpgroups (launched with 128 each): with 64-row
+  // tiles the compute threads hold half as much, and at 64 the issuing threads spill their descriptors (slower by 12 %)
+  static constexpr int REGS_COMPUTE = QT == 64 ? 160 : 192, REGS_MOVE = 256 - REGS_COMPUTE;
   static constexpr bool FITS = SMEM <= 227 * 1024 && T_DQ + DQ_COLS <= 512;
 };
 
@@ -84,7 +87,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                  all_done = bar0 + 112, pds_free = bar0 + 120, pds_ready = bar0 + 136 /*2*/,
                  dq_drained = bar0 + 152 /*2*/, aux_ready = bar0 + 168 /*3*/;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 96);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 104);
+  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 104;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -113,7 +116,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 12) {
     if (lane == 0) {
-      *abort_flag = 0;
+      st_shared_flag(abort_flag, 0u);
       mbar_init(kv_full, 1);
       mbar_init(dp_full, 1);
       mbar_init(sdp_read, 8);   // every compute warp has S^T and dP^T of the tile in registers
@@ -149,7 +152,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t tmem = *tmem_slot;
 
   if (warp >= 12) {
-    setmaxnreg_dec<64>();
+    setmaxnreg_dec<Cfg::REGS_MOVE>();
     if (lane == 0 && n_it > 0) {
       // B operands read transposed (MN-major: rows are the contraction index), A of dQ likewise
       constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, QT);   // S^T, dP^T: both operands K-major
@@ -230,7 +233,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       umma_commit(all_done);  // every MMA of this thread
     }
   } else if (warp >= 8) {
-    setmaxnreg_dec<64>();
+    setmaxnreg_dec<Cfg::REGS_MOVE>();
     // ------------------------------------------------------------------ drain warpgroup (thread = query row, or column)
     if (n_it > 0) {
       const int row = (warp & 3) * 32 + lane;
@@ -291,7 +294,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   } else if (n_it > 0) {
     // ------------------------------------------------------------------ compute warpgroups (warps 0-7)
-    setmaxnreg_inc<192>();
+    setmaxnreg_inc<Cfg::REGS_COMPUTE>();
     const int wg = warp >> 2;
     const int row = (warp & 3) * 32 + lane;  // key of this thread within the tile
     const int key = k0 + row;
@@ -418,29 +421,28 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                     kLog2e;
           }
         }
-        auto elems = [&](auto masked) {
+        // dead pairs become -inf logits ahead of the one straight-line loop (as in the query-major kernel)
+        if (need_mask) {
+          const int first = key >= a.Sk ? 32 : a.causal ? key - (q0 + col0) : 0;  // first live column of the chunk
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
-            float a0, a1;
-            f2_unpack(MODE == BWD_ALIBI  ? f2_fma(sp, sl2p, akp)
-                      : MODE == BWD_MASK ? f2_fma(sp, sl2p, f2(mv[i], mv[i + 1]))
-                                         : f2_mul(sp, sl2p),
-                      a0, a1);
-            float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
-            if (decltype(masked)::value) {
-              const int q = q0 + col0 + i;
-              if (key >= a.Sk || (a.causal && key > q)) p0 = 0.f;
-              if (key >= a.Sk || (a.causal && key > q + 1)) p1 = 0.f;
-            }
-            const uint64_t ds = f2_mul(f2(p0, p1), f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])));
-            float d0, d1;
-            f2_unpack(ds, d0, d1);
-            pk[i / 2] = Pack2<T>::pack(p0, p1);
-            dk[i / 2] = Pack2<T>::pack(d0, d1);
-          }
-        };
-        if (need_mask) elems(std::true_type{}); else elems(std::false_type{});
+          for (int i = 0; i < 32; ++i)
+            if (i < first) rs[i] = __float_as_uint(-INFINITY);
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const uint64_t sp = f2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1]));
+          float a0, a1;
+          f2_unpack(MODE == BWD_ALIBI  ? f2_fma(sp, sl2p, akp)
+                    : MODE == BWD_MASK ? f2_fma(sp, sl2p, f2(mv[i], mv[i + 1]))
+                                       : f2_mul(sp, sl2p),
+                    a0, a1);
+          const float p0 = fast_exp2(a0), p1 = fast_exp2(a1);
+          const uint64_t ds = f2_mul(f2(p0, p1), f2(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])));
+          float d0, d1;
+          f2_unpack(ds, d0, d1);
+          pk[i / 2] = Pack2<T>::pack(p0, p1);
+          dk[i / 2] = Pack2<T>::pack(d0, d1);
+        }
       };
       uint32_t pk0[16], pk1[16], dk0[16], dk1[16];
       chunk(rs0, rd0, pk0, dk0, 0);

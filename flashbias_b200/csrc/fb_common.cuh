@@ -84,24 +84,32 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  `abort_flag` lives in shared memory: once any wait of the CTA has expired every later wait returns at
+// Bounded wait.  `abort_flag` is a word in shared memory (its address): once any wait of the CTA has expired every later wait returns at
 // once, so a broken pipeline drains in bounded time; the kernel reports it at its end (report_expired_wait).  Returns
 // false on expiry.  Kept to a handful of instructions: a kernel has some thirty waits, and with the status write and an
 // unrolled poll loop in each of them they were a third of the backward's code, whose roles together overflow the
 // instruction cache (windowed backward: 4.6 of 9 stall cycles per instruction were instruction fetch).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ uint32_t ld_shared_flag(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_flag(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
 #pragma unroll 1
   for (uint32_t n = kSpinLimit; !mbar_try_wait(bar, parity); --n) {
-    if (n == 0 || *abort_flag) {
-      *abort_flag = 1;
+    if (n == 0 || ld_shared_flag(abort_flag)) {
+      st_shared_flag(abort_flag, 1u);
       return false;
     }
   }
   return true;
 }
 // At the end of a kernel, after its last CTA-wide barrier.
-__device__ __forceinline__ void report_expired_wait(volatile int* abort_flag, int* status) {
-  if (threadIdx.x == 0 && *abort_flag && status) atomicExch(status, FB_DEV_WAIT_TIMEOUT);
+__device__ __forceinline__ void report_expired_wait(uint32_t abort_flag, int* status) {
+  if (threadIdx.x == 0 && status && ld_shared_flag(abort_flag)) atomicExch(status, FB_DEV_WAIT_TIMEOUT);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -50,6 +50,7 @@ struct FwdArgs {
   const void* mask;  // additive mask, (batch, head, row) element strides; row stride 0 for a (1, Sk) mask
   int64_t mask_stride[3];
   int mask_kind, mask_dtype, mask_batch_period;
+  uint32_t zero;  // 0, unknown to the compiler
   int mask_tma, mask_b1, mask_h1;  // mask tiles come by TMA; the mask has extent 1 on batch / heads
   const float* alibi_slopes;
 };
@@ -129,7 +130,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t k_full = bar0 + 32, k_free = bar0 + 64, v_full = bar0 + 96, v_free = bar0 + 128;  // 4 slots each
   const uint32_t m_full = bar0 + 192, m_free = bar0 + 224;  // likewise
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 160);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::OFF_BAR + 168);
+  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 168;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -163,7 +164,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (warp == 4) {
     if (lane == 0) {
-      *abort_flag = 0;
+      st_shared_flag(abort_flag, 0u);
       mbar_init(q_full, 1);
       mbar_init(s_full, 1);
       mbar_init(p_ready, 4);  // one arrival per softmax warp
@@ -332,15 +333,21 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int st = mc % (MST > 0 ? MST : 1);
         if (V == 8 || (c & 1) == 0) mbar_wait(m_full + 8 * st, (mc / (MST > 0 ? MST : 1)) & 1, abort_flag);
         const uint32_t base = sM + st * Cfg::M_STAGE + row * 128;
+        uint32_t seen = 0u;
 #pragma unroll
         for (int g = 0; g < V; ++g) {
           const int ch = (V == 8 ? 0 : (c & 1) * 4) + g;
           uint32_t w[4];
           ld_shared_v4(base + ((ch ^ (row & 7)) << 4), w[0], w[1], w[2], w[3]);
+          seen |= w[0] | w[1] | w[2] | w[3];
           const MT* e = reinterpret_cast<const MT*>(w);
 #pragma unroll
           for (int i = 0; i < 32 / V; ++i) mv[g * (32 / V) + i] = to_f32(e[i]) * kLog2e;
         }
+        // The stage may only be released once the values are in registers: the arrival is not ordered behind shared-memory
+        // reads that are still in flight (TMA then overwrote 9 % of the rows' masks).  a.zero is 0: the branch is never
+        // taken, but it cannot be decided before every read has returned.
+        if (seen & a.zero) st_shared_flag(abort_flag, 1u);
         if (V == 8 || (c & 1) == 1) {
           mbar_arrive_warp(m_free + 8 * st);
           ++mc;
@@ -351,9 +358,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     };
 
-    // One key tile.  DEAD: the tile has columns beyond Sk or above the causal diagonal.
-    auto tile = [&](int j, auto dead_c, auto mask_c) {
-      constexpr bool DEAD = decltype(dead_c)::value;
+    // One key tile.  dead: it has columns beyond Sk or above the causal diagonal, which become -inf logits (one copy of
+    // the tile's code: the instruction cache is short, see mbar_wait).
+    auto tile = [&](int j, bool dead, auto mask_c) {
       const int k0 = j * 128;
       // ---- logits from tensor memory (the load of one 32-column chunk overlaps the arithmetic of the previous
       // one), completed (log2 units for MODE != PLAIN), and the row maximum, four chains
@@ -364,6 +371,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto complete = [&](int c) {
         float mv[32];
         if constexpr (MODE == FWD_MASK) mask_chunk(k0, c, mask_c, mv);
+        if (dead) {
+          const int last = (a.causal ? min(grow, a.Sk - 1) : a.Sk - 1) - (k0 + c * 32);  // last live column of the chunk
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i > last) s[c][i] = __float_as_uint(-INFINITY);
+        }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float v0 = __uint_as_float(s[c][i]), v1 = __uint_as_float(s[c][i + 1]);
@@ -372,12 +385,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             f2_unpack(f2_fma(f2(v0, v1), sl2p,
                              f2(fmaf((float)(c * 32 + i), slope2, abase), fmaf((float)(c * 32 + i + 1), slope2, abase))),
                       v0, v1);
-          if (DEAD) {
-            const int col = k0 + c * 32 + i;
-            if (col >= a.Sk || (a.causal && col > grow)) v0 = -INFINITY;
-            if (col + 1 >= a.Sk || (a.causal && col + 1 > grow)) v1 = -INFINITY;
-          }
-          if (MODE != FWD_PLAIN || DEAD) {
+          if (MODE != FWD_PLAIN) {
             s[c][i] = __float_as_uint(v0);
             s[c][i + 1] = __float_as_uint(v1);
           }
@@ -472,8 +480,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_after_sync();
       const bool dead = (a.causal && k0 + 127 > q0) || (k0 + 128 > a.Sk);
       auto step = [&](auto mask_c) {
-        if (dead) tile(j, std::true_type{}, mask_c);
-        else tile(j, std::false_type{}, mask_c);
+        tile(j, dead, mask_c);
       };
       if (MODE == FWD_MASK && a.mask_dtype == FB_DTYPE_F16) step(__half{});
       else if (MODE == FWD_MASK && a.mask_dtype == FB_DTYPE_BF16) step(__nv_bfloat16{});
@@ -587,6 +594,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     a.mask_kind = p->mask_kind;
     a.mask_dtype = p->mask_dtype;
     a.mask_batch_period = p->mask_batch_period;
+    a.zero = 0u;
     a.mask_b1 = p->mask_stride[0] == 0;
     a.mask_h1 = p->mask_stride[1] == 0;
     CUtensorMap tM = tQ;

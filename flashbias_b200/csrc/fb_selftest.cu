@@ -47,13 +47,13 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
   uint8_t* sB2 = smem + 65536 + 16384; // 16 KB
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 98304);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 98304 + 64);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 98304 + 72);
+  const uint32_t abort_flag = smem_u32(smem) + 98304 + 72;
   constexpr int N = MODE == 0 ? 128 : C;
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const uint32_t bar_tma = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);
   if (tid == 0) {
-    *abort_flag = 0;
+    st_shared_flag(abort_flag, 0u);
     mbar_init(bar_tma, 1);
     mbar_init(bar_mma, 1);
     mbar_fence_init();
