@@ -692,10 +692,11 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // dS are then exactly zero.  (A second copy of the loop for tiles with dead columns doubled the hottest code, and the
         // roles of this kernel together already overflow the instruction cache.)
         if (need_mask) {
-          const int last = (a.causal ? min(grow, a.Sk - 1) : a.Sk - 1) - (k0 + col0);  // last live column of the chunk
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (i > last) rs[i] = __float_as_uint(-INFINITY);
+          for (int i = 0; i < 32; ++i) {
+            const int col = k0 + col0 + i;
+            if (col >= a.Sk || (a.causal && col > grow)) rs[i] = __float_as_uint(-INFINITY);
+          }
         }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
