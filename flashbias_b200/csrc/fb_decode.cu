@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kDecodeThreads, kDecodeCtas) decode_kernel(con
       if (key >= k_end) s[u] = -INFINITY;
       mx = fmaxf(mx, s[u]);
     }
-    const float msub = fmaxf(mx, -1e38f);  // no visible key yet: every exponential below is zero
+    const float msub = mx == -INFINITY ? 0.f : mx;  // no visible key yet: every exponential below is zero
     const float alpha = fast_exp2(m - msub);  // 0 while m is still -inf
     m = mx;
     l *= alpha;

@@ -72,3 +72,16 @@ def test_single_query_without_a_visible_key():
     mask = torch.full((2, 1, 1, 400), float("-inf"), device="cuda")
     o, lse, _ = flash_bias_forward(q, k, k, None, None, mask)
     assert (o == 0).all() and (lse[..., 0] == float("-inf")).all()
+
+
+@pytest.mark.parametrize("level", [-1e37, -8e37, -2e38])
+@pytest.mark.parametrize("Sk", [3, 400])
+def test_single_query_under_a_large_finite_mask(level, Sk):
+    """Every key carries the same finite mask, however large: the probabilities are those of the unmasked row."""
+    g = torch.Generator().manual_seed(11)
+    q, k, v = (torch.randn(2, S, 2, 32, generator=g).half().cuda() for S in (1, Sk, Sk))
+    o, lse, _ = flash_bias_forward(q, k, v, None, None, torch.full((2, 1, 1, Sk), level, device="cuda"))
+    # next to such a mask every q.k vanishes (an fp32 ulp is 2^100 or more): the mean of the values
+    want = v.float().mean(1, keepdim=True)
+    assert (o.float() - want).abs().max().item() <= 2.0 ** -10 * want.abs().max().item()  # one rounding to fp16, fp32 sums
+    assert ((lse[..., 0] - level) / level).abs().max().item() <= 2.0 ** -21  # two products by log2 e and ln 2, one sum
