@@ -334,8 +334,25 @@ struct FlashBiasNode : torch::autograd::Function<FlashBiasNode> {
 
 bool wants_grad(const OptTensor& t) { return t && t->requires_grad(); }
 
+// There is no forward-mode derivative: a tangent is refused, as torch.autograd.Function does without a jvp, and not
+// dropped by the calls that need no node.
+struct NoForwardMode : std::exception {
+  const char* what() const noexcept override { return "flash_bias has no forward-mode derivative"; }
+};
+void refuse_tangent(const Tensor& t) {
+  if (t._fw_grad(/*level=*/0).defined()) throw NoForwardMode();
+}
+void refuse_tangent(const OptTensor& t) {
+  if (t) refuse_tangent(*t);
+}
+template <typename... Ts>
+void refuse_tangents(const Ts&... t) {
+  (refuse_tangent(t), ...);
+}
+
 Tensor flash_bias(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& q_bias, const OptTensor& k_bias,
                   const OptTensor& mask, bool causal, std::optional<double> softmax_scale) {
+  refuse_tangents(q, k, v, q_bias, k_bias, mask);
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() ||
                                      wants_grad(q_bias) || wants_grad(k_bias) || wants_grad(mask)))
     return FlashBiasNode::apply(q, k, v, q_bias, k_bias, mask, OptTensor(), causal, softmax_scale);
@@ -348,6 +365,7 @@ Tensor flash_bias(const Tensor& q, const Tensor& k, const Tensor& v, const OptTe
 // gradient) go in directly, the positions never exist as tensors and are never rounded to 16 bits.
 Tensor flash_bias_alibi(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& slopes_, bool causal,
                         std::optional<double> softmax_scale) {
+  refuse_tangents(q, k, v, slopes_);
   const Tensor slopes = slopes_.detach().to(q.device(), at::kFloat).reshape({-1}).contiguous();
   FB_ASSERT(q.dim() == 4 && slopes.numel() == q.size(2), "one slope per head");
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
@@ -387,6 +405,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       if (e) std::rethrow_exception(e);
     } catch (const AssertionFailure& x) {
       PyErr_SetString(PyExc_AssertionError, x.what());
+    } catch (const NoForwardMode& x) {
+      PyErr_SetString(PyExc_NotImplementedError, x.what());
     }
   });
   m.def("status_word", &status_word, release());
