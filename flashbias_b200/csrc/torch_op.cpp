@@ -162,7 +162,8 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const OptTe
       throw std::runtime_error("Last 2 dimensions of mask must be (1, seqlen_k) or (seqlen_q, seqlen_k)");
     // the reference expands the mask over batch and heads (:1128); a mask of n batch entries with n dividing the
     // batch is also taken and read periodically, which is what Swin's repeat() produces
-    FB_ASSERT((mask->size(0) == 1 || batch % mask->size(0) == 0) && (mask->size(1) == 1 || mask->size(1) == nheads), "");
+    const int64_t entries = mask->size(0);  // (none: not a divisor, and an integer division by zero ends the process)
+    FB_ASSERT((entries == 1 || (entries > 0 && batch % entries == 0)) && (mask->size(1) == 1 || mask->size(1) == nheads), "");
   }
 }
 

@@ -30,6 +30,12 @@ def test_mask_gradient_is_refused_in_backward():
     assert torch.isfinite(dq).all()
 
 
+def test_mask_without_batch_entries_is_refused():
+    q, k, v, _, _, _ = (t.cuda() for t in _inputs(2, 32, 2, 32, 4, torch.float16, 1))
+    with pytest.raises(AssertionError):
+        flash_bias_func(q, k, v, None, None, torch.zeros(0, 1, 32, 32, device="cuda"))
+
+
 def test_mask_with_strided_rows_is_read_right_in_both_directions():
     q, k, v, qb, kb, do = _inputs(2, 160, 2, 32, 4, torch.float16, 2)
     base = torch.randn(2, 1, 160, 320, generator=torch.Generator().manual_seed(3))
