@@ -36,6 +36,13 @@ def test_mask_without_batch_entries_is_refused():
         flash_bias_func(q, k, v, None, None, torch.zeros(0, 1, 32, 32, device="cuda"))
 
 
+@pytest.mark.parametrize("on_host", ["q", "k"])
+def test_factors_in_host_memory_are_refused(on_host):
+    q, k, v, qb, kb, _ = (t.cuda() for t in _inputs(1, 32, 2, 32, 4, torch.float16, 1))
+    with pytest.raises(AssertionError):
+        flash_bias_func(q, k, v, qb.cpu() if on_host == "q" else qb, kb.cpu() if on_host == "k" else kb)
+
+
 def test_mask_with_strided_rows_is_read_right_in_both_directions():
     q, k, v, qb, kb, do = _inputs(2, 160, 2, 32, 4, torch.float16, 2)
     base = torch.randn(2, 1, 160, 320, generator=torch.Generator().manual_seed(3))
