@@ -146,7 +146,7 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const OptTe
   if (q_bias) {
     FB_ASSERT(q_bias->scalar_type() == q.scalar_type() && k_bias->scalar_type() == q.scalar_type(),
               "All tensors must have the same type");
-    FB_ASSERT(q_bias->is_cuda() && k_bias->is_cuda(), "");
+    for (const Tensor& t : {*q_bias, *k_bias}) FB_ASSERT(t.is_cuda() || t.is_pinned(), "");  // pinned: read in place
     FB_ASSERT(q_bias->dim() == 4 && k_bias->dim() == 4, "");
     FB_ASSERT(k_bias->size(3) == q_bias->size(3), "");
     auto fits = [&](const Tensor& t, int64_t rows) {

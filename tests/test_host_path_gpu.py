@@ -43,6 +43,11 @@ def test_factors_in_host_memory_are_refused(on_host):
         flash_bias_func(q, k, v, qb.cpu() if on_host == "q" else qb, kb.cpu() if on_host == "k" else kb)
 
 
+def test_pinned_factors_are_read_in_place():
+    q, k, v, qb, kb, _ = (t.cuda() for t in _inputs(1, 32, 2, 32, 4, torch.float16, 1))
+    assert torch.equal(flash_bias_func(q, k, v, qb.cpu().pin_memory(), kb.cpu().pin_memory()), flash_bias_func(q, k, v, qb, kb))
+
+
 def test_mask_with_strided_rows_is_read_right_in_both_directions():
     q, k, v, qb, kb, do = _inputs(2, 160, 2, 32, 4, torch.float16, 2)
     base = torch.randn(2, 1, 160, 320, generator=torch.Generator().manual_seed(3))
