@@ -215,9 +215,13 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor, OptTensor> backward(
     const OptTensor& k_bias, const Tensor& lse, OptTensor mask, bool causal, std::optional<double> softmax_scale,
     int flags, const OptTensor& slopes) {
   check_device_status();
+  check_inputs(q, k, v, q_bias, k_bias, mask);
+  for (const Tensor& t : {dout, o})  // (what the kernels address with q's sizes)
+    FB_ASSERT(t.sizes() == q.sizes() && t.scalar_type() == q.scalar_type() && t.is_cuda(), "");
+  FB_ASSERT(!q_bias || (q_bias->is_cuda() && k_bias->is_cuda()), "");  // their gradients lie where they do
+  FB_ASSERT(lse.is_cuda() && lse.scalar_type() == at::kFloat && lse.is_contiguous(), "");
   if (dout.stride(-1) != 1) dout = dout.contiguous();
   const int64_t rows = rounded_rows(q.size(1));
-  FB_ASSERT(q.size(3) <= 128, "");
   FB_ASSERT(lse.dim() == 3 && lse.size(0) == q.size(0) && lse.size(1) == q.size(2) && lse.size(2) == rows, "");
   FB_ASSERT(q.stride(-1) == 1 && k.stride(-1) == 1 && v.stride(-1) == 1 && o.stride(-1) == 1, "");
   const double scale = scale_or_default(softmax_scale, q.size(3));

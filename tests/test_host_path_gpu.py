@@ -48,6 +48,20 @@ def test_pinned_factors_are_read_in_place():
     assert torch.equal(flash_bias_func(q, k, v, qb.cpu().pin_memory(), kb.cpu().pin_memory()), flash_bias_func(q, k, v, qb, kb))
 
 
+@pytest.mark.parametrize("what", ["do_rows", "do_type", "o_rows", "k_heads", "factor_rows", "factors_on_host", "lse_type"])
+def test_backward_refuses_what_its_kernels_would_misread(what):
+    from flashbias_b200.flash_bias import flash_bias_backward, flash_bias_forward
+    q, k, v, qb, kb, do = (t.cuda() for t in _inputs(2, 64, 2, 32, 4, torch.float16, 1))
+    o, lse, _ = flash_bias_forward(q, k, v, qb, kb)
+    args = dict(do=do, q=q, k=k, v=v, o=o, q_bias=qb, k_bias=kb, lse=lse)
+    assert torch.isfinite(flash_bias_backward(**args)[0]).all()
+    bad = {"do_rows": dict(do=do[:, :32]), "do_type": dict(do=do.float()), "o_rows": dict(o=o[:1]), "k_heads": dict(k=k[:, :, :1]),
+           "factor_rows": dict(k_bias=kb[:, :32]), "factors_on_host": dict(q_bias=qb.cpu(), k_bias=kb.cpu()),
+           "lse_type": dict(lse=lse.half())}[what]
+    with pytest.raises(AssertionError):
+        flash_bias_backward(**{**args, **bad})
+
+
 def test_mask_with_strided_rows_is_read_right_in_both_directions():
     q, k, v, qb, kb, do = _inputs(2, 160, 2, 32, 4, torch.float16, 2)
     base = torch.randn(2, 1, 160, 320, generator=torch.Generator().manual_seed(3))
