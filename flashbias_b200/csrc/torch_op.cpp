@@ -419,6 +419,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("check_device_status", &check_device_status, release());
   m.def("forward", &forward, release());
   m.def("backward", &backward, release());
+  m.def("narrow_expanded", &narrow_expanded, release());
+  m.def("widen_grad", [](const Tensor& g, const std::vector<int64_t>& shape) { return widen_grad(g, shape); }, release());
   m.def("flash_bias", &flash_bias, release(), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("q_bias") = py::none(),
         py::arg("k_bias") = py::none(), py::arg("mask") = py::none(), py::arg("causal") = false,
         py::arg("softmax_scale") = py::none());

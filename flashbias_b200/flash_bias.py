@@ -109,38 +109,90 @@ def flash_bias_backward(do, q, k, v, o, q_bias, k_bias, lse, mask=None, causal=F
     return _op().backward(do, q, k, v, o, q_bias, k_bias, lse, mask, causal, softmax_scale, flags, alibi_slopes)
 
 
-class FlashBiasFunc:
-    """The differentiable operator; ``FlashBiasFunc.apply`` is ``flash_bias_func``."""
+def _unit_rows(*ts):
+    return [t if t is None or t.stride(-1) == 1 else t.contiguous() for t in ts]
+
+
+class FlashBiasFunc(torch.autograd.Function):
+    """The differentiable operator of ``flash_bias_func``.
+
+    ``apply`` of this class is ``flash_bias_func``, the native node (csrc/torch_op.cpp).  ``forward`` and ``backward``
+    are the same operator as static methods, for code that derives from the class or calls them with a context of its
+    own.
+    """
 
     @staticmethod
-    def apply(q, k, v, q_bias=None, k_bias=None, mask=None, causal=False, softmax_scale=None):
-        """
-        q: (batch_size, seqlen_q, nheads, headdim)
-        k, v: (batch_size, seqlen_k, nheads, headdim)
-        q_bias: (batch_size | 1, seqlen_q, nheads | 1, rankdim)
-        k_bias: (batch_size | 1, seqlen_k, nheads | 1, rankdim)
-        mask: optional, (batch | 1, nheads | 1, 1 | seqlen_q, seqlen_k), added to the logits.
-        softmax_scale: multiplies q.k only; defaults to 1 / sqrt(headdim).
-        """
-        return (_torch_op or _op()).flash_bias(q, k, v, q_bias, k_bias, mask, causal, softmax_scale)
+    def forward(ctx, q, k, v, q_bias=None, k_bias=None, mask=None, causal=False, softmax_scale=None):
+        q, k, v, q_bias, k_bias = _unit_rows(q, k, v, q_bias, k_bias)
+        ctx.factor_shapes = [None if t is None else t.shape for t in (q_bias, k_bias)]
+        q_bias, k_bias = _op().narrow_expanded(q_bias), _op().narrow_expanded(k_bias)
+        o, lse, ctx.softmax_scale = flash_bias_forward(q, k, v, q_bias, k_bias, mask, causal, softmax_scale)
+        ctx.save_for_backward(q, k, v, o, q_bias, k_bias, lse, mask)
+        ctx.causal = causal
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, o, q_bias, k_bias, lse, mask = ctx.saved_tensors
+        assert not any(ctx.needs_input_grad[5:6]), "FlashBias does not support mask gradient yet"
+        with torch.no_grad():
+            dq, dk, dv, dq_bias, dk_bias = flash_bias_backward(do, q, k, v, o, q_bias, k_bias, lse, mask, ctx.causal,
+                                                               ctx.softmax_scale)
+            dq_bias, dk_bias = (g if g is None else _op().widen_grad(g, s)
+                                for g, s in zip((dq_bias, dk_bias), ctx.factor_shapes))
+        return dq, dk, dv, dq_bias, dk_bias, None, None, None
+
+    @classmethod
+    def apply(cls, *args, **kwargs):
+        return flash_bias_func(*args, **kwargs) if cls is FlashBiasFunc else super().apply(*args, **kwargs)
 
 
-flash_bias_func = FlashBiasFunc.apply
+def flash_bias_func(q, k, v, q_bias=None, k_bias=None, mask=None, causal=False, softmax_scale=None):
+    """
+    q: (batch_size, seqlen_q, nheads, headdim)
+    k, v: (batch_size, seqlen_k, nheads, headdim)
+    q_bias: (batch_size | 1, seqlen_q, nheads | 1, rankdim)
+    k_bias: (batch_size | 1, seqlen_k, nheads | 1, rankdim)
+    mask: optional, (batch | 1, nheads | 1, 1 | seqlen_q, seqlen_k), added to the logits.
+    softmax_scale: multiplies q.k only; defaults to 1 / sqrt(headdim).
+    """
+    return (_torch_op or _op()).flash_bias(q, k, v, q_bias, k_bias, mask, causal, softmax_scale)
 
 
-class FlashBiasAlibiFunc:
+class FlashBiasAlibiFunc(torch.autograd.Function):
     """Attention with the ALiBi bias ``slopes[h] * (j - i)`` generated inside the kernels.
 
     The reference's language-model call site builds this bias as rank-2 factors from the positions and the
     per-head slopes (1_Language_Model/attention_with_alibi_bias.py:47-52) and feeds them to
     ``flash_bias_func``; here the slopes go in directly, the positions never exist as tensors and are never
     rounded to 16 bits.  ``slopes`` is an fp32 tensor of ``nheads`` values, a constant (the reference
-    registers it as a buffer): it gets no gradient.
+    registers it as a buffer): it gets no gradient.  ``apply``, ``forward`` and ``backward``: as in ``FlashBiasFunc``.
     """
 
     @staticmethod
-    def apply(q, k, v, slopes, causal=True, softmax_scale=None):
-        return (_torch_op or _op()).flash_bias_alibi(q, k, v, slopes, causal, softmax_scale)
+    def forward(ctx, q, k, v, slopes, causal=True, softmax_scale=None):
+        q, k, v = _unit_rows(q, k, v)
+        slopes = slopes.detach().to(device=q.device, dtype=torch.float32).reshape(-1).contiguous()
+        assert slopes.numel() == q.shape[2], "one slope per head"
+        o, lse, ctx.softmax_scale = flash_bias_forward(q, k, v, causal=causal, softmax_scale=softmax_scale,
+                                                       alibi_slopes=slopes)
+        ctx.save_for_backward(q, k, v, o, lse, slopes)
+        ctx.causal = causal
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, o, lse, slopes = ctx.saved_tensors
+        with torch.no_grad():
+            dq, dk, dv, _, _ = flash_bias_backward(do, q, k, v, o, None, None, lse, None, ctx.causal, ctx.softmax_scale,
+                                                   alibi_slopes=slopes)
+        return dq, dk, dv, None, None, None
+
+    @classmethod
+    def apply(cls, *args, **kwargs):
+        return flash_bias_alibi_func(*args, **kwargs) if cls is FlashBiasAlibiFunc else super().apply(*args, **kwargs)
 
 
-flash_bias_alibi_func = FlashBiasAlibiFunc.apply
+def flash_bias_alibi_func(q, k, v, slopes, causal=True, softmax_scale=None):
+    """The operator of ``FlashBiasAlibiFunc``."""
+    return (_torch_op or _op()).flash_bias_alibi(q, k, v, slopes, causal, softmax_scale)

@@ -62,6 +62,57 @@ def test_backward_refuses_what_its_kernels_would_misread(what):
         flash_bias_backward(**{**args, **bad})
 
 
+@pytest.mark.parametrize("expanded", [False, True])
+def test_a_derived_function_gives_the_operator_s_results(expanded):
+    """Code may derive from FlashBiasFunc and call its forward and backward: the same values as the native node."""
+    from flashbias_b200 import FlashBiasFunc
+    seen = []
+
+    class Logged(FlashBiasFunc):
+        @staticmethod
+        def forward(ctx, *args):
+            seen.append("forward")
+            return FlashBiasFunc.forward(ctx, *args)
+
+        @staticmethod
+        def backward(ctx, do):
+            seen.append("backward")
+            return FlashBiasFunc.backward(ctx, do)
+
+    q, k, v, qb, kb, do = (t.cuda() for t in _inputs(2, 130, 2, 32, 4, torch.float16, 4))
+    results = []
+    for fn in (FlashBiasFunc, Logged):
+        leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v, qb, kb)]
+        factors = [t.expand(2, -1, -1, -1) if expanded else t for t in leaves[3:]]
+        o = fn.apply(*leaves[:3], *factors)
+        results.append((o, *torch.autograd.grad(o, leaves, do)))
+    assert seen == ["forward", "backward"]
+    for a, b in zip(*results):  # fp32 sums over key tiles are not ordered: equal up to one rounding
+        assert a.shape == b.shape and (a.float() - b.float()).abs().max() <= 2.0 ** -10 * b.float().abs().max()
+
+
+def test_a_derived_function_takes_three_arguments():
+    from flashbias_b200 import FlashBiasFunc
+    q, k, v, _, _, do = (t.cuda() for t in _inputs(1, 64, 2, 32, 4, torch.float16, 4))
+    o = type("Derived", (FlashBiasFunc,), {}).apply(q.requires_grad_(True), k, v)
+    (dq,) = torch.autograd.grad(o, [q], do)
+    (want,) = torch.autograd.grad(flash_bias_func(q, k, v), [q], do)
+    assert (dq.float() - want.float()).abs().max() <= 2.0 ** -10 * want.float().abs().max()
+
+
+def test_a_function_derived_from_the_slope_form():
+    from flashbias_b200 import FlashBiasAlibiFunc
+    q, k, v, _, _, do = (t.cuda() for t in _inputs(1, 130, 2, 32, 4, torch.float16, 4))
+    slopes = torch.tensor([0.5, 0.25], device="cuda")
+    results = []
+    for fn in (FlashBiasAlibiFunc, type("Derived", (FlashBiasAlibiFunc,), {})):
+        leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        o = fn.apply(*leaves, slopes)
+        results.append((o, *torch.autograd.grad(o, leaves, do)))
+    for a, b in zip(*results):
+        assert (a.float() - b.float()).abs().max() <= 2.0 ** -10 * b.float().abs().max()
+
+
 def test_mask_with_strided_rows_is_read_right_in_both_directions():
     q, k, v, qb, kb, do = _inputs(2, 160, 2, 32, 4, torch.float16, 2)
     base = torch.randn(2, 1, 160, 320, generator=torch.Generator().manual_seed(3))

@@ -3,7 +3,7 @@ import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
 
-from flashbias_b200 import flash_bias_alibi_func, flash_bias_func
+from flashbias_b200 import FlashBiasAlibiFunc, FlashBiasFunc, flash_bias_alibi_func, flash_bias_func
 
 
 @pytest.mark.parametrize("with_grad", [False, True])
@@ -25,3 +25,10 @@ def test_tangents_are_refused_by_the_slope_form(which):
         t[which] = fwAD.make_dual(t[which], torch.ones_like(t[which]))
         with pytest.raises(NotImplementedError, match="forward-mode"):
             flash_bias_alibi_func(*t)
+
+
+@pytest.mark.parametrize("cls", [FlashBiasFunc, FlashBiasAlibiFunc])
+def test_operators_are_autograd_functions(cls):
+    assert issubclass(cls, torch.autograd.Function)
+    for name in ("forward", "backward"):
+        assert name in cls.__dict__
