@@ -64,3 +64,35 @@ def test_repeated_masked_forward_is_bit_identical(mdtype):
     for _ in range(50):
         got, _, _ = flash_bias_forward(q, k, v, qb, kb, mask)
         assert torch.equal(got, want)
+
+
+# (head_dim, rank, softmax_scale, dtype): each number of mask stages (1 to 4), beside one and two CTAs per SM
+RINGS = [
+    (32, 0, None, torch.float16),     # 4 stages, two CTAs
+    (32, 20, None, torch.bfloat16),   # 2 stages, two CTAs
+    (32, 40, 0.25, torch.bfloat16),   # 1 stage, two CTAs
+    (64, 0, None, torch.float16),     # 1 stage, two CTAs
+    (32, 70, None, torch.bfloat16),   # 4 stages, one CTA
+    (64, 70, 0.125, torch.bfloat16),  # 3 stages, one CTA
+    (128, 0, None, torch.bfloat16),   # 4 stages, one CTA
+    (128, 20, 0.25, torch.bfloat16),  # 2 stages, one CTA
+    (128, 12, None, torch.float16),   # 1 stage, one CTA
+]
+
+
+@pytest.mark.parametrize("wide", [True, False], ids=["fp32", "16bit"])
+@pytest.mark.parametrize("ring", RINGS, ids=lambda r: "D%dR%d" % r[:2])
+def test_every_ring_depth_repeats_bit_identical(ring, wide):
+    D, R, scale, dtype = ring
+    mdtype = torch.float32 if wide else dtype
+    g = torch.Generator().manual_seed(D + R)
+    q, k, v = (torch.randn(48, 384, 8, D, generator=g).to(dtype).cuda() for _ in range(3))
+    qb = kb = None
+    if R:
+        qb, kb = ((torch.randn(1, 384, 8, R, generator=g) * 0.3).to(dtype).cuda() for _ in range(2))
+    mask = torch.randn(4, 1, 384, 384, generator=g).to(mdtype).cuda()
+    unaligned = torch.zeros(4, 1, 384, 385, dtype=mdtype, device="cuda")[..., :384].copy_(mask)  # read without the ring
+    want, _, _ = flash_bias_forward(q, k, v, qb, kb, unaligned, False, scale)
+    for _ in range(30):
+        got, _, _ = flash_bias_forward(q, k, v, qb, kb, mask, False, scale)
+        assert torch.equal(got, want)
