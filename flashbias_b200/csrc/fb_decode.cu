@@ -9,6 +9,8 @@
 // fp32 on the given 16-bit values (probabilities are not rounded), and no operand is packed.
 // B16 H50 Sk5001 D32 R2: 233 us with the tiled kernel (2.2 TB/s), 86 us here (5.9 TB/s; 124 us when the rounds in flight
 // were held in registers, 92 us with 3 CTAs and rounds of 2 keys).
+#include <float.h>
+
 #include <mutex>
 #include <type_traits>
 
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(kDecodeThreads, kDecodeCtas) decode_kernel(con
       if (key >= k_end) s[u] = -INFINITY;
       mx = fmaxf(mx, s[u]);
     }
-    const float msub = mx == -INFINITY ? 0.f : mx;  // no visible key yet: every exponential below is zero
+    const float msub = fmaxf(mx, -FLT_MAX);  // no visible key yet: every exponential below is zero
     const float alpha = fast_exp2(m - msub);  // 0 while m is still -inf
     m = mx;
     l *= alpha;
