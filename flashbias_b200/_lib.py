@@ -19,6 +19,7 @@ FB_FLAG_BWD_QUERY_MAJOR = 2
 FB_FLAG_BWD_ONE_ITEM = 4
 FB_FLAG_BWD_PERSISTENT = 8
 FB_FLAG_BWD_FUSED_DELTA = 16
+KERNELS = ("general", "fwd_tiled", "fwd_one_query", "bwd_query_major", "bwd_persistent", "bwd_key_major")  # FB_KERNEL_*
 
 I64x3 = C.c_int64 * 3
 
@@ -51,6 +52,8 @@ EXPORTS = {
     "fb_version": (C.c_int, []),
     "fb_params_size": (C.c_size_t, []),
     "fb_strerror": (C.c_char_p, [C.c_int]),
+    "fb_fwd_kernel": (C.c_int, [C.POINTER(FbParams)]),
+    "fb_bwd_kernel": (C.c_int, [C.POINTER(FbParams)]),
     "fb_fwd_uses_tensor_path": (C.c_int, [C.POINTER(FbParams)]),
     "fb_bwd_uses_tensor_path": (C.c_int, [C.POINTER(FbParams)]),
     "fb_fwd_workspace_bytes": (C.c_size_t, [C.POINTER(FbParams)]),

@@ -190,6 +190,27 @@ extern "C" int fb_read_status(const int32_t* status, int32_t* value, void* cuda_
   return host == FB_DEV_OK ? FB_OK : FB_EDEVICE;
 }
 
+// The kernel a valid problem takes: the one place that decides it, for the launches, the workspace sizes and the queries.
+static int fwd_kernel_of(const fb_params* p, PackPlan* plan) {
+  if (decode_supported(p)) return FB_KERNEL_FWD_ONE_QUERY;
+  return fwd_sm100_supported(p, plan) ? FB_KERNEL_FWD_TILED : FB_KERNEL_GENERAL;
+}
+static int bwd_kernel_of(const fb_params* p, PackPlan* plan) {
+  return bwd_sm100_supported(p, plan) ? bwd_sm100_form(p, *plan) : FB_KERNEL_GENERAL;
+}
+
+extern "C" int fb_fwd_kernel(const fb_params* p) {
+  const int rc = validate_common(p);
+  PackPlan plan;
+  return rc ? rc : fwd_kernel_of(p, &plan);
+}
+
+extern "C" int fb_bwd_kernel(const fb_params* p) {
+  const int rc = validate_common(p);
+  PackPlan plan;
+  return rc ? rc : bwd_kernel_of(p, &plan);
+}
+
 extern "C" int fb_fwd_uses_tensor_path(const fb_params* p) {
   int rc = validate_common(p);
   if (rc) return rc;
@@ -207,9 +228,11 @@ extern "C" int fb_bwd_uses_tensor_path(const fb_params* p) {
 
 extern "C" size_t fb_fwd_workspace_bytes(const fb_params* p) {
   if (validate_common(p)) return 0;
-  if (decode_supported(p)) return decode_workspace(p);
   PackPlan plan;
-  if (fwd_sm100_supported(p, &plan)) return plan.q_bytes + plan.k_bytes + plan.qs_bytes;
+  switch (fwd_kernel_of(p, &plan)) {
+    case FB_KERNEL_FWD_ONE_QUERY: return decode_workspace(p);
+    case FB_KERNEL_FWD_TILED: return plan.q_bytes + plan.k_bytes + plan.qs_bytes;
+  }
   return 0;
 }
 
@@ -217,14 +240,14 @@ extern "C" int fb_fwd(const fb_params* p, void* cuda_stream) {
   int rc = validate_common(p);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
-  if (decode_supported(p)) {
-    if ((rc = check_workspace(p, decode_workspace(p)))) return rc;
-    return launch_decode(p, st);
-  }
   PackPlan plan;
-  if (fwd_sm100_supported(p, &plan)) {
-    if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes + plan.qs_bytes))) return rc;
-    return launch_fwd_sm100(p, plan, st);
+  switch (fwd_kernel_of(p, &plan)) {
+    case FB_KERNEL_FWD_ONE_QUERY:
+      if ((rc = check_workspace(p, decode_workspace(p)))) return rc;
+      return launch_decode(p, st);
+    case FB_KERNEL_FWD_TILED:
+      if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes + plan.qs_bytes))) return rc;
+      return launch_fwd_sm100(p, plan, st);
   }
   return launch_fwd_general(p, st);
 }
@@ -232,7 +255,7 @@ extern "C" int fb_fwd(const fb_params* p, void* cuda_stream) {
 extern "C" size_t fb_bwd_workspace_bytes(const fb_params* p) {
   if (validate_common(p)) return 0;
   PackPlan plan;
-  if (bwd_sm100_supported(p, &plan)) return bwd_sm100_workspace(p, plan);
+  if (bwd_kernel_of(p, &plan) != FB_KERNEL_GENERAL) return bwd_sm100_workspace(p, plan);
   return bwd_general_workspace(p);
 }
 
@@ -247,7 +270,7 @@ extern "C" int fb_bwd(const fb_params* p, void* cuda_stream) {
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   PackPlan plan;
-  if (bwd_sm100_supported(p, &plan)) {
+  if (bwd_kernel_of(p, &plan) != FB_KERNEL_GENERAL) {
     if ((rc = check_workspace(p, bwd_sm100_workspace(p, plan)))) return rc;
     return launch_bwd_sm100(p, plan, st);
   }

@@ -54,13 +54,21 @@ static bool bwd_prefers_persistent(const fb_params* p) {
   return sms > 0 && tiles_per_item <= 8 && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
 }
 
-int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+int bwd_sm100_form(const fb_params* p, const PackPlan& plan) {
+  // without factor operands: key-major where it is built, unless the caller asks for the other form
+  if (plan.RP == 0 && (plan.TD == 128 || (plan.TD == 32 && !(p->flags & FB_FLAG_BWD_QUERY_MAJOR))))
+    return FB_KERNEL_BWD_KEY_MAJOR;
   // (the persistent form writes dK and dV with tile stores: their layout must be one a tensor map can describe)
   if (plan.TD == 32 && plan.RP > 0 && !p->alibi_slopes && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
       ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p)) &&
-      tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B) &&
-      tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B))
-    return dispatch_bwd_d32p(p, plan, st);
+      (!p->dk || tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B)) &&
+      (!p->dv || tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B)))
+    return FB_KERNEL_BWD_PERSISTENT;
+  return FB_KERNEL_BWD_QUERY_MAJOR;
+}
+
+int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+  if (bwd_sm100_form(p, plan) == FB_KERNEL_BWD_PERSISTENT) return dispatch_bwd_d32p(p, plan, st);
   switch (plan.TD) {
     case 32: return dispatch_bwd_d32(p, plan, st);
     case 64: return dispatch_bwd_d64(p, plan, st);

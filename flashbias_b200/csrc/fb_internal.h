@@ -92,6 +92,7 @@ bool fwd_sm100_supported(const fb_params* p, PackPlan* plan);
 int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 
 bool bwd_sm100_supported(const fb_params* p, PackPlan* plan);
+int bwd_sm100_form(const fb_params* p, const PackPlan& plan);  // FB_KERNEL_BWD_*
 size_t bwd_sm100_workspace(const fb_params* p, const PackPlan& plan);
 int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 

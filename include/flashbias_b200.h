@@ -128,9 +128,23 @@ int fb_version(void);
 size_t fb_params_size(void); /* sizeof(fb_params) as compiled, for bindings to check their mirror of the struct */
 const char *fb_strerror(int code);
 
-/* 1 if the tcgen05/TMA kernels handle this problem, 0 if the shape-generic kernels do, <0 on invalid arguments.
- * (fb_bwd_uses_tensor_path answers for head dimensions up to 64; without factor operands the tcgen05 kernels also
- * take 65..128, for which it keeps answering 0.) */
+/*
+ * The kernel that fb_fwd / fb_bwd takes for this problem (FB_KERNEL_*), or <0 on invalid arguments.  No counterpart in the
+ * reference, which has one kernel per direction.  Fill in every pointer and stride of the call: alignment counts.  (Gradient
+ * pointers that are null count as aligned.)
+ */
+#define FB_KERNEL_GENERAL 0         /* shape-generic CUDA-core kernels, either direction */
+#define FB_KERNEL_FWD_TILED 1       /* forward, tcgen05: tiles of 128 query rows */
+#define FB_KERNEL_FWD_ONE_QUERY 2   /* forward, CUDA cores: one query row per (batch, head), split over the keys */
+#define FB_KERNEL_BWD_QUERY_MAJOR 3 /* backward, tcgen05: thread = query row, one work item per CTA */
+#define FB_KERNEL_BWD_PERSISTENT 4  /* ... one persistent CTA per SM walking the work items */
+#define FB_KERNEL_BWD_KEY_MAJOR 5   /* backward, tcgen05: thread = key, no factor operands */
+int fb_fwd_kernel(const fb_params *p);
+int fb_bwd_kernel(const fb_params *p);
+
+/* 1 if the shape is one that the tcgen05/TMA kernels are built for, 0 if not, <0 on invalid arguments.  Not the kernel
+ * that a call takes: a single query row answers 1 and runs on the one-query kernel; head dimensions 65..128 without factor
+ * operands answer 0 for the backward and run on the key-major one.  fb_fwd_kernel / fb_bwd_kernel name the kernel. */
 int fb_fwd_uses_tensor_path(const fb_params *p);
 int fb_bwd_uses_tensor_path(const fb_params *p);
 

@@ -66,3 +66,26 @@ def check_close(name, got, want_fp32, out_dtype, max_abs_tol=MAX_ABS_TOL, rel_l2
     gate = rel_l2_tol * (4.0 if out_dtype == torch.bfloat16 else 1.0)
     assert rl <= gate, f"{name}: rel-l2 {rl:.3e} > {gate:.1e} (max-abs {ma:.3e})"
     return ma, rl
+
+
+def kernels_taken(q, k, v, q_bias=None, k_bias=None, mask=None, causal=False, flags=0, slopes=None):
+    """The names (flashbias_b200._lib.KERNELS) of the kernels that the operator takes for these device tensors, forward
+    and backward."""
+    import ctypes as C
+    import math
+
+    from flashbias_b200 import _lib
+    from flashbias_b200.flash_bias import _fill_common, _strides_bhs
+    p = _lib.FbParams()
+    _fill_common(p, q, k, v, q_bias, k_bias, mask, causal, 1.0 / math.sqrt(q.shape[-1]), flags, slopes)
+    o, dq, dk, dv = (torch.empty_like(t) for t in (q, q, k, v))
+    lse = torch.empty(q.shape[0], q.shape[2], -(-q.shape[1] // 128) * 128, device=q.device)
+    p.o, p.o_stride, p.lse, p.lse_stride_bh = o.data_ptr(), _strides_bhs(o), lse.data_ptr(), lse.shape[-1]
+    p.dout, p.dout_stride = o.data_ptr(), _strides_bhs(o)
+    for name, t in (("dq", dq), ("dk", dk), ("dv", dv)):
+        setattr(p, name, t.data_ptr())
+        setattr(p, name + "_stride", _strides_bhs(t))
+    lib = _lib.load()
+    codes = lib.fb_fwd_kernel(C.byref(p)), lib.fb_bwd_kernel(C.byref(p))
+    assert min(codes) >= 0, codes
+    return tuple(_lib.KERNELS[c] for c in codes)

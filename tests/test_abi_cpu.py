@@ -61,6 +61,58 @@ def test_host_side_validation(mutate, code):
     assert _lib.strerror(code)
 
 
+def _problem(D=32, Sq=256, R=0, dtype=_lib.FB_DTYPE_BF16, scale=None, flags=0, slopes=False, mask=False, odd=False):
+    p = _valid_params()
+    p.D, p.Sq, p.Sk, p.R, p.dtype, p.flags = D, Sq, 256, R, dtype, flags
+    p.softmax_scale = scale or D ** -0.5
+    row = 2 * D + (1 if odd else 0)
+    for name in ("q_stride", "k_stride", "v_stride", "o_stride"):
+        setattr(p, name, _lib.I64x3(256 * row, D, row))
+    p.lse_stride_bh = 256
+    if R:
+        p.q_bias = p.k_bias = 0x1000
+        p.q_bias_stride = p.k_bias_stride = _lib.I64x3(0, R, 2 * R)
+    if slopes:
+        p.alibi_slopes = 0x1000
+    if mask:
+        p.mask, p.mask_kind, p.mask_dtype = 0x1000, _lib.FB_MASK_VECTOR, _lib.FB_DTYPE_F32
+    return p
+
+
+@pytest.mark.parametrize("problem,fwd,bwd", [
+    (dict(R=2), "fwd_tiled", "bwd_query_major"),
+    (dict(R=2, flags=_lib.FB_FLAG_BWD_PERSISTENT), "fwd_tiled", "bwd_persistent"),
+    (dict(R=2, flags=_lib.FB_FLAG_BWD_PERSISTENT | _lib.FB_FLAG_BWD_ONE_ITEM), "fwd_tiled", "bwd_query_major"),
+    (dict(slopes=True), "fwd_tiled", "bwd_key_major"),
+    (dict(mask=True, flags=_lib.FB_FLAG_BWD_QUERY_MAJOR), "fwd_tiled", "bwd_query_major"),
+    (dict(D=64), "fwd_tiled", "bwd_query_major"),
+    (dict(D=72), "fwd_tiled", "bwd_key_major"),
+    (dict(D=128, slopes=True), "fwd_tiled", "bwd_key_major"),
+    (dict(D=128, R=2), "fwd_tiled", "general"),
+    (dict(D=64, R=12, dtype=_lib.FB_DTYPE_F16), "fwd_tiled", "general"),
+    (dict(R=40), "fwd_tiled", "general"),
+    (dict(R=130), "general", "general"),
+    (dict(D=20), "general", "general"),
+    (dict(odd=True), "general", "general"),
+    (dict(slopes=True, mask=True), "general", "general"),
+    (dict(flags=_lib.FB_FLAG_FORCE_GENERAL), "general", "general"),
+    (dict(Sq=1), "fwd_one_query", "bwd_key_major"),
+    (dict(Sq=1, slopes=True, mask=True), "fwd_one_query", "general"),
+    (dict(Sq=1, R=17), "fwd_tiled", "bwd_query_major"),
+    (dict(Sq=1, scale=-1.0), "fwd_one_query", "general"),
+    (dict(scale=-1.0), "general", "general"),
+], ids=str)
+def test_kernel_queries_name_the_kernel_taken(problem, fwd, bwd):
+    lib, p = _lib.load(), _problem(**problem)
+    assert _lib.KERNELS[lib.fb_fwd_kernel(C.byref(p))] == fwd
+    assert _lib.KERNELS[lib.fb_bwd_kernel(C.byref(p))] == bwd
+
+
+def test_kernel_queries_reject_what_the_launches_reject():
+    lib, p = _lib.load(), _problem(D=129)
+    assert lib.fb_fwd_kernel(C.byref(p)) == lib.fb_bwd_kernel(C.byref(p)) == -2
+
+
 def test_backward_requires_gradient_buffers():
     lib = _lib.load()
     p = _valid_params()

@@ -8,7 +8,7 @@ import torch
 from flashbias_b200 import check_device_status, flash_bias_alibi_func
 from flashbias_b200.flash_bias import flash_bias_forward
 from oracle import flashbias_oracle as orc
-from tests.helpers import check_close
+from tests.helpers import check_close, kernels_taken
 
 pytestmark = pytest.mark.gpu
 
@@ -41,6 +41,7 @@ def test_single_query_forward(case):
         mask[..., Sk // 2:] = float("-inf") if mkind == "vector" else -50.0
         mask = mask.to(dtype if mkind == "matrix" else torch.float32)
     dev = [t.cuda() if t is not None else None for t in (q, k, v, qb, kb, mask)]
+    assert kernels_taken(*dev, causal)[0] == ("fwd_tiled" if R == 96 else "fwd_one_query")
     o, lse, _ = flash_bias_forward(*dev, causal, None)
     torch.cuda.synchronize()
     check_device_status()

@@ -7,7 +7,7 @@ import torch
 
 from flashbias_b200 import check_device_status, flash_bias_alibi_func, flash_bias_func
 from oracle import flashbias_oracle as orc
-from tests.helpers import check_close
+from tests.helpers import check_close, kernels_taken
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +43,11 @@ def test_head_dims(case):
         mask = torch.where(torch.rand(B, 1, Sq, Sk, generator=g) < 0.3, -100.0, torch.randn(B, 1, Sq, Sk, generator=g))
     leaves = [t.cuda().requires_grad_(True) for t in (q, k, v, qb, kb) if t is not None]
     f = [t.float() for t in (q, k, v)] + [t.float() if t is not None else None for t in (qb, kb)]
+    slopes_dev = torch.ones(H, device="cuda") if mode == "slopes" else None
+    dev = [t.detach() for t in leaves] + [None] * (5 - len(leaves))
+    bwd = "bwd_key_major" if D > 64 else "bwd_persistent" if B == 40 else "bwd_query_major"
+    assert kernels_taken(*dev, mask.cuda() if mask is not None else None, causal, 0, slopes_dev) == (
+        "fwd_one_query" if Sq == 1 else "fwd_tiled", bwd)
     if mode == "slopes":
         slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)])
         o = flash_bias_alibi_func(*leaves, slopes.cuda(), causal)
