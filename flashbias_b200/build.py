@@ -1,6 +1,10 @@
 """Build libflashbias_b200.so in-tree with nvcc for sm_100a.
 
     python -m flashbias_b200.build [--force] [--verbose]
+    python flashbias_b200/build.py        (the same, without importing the package)
+
+The C library needs nvcc alone.  The PyTorch extension with the operators' host path is built beside it where torch is
+installed; without torch the C library is all there is.
 
 The shared library lands next to the package (``flashbias_b200/libflashbias_b200.so``) so that it
 travels with the source tree; nothing is installed into site-packages and nothing is JIT-cached.
@@ -55,10 +59,16 @@ def _build_torch_op(verbose: bool) -> None:
         sys.stderr.write(r.stderr)
 
 
-def _digest(paths) -> str:
-    import torch
-    h = hashlib.sha256()
-    h.update(torch.__version__.encode())
+def _torch_version() -> str | None:
+    try:
+        import torch
+    except ImportError:
+        return None
+    return torch.__version__
+
+
+def _digest(paths, salt: str = "") -> str:
+    h = hashlib.sha256(salt.encode())
     for p in sorted(paths):
         with open(p, "rb") as f:
             h.update(p.encode() + b"\0" + f.read())
@@ -84,11 +94,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
     srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(ROOT, "include", "flashbias_b200.h"))
-    stamp = os.path.join(OBJ, "stamp")
-    digest = _digest([os.path.join(CSRC, s) for s in srcs + ["torch_op.cpp"]] + headers)
-    if not force and os.path.exists(LIB) and os.path.exists(TORCH_OP) and os.path.exists(stamp) and open(stamp).read() == digest:
-        return LIB
     os.makedirs(OBJ, exist_ok=True)
+    stamp, op_stamp = os.path.join(OBJ, "stamp"), os.path.join(OBJ, "torch_op.stamp")
+    digest = _digest([os.path.join(CSRC, s) for s in srcs] + headers)
+    torch_version = _torch_version()
+    op_digest = torch_version and _digest(_with_headers(os.path.join(CSRC, "torch_op.cpp")), torch_version)
+
+    def is_current(target, stamp_path, want):
+        return not force and os.path.exists(target) and os.path.exists(stamp_path) and open(stamp_path).read() == want
+
+    if not is_current(LIB, stamp, digest):
+        _build_library(srcs, force, verbose)
+        with open(stamp, "w") as f:
+            f.write(digest)
+    if op_digest and not is_current(TORCH_OP, op_stamp, op_digest):
+        _build_torch_op(verbose)
+        with open(op_stamp, "w") as f:
+            f.write(op_digest)
+    return LIB
+
+
+def _build_library(srcs, force: bool, verbose: bool) -> None:
     nvcc = _nvcc()
     extra = ["-Xptxas", "-v"] if verbose else []
 
@@ -114,10 +140,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
                        capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _build_torch_op(verbose)
-    with open(stamp, "w") as f:
-        f.write(digest)
-    return LIB
 
 
 if __name__ == "__main__":
