@@ -7,8 +7,8 @@
 // of a CTA cover neighbouring heads of the same key, so that a (B, S, H, D) cache is read as whole contiguous rows; the
 // keys are split over enough CTAs to fill the GPU once, and a second small kernel merges the splits.  All arithmetic is
 // fp32 on the given 16-bit values (probabilities are not rounded), and no operand is packed.
-// B16 H50 Sk5001 D32 R2: 233 us with the tiled kernel (2.2 TB/s), 86 us here (5.9 TB/s; 124 us when the rounds in flight
-// were held in registers, 92 us with 3 CTAs and rounds of 2 keys).
+// B16 H50 Sk5001 D32 R2: 233 us a call with the tiled kernel (2.2 TB/s), 87 to 91 us here (5.6 to 5.9 TB/s; 85 us of it this
+// kernel; 124 us when the rounds in flight were held in registers, 92 us with 3 CTAs and rounds of 2 keys).
 #include <float.h>
 
 #include <mutex>
@@ -326,7 +326,10 @@ DecodePlan plan_decode(const fb_params* p) {
   d.nhg = (p->H + fit - 1) / fit;
   d.hg = (p->H + d.nhg - 1) / d.nhg;
   d.kp = fit / d.hg;
-  // as many key ranges as fill the resident CTA slots once, none shorter than 8 rounds
+  // The largest number of key ranges with which all CTAs are resident at once, none shorter than 8 rounds.  Rounded down: where
+  // it does not divide, slots stay empty, up to half of them just above one CTA per SM (rates per call, 296 slots: B37 H16
+  // Sk5000 D128, 296 used, 6.6 TB/s; B25 H50 Sk5001 D128, 200 used, 5.5; B148 H16 Sk2000 D128, 296 used, 6.6; B149, 149 used,
+  // 5.4; B149 H50 Sk1000 D32, 149 used, 4.1).
   int dev = 0;
   cudaGetDevice(&dev);
   const int slots = kDecodeCtas * (device_sm_count(dev) > 0 ? device_sm_count(dev) : 148);

@@ -2,7 +2,7 @@
 
 Every tensor is drawn on the CPU in fp32 from ``torch.Generator().manual_seed(seed)``
 with ``seed = 1000 * workload + k`` (k: 0 q, 1 k, 2 v, 3 dO, 4+ factor sources) and
-then rounded once to the run dtype, so the CPU checker and the CUDA kernels consume
+then rounded once to the run dtype, so the CPU oracle and the CUDA kernels consume
 bit-identical values.  The public workloads these stand in for (ImageNet/Swin
 checkpoints, car-design meshes, PDB structures) are not reproduced; only their
 shapes and value distributions are.

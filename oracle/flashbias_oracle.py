@@ -1,6 +1,6 @@
 """CPU restatement of the FlashBias attention path.  TEST INFRASTRUCTURE ONLY.
 
-This module is the checker for the CUDA kernels: only the test-suite, the smoke
+This module is the oracle for the CUDA kernels: only the test-suite, the smoke
 entry and the benchmark's CPU-baseline leg may import it.  Nothing in the
 product package routes through it.
 
