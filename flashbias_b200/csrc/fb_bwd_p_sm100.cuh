@@ -263,16 +263,14 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int it = 0; it < x.n_it; ++it, ++tn) {
           issue_dQ(tn);
           if (lx.valid) {  // the S|dP, dV and dK chains have finished reading the stage of tile tn: tile tn + NSTAGE
-            mbar_wait(qdo_free + 8 * (tn % Cfg::NSTAGE), (tn / Cfg::NSTAGE) & 1, abort_flag);
-            load_next();
+            if (mbar_wait(qdo_free + 8 * (tn % Cfg::NSTAGE), (tn / Cfg::NSTAGE) & 1, abort_flag)) load_next();
           }
         }
         if (!ASYNC) umma_commit(all_done);
         const BwdItem nx = get_item(w + 1, pa.active_items);
         if (nx.valid) {  // K and Kc are free once the dQ | dQb products of the item's last tile have completed
           const uint32_t tl = tn - 1;
-          mbar_wait(dq_full + 8 * (tl % Cfg::NDQ), (tl / Cfg::NDQ) & 1, abort_flag);
-          load_kvb(nx);
+          if (mbar_wait(dq_full + 8 * (tl % Cfg::NDQ), (tl / Cfg::NDQ) & 1, abort_flag)) load_kvb(nx);
         }
         ++n;
       }
@@ -363,8 +361,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           {
             const BwdItem nx = get_item(w + 1, pa.active_items);
             if (nx.valid) {  // group A of the next item, while the compute warps are on this item's last tile
-              mbar_wait(sdp_done, n & 1, abort_flag);
-              load_kva(nx);
+              if (mbar_wait(sdp_done, n & 1, abort_flag)) load_kva(nx);
             }
           }
           if (Cfg::SEP_DKB) {
@@ -852,6 +849,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
+    settle_expired_wait(abort_flag);
     __syncwarp();
     tmem_dealloc(tmem, 512);
   }

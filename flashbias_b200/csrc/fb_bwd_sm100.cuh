@@ -345,10 +345,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll 1
       for (int it = 0; it < n_it; ++it) {
         issue_dQ(it);
-        if (it + Cfg::NSTAGE < n_it) {  // the S|dP, dV and dK chains have finished reading the stage of tile it
-          mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag);
+        // the S|dP, dV and dK chains have finished reading the stage of tile it
+        if (it + Cfg::NSTAGE < n_it && mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag))
           load_tile(it + Cfg::NSTAGE);
-        }
       }
       umma_commit(all_done);
     }
@@ -800,6 +799,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
+    settle_expired_wait(abort_flag);
     __syncwarp();
     tmem_dealloc(tmem, 512);
   }

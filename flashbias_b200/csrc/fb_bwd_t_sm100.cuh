@@ -178,10 +178,9 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
           umma_commit(dq_full + 8 * qb);
           umma_commit(pds_free);
-          if (it + Cfg::NSTAGE < n_it) {  // the S^T|dP^T, dV and dK chains have finished reading the stage of tile it
-            mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag);
+          // the S^T|dP^T, dV and dK chains have finished reading the stage of tile it
+          if (it + Cfg::NSTAGE < n_it && mbar_wait(qdo_free + 8 * (it % Cfg::NSTAGE), (it / Cfg::NSTAGE) & 1, abort_flag))
             load_tile(it + Cfg::NSTAGE);
-          }
         }
       } else if (warp == 13) {
         // ------------------------------------------------------------------ S^T = K.Q^T, dP^T = V.dO^T
@@ -537,6 +536,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   report_expired_wait(abort_flag, a.status);
   if (warp == 13) {
+    settle_expired_wait(abort_flag);
     __syncwarp();
     tmem_dealloc(tmem, 512);
   }

@@ -107,9 +107,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
   return true;
 }
+// A thread that starts copies does so only behind waits that have succeeded: behind an expired one it would pile loads on
+// barriers and stages still in use.
+//
 // At the end of a kernel, after its last CTA-wide barrier.
 __device__ __forceinline__ void report_expired_wait(uint32_t abort_flag, int* status) {
   if (threadIdx.x == 0 && status && ld_shared_flag(abort_flag)) atomicExch(status, FB_DEV_WAIT_TIMEOUT);
+}
+// By the warp that frees tensor memory, before it does: where a wait has expired, copies and products of the CTA may still
+// be in flight, and must not outlive its shared and tensor memory.  Their barriers tell nothing any more, so they get a
+// fixed time, about 20 ms, far more than any of them takes.
+__device__ __forceinline__ void settle_expired_wait(uint32_t abort_flag) {
+  if (ld_shared_flag(abort_flag)) {
+#pragma unroll 1
+    for (int i = 0; i < 2000; ++i) __nanosleep(10000);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -197,29 +197,30 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if constexpr (Cfg::MINB == 2) setmaxnreg_dec<48>();
     if (warp == 4) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
+      auto produce = [&] {
         int kc = 0, vc = 0, n = 0;  // K and V tiles loaded so far (ring positions), items started
         for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w, ++n) {
           const Item it = item_of(idx);
           const int hq = a.hq_bcast ? 0 : it.h, bq = a.bq_bcast ? 0 : it.b;
           const int hk = a.hk_bcast ? 0 : it.h, bk = a.bk_bcast ? 0 : it.b;
-          if (n > 0) mbar_wait(q_free, (n - 1) & 1, abort_flag);
+          if (n > 0 && !mbar_wait(q_free, (n - 1) & 1, abort_flag)) return;
           mbar_expect_tx(q_full, NQ * Cfg::Q_BYTES + Cfg::QB_BYTES);
 #pragma unroll
           for (int t = 0; t < NQ; ++t) tma_tile_4d<D>(sQ + t * Cfg::Q_BYTES, &tmQ, q_full, it.q0, it.h, it.b, t * D);
           if (RP) tma_tile_4d<RPX>(sQb, &tmQb, q_full, it.q0, hq, bq);
           for (int j = 0; j < it.n_kv; ++j, ++kc, ++vc) {
             const int ks = kc % KST, vs = vc % VST;
-            if (kc >= KST) mbar_wait(k_free + 8 * ks, ((kc / KST) - 1) & 1, abort_flag);
+            if (kc >= KST && !mbar_wait(k_free + 8 * ks, ((kc / KST) - 1) & 1, abort_flag)) return;
             mbar_expect_tx(k_full + 8 * ks, Cfg::Q_BYTES + Cfg::QB_BYTES);
             tma_tile_4d<D>(sK + ks * Cfg::Q_BYTES, &tmK, k_full + 8 * ks, j * 128, it.h, it.b);
             if (RP) tma_tile_4d<RPX>(sKb + ks * Cfg::QB_BYTES, &tmKb, k_full + 8 * ks, j * 128, hk, bk);
-            if (vc >= VST) mbar_wait(v_free + 8 * vs, ((vc / VST) - 1) & 1, abort_flag);
+            if (vc >= VST && !mbar_wait(v_free + 8 * vs, ((vc / VST) - 1) & 1, abort_flag)) return;
             mbar_expect_tx(v_full + 8 * vs, Cfg::Q_BYTES);
             tma_tile_4d<D>(sV + vs * Cfg::Q_BYTES, &tmV, v_full + 8 * vs, j * 128, it.h, it.b);
           }
         }
-      }
+      };
+      if (lane == 0) produce();
     } else if (warp == 5) {
       // ------------------------------------------------------------------ MMA issuer: S = [Q|Qb].[K|Kb]^T
       if (lane == 0) {
@@ -287,7 +288,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
     if constexpr (MST > 0) {
-      if (warp == 7 && lane == 0 && a.mask_tma) {
+      auto produce_mask = [&] {
         // ---------------------------------------------------------------- mask tiles, 128 bytes of every row at a time
         const int per = a.mask_dtype == FB_DTYPE_F32 ? 32 : 64;  // columns of a stage
         int mc = 0;
@@ -297,12 +298,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int mh = a.mask_h1 ? 0 : it.h;
           for (int col = 0; col < it.n_kv * 128; col += per, ++mc) {
             const int st = mc % MST;
-            if (mc >= MST) mbar_wait(m_free + 8 * st, ((mc / MST) - 1) & 1, abort_flag);
+            if (mc >= MST && !mbar_wait(m_free + 8 * st, ((mc / MST) - 1) & 1, abort_flag)) return;
             mbar_expect_tx(m_full + 8 * st, Cfg::M_STAGE);
             tma_load_4d(sM + st * Cfg::M_STAGE, &tmM, m_full + 8 * st, col, it.q0, mh, mb);
           }
         }
-      }
+      };
+      if (warp == 7 && lane == 0 && a.mask_tma) produce_mask();
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
@@ -523,6 +525,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   report_expired_wait(abort_flag, a.status);
   if (warp == 5) {
+    settle_expired_wait(abort_flag);
     __syncwarp();
     tmem_dealloc(tmem, Cfg::TMEM_COLS);
   }

@@ -139,7 +139,11 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
   tc_fence_before_sync();
   __syncthreads();
   report_expired_wait(abort_flag, status);
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  if (warp == 0) {
+    settle_expired_wait(abort_flag);
+    __syncwarp();
+    tmem_dealloc(tmem, 256);
+  }
 }
 
 template <int MODE, int C, int C2>
