@@ -307,7 +307,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   setmaxnreg_dec<64>();
   if (warp == 12) {
     // ------------------------------------------------------------------ TMA producer, dQ | dQb chain
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       // The same thread issues the dQ | dQb products: they become due when a query tile's P/dS are written,
       // the next load when the other chains have finished with that tile's stage -- in this order, every tile.
       constexpr uint32_t idQD = instr_desc(kBf16, false, true, 128, D);             // dQ: A K-major, B MN-major
@@ -361,7 +361,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     //   warp 13  also dKb when it is a separate accumulator      warp 14  dV
     //   warp 15  dK (or dK | dKb merged)
     // Every accumulator is only ever touched by one thread, which keeps its MMAs ordered.
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       const int role = warp - 13;
       constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, 128);  // S, dP: both operands K-major
       constexpr uint32_t idTD = instr_desc(kBf16, true, true, 128, D);     // dV, dK: A^T (MN-major), B MN-major

@@ -153,7 +153,7 @@ bwd_t_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp >= 12) {
     setmaxnreg_dec<Cfg::REGS_MOVE>();
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       // B operands read transposed (MN-major: rows are the contraction index), A of dQ likewise
       constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, QT);   // S^T, dP^T: both operands K-major
       constexpr uint32_t idTS = instr_desc(kBf16, false, true, 128, D);    // dV, dK: A in TMEM, B MN-major

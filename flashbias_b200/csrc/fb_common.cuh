@@ -27,6 +27,11 @@ __device__ __forceinline__ uint32_t lane_id() {
   return l;
 }
 
+// The one thread of a warp that issues copies and products.  Branches on elect.sync, not on the lane index: the compiler then
+// knows that a single thread runs and feeds the tensor instructions from uniform registers.  Alone on an SM a product issued
+// behind `lane == 0` takes 59 to 67 clocks to issue, behind elect.sync 16 (A in tensor memory, N = 32) to 48 (both operands
+// in shared memory, N = 64, the operand fetch).  Windowed training shape (B4096 H24 S256 D32 R16): backward kernel 7150 -> 6820
+// us, forward kernel 3035 -> 2943 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(

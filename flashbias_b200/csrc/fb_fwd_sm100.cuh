@@ -220,10 +220,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       };
-      if (lane == 0) produce();
+      if (elect_one()) produce();
     } else if (warp == 5) {
       // ------------------------------------------------------------------ MMA issuer: S = [Q|Qb].[K|Kb]^T
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, 128);
         // descriptor views built once; each MMA only adds a constant to the start-address field
         const DescBase dQ = kmajor_base<D>(sQ), dQb = kmajor_base<RPX>(sQb), dK = kmajor_base<D>(sK),
@@ -266,7 +266,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ------------------------------------------------------------------ MMA issuer: O += P.V
       // A second issuing thread on another warp scheduler: S of the next key tile and P.V of this one are
       // issued concurrently (an issuing thread only gets a slot when the softmax warps of its scheduler stall).
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idO = instr_desc(kBf16, false, true, 128, D);
         const DescBase dV = mnmajor_base<D>(sV);
         int t = 0;
@@ -304,7 +304,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       };
-      if (warp == 7 && lane == 0 && a.mask_tma) produce_mask();
+      if (warp == 7 && a.mask_tma && elect_one()) produce_mask();
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
