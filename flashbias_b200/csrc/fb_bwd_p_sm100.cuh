@@ -425,12 +425,12 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
       float* s_kbc = reinterpret_cast<float*>(smem + Cfg::OFF_KBC);
-      // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32, laid out [column][key
-      // group]: one entry per thread, fetched one item ahead so that the load is not waited for at the item's head
+      // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32, laid out [column pair]
+      // [key group][2]: one entry per thread, fetched one item ahead so that the load is not waited for at the item's head
       float kbc_next = 0.f;
       auto fetch_kbc = [&](const BwdItem& y) {
         const int i = (int)threadIdx.x - 256;
-        const int c = i >> 2, g = i & 3;
+        const int c = (i >> 3) * 2 + (i & 1), g = (i >> 1) & 3;
         kbc_next = 0.f;
         if (i < 2 * Cfg::RCX && c < a.R) {
           const T* kb_bh = a.k_bias_t<T>() + (a.bk_bcast ? 0 : y.b) * a.kb_stride[0] + (a.hk_bcast ? 0 : y.h) * a.kb_stride[1];
@@ -509,13 +509,12 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
         }
         if (RP) {
-          const float* s_rowsum = reinterpret_cast<const float*>(smem + Cfg::OFF_ROWSUM) + (tn & 3) * 512;
           const int bq = a.bq_bcast ? 0 : b, hq = a.hq_bcast ? 0 : h;
           // accumulator laid out (Bq, Hq, query tiles, R, 128 rows): a tile is contiguous
           float* tileb = a.dqb_acc + (bh % a.dqb_slots) * a.dqb_slot_stride +
                          (((int64_t)bq * a.Hq + hq) * a.nq_tiles + (i_begin + it)) * (128 * a.R);
-          float* stgb = reinterpret_cast<float*>(smem + Cfg::OFF_STG + 128 * D * 4) + row;
-          drain_dq_bias<Cfg>(tq + Cfg::T_DQB, s_rowsum, sbase + Cfg::OFF_KBC, stgb, tileb, row, grow < a.Sq, a.R);
+          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (tn & 3) * 2048 + row * 4,
+                                                   sbase + Cfg::OFF_KBC, sStgB + row * 4, tileb + row, grow < a.Sq, a.R);
         }
         tc_fence_before_sync();
         mbar_arrive_warp(dq_drained + 8 * qb);  // every tensor-memory read of the tile is done

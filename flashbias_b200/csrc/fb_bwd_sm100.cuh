@@ -159,17 +159,21 @@ __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk
 // dS16 . (k_bias - c) + c * rowsum_fp32(dS) with c the k_bias of the group's middle key (rows of dS sum to ~0, so
 // rounding dS to 16 bits against a large, slowly varying factor -- ALiBi positions -- would otherwise dominate the
 // result).  The accumulator holds dS16 . hi(k_bias - c) in columns [0, R) and dS16 . lo(k_bias - c) in columns
-// [RCX/2, RCX/2 + R); s_kbc holds c as [column][key group] (4 floats per column, one vector load).
-// The result goes rank-major ([R][128 rows]) into the staging tile (STAGED) or straight into the accumulator in
-// global memory: consecutive threads then write consecutive floats.
-template <typename Cfg>
-__device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, const float* s_rowsum, uint32_t s_kbc, float* stgb,
-                                              float* tileb, int row, bool row_ok, int R) {
-  constexpr int HALF = Cfg::RCX / 2;
-  constexpr int W = HALF >= 16 ? 16 : 8;
-  float rsum[4];
+// [HALF, HALF + R); s_kbc holds c as [column pair][key group][2], s_rowsum the row sums as [key group][128 rows].
+// The result goes rank-major ([R][128 rows]) into the staging tile (stg: this thread's row of it): consecutive threads then
+// write consecutive floats.  Eight columns are evaluated at a time, also those beyond the rank: a branch per column
+// serialised the loads of the centre keys and paced the whole kernel (B512 H24 S144 D32 R8: backward kernel 1094 -> 771 us).
+// Without a staging tile it is added straight to the accumulator in global memory (STAGED false).
+template <int HALF, bool STAGED = true>
+__device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, uint32_t s_rowsum, uint32_t s_kbc, uint32_t stg,
+                                              float* tileb = nullptr, bool row_ok = true, int R = HALF) {
+  constexpr int W = 8;
+  uint64_t rsum[4];
 #pragma unroll
-  for (int g = 0; g < 4; ++g) rsum[g] = s_rowsum[g * 128 + row];
+  for (int g = 0; g < 4; ++g) {
+    const float v = __uint_as_float(ld_shared_flag(s_rowsum + g * 512));
+    rsum[g] = f2(v, v);
+  }
 #pragma unroll 1
   for (int c0 = 0; c0 < HALF && c0 < R; c0 += W) {
     uint32_t rh[W], rl[W];
@@ -178,17 +182,22 @@ __device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, const float* s_ro
     tmem_wait_ld(rh);
     tmem_wait_ld(rl);
 #pragma unroll
-    for (int i = 0; i < W; ++i) {
-      const int c = c0 + i;
-      if (c < R) {
-        const float4 kc = ld_shared_v4f(s_kbc + c * 16);
-        float v = __uint_as_float(rh[i]) + __uint_as_float(rl[i]);
-        v = fmaf(kc.x, rsum[0], v);
-        v = fmaf(kc.y, rsum[1], v);
-        v = fmaf(kc.z, rsum[2], v);
-        v = fmaf(kc.w, rsum[3], v);
-        if (Cfg::STAGED) stgb[c * 128] = v;
-        else if (row_ok) atomicAdd(tileb + c * 128 + row, v);
+    for (int i = 0; i < W; i += 2) {
+      const float4 x = ld_shared_v4f(s_kbc + (c0 + i) * 16), y = ld_shared_v4f(s_kbc + (c0 + i) * 16 + 16);
+      uint64_t v = f2_add(f2(__uint_as_float(rh[i]), __uint_as_float(rh[i + 1])),
+                          f2(__uint_as_float(rl[i]), __uint_as_float(rl[i + 1])));
+      v = f2_fma(f2(x.x, x.y), rsum[0], v);
+      v = f2_fma(f2(x.z, x.w), rsum[1], v);
+      v = f2_fma(f2(y.x, y.y), rsum[2], v);
+      v = f2_fma(f2(y.z, y.w), rsum[3], v);
+      float v0, v1;
+      f2_unpack(v, v0, v1);
+      if (STAGED) {
+        st_shared_f32(stg + (c0 + i) * 512, v0);
+        st_shared_f32(stg + (c0 + i) * 512 + 512, v1);
+      } else if (row_ok) {
+        if (c0 + i < R) atomicAdd(tileb + (c0 + i) * 128, v0);
+        if (c0 + i + 1 < R) atomicAdd(tileb + (c0 + i + 1) * 128, v1);
       }
     }
   }
@@ -524,13 +533,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
         if (RP) {
-          const float* s_rowsum = reinterpret_cast<const float*>(smem + Cfg::OFF_ROWSUM) + (it & 3) * 512;
           const int bq = a.bq_bcast ? 0 : b, hq = a.hq_bcast ? 0 : h;
           // accumulator laid out (Bq, Hq, query tiles, R, 128 rows): a tile is contiguous
           float* tileb = a.dqb_acc + (bh % a.dqb_slots) * a.dqb_slot_stride +
                          (((int64_t)bq * a.Hq + hq) * a.nq_tiles + (i_begin + it)) * (128 * a.R);
-          float* stgb = reinterpret_cast<float*>(smem + Cfg::OFF_STG + 128 * D * 4) + row;
-          drain_dq_bias<Cfg>(tq + Cfg::T_DQB, s_rowsum, sbase + Cfg::OFF_KBC, stgb, tileb, row, grow < a.Sq, a.R);
+          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (it & 3) * 2048 + row * 4,
+                                                   sbase + Cfg::OFF_KBC, sStgB + row * 4, tileb + row, grow < a.Sq, a.R);
         }
         tc_fence_before_sync();
         mbar_arrive_warp(dq_drained + 8 * qb);  // every tensor-memory read of the tile is done
@@ -568,8 +576,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32; read by the drain
       // warpgroup, which is ordered after this through the first pds_ready -> dq_full chain
       const T* kb_bh = a.k_bias_t<T>() + (a.bk_bcast ? 0 : b) * a.kb_stride[0] + (a.hk_bcast ? 0 : h) * a.kb_stride[1];
-      for (int i = threadIdx.x; i < 2 * Cfg::RCX; i += 256) {  // [column][key group]
-        const int c = i >> 2, g = i & 3;
+      for (int i = threadIdx.x; i < 2 * Cfg::RCX; i += 256) {  // [column pair][key group][2]
+        const int c = (i >> 3) * 2 + (i & 1), g = (i >> 1) & 3;
         s_kbc[i] = c < a.R ? to_f32(kb_bh[(int64_t)min(k0 + 32 * g + 16, a.Sk - 1) * a.kb_stride[2] + c]) : 0.f;
       }
     }
