@@ -1,0 +1,23 @@
+// Two-stream backward kernels for head_dim up to 32 (without a mask, both 16-bit types).
+#include "fb_bwd_s_sm100.cuh"
+
+namespace fb {
+
+template <typename T>
+static int dispatch_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+  if (p->alibi_slopes) return launch_bwd_s<T, 32, 0, 0, 1, BWD_ALIBI>(p, plan, st);
+  switch (plan.RC) {
+    case 0: return launch_bwd_s<T, 32, 0, 0, 1, BWD_PLAIN>(p, plan, st);
+    case 32: return plan.nq == 2 ? launch_bwd_s<T, 32, 16, 32, 2, BWD_PLAIN>(p, plan, st)
+                                 : launch_bwd_s<T, 32, 16, 32, 1, BWD_PLAIN>(p, plan, st);
+    case 64: return plan.nq == 2 ? launch_bwd_s<T, 32, 32, 64, 2, BWD_PLAIN>(p, plan, st)
+                                 : launch_bwd_s<T, 32, 32, 64, 1, BWD_PLAIN>(p, plan, st);
+  }
+  return FB_ENOTBUILT;
+}
+
+int dispatch_bwd_s32(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+  return p->dtype == FB_DTYPE_F16 ? dispatch_t<__half>(p, plan, st) : dispatch_t<__nv_bfloat16>(p, plan, st);
+}
+
+}  // namespace fb

@@ -22,6 +22,15 @@ bool bwd_cfg_fits(int D, int RP, int nq) {
   return false;
 }
 
+// The two-stream kernel takes every problem without a mask at head_dim up to 64, except the short items of the persistent
+// form, calls that ask for another form by flag (head_dim 32), and ranks 9 to 16 above head_dim 32, whose accumulators leave
+// no room for dS^T in tensor memory.
+static bool takes_two_stream(const fb_params* p, const PackPlan& plan) {
+  if (plan.TD > 64 || p->mask_kind != FB_MASK_NONE || (plan.TD == 64 && plan.RP > 16)) return false;
+  if (plan.TD == 32 && (p->flags & (plan.RP ? FB_FLAG_BWD_ONE_ITEM : FB_FLAG_BWD_QUERY_MAJOR))) return false;
+  return bwd_sm100_form(p, plan) != FB_KERNEL_BWD_PERSISTENT;
+}
+
 bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->flags & FB_FLAG_FORCE_GENERAL) return false;
   if (p->alibi_slopes && p->mask_kind != FB_MASK_NONE) return false;  // both at once: shape-generic kernels
@@ -38,6 +47,7 @@ bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->dk && !rows_16b_ok(p->dk, p->dk_stride)) return false;
   if (p->dv && !rows_16b_ok(p->dv, p->dv_stride)) return false;
   if ((int64_t)p->B * p->H * ((p->Sk + 127) / 128) > 0x7fffffffLL) return false;
+  if (takes_two_stream(p, *plan)) plan_two_stream(p, plan);
   return true;
 }
 
@@ -68,6 +78,7 @@ int bwd_sm100_form(const fb_params* p, const PackPlan& plan) {
 }
 
 int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+  if (plan.two_stream) return plan.TD == 32 ? dispatch_bwd_s32(p, plan, st) : dispatch_bwd_s64(p, plan, st);
   if (bwd_sm100_form(p, plan) == FB_KERNEL_BWD_PERSISTENT) return dispatch_bwd_d32p(p, plan, st);
   switch (plan.TD) {
     case 32: return dispatch_bwd_d32(p, plan, st);

@@ -848,6 +848,49 @@ inline BwdWs bwd_layout(const fb_params* p, const PackPlan& plan) {
   return w;
 }
 
+inline BwdArgs bwd_args(const fb_params* p, const PackPlan& plan, const BwdWs& w) {
+  uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
+  BwdArgs a;
+  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
+  a.nq_tiles = (p->Sq + 127) / 128;
+  a.nk_tiles = (p->Sk + 127) / 128;
+  a.causal = p->causal;
+  a.R = p->R;
+  a.hq_bcast = plan.Hq == 1; a.bq_bcast = plan.Bq == 1; a.hk_bcast = plan.Hk == 1; a.bk_bcast = plan.Bk == 1;
+  a.Hq = plan.Hq; a.Hk = plan.Hk;
+  // with a split key operand the scale is already inside S
+  a.dk_scale = p->softmax_scale;                     // dK accumulates dS^T.q
+  a.dkb_scale = plan.nq == 2 ? 1.f : p->softmax_scale;    // the packed q-side factor carries 1/scale when nq == 1
+  a.scale_log2 = (plan.nq == 2 ? 1.f : p->softmax_scale) * 1.4426950408889634f;
+  a.lse = p->lse;
+  a.delta = p->delta;
+  a.lse_stride_bh = p->lse_stride_bh;
+  a.dq_acc = reinterpret_cast<float*>(ws + w.off_dq);
+  a.dqb_acc = reinterpret_cast<float*>(ws + w.off_dqb);
+  a.dqb_slots = w.dqb_slots;
+  a.dqb_slot_stride = (int64_t)(w.dqb_slot_bytes / 4);
+  a.dkb_acc = reinterpret_cast<float*>(ws + w.off_dkb);
+  a.dkb_slots = w.dkb_slots;
+  a.dkb_slot_stride = (int64_t)(w.dkb_slot_bytes / 4);
+  a.dk = p->dk;
+  a.dv = p->dv;
+  for (int i = 0; i < 3; ++i) {
+    a.dk_stride[i] = p->dk_stride[i];
+    a.dv_stride[i] = p->dv_stride[i];
+  }
+  a.k_bias = p->k_bias;
+  for (int i = 0; i < 3; ++i) a.kb_stride[i] = p->k_bias_stride[i];
+  a.status = p->status;
+  a.mask = p->mask;
+  for (int i = 0; i < 3; ++i) a.mask_stride[i] = p->mask_stride[i];
+  if (p->mask_kind == FB_MASK_VECTOR) a.mask_stride[2] = 0;
+  a.mask_kind = p->mask_kind;
+  a.mask_dtype = p->mask_dtype;
+  a.mask_batch_period = p->mask_batch_period;
+  a.alibi_slopes = p->alibi_slopes;
+  return a;
+}
+
 // everything a launch of a backward main kernel needs: tensor maps and arguments
 struct BwdLaunch {
   CUtensorMap tQ, tK, tV, tDO, tQb, tKb, tKc, tKs;
@@ -899,44 +942,7 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
     tKb = tK;
     tKc = tK;
   }
-  BwdArgs& a = L.a;
-  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
-  a.nq_tiles = (p->Sq + 127) / 128;
-  a.nk_tiles = (p->Sk + 127) / 128;
-  a.causal = p->causal;
-  a.R = p->R;
-  a.hq_bcast = plan.Hq == 1; a.bq_bcast = plan.Bq == 1; a.hk_bcast = plan.Hk == 1; a.bk_bcast = plan.Bk == 1;
-  a.Hq = plan.Hq; a.Hk = plan.Hk;
-  // with a split key operand the scale is already inside S
-  a.dk_scale = p->softmax_scale;                     // dK accumulates dS^T.q
-  a.dkb_scale = NQ == 2 ? 1.f : p->softmax_scale;    // the packed q-side factor carries 1/scale when nq == 1
-  a.scale_log2 = (NQ == 2 ? 1.f : p->softmax_scale) * 1.4426950408889634f;
-  a.lse = p->lse;
-  a.delta = p->delta;
-  a.lse_stride_bh = p->lse_stride_bh;
-  a.dq_acc = reinterpret_cast<float*>(ws + w.off_dq);
-  a.dqb_acc = reinterpret_cast<float*>(ws + w.off_dqb);
-  a.dqb_slots = w.dqb_slots;
-  a.dqb_slot_stride = (int64_t)(w.dqb_slot_bytes / 4);
-  a.dkb_acc = reinterpret_cast<float*>(ws + w.off_dkb);
-  a.dkb_slots = w.dkb_slots;
-  a.dkb_slot_stride = (int64_t)(w.dkb_slot_bytes / 4);
-  a.dk = p->dk;
-  a.dv = p->dv;
-  for (int i = 0; i < 3; ++i) {
-    a.dk_stride[i] = p->dk_stride[i];
-    a.dv_stride[i] = p->dv_stride[i];
-  }
-  a.k_bias = p->k_bias;
-  for (int i = 0; i < 3; ++i) a.kb_stride[i] = p->k_bias_stride[i];
-  a.status = p->status;
-  a.mask = p->mask;
-  for (int i = 0; i < 3; ++i) a.mask_stride[i] = p->mask_stride[i];
-  if (p->mask_kind == FB_MASK_VECTOR) a.mask_stride[2] = 0;
-  a.mask_kind = p->mask_kind;
-  a.mask_dtype = p->mask_dtype;
-  a.mask_batch_period = p->mask_batch_period;
-  a.alibi_slopes = p->alibi_slopes;
+  L.a = bwd_args(p, plan, w);
   // launches last: the tensor maps and arguments above are ready when the main kernel's turn comes
   return launch_prepare(p, plan, {qpack, kpack, kcenter, ws + w.off_qs, true, fused_delta(p), ws + w.off_dq, w.zero_bytes},
                         st);
@@ -991,6 +997,9 @@ bool bwd_cfg_fits(int D, int RP, int nq);
 int dispatch_bwd_d32(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_bwd_d64(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_bwd_d128(const fb_params* p, const PackPlan& plan, cudaStream_t st);  // without factor operands
+// two-stream form (head_dim up to 64, no mask)
+int dispatch_bwd_s32(const fb_params* p, const PackPlan& plan, cudaStream_t st);
+int dispatch_bwd_s64(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 // persistent form (head_dim 32 with factor operands, plain or masked logits)
 int dispatch_bwd_d32p(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 

@@ -1,5 +1,5 @@
 // Backward FlashBias attention for sm_100a, key-major ("transposed") form, for problems without factor operands
-// (no bias, an additive mask tensor, or the fused ALiBi producer) at head_dim 32 and 128.
+// (no bias, an additive mask tensor, or the fused ALiBi producer) at head_dim 128, and with a mask at head_dim 32.
 //
 // At head_dim 32 the backward is bound by shared-memory bandwidth (128 bytes per clock feed both the tensor
 // core's operand fetches and the threads' stores): in the query-major kernel of fb_bwd_sm100.cuh every query

@@ -56,12 +56,15 @@ struct PackPlan {
   int TD;          // head_dim padded to the tile width: 32, 64 or 128 (missing columns are read as zero)
   int RP;          // packed factor width: 0 (no bias), 16, 32 or 64
   int RC;          // width of the centred k-side copy of the backward (>= RP; 32 beside a head_dim-32 K tile)
+  bool two_stream; // backward: the two-stream kernel (its factor tiles are narrower)
   int Bq, Hq, Bk, Hk;
   size_t q_bytes, k_bytes, kc_bytes, qs_bytes;  // packed q factor, packed k factor, centred k factor, scaled-query
                                                // copy (each rounded to 256)
 };
 // false if the rank does not fit the tensor path; for_bwd reserves room for the centred (hi, lo) k-side copy
 bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd = false);
+// a backward plan with factors, re-planned for the two-stream kernel: factor tiles as wide as the rank asks
+void plan_two_stream(const fb_params* p, PackPlan* plan);
 // What one launch prepares for a call: packed q/k factors, kcenter (optional, rows of plan.RC columns: k_bias minus the
 // k_bias of the middle key of each group of 32 keys), when plan.nq == 2 the (hi, lo) split of q*scale (forward) or
 // k*scale (backward; scaled_is_key), laid out (B, H, S, 2 TD), and for the backward delta (optional) and the zeroed
