@@ -53,15 +53,20 @@ bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
 
 size_t bwd_sm100_workspace(const fb_params* p, const PackPlan& plan) { return bwd_layout(p, plan).total; }
 
-// Whether the persistent form of the query-major kernel is the better one: few query tiles per work item (a CTA
-// that handles one item then spends more time starting and draining than on its tiles) and more items than SMs.
+// Whether the persistent form of the query-major kernel is the better one for a problem with factors at head_dim 32.  What it
+// saves is the start and the drain of a CTA per work item, so: at least two items per SM, and few query tiles per item (mean):
+//  - up to rank 16, up to 20 (persistent / two-stream kernel, us: B256 H24 S256 R16 369 / 805, B1 H50 S1280 R2 80 / 88, S2304
+//    causal 119 / 134, S4096 causal 319 / 336; at 32 tiles, S8192 causal 1182 / 1179; B2 H8 S16384 R5 3058 / 2789);
+//  - above, where it has no staging tile to drain through, up to 4 (B16 H16 S512 R24 99 / 105, S2048 R32 107 / 86);
+//  - with a mask, where the other choice is the one-item form of the same kernel, up to 8.
 static bool bwd_prefers_persistent(const fb_params* p) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = device_sm_count(dev);
   const int nq = (p->Sq + 127) / 128, nk = (p->Sk + 127) / 128;
   const int tiles_per_item = p->causal ? (nq + 1) / 2 : nq;  // mean, under causal masking
-  return sms > 0 && tiles_per_item <= 8 && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
+  const int most = p->mask_kind != FB_MASK_NONE ? 8 : p->R <= 16 ? 20 : 4;
+  return sms > 0 && tiles_per_item <= most && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
 }
 
 int bwd_sm100_form(const fb_params* p, const PackPlan& plan) {
