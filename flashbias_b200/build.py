@@ -27,7 +27,7 @@ LIB = os.path.join(PKG, "libflashbias_b200.so")
 TORCH_OP = os.path.join(PKG, "_torch_op.so")  # the operators' host path (csrc/torch_op.cpp), linked against LIB
 
 SOURCES = ["fb_api.cu", "fb_tmap.cu", "fb_pack.cu", "fb_finish.cu", "fb_general.cu", "fb_selftest.cu",
-           "fb_fwd_sm100.cu", "fb_fwd_inst_d32.cu", "fb_fwd_inst_d64.cu", "fb_fwd_inst_d128.cu",
+           "fb_fwd_sm100.cu", "fb_fwd_inst_d32.cu", "fb_fwd_inst_d64.cu", "fb_fwd_inst_d128.cu", "fb_fwd_inst_s128.cu",
            "fb_bwd_sm100.cu", "fb_bwd_inst_d32.cu", "fb_bwd_inst_d32p.cu", "fb_bwd_inst_d64.cu", "fb_bwd_inst_d128.cu", "fb_bwd_inst_s32.cu", "fb_bwd_inst_s64.cu",
            "fb_decode.cu", "fb_noalloc.cu", "fb_prepare.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -39,7 +39,8 @@ int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) 
   switch (plan.TD) {
     case 32: return dispatch_fwd_d32(p, plan, st);
     case 64: return dispatch_fwd_d64(p, plan, st);
-    case 128: return dispatch_fwd_d128(p, plan, st);
+    case 128:
+      return p->mask_kind == FB_MASK_NONE && plan.RP <= 32 ? dispatch_fwd_s(p, plan, st) : dispatch_fwd_d128(p, plan, st);
   }
   return FB_ENOTBUILT;
 }

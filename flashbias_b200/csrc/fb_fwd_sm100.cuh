@@ -539,6 +539,34 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
+inline FwdArgs fwd_args(const fb_params* p, const PackPlan& plan) {
+  FwdArgs a;
+  a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
+  a.nq_tiles = (p->Sq + 127) / 128;
+  a.total_items = (int)((int64_t)a.nq_tiles * p->B * p->H);
+  a.causal = p->causal;
+  a.hq_bcast = plan.Hq == 1; a.bq_bcast = plan.Bq == 1; a.hk_bcast = plan.Hk == 1; a.bk_bcast = plan.Bk == 1;
+  // logits = a.scale * S: the scale is already inside the query operand when it is split
+  a.scale = plan.nq == 2 ? 1.f : p->softmax_scale;
+  a.scale_log2 = a.scale * 1.4426950408889634f;
+  a.o = p->o;
+  for (int i = 0; i < 3; ++i) a.o_stride[i] = p->o_stride[i];
+  a.lse = p->lse;
+  a.lse_stride_bh = p->lse_stride_bh;
+  a.status = p->status;
+  a.mask = p->mask;
+  for (int i = 0; i < 3; ++i) a.mask_stride[i] = p->mask_stride[i];
+  if (p->mask_kind == FB_MASK_VECTOR) a.mask_stride[2] = 0;
+  a.mask_kind = p->mask_kind;
+  a.mask_dtype = p->mask_dtype;
+  a.mask_batch_period = p->mask_batch_period;
+  a.mask_b1 = p->mask_stride[0] == 0;
+  a.mask_h1 = p->mask_stride[1] == 0;
+  a.mask_tma = 0;
+  a.alibi_slopes = p->alibi_slopes;
+  return a;
+}
+
 template <typename T, int D, int RP, int NQ, int MODE>
 int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   using Cfg = FwdCfg<D, RP, NQ, MODE == FWD_MASK>;
@@ -579,31 +607,9 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       tQb = tQ;
       tKb = tK;
     }
-    FwdArgs a;
-    a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk; a.D = p->D;
-    a.nq_tiles = (p->Sq + 127) / 128;
-    a.total_items = (int)((int64_t)a.nq_tiles * p->B * p->H);
-    a.causal = p->causal;
-    a.hq_bcast = plan.Hq == 1; a.bq_bcast = plan.Bq == 1; a.hk_bcast = plan.Hk == 1; a.bk_bcast = plan.Bk == 1;
-    // logits = a.scale * S: the scale is already inside the query operand when it is split
-    a.scale = NQ == 2 ? 1.f : p->softmax_scale;
-    a.scale_log2 = a.scale * 1.4426950408889634f;
-    a.o = p->o;
-    for (int i = 0; i < 3; ++i) a.o_stride[i] = p->o_stride[i];
-    a.lse = p->lse;
-    a.lse_stride_bh = p->lse_stride_bh;
-    a.status = p->status;
-    a.mask = p->mask;
-    for (int i = 0; i < 3; ++i) a.mask_stride[i] = p->mask_stride[i];
-    if (p->mask_kind == FB_MASK_VECTOR) a.mask_stride[2] = 0;
-    a.mask_kind = p->mask_kind;
-    a.mask_dtype = p->mask_dtype;
-    a.mask_batch_period = p->mask_batch_period;
-    a.mask_b1 = p->mask_stride[0] == 0;
-    a.mask_h1 = p->mask_stride[1] == 0;
+    FwdArgs a = fwd_args(p, plan);
     CUtensorMap tM = tQ;
     a.mask_tma = MODE == FWD_MASK && Cfg::MST > 0 && make_tmap_mask(&tM, p);
-    a.alibi_slopes = p->alibi_slopes;
     // (the tensor maps above are encoded first: the host then has the main kernel's launch ready while the operand
     // preparation runs)
     if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, qs, false, nullptr, nullptr, 0}, st))) return rc;
@@ -641,6 +647,7 @@ bool fwd_cfg_fits(int D, int RP, int nq);
 int dispatch_fwd_d32(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_fwd_d64(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 int dispatch_fwd_d128(const fb_params* p, const PackPlan& plan, cudaStream_t st);
+int dispatch_fwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st);  // head_dim 128, two softmax streams
 
 #define FB_FWD_DISPATCH_BODY(DD)                                                                            \
   template <typename T, int MODE>                                                                           \

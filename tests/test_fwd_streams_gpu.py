@@ -1,0 +1,59 @@
+"""The two-stream forward kernel (head_dim 65 to 128) at odd and even numbers of key tiles, the edges of its tiles, ranks and
+scale kinds, against the CPU checker; and repeated, since a race between its streams would show as different bits."""
+import math
+
+import pytest
+import torch
+
+from flashbias_b200 import check_device_status, flash_bias_alibi_func
+from flashbias_b200.flash_bias import flash_bias_forward
+from oracle import flashbias_oracle as orc
+from tests.helpers import check_close
+
+pytestmark = pytest.mark.gpu
+BF, HF = torch.bfloat16, torch.float16
+
+# (B, H, Sq, Sk, D, R, causal, scale, dtype); R < 0: slopes
+CASES = [
+    (1, 2, 2, 1, 128, 0, False, None, BF),        # one key: the second stream has no tile
+    (1, 2, 128, 128, 72, 2, False, None, HF),     # exactly one tile
+    (1, 2, 129, 129, 128, 16, False, 0.125, BF),  # one past a tile, power-of-two scale (bf16: no split), full packed rank
+    (2, 2, 200, 385, 128, 17, False, None, HF),   # four key tiles, packed rank 32
+    (1, 2, 300, 300, 96, 32, True, None, BF),     # causal, 1 to 3 key tiles per item
+    (1, 2, 450, 260, 128, 3, True, None, HF),     # causal, Sq > Sk
+    (1, 2, 100, 700, 80, 0, True, None, BF),      # causal, Sq < Sk
+    (3, 60, 257, 257, 128, 2, True, None, BF),    # more items than SMs
+    (1, 4, 640, 640, 128, -1, True, None, HF),    # slopes
+    (1, 4, 333, 641, 104, -1, False, None, BF),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "B%dH%dSq%dSk%dD%dR%d%s" % (*c[:6], "c" if c[6] else ""))
+def test_edges(case):
+    B, H, Sq, Sk, D, R, causal, scale, dtype = case
+    scale = scale or 1.0 / math.sqrt(D)
+    g = torch.Generator().manual_seed(Sq * 5 + Sk + D)
+    q = torch.randn(B, Sq, H, D, generator=g).to(dtype)
+    k, v = (torch.randn(B, Sk, H, D, generator=g).to(dtype) for _ in range(2))
+    qb = kb = None
+    if R > 0:
+        qb, kb = ((torch.randn(1, S, H, R, generator=g) * 0.5).to(dtype) for S in (Sq, Sk))
+    dev = [t.cuda() if t is not None else None for t in (q, k, v, qb, kb)]
+    f = [t.float() if t is not None else None for t in (q, k, v, qb, kb)]
+    if R < 0:
+        m = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)])
+        run = lambda: (flash_bias_alibi_func(*dev[:3], m.cuda(), causal, scale), None)
+        m, i, j = m.double(), torch.arange(Sq).double(), torch.arange(Sk).double()
+        f[3] = torch.stack([-(m[None] * i[:, None]), torch.ones(Sq, H).double()], dim=-1)[None]
+        f[4] = torch.stack([torch.ones(Sk, H).double(), m[None] * j[:, None]], dim=-1)[None]
+    else:
+        run = lambda: flash_bias_forward(*dev, None, causal, scale)[:2]
+    o, lse = run()
+    torch.cuda.synchronize()
+    check_device_status()
+    o_ref, lse_ref = orc.attention_forward(*f, None, causal, scale, dtype=torch.float64)
+    check_close("fwd_streams/Sq%dSk%dD%dR%d" % (Sq, Sk, D, R), o, o_ref, dtype)
+    if lse is not None:  # fp32 sums of 16-bit products: 2^-22 of logits up to about 30
+        assert (lse[..., :Sq].cpu().double() - lse_ref.double().reshape(B, H, -1)[..., :Sq]).abs().max() < 2e-5
+    for _ in range(20):
+        assert torch.equal(run()[0], o)
