@@ -203,7 +203,8 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // 8-row group.  The same bytes can be read by the tensor core
 //   * K-major  : rows are the M/N index, columns the contraction index, or
 //   * MN-major : columns are the M/N index, rows the contraction index.
-constexpr __host__ __device__ int swizzle_bytes(int cols) { return cols * 2 >= 128 ? 128 : cols * 2; }
+// (A width that is no multiple of 64 columns is stored in blocks of 32: 96 = 3 x 32.)
+constexpr __host__ __device__ int swizzle_bytes(int cols) { return cols % 64 == 0 ? 128 : cols % 32 == 0 ? 64 : cols * 2; }
 constexpr __host__ __device__ int tile_bytes(int cols, int rows = 128) { return rows * cols * 2; }
 
 // sm_100 shared-memory matrix descriptor: start address [0,14), leading byte offset [16,30),

@@ -14,7 +14,7 @@ static bool o_store_ok(const fb_params* p) {
 bool fwd_cfg_fits(int D, int RP, int nq) {
 #define FB_FIT(DD, RR) \
   if (D == DD && RP == RR) return nq == 2 ? FwdCfg<DD, RR, 2>::FITS : FwdCfg<DD, RR, 1>::FITS;
-  FB_FIT(32, 0) FB_FIT(32, 16) FB_FIT(32, 32) FB_FIT(32, 64) FB_FIT(32, 128)
+  FB_FIT(32, 0) FB_FIT(32, 16) FB_FIT(32, 32) FB_FIT(32, 64) FB_FIT(32, 96) FB_FIT(32, 128)
   FB_FIT(64, 0) FB_FIT(64, 16) FB_FIT(64, 32) FB_FIT(64, 64) FB_FIT(64, 128)
   FB_FIT(128, 0) FB_FIT(128, 16) FB_FIT(128, 32) FB_FIT(128, 64) FB_FIT(128, 128)
 #undef FB_FIT

@@ -69,7 +69,8 @@ struct FwdCfg {
   static constexpr int TMEM_COLS = (T_O + D <= 256) ? 256 : 512;
   // Two CTAs per SM (each CTA reserves 1 KB of the 228 KB) when two stages of each ring fit; else one.
   static constexpr int LIM2 = 113 * 1024, LIM1 = 227 * 1024;
-  static constexpr bool TWO = TMEM_COLS == 256 && smem_for(2, 2) <= LIM2;
+  // (packed rank 96: with one stage of V, whose next load has a whole tile's softmax to arrive)
+  static constexpr bool TWO = TMEM_COLS == 256 && (smem_for(2, 2) <= LIM2 || (RP == 96 && !MASKED && smem_for(2, 1) <= LIM2));
   static constexpr int LIM = TWO ? LIM2 : LIM1;
   static constexpr int MINB = TWO ? 2 : 1;
   // as many K|Kb and V stages (up to 4) as fit: the TMA producer runs that many key tiles ahead, which is
@@ -580,7 +581,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     void* qs = ws + plan.q_bytes + plan.k_bytes;
     CUtensorMap tQ, tK, tV, tQb, tKb;
     constexpr int BOXD = D > 64 ? 64 : D;
-    constexpr int BOXR = RP > 64 ? 64 : (RP ? RP : 16);
+    constexpr int BOXR = RP ? swizzle_bytes(RP) / 2 : 16;
     if (NQ == 2) {
       // query operand = (hi, lo) of q*scale, laid out (B, H, Sq, 2D) in the workspace
       if ((rc = make_tmap_4d(&tQ, qs, 2 * D, p->Sq, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sq,
@@ -660,6 +661,11 @@ int dispatch_fwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st);  
                                    : launch_fwd_t<T, DD, 32, 1, MODE>(p, plan, st);                         \
       case 64: return plan.nq == 2 ? launch_fwd_t<T, DD, 64, 2, MODE>(p, plan, st)                          \
                                    : launch_fwd_t<T, DD, 64, 1, MODE>(p, plan, st);                         \
+      case 96: /* head_dim 32 only */                                                                       \
+        if constexpr (DD == 32)                                                                             \
+          return plan.nq == 2 ? launch_fwd_t<T, DD, 96, 2, MODE>(p, plan, st)                               \
+                              : launch_fwd_t<T, DD, 96, 1, MODE>(p, plan, st);                              \
+        break;                                                                                              \
       case 128: return plan.nq == 2 ? launch_fwd_t<T, DD, 128, 2, MODE>(p, plan, st)                        \
                                     : launch_fwd_t<T, DD, 128, 1, MODE>(p, plan, st);                       \
     }                                                                                                       \

@@ -9,7 +9,7 @@
 //     terms as large as an ALiBi position cancel inside one MMA instead of being rounded first.
 // The backward keeps its key tile resident and streams the query tiles, so it puts the split on the key side
 // instead: S = q.(k*scale), with k*scale as a (hi, lo) pair.
-// Factors are zero-padded to RP columns (16/32/64; the forward also takes 128).  The backward also gets a centred k-side copy
+// Factors are zero-padded to RP columns (16/32/64; the forward also takes 96 and 128).  The backward also gets a centred k-side copy
 // (k_bias minus the k_bias of the middle key of its group of 32 keys, as a (hi, lo) pair).
 #include <math.h>
 
@@ -50,6 +50,8 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   }
   // the centred k-side copy of the backward holds a (hi, lo) pair: twice the rank
   plan->RP = pad_pow2_16(for_bwd ? 2 * p->R : p->R);
+  // forward at head_dim 32: ranks up to 96 fit two CTAs per SM where 128 packed columns fit one
+  if (!for_bwd && plan->TD == 32 && p->R > 64 && p->R <= 96) plan->RP = 96;
   // backward at head_dim 32: factor tiles as wide as the Q/K tiles, so that [Q | Qb] and [K | Kc] are read as one
   // MMA operand each (one product instead of two per 16 query rows / keys)
   if (for_bwd && plan->TD == 32 && plan->RP < 32) plan->RP = 32;
