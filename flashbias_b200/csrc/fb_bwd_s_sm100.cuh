@@ -713,7 +713,7 @@ int launch_bwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       attr_done[dev & 63] = true;
     }
   }
-  if ((rc = launch_prepare(p, plan, {qpack, kpack, RP ? kcenter : nullptr, ks, true, fused_delta(p), ws + w.off_dq, w.zero_bytes},
+  if ((rc = launch_prepare(p, plan, {qpack, kpack, RP ? kcenter : nullptr, ks, fused_delta(p), ws + w.off_dq, w.zero_bytes},
                            st)))
     return rc;
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);

@@ -944,7 +944,7 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
   }
   L.a = bwd_args(p, plan, w);
   // launches last: the tensor maps and arguments above are ready when the main kernel's turn comes
-  return launch_prepare(p, plan, {qpack, kpack, kcenter, ws + w.off_qs, true, fused_delta(p), ws + w.off_dq, w.zero_bytes},
+  return launch_prepare(p, plan, {qpack, kpack, kcenter, ws + w.off_qs, fused_delta(p), ws + w.off_dq, w.zero_bytes},
                         st);
 }
 

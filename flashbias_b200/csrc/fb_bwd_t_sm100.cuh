@@ -603,7 +603,7 @@ int launch_bwd_t_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     }
   }
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);
-  if ((rc = launch_prepare(p, plan, {nullptr, nullptr, nullptr, nullptr, true, fused_delta(p), ws + w.off_dq, w.zero_bytes}, st)))
+  if ((rc = launch_prepare(p, plan, {nullptr, nullptr, nullptr, nullptr, fused_delta(p), ws + w.off_dq, w.zero_bytes}, st)))
     return rc;
   prof_before(KC_BWD_MAIN, st);
   rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, tQ, tK, tV, tDO, a);

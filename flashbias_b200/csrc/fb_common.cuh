@@ -514,6 +514,24 @@ __device__ __forceinline__ uint32_t tile_chunk_offset(int row, int col) {
   return blk * (ROWS * SWB) + row * SWB + (((chunk ^ x) & (CHUNKS - 1)) << 4);
 }
 
+// The 16-byte chunk of eight values at `hi`, times scale, as a (hi, lo) pair of 16-bit terms: hi in place, lo at `lo`.
+template <typename T>
+__device__ __forceinline__ void split_scaled_chunk(uint32_t hi, uint32_t lo, float scale) {
+  uint32_t w[4], l[4];
+  ld_shared_v4(hi, w[0], w[1], w[2], w[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const T* x = reinterpret_cast<const T*>(&w[i]);
+    const float v0 = to_f32(x[0]) * scale, v1 = to_f32(x[1]) * scale;
+    const uint32_t h = Pack2<T>::pack(v0, v1);
+    const T* y = reinterpret_cast<const T*>(&h);
+    l[i] = Pack2<T>::pack(v0 - to_f32(y[0]), v1 - to_f32(y[1]));
+    w[i] = h;
+  }
+  st_shared_v4(hi, w[0], w[1], w[2], w[3]);
+  st_shared_v4(lo, l[0], l[1], l[2], l[3]);
+}
+
 // Byte offset of 16-byte chunk `ch` of row `r` in a staged [128][D] fp32 dQ tile: 128-byte lines, chunks XOR-swizzled
 // by row so that one row per thread writes without bank conflicts.  The fp32 dQ accumulator in global memory keeps
 // this arrangement per (batch, head, query tile) when the tile is reduced in bulk.

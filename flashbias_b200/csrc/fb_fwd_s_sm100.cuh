@@ -55,7 +55,7 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   // (two slots: one per stream)
   const uint32_t q_full = bar0, q_free = bar0 + 8, o_free = bar0 + 16, s_full = bar0 + 24, p_ready = bar0 + 40,
                  pv_done = bar0 + 56, k_full = bar0 + 72 /*3*/, k_free = bar0 + 96 /*3*/, v_full = bar0 + 120 /*3*/,
-                 v_free = bar0 + 144 /*3*/, s_read = bar0 + 176;
+                 v_free = bar0 + 144 /*3*/, s_read = bar0 + 176, q_ready = bar0 + 192;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 168);
   const uint32_t abort_flag = bar0 + 172;
 
@@ -95,6 +95,7 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       st_shared_flag(abort_flag, 0u);
       mbar_init(q_full, 1);
       mbar_init(q_free, 1);
+      mbar_init(q_ready, 8);  // the softmax warps have split the item's q*scale
       mbar_init(o_free, 8);  // every softmax warp has read the accumulators of the item
       for (int i = 0; i < 2; ++i) {
         mbar_init(s_full + 8 * i, 1);
@@ -131,9 +132,8 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int hq = a.hq_bcast ? 0 : it.h, bq = a.bq_bcast ? 0 : it.b;
           const int hk = a.hk_bcast ? 0 : it.h, bk = a.bk_bcast ? 0 : it.b;
           if (n > 0 && !mbar_wait(q_free, (n - 1) & 1, abort_flag)) return;
-          mbar_expect_tx(q_full, NQ * Cfg::Q_BYTES + Cfg::QB_BYTES);
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) tma_tile_4d<D>(sQ + q * Cfg::Q_BYTES, &tmQ, q_full, it.q0, it.h, it.b, q * D);
+          mbar_expect_tx(q_full, Cfg::Q_BYTES + Cfg::QB_BYTES);
+          tma_tile_4d<D>(sQ, &tmQ, q_full, it.q0, it.h, it.b);
           if (RP) tma_tile_4d<RPX>(sQb, &tmQb, q_full, it.q0, hq, bq);
           for (int j = 0; j < it.n_kv; ++j, ++t) {
             const int st = t % ST;
@@ -157,7 +157,8 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         int t = 0, n = 0, c0 = 0, c1 = 0;  // key tiles, items; key tiles of either stream
         for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w, ++n) {
           const Item it = item_of(idx);
-          mbar_wait(q_full, n & 1, abort_flag);
+          mbar_wait(NQ == 2 ? q_ready : q_full, n & 1, abort_flag);
+          tc_fence_after_sync();
           for (int j = 0; j < it.n_kv; ++j, ++t) {
             const int x = j & 1, c = x ? c1++ : c0++, st = t % ST;
             if (c > 0) mbar_wait(s_read + 8 * x, (c - 1) & 1, abort_flag);
@@ -219,6 +220,20 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint64_t sl2p = f2(sl2, sl2);
     int c = 0, co = 0, n = 0;  // key tiles of this stream and of the other, items so far
     uint32_t s[4][32];  // the thread's row of the logit tile
+    // The split of q*scale, half a row per thread, in place and into the tile behind; the next item's ahead of this one's
+    // epilogue, under the wait for the last products.
+    int n_split = 0;
+    auto split_q = [&] {
+      mbar_wait(q_full, n_split++ & 1, abort_flag);
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        const uint32_t at = sQ + tile_chunk_offset<D>(row, 64 * x + 8 * ch);
+        split_scaled_chunk<T>(at, at + Cfg::Q_BYTES, a.q_scale);
+      }
+      fence_proxy_async_smem();
+      mbar_arrive_warp(q_ready);
+    };
+    if (NQ == 2 && item_index(0) < a.total_items) split_q();
     for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w, ++n) {
       const Item it = item_of(idx);
       const int grow = it.q0 + row;
@@ -331,6 +346,7 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc_fence_before_sync();
         mbar_arrive_warp(p_ready + 8 * x);
       }
+      if (NQ == 2 && item_index(w + 1) < a.total_items) split_q();
       // ---- epilogue: O / l -> global, this warpgroup's half of the columns; lse.  (The last product's commit covers the ones
       // before it, which the same thread issued.)
       c = c0 + ((it.n_kv + 1 - x) >> 1);
@@ -388,15 +404,9 @@ int launch_fwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   constexpr int D = Cfg::D;
   int rc;
   uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
-  void *qpack = ws, *kpack = ws + plan.q_bytes, *qs = ws + plan.q_bytes + plan.k_bytes;
+  void *qpack = ws, *kpack = ws + plan.q_bytes;
   CUtensorMap tQ, tK, tV, tQb, tKb;
-  if (NQ == 2) {  // (hi, lo) of q*scale, laid out (B, H, Sq, 2D) in the workspace
-    if ((rc = make_tmap_4d(&tQ, qs, 2 * D, p->Sq, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sq, (int64_t)2 * D * p->Sq * p->H, 64,
-                           128)))
-      return rc;
-  } else if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], 64, 128))) {
-    return rc;
-  }
+  if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], 64, 128))) return rc;
   if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], 64, 128))) return rc;
   if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], 64, 128))) return rc;
   tQb = tKb = tK;
@@ -409,7 +419,7 @@ int launch_fwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       return rc;
   }
   const FwdArgs a = fwd_args(p, plan);
-  if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, qs, false, nullptr, nullptr, 0}, st))) return rc;
+  if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, nullptr, nullptr, nullptr, 0}, st))) return rc;
   auto kern = fwd_s_sm100_kernel<T, RP, NQ, MODE>;
   // per kernel instantiation and device: raise the dynamic shared-memory limit once
   static std::mutex mu;

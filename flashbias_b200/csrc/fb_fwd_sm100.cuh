@@ -9,7 +9,7 @@
 // softmax and the P.V products of this one, and the per-CTA set-up is paid once per SM slot instead of once per
 // query tile -- which is what a short sequence (Swin windows: two key tiles per item) needs.
 // For one item the CTA walks the key/value tiles:
-//   warp 4      TMA producer: Q (or the (hi, lo) split of q*scale) | packed q_bias once per item, then K|packed k_bias
+//   warp 4      TMA producer: Q | packed q_bias once per item, then K|packed k_bias
 //               and V tiles through rings of shared-memory stages.
 //   warp 5      MMA issuer (one thread): S = [Q|Qb].[K|Kb]^T into TMEM, bias products first.
 //   warp 6      MMA issuer (one thread, another warp scheduler): O += P.V with P read from TMEM.
@@ -22,7 +22,8 @@
 //               O is rescaled in TMEM only when the running maximum has grown by more than 2^8 ("lazy
 //               rescale"), which is exact because the row sum carries the same reference maximum.
 // All logit terms share one accumulator: S' = qs.k + qb.k_bias, with qs = q and qb = q_bias/scale when the
-// scale is a power of two (p = exp2((S' - m) * scale * log2 e)), else qs = (hi, lo) of q*scale and qb = q_bias.
+// scale is a power of two (p = exp2((S' - m) * scale * log2 e)), else qs = (hi, lo) of q*scale, which the softmax warps form from
+// the Q tile, and qb = q_bias.
 // An additive mask tensor is added in registers (one mask row per thread, through a TMA ring where the mask's rows are aligned); the fused
 // ALiBi producer adds slope * (col - row) with one FMA per logit and needs no factor operands at all.
 // Two CTAs share an SM when their tiles fit (256 TMEM columns each) so one CTA's softmax overlaps the
@@ -42,6 +43,7 @@ struct FwdArgs {
   int total_items;  // query tiles x batch x heads: the CTAs walk them with a stride of the grid size
   int hq_bcast, bq_bcast, hk_bcast, bk_bcast;  // 1 = the packed factor has extent 1 on that dim
   float scale, scale_log2;
+  float q_scale;  // multiplies q where it is split
   void* o;
   int64_t o_stride[3];
   float* lse;
@@ -130,7 +132,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t k_full = bar0 + 32, k_free = bar0 + 64, v_full = bar0 + 96, v_free = bar0 + 128;  // 4 slots each
   const uint32_t m_full = bar0 + 192, m_free = bar0 + 224;  // likewise
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 160);
-  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 168;
+  const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 164, q_ready = bar0 + 168;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -185,6 +187,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_init(m_free + 8 * i, 4);  // one arrival per softmax warp
       }
       mbar_init(q_free, 1);
+      mbar_init(q_ready, 4);  // the softmax warps have split the item's q*scale
       mbar_fence_init();
     }
   } else if (warp == 5) {
@@ -211,9 +214,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int hq = a.hq_bcast ? 0 : it.h, bq = a.bq_bcast ? 0 : it.b;
           const int hk = a.hk_bcast ? 0 : it.h, bk = a.bk_bcast ? 0 : it.b;
           if (n > 0 && !mbar_wait(q_free, (n - 1) & 1, abort_flag)) return;
-          mbar_expect_tx(q_full, NQ * Cfg::Q_BYTES + Cfg::QB_BYTES);
-#pragma unroll
-          for (int t = 0; t < NQ; ++t) tma_tile_4d<D>(sQ + t * Cfg::Q_BYTES, &tmQ, q_full, it.q0, it.h, it.b, t * D);
+          mbar_expect_tx(q_full, Cfg::Q_BYTES + Cfg::QB_BYTES);
+          tma_tile_4d<D>(sQ, &tmQ, q_full, it.q0, it.h, it.b);
           if (RP) tma_tile_4d<RPX>(sQb, &tmQb, q_full, it.q0, hq, bq);
           for (int j = 0; j < it.n_kv; ++j, ++kc, ++vc) {
             const int ks = kc % KST, vs = vc % VST;
@@ -238,7 +240,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         int t = 0, n = 0;  // key tiles and items issued so far
         for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w, ++n) {
           const Item it = item_of(idx);
-          mbar_wait(q_full, n & 1, abort_flag);
+          mbar_wait(NQ == 2 ? q_ready : q_full, n & 1, abort_flag);
+          tc_fence_after_sync();
           for (int j = 0; j < it.n_kv; ++j, ++t) {
             if (t > 0) {  // the softmax warps hold the logits of the previous key tile in registers
               mbar_wait(s_read, (t - 1) & 1, abort_flag);
@@ -463,6 +466,21 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     };
 
+    // The split of q*scale, a row per thread, in place and into the tile behind.  The next item's is formed ahead of this
+    // item's epilogue, under the wait for the last product.  (As a pass over q ahead of the kernel it cost B4096 H24 S256 D32
+    // 750 us, and the kernel the reads of twice the bytes.)
+    int n_split = 0;
+    auto split_q = [&] {
+      mbar_wait(q_full, n_split++ & 1, abort_flag);
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c) {
+        const uint32_t at = sQ + tile_chunk_offset<D>(row, 8 * c);
+        split_scaled_chunk<T>(at, at + Cfg::Q_BYTES, a.q_scale);
+      }
+      fence_proxy_async_smem();
+      mbar_arrive_warp(q_ready);
+    };
+    if (NQ == 2 && item_index(0) < a.total_items) split_q();
     for (int w = 0, idx; (idx = item_index(w)) < a.total_items; ++w) {
     const Item item = item_of(idx);
     const int b = item.b, h = item.h, bh = item.bh, n_kv = item.n_kv;
@@ -494,6 +512,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before_sync();
       mbar_arrive_warp(p_ready);
     }
+    if (NQ == 2 && item_index(w + 1) < a.total_items) split_q();
     // ---- epilogue: O / l -> global, lse
     mbar_wait(pv_done, (t - 1) & 1, abort_flag);
     tc_fence_after_sync();
@@ -550,6 +569,7 @@ inline FwdArgs fwd_args(const fb_params* p, const PackPlan& plan) {
   // logits = a.scale * S: the scale is already inside the query operand when it is split
   a.scale = plan.nq == 2 ? 1.f : p->softmax_scale;
   a.scale_log2 = a.scale * 1.4426950408889634f;
+  a.q_scale = p->softmax_scale;
   a.o = p->o;
   for (int i = 0; i < 3; ++i) a.o_stride[i] = p->o_stride[i];
   a.lse = p->lse;
@@ -578,19 +598,12 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
     void* qpack = ws;
     void* kpack = ws + plan.q_bytes;
-    void* qs = ws + plan.q_bytes + plan.k_bytes;
     CUtensorMap tQ, tK, tV, tQb, tKb;
     constexpr int BOXD = D > 64 ? 64 : D;
     constexpr int BOXR = RP ? swizzle_bytes(RP) / 2 : 16;
-    if (NQ == 2) {
-      // query operand = (hi, lo) of q*scale, laid out (B, H, Sq, 2D) in the workspace
-      if ((rc = make_tmap_4d(&tQ, qs, 2 * D, p->Sq, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sq,
-                             (int64_t)2 * D * p->Sq * p->H, BOXD, 128)))
-        return rc;
-    } else if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0],
-                                  BOXD, 128))) {
+    if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], BOXD,
+                           128)))
       return rc;
-    }
     if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], BOXD,
                            128)))
       return rc;
@@ -613,7 +626,7 @@ int launch_fwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     a.mask_tma = MODE == FWD_MASK && Cfg::MST > 0 && make_tmap_mask(&tM, p);
     // (the tensor maps above are encoded first: the host then has the main kernel's launch ready while the operand
     // preparation runs)
-    if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, qs, false, nullptr, nullptr, 0}, st))) return rc;
+    if ((rc = launch_prepare(p, plan, {qpack, kpack, nullptr, nullptr, nullptr, nullptr, 0}, st))) return rc;
     auto kern = fwd_sm100_kernel<T, D, RP, NQ, MODE>;
     // per kernel instantiation and device: raise the dynamic shared-memory limit once
     static std::mutex mu;

@@ -46,9 +46,8 @@ bool tma_compatible(const void* ptr, int64_t stride_row, int64_t stride_head, in
 // The tensor-core kernels contract over [scaled query terms | packed rank] in one fp32 accumulator.
 //   nq == 1 (softmax_scale an exact power of two): the query operand is the caller's q, the q-side factor is
 //           q_bias / scale (exact), logits = scale * S.
-//   nq == 2: the query operand is q*scale as a (hi, lo) pair of 16-bit terms, laid out (B, H, Sq, 2 TD); factors
-//           are used as given, logits = S.  (The backward splits k*scale instead: its key tile is the resident
-//           one.)
+//   nq == 2: the query operand is q*scale as a (hi, lo) pair of 16-bit terms, formed on chip; factors are used as given,
+//           logits = S.  (The backward splits k*scale instead: its key tile is the resident one.)
 // Packed factors: (Bb, Hb, S, RP) contiguous, Bb/Hb = 1 on broadcast dims, zero-padded to RP columns.
 struct PackPlan {
   int nq;          // 1 or 2 query terms
@@ -58,7 +57,7 @@ struct PackPlan {
   int RC;          // width of the centred k-side copy of the backward (>= RP; 32 beside a head_dim-32 K tile)
   bool two_stream; // backward: the two-stream kernel (its factor tiles are narrower)
   int Bq, Hq, Bk, Hk;
-  size_t q_bytes, k_bytes, kc_bytes, qs_bytes;  // packed q factor, packed k factor, centred k factor, scaled-query
+  size_t q_bytes, k_bytes, kc_bytes, qs_bytes;  // packed q factor, packed k factor, centred k factor, scaled-key
                                                // copy (each rounded to 256)
 };
 // false if the rank does not fit the tensor path; for_bwd reserves room for the centred (hi, lo) k-side copy
@@ -66,12 +65,10 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd = false);
 // a backward plan with factors, re-planned for the two-stream kernel: factor tiles as wide as the rank asks
 void plan_two_stream(const fb_params* p, PackPlan* plan);
 // What one launch prepares for a call: packed q/k factors, kcenter (optional, rows of plan.RC columns: k_bias minus the
-// k_bias of the middle key of each group of 32 keys), when plan.nq == 2 the (hi, lo) split of q*scale (forward) or
-// k*scale (backward; scaled_is_key), laid out (B, H, S, 2 TD), and for the backward delta (optional) and the zeroed
-// accumulators.
+// k_bias of the middle key of each group of 32 keys), when plan.nq == 2 the (hi, lo) split of k*scale (optional), laid out
+// (B, H, Sk, 2 TD), and for the backward delta (optional) and the zeroed accumulators.
 struct PrepBuffers {
   void *qpack, *kpack, *kcenter, *scaled;
-  bool scaled_is_key;
   float* delta;
   void* zero;
   size_t zero_bytes;

@@ -4,11 +4,11 @@
 // scale has to live inside an operand:
 //   * scale an exact power of two: qs = q (the caller's tensor, untouched) and qb = q_bias / scale,
 //     which is exact in the 16-bit type; the exponent argument is S * scale * log2(e);
-//   * otherwise: qs = q * scale, stored as a (hi, lo) pair of 16-bit terms (contraction 2*head_dim),
+//   * otherwise: qs = q * scale as a (hi, lo) pair of 16-bit terms (contraction 2*head_dim), which the forward forms on chip,
 //     and qb = q_bias as given, so that the products of the bias factors stay exact and un-scaled --
 //     terms as large as an ALiBi position cancel inside one MMA instead of being rounded first.
 // The backward keeps its key tile resident and streams the query tiles, so it puts the split on the key side
-// instead: S = q.(k*scale), with k*scale as a (hi, lo) pair.
+// instead: S = q.(k*scale), with k*scale as a (hi, lo) pair that is prepared here.
 // Factors are zero-padded to RP columns (16/32/64; the forward also takes 96 and 128).  The backward also gets a centred k-side copy
 // (k_bias minus the k_bias of the middle key of its group of 32 keys, as a (hi, lo) pair).
 #include <math.h>
@@ -39,8 +39,8 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   if (p->R <= 0) pow2 = true;
   plan->nq = pow2 ? 1 : 2;
   plan->qb_mult = (pow2 && p->R > 0) ? (float)(1.0 / (double)p->softmax_scale) : 1.f;
-  // forward: scaled-query copy; backward: scaled-key copy
-  plan->qs_bytes = pow2 ? 0 : round256((size_t)p->B * p->H * (for_bwd ? p->Sk : p->Sq) * 2 * plan->TD * 2);
+  // backward: scaled-key copy (the forward splits q*scale on chip)
+  plan->qs_bytes = pow2 || !for_bwd ? 0 : round256((size_t)p->B * p->H * p->Sk * 2 * plan->TD * 2);
   plan->RC = 0;
   plan->kc_bytes = 0;
   if (p->R <= 0) {
@@ -168,8 +168,7 @@ __device__ __forceinline__ void pack_factor_chunk(const FactorJob<T>& j, int64_t
   *reinterpret_cast<uint4*>(j.dst + row * j.W + c0) = w;
 }
 
-// qs[b][h][s][0:W] = T(x * scale), qs[b][h][s][W:2W] = T(x * scale - hi): the scaled query (or key) as two 16-bit
-// terms.
+// ks[b][h][s][0:W] = T(x * scale), ks[b][h][s][W:2W] = T(x * scale - hi): the scaled key as two 16-bit terms.
 // One thread converts 8 consecutive elements (16-byte load, two 16-byte stores).
 template <typename T>
 __device__ __forceinline__ void pack_scaled_chunk(const ScaledJob<T>& j, int64_t idx, float scale) {
@@ -231,7 +230,7 @@ __device__ __forceinline__ void delta_chunk(const DeltaJob<T>& j, int64_t idx) {
 }
 
 // Everything a call needs before its main kernel, in one launch: block ranges pack the q-side factor, the k-side
-// factor and its centred copy, split the scaled query (forward) or key (backward), take delta = rowsum(o * dout) and
+// factor and its centred copy, split the scaled key (backward), take delta = rowsum(o * dout) and
 // zero the fp32 accumulators (backward).  Three launches and a memset before; at small sizes each of them costs more in
 // launch and drain than in work.
 template <typename T>
@@ -296,12 +295,11 @@ static int launch_prepare_t(const fb_params* p, const PackPlan& plan, const Prep
   j.end_q = n += blocks_for(j.fq.units);
   j.end_k = n += blocks_for(j.fk.units);
   j.end_c = n += blocks_for(j.fc.units);
-  if (plan.nq == 2) {
+  if (plan.nq == 2 && buf.scaled) {
     ScaledJob<T>& s = j.sc;
-    const int64_t* stv = buf.scaled_is_key ? p->k_stride : p->q_stride;
-    s.src = reinterpret_cast<const T*>(buf.scaled_is_key ? p->k : p->q);
-    s.sb = stv[0]; s.sh = stv[1]; s.ss = stv[2];
-    s.S = buf.scaled_is_key ? p->Sk : p->Sq;
+    s.src = reinterpret_cast<const T*>(p->k);
+    s.sb = p->k_stride[0]; s.sh = p->k_stride[1]; s.ss = p->k_stride[2];
+    s.S = p->Sk;
     s.D = p->D; s.W = plan.TD;
     s.dst = reinterpret_cast<T*>(buf.scaled);
     s.div_w8 = Div(plan.TD / 8); s.div_s = Div(s.S); s.div_h = Div(p->H);
