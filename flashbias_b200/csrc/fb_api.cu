@@ -231,7 +231,7 @@ extern "C" size_t fb_fwd_workspace_bytes(const fb_params* p) {
   PackPlan plan;
   switch (fwd_kernel_of(p, &plan)) {
     case FB_KERNEL_FWD_ONE_QUERY: return decode_workspace(p);
-    case FB_KERNEL_FWD_TILED: return plan.q_bytes + plan.k_bytes + plan.qs_bytes;
+    case FB_KERNEL_FWD_TILED: return plan.q_bytes + plan.k_bytes;
   }
   return 0;
 }
@@ -246,7 +246,7 @@ extern "C" int fb_fwd(const fb_params* p, void* cuda_stream) {
       if ((rc = check_workspace(p, decode_workspace(p)))) return rc;
       return launch_decode(p, st);
     case FB_KERNEL_FWD_TILED:
-      if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes + plan.qs_bytes))) return rc;
+      if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes))) return rc;
       return launch_fwd_sm100(p, plan, st);
   }
   return launch_fwd_general(p, st);

@@ -48,7 +48,7 @@ struct BwdSCfg {
   static constexpr int KC_BLOCKS = RC ? (RC + D - 1) / D : 0;
   // resident: K, (hi, lo) of k*scale when the scale is not a power of two, Kb, V
   static constexpr int OFF_K = 0, OFF_KC = KT, OFF_KS = OFF_KC + KC_BLOCKS * KT, OFF_V = OFF_KS + (NQ == 2 ? 2 * KT : 0),
-                       OFF_KB = OFF_V + KT, KV_BYTES = OFF_KB + RT;
+                       OFF_KB = OFF_V + KT, KV_BYTES = OFF_KB + RT, KV_TMA_BYTES = KV_BYTES - (NQ == 2 ? KT : 0);  // (lo is computed)
   // one stage of the ring: Q, dO, Qb of 64 queries
   static constexpr int OFF_DO = tile_bytes(D, HALF), OFF_QB = 2 * OFF_DO;
   static constexpr int STAGE_BYTES = OFF_QB + (RP ? tile_bytes(RPX, HALF) : 0);
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBwdSThreads, 1)
 bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                    const __grid_constant__ CUtensorMap tmQb, const __grid_constant__ CUtensorMap tmKb,
-                   const __grid_constant__ CUtensorMap tmKc, const __grid_constant__ CUtensorMap tmKs, const BwdArgs a) {
+                   const __grid_constant__ CUtensorMap tmKc, const BwdArgs a) {
   using Cfg = BwdSCfg<D, RP, RC, NQ>;
   constexpr int RPX = Cfg::RPX, HALF = Cfg::HALF, NST = Cfg::NSTAGE;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
@@ -146,7 +146,7 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   // barriers; those of two slots belong to a stream each
   const uint32_t kv_full = bar0, all_done = bar0 + 8, dq_full = bar0 + 16, dq_drained = bar0 + 24, s_full = bar0 + 32,
                  dp_full = bar0 + 48, p_ready = bar0 + 64, ds_ready = bar0 + 80, dv_done = bar0 + 96, dk_done = bar0 + 112,
-                 full = bar0 + 128 /*6*/, free_ = bar0 + 176 /*6*/, rs_ready = bar0 + 256 /*4*/;
+                 full = bar0 + 128 /*6*/, free_ = bar0 + 176 /*6*/, rs_ready = bar0 + 256 /*4*/, ks_ready = bar0 + 288;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 232);
   const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 236;
 
@@ -181,6 +181,7 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (lane == 0) {
       st_shared_flag(abort_flag, 0u);
       mbar_init(kv_full, 1);
+      mbar_init(ks_ready, 4);  // the drain warps have split k*scale
       mbar_init(all_done, 2);  // the threads that issue into dV and into dK|dkb
       mbar_init(dq_full, 1);
       mbar_init(dq_drained, 4);  // the drain warps
@@ -203,11 +204,8 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       grid_dep_wait();
       if (n_it > 0) {
         const int hk = a.hk_bcast ? 0 : h, bk = a.bk_bcast ? 0 : b;
-        mbar_expect_tx(kv_full, Cfg::KV_BYTES);
-        if (NQ == 2) {
-          tma_tile_bwd<D>(sKs, &tmKs, kv_full, k0, h, b);
-          tma_tile_bwd<D>(sKs + Cfg::KT, &tmKs, kv_full, k0, h, b, D);
-        }
+        mbar_expect_tx(kv_full, Cfg::KV_TMA_BYTES);
+        if (NQ == 2) tma_tile_bwd<D>(sKs, &tmK, kv_full, k0, h, b);  // (split in place)
         if (RP) tma_tile_bwd<RPX>(sKb, &tmKb, kv_full, k0, hk, bk);
         tma_tile_bwd<D>(sV, &tmV, kv_full, k0, h, b);
         tma_tile_bwd<D>(sK, &tmK, kv_full, k0, h, b);
@@ -279,6 +277,7 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                        kK = kmajor_base<D>(NQ == 2 ? sKs : sK), kKb = kmajor_base<RPX>(sKb), kV = kmajor_base<D>(sV),
                        kDO = kmajor_base<D, HALF>(sStage + Cfg::OFF_DO);
         mbar_wait(kv_full, 0, abort_flag);
+        if (NQ == 2) mbar_wait(ks_ready, 0, abort_flag);
 #pragma unroll 1
         for (int x = 0; x < n_half; ++x) {
           const int w = x & 1, n = x >> 1, st = x % NST;
@@ -375,6 +374,11 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
       const int bq = a.bq_bcast ? 0 : b, hq = a.hq_bcast ? 0 : h;
+      if (NQ == 2) {
+        mbar_wait(kv_full, 0, abort_flag);
+        split_scaled_row<T, D>(sKs, row, a.k_scale);
+        mbar_arrive_warp(ks_ready);
+      }
       if (RP) {
         // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32: [column pair][key group][2]
         float* s_kbc = reinterpret_cast<float*>(smem + Cfg::OFF_KBC);
@@ -670,8 +674,8 @@ int launch_bwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   int rc;
   const BwdWs w = bwd_layout(p, plan);
   uint8_t* ws = reinterpret_cast<uint8_t*>(p->workspace);
-  void *qpack = ws + w.off_qpack, *kpack = ws + w.off_kpack, *kcenter = ws + w.off_kcenter, *ks = ws + w.off_qs;
-  CUtensorMap tQ, tK, tV, tDO, tQb, tKb, tKc, tKs;
+  void *qpack = ws + w.off_qpack, *kpack = ws + w.off_kpack, *kcenter = ws + w.off_kcenter;
+  CUtensorMap tQ, tK, tV, tDO, tQb, tKb, tKc;
   if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, Cfg::HALF)))
     return rc;
   if ((rc = make_tmap_4d(&tDO, p->dout, p->D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1], p->dout_stride[0],
@@ -681,12 +685,7 @@ int launch_bwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
     return rc;
   if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], D, 128)))
     return rc;
-  tKs = tQb = tKb = tKc = tK;
-  if (NQ == 2) {  // (hi, lo) of k*scale, laid out (B, H, Sk, 2D) in the workspace
-    if ((rc = make_tmap_4d(&tKs, ks, 2 * D, p->Sk, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sk, (int64_t)2 * D * p->Sk * p->H,
-                           D, 128)))
-      return rc;
-  }
+  tQb = tKb = tKc = tK;
   if (RP) {
     if ((rc = make_tmap_4d(&tQb, qpack, RP, p->Sq, plan.Hq, plan.Bq, RP, (int64_t)RP * p->Sq, (int64_t)RP * p->Sq * plan.Hq,
                            Cfg::RPX, Cfg::HALF)))
@@ -713,12 +712,12 @@ int launch_bwd_s(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
       attr_done[dev & 63] = true;
     }
   }
-  if ((rc = launch_prepare(p, plan, {qpack, kpack, RP ? kcenter : nullptr, ks, fused_delta(p), ws + w.off_dq, w.zero_bytes},
+  if ((rc = launch_prepare(p, plan, {qpack, kpack, RP ? kcenter : nullptr, nullptr, fused_delta(p), ws + w.off_dq, w.zero_bytes},
                            st)))
     return rc;
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);
   prof_before(KC_BWD_MAIN, st);
-  rc = launch_pdl(kern, grid, kBwdSThreads, Cfg::SMEM, st, tQ, tK, tV, tDO, tQb, tKb, tKc, tKs, a);
+  rc = launch_pdl(kern, grid, kBwdSThreads, Cfg::SMEM, st, tQ, tK, tV, tDO, tQb, tKb, tKc, a);
   prof_after(KC_BWD_MAIN, st);
   if (rc) return rc;
   return launch_store_grads(p, {a.dq_acc, DQ_SWIZZLED, D, a.dqb_acc, a.dkb_acc,

@@ -48,6 +48,7 @@ bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->dv && !rows_16b_ok(p->dv, p->dv_stride)) return false;
   if ((int64_t)p->B * p->H * ((p->Sk + 127) / 128) > 0x7fffffffLL) return false;
   if (takes_two_stream(p, *plan)) plan_two_stream(p, plan);
+  if (plan->two_stream || bwd_sm100_form(p, *plan) != FB_KERNEL_BWD_PERSISTENT) plan->qs_bytes = 0;  // k*scale is split on chip
   return true;
 }
 

@@ -36,6 +36,7 @@ struct BwdArgs {
   int B, H, Sq, Sk, D, nq_tiles, nk_tiles, causal, R;  // D <= the tile's head_dim (columns beyond it are zeros)
   int hq_bcast, bq_bcast, hk_bcast, bk_bcast;
   int Hq, Hk;  // head extents of the un-expanded factors
+  float k_scale;     // multiplies k where it is split
   float dk_scale;    // applied to dK on store
   float dkb_scale;   // applied to dk_bias on store
   float scale_log2;  // logits * log2(e) = S * scale_log2
@@ -89,7 +90,7 @@ struct BwdCfg {
   static constexpr int OFF_KB = OFF_KS + (NQ == 2 ? 2 * D_BYTES : 0);
   static constexpr int OFF_KC = OFF_KB + R_BYTES;  // centred k_bias tile (dq_bias only)
   static constexpr int OFF_V = OFF_KC + RC_BYTES;
-  static constexpr int KV_BYTES = OFF_V + D_BYTES;
+  static constexpr int KV_BYTES = OFF_V + D_BYTES, KV_TMA_BYTES = KV_BYTES - (NQ == 2 ? D_BYTES : 0);  // (lo is computed)
   static constexpr int OFF_STAGE = KV_BYTES;
   static constexpr int TAIL_BYTES = 256 + 8192 + 4 * RCX * 4 + 1024;  // barriers, row sums, centre keys, alignment
   // P and dS buffers: the compute warps keep the 16-bit P and dS of a query tile in registers until the tile's
@@ -136,6 +137,19 @@ __device__ __forceinline__ void tma_tile_bwd(uint32_t dst, const CUtensorMap* m,
   constexpr int NB = C * 2 / SWB;
 #pragma unroll
   for (int blk = 0; blk < NB; ++blk) tma_load_4d(dst + blk * ROWS * SWB, m, bar, col0 + blk * (SWB / 2), row0, h, b);
+}
+
+// Row `row` of a [128][D] tile, times scale, as a (hi, lo) pair: hi in place, lo in the tile behind; ready for the tensor core.
+// (The persistent form reads k*scale split by a pass ahead of it: short items wait for the split between their tiles, B512 H24
+// S144 R8 996 instead of 701 us, which is more than the pass takes.)
+template <typename T, int D>
+__device__ __forceinline__ void split_scaled_row(uint32_t tile, int row, float scale) {
+#pragma unroll
+  for (int c = 0; c < D / 8; ++c) {
+    const uint32_t at = tile + tile_chunk_offset<D>(row, 8 * c);
+    split_scaled_chunk<T>(at, at + tile_bytes(D), scale);
+  }
+  fence_proxy_async_smem();
 }
 
 __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
@@ -213,8 +227,7 @@ __global__ void __launch_bounds__(512, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                  const __grid_constant__ CUtensorMap tmQb, const __grid_constant__ CUtensorMap tmKb,
-                 const __grid_constant__ CUtensorMap tmKc, const __grid_constant__ CUtensorMap tmKs,
-                 const BwdArgs a) {
+                 const __grid_constant__ CUtensorMap tmKc, const BwdArgs a) {
   using Cfg = BwdCfg<D, RP, NQ>;
   constexpr int RPX = Cfg::RPX;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
@@ -231,7 +244,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t kv_full = bar0, dp_full = bar0 + 16, sdp_read = bar0 + 24,
                  dq_full = bar0 + 32 /*2*/, qdo_full = bar0 + 48 /*3*/, qdo_free = bar0 + 72 /*3*/,
                  all_done = bar0 + 112, pds_free = bar0 + 120, pds_ready = bar0 + 136 /*2*/,
-                 dq_drained = bar0 + 152 /*2*/;
+                 dq_drained = bar0 + 152 /*2*/, ks_ready = bar0 + 168;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 96);
   const uint32_t abort_flag = sbase + Cfg::OFF_BAR + 104;
 
@@ -266,6 +279,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (lane == 0) {
       st_shared_flag(abort_flag, 0u);
       mbar_init(kv_full, 1);
+      mbar_init(ks_ready, 4);  // the drain warps have split k*scale
       mbar_init(dp_full, 1);
       mbar_init(sdp_read, 8);  // every compute warp has S and dP of the tile in registers
       mbar_init(all_done, 4);  // one commit per issuing thread
@@ -286,12 +300,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (n_it > 0) {
         // the first loads start before the rest of the CTA has finished its set-up
         const int hk = a.hk_bcast ? 0 : h, bk = a.bk_bcast ? 0 : b;
-        mbar_expect_tx(kv_full, Cfg::KV_BYTES);
+        mbar_expect_tx(kv_full, Cfg::KV_TMA_BYTES);
         tma_tile_bwd<D>(sK, &tmK, kv_full, k0, h, b);
-        if (NQ == 2) {
-          tma_tile_bwd<D>(sKs, &tmKs, kv_full, k0, h, b);
-          tma_tile_bwd<D>(sKs + Cfg::D_BYTES, &tmKs, kv_full, k0, h, b, D);
-        }
+        if (NQ == 2) tma_tile_bwd<D>(sKs, &tmK, kv_full, k0, h, b);  // (split in place)
         if (RP) tma_tile_bwd<RPX>(sKb, &tmKb, kv_full, k0, hk, bk);
         tma_tile_bwd<D>(sV, &tmV, kv_full, k0, h, b);
         load_tile(0);
@@ -379,6 +390,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_wait(kv_full, 0, abort_flag);
       tc_fence_after_sync();
       if (role == 0) {
+        if (NQ == 2) {
+          mbar_wait(ks_ready, 0, abort_flag);
+          tc_fence_after_sync();
+        }
         // descriptor views built once (stage 0); each MMA adds a constant to the address field
         const DescBase kQ = kmajor_base<D>(sStage), kDO = kmajor_base<D>(sStage + Cfg::OFF_DO),
                        kQb = kmajor_base<RPX>(sStage + Cfg::OFF_QB), kK = kmajor_base<D>(NQ == 2 ? sKs : sK),
@@ -481,6 +496,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (n_it > 0) {
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+      if (NQ == 2) {
+        mbar_wait(kv_full, 0, abort_flag);
+        split_scaled_row<T, D>(sKs, row, a.k_scale);
+        mbar_arrive_warp(ks_ready);
+      }
 #pragma unroll 1
       for (int it = 0; it < n_it; ++it) {
         const int grow = (i_begin + it) * 128 + row;
@@ -859,6 +879,7 @@ inline BwdArgs bwd_args(const fb_params* p, const PackPlan& plan, const BwdWs& w
   a.hq_bcast = plan.Hq == 1; a.bq_bcast = plan.Bq == 1; a.hk_bcast = plan.Hk == 1; a.bk_bcast = plan.Bk == 1;
   a.Hq = plan.Hq; a.Hk = plan.Hk;
   // with a split key operand the scale is already inside S
+  a.k_scale = p->softmax_scale;
   a.dk_scale = p->softmax_scale;                     // dK accumulates dS^T.q
   a.dkb_scale = plan.nq == 2 ? 1.f : p->softmax_scale;    // the packed q-side factor carries 1/scale when nq == 1
   a.scale_log2 = (plan.nq == 2 ? 1.f : p->softmax_scale) * 1.4426950408889634f;
@@ -911,16 +932,13 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
   CUtensorMap &tQ = L.tQ, &tK = L.tK, &tV = L.tV, &tDO = L.tDO, &tQb = L.tQb, &tKb = L.tKb, &tKc = L.tKc, &tKs = L.tKs;
   if ((rc = make_tmap_4d(&tQ, p->q, p->D, p->Sq, p->H, p->B, p->q_stride[2], p->q_stride[1], p->q_stride[0], D, 128)))
     return rc;
-  if (NQ == 2) {
-    // key operand of S = (hi, lo) of k*scale, laid out (B, H, Sk, 2D) in the workspace
-    void* ks = ws + w.off_qs;
-    if ((rc = make_tmap_4d(&tKs, ks, 2 * D, p->Sk, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sk,
-                           (int64_t)2 * D * p->Sk * p->H, D, 128)))
-      return rc;
-  }
   if ((rc = make_tmap_4d(&tK, p->k, p->D, p->Sk, p->H, p->B, p->k_stride[2], p->k_stride[1], p->k_stride[0], D, 128)))
     return rc;
-  if (NQ != 2) tKs = tK;
+  tKs = tK;
+  void* ks = plan.qs_bytes ? ws + w.off_qs : nullptr;  // persistent form: (hi, lo) of k*scale, laid out (B, H, Sk, 2D)
+  if (ks && (rc = make_tmap_4d(&tKs, ks, 2 * D, p->Sk, p->H, p->B, 2 * D, (int64_t)2 * D * p->Sk,
+                               (int64_t)2 * D * p->Sk * p->H, D, 128)))
+    return rc;
   if ((rc = make_tmap_4d(&tV, p->v, p->D, p->Sk, p->H, p->B, p->v_stride[2], p->v_stride[1], p->v_stride[0], D, 128)))
     return rc;
   if ((rc = make_tmap_4d(&tDO, p->dout, p->D, p->Sq, p->H, p->B, p->dout_stride[2], p->dout_stride[1],
@@ -944,7 +962,7 @@ int bwd_prepare(const fb_params* p, const PackPlan& plan, cudaStream_t st, BwdLa
   }
   L.a = bwd_args(p, plan, w);
   // launches last: the tensor maps and arguments above are ready when the main kernel's turn comes
-  return launch_prepare(p, plan, {qpack, kpack, kcenter, ws + w.off_qs, fused_delta(p), ws + w.off_dq, w.zero_bytes},
+  return launch_prepare(p, plan, {qpack, kpack, kcenter, ks, fused_delta(p), ws + w.off_dq, w.zero_bytes},
                         st);
 }
 
@@ -986,7 +1004,7 @@ int launch_bwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   }
   const unsigned grid = (unsigned)((int64_t)a.nk_tiles * p->B * p->H);
   prof_before(KC_BWD_MAIN, st);
-  rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, L.tKs, a);
+  rc = launch_pdl(kern, grid, 512, Cfg::SMEM, st, L.tQ, L.tK, L.tV, L.tDO, L.tQb, L.tKb, L.tKc, a);
   prof_after(KC_BWD_MAIN, st);
   if (rc) return rc;
   return bwd_finish<T, D, RP, NQ>(p, L, st);

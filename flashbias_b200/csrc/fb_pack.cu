@@ -8,7 +8,7 @@
 //     and qb = q_bias as given, so that the products of the bias factors stay exact and un-scaled --
 //     terms as large as an ALiBi position cancel inside one MMA instead of being rounded first.
 // The backward keeps its key tile resident and streams the query tiles, so it puts the split on the key side
-// instead: S = q.(k*scale), with k*scale as a (hi, lo) pair that is prepared here.
+// instead: S = q.(k*scale), with k*scale as a (hi, lo) pair, formed on chip as well, or here for the persistent form.
 // Factors are zero-padded to RP columns (16/32/64; the forward also takes 96 and 128).  The backward also gets a centred k-side copy
 // (k_bias minus the k_bias of the middle key of its group of 32 keys, as a (hi, lo) pair).
 #include <math.h>
@@ -39,7 +39,7 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   if (p->R <= 0) pow2 = true;
   plan->nq = pow2 ? 1 : 2;
   plan->qb_mult = (pow2 && p->R > 0) ? (float)(1.0 / (double)p->softmax_scale) : 1.f;
-  // backward: scaled-key copy (the forward splits q*scale on chip)
+  // persistent backward: scaled-key copy (the other kernels split q*scale or k*scale on chip)
   plan->qs_bytes = pow2 || !for_bwd ? 0 : round256((size_t)p->B * p->H * p->Sk * 2 * plan->TD * 2);
   plan->RC = 0;
   plan->kc_bytes = 0;
