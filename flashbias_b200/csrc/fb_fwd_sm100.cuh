@@ -140,10 +140,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   struct Item {
     int bh, b, h, q0, n_kv;
     // First key of the j-th key tile visited.  Under causal masking from the diagonal down: a bias that falls with the distance
-    // (ALiBi) then shows its maximum first, and O is hardly ever rescaled (B1 H50 S8192 D32 R2: 610 -> 588 us).  Masks come in
-    // ascending order through their ring.
+    // (ALiBi) then shows its maximum first, and O is hardly ever rescaled.  Not with factor operands, where it would take 23 of
+    // 611 us (B1 H50 S8192 D32 R2): the order decides against which maximum P is rounded, so o moves within its rounding
+    // (1.2e-3), and dq_bias, which cancels down to that rounding where factors are as large as ALiBi's, by 40 %.  Masks come
+    // in ascending order through their ring.
     __device__ __forceinline__ int key0(int j, int causal) const {
-      return (MODE != FWD_MASK && causal ? n_kv - 1 - j : j) * 128;
+      return (RP == 0 && MODE != FWD_MASK && causal ? n_kv - 1 - j : j) * 128;
     }
   };
   // The w-th work item of this CTA.  Items are ordered heaviest first (causal); the CTAs take them in snake order

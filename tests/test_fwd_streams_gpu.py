@@ -57,3 +57,18 @@ def test_edges(case):
         assert (lse[..., :Sq].cpu().double() - lse_ref.double().reshape(B, H, -1)[..., :Sq]).abs().max() < 2e-5
     for _ in range(20):
         assert torch.equal(run()[0], o)
+
+
+@pytest.mark.parametrize("D", [32, 64])
+def test_causal_visits_keys_in_ascending_order_with_factors(D):
+    """The last query sees every key with and without causal masking: the same tiles in the same order give the same bits.  (In
+    another order P is rounded against another maximum; o then moves within its rounding, and an ALiBi dq_bias by 40 %.)"""
+    B, H, S = 1, 8, 900
+    g = torch.Generator().manual_seed(D)
+    q, k, v = (torch.randn(B, S, H, D, generator=g).to(BF).cuda() for _ in range(3))
+    m, i = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)]), torch.arange(S).float()
+    one = torch.ones(S, H)
+    qb = torch.stack([-(m[None] * i[:, None]), one], dim=-1)[None].to(BF).cuda()
+    kb = torch.stack([one, m[None] * i[:, None]], dim=-1)[None].to(BF).cuda()
+    run = lambda causal: flash_bias_forward(q, k, v, qb, kb, None, causal, 1.0 / math.sqrt(D))[0]
+    assert torch.equal(run(True)[:, -1], run(False)[:, -1])
