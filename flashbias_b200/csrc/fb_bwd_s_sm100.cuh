@@ -27,8 +27,8 @@
 // threads have read this one's (dS^T in columns of its own: behind the dK product they came 1400 clk later); satisfied waits
 // tested ahead of use (85 to 290 clk each); the next S^T loaded under the row sums.  Sixteen compute warps of 32 x 32 took
 // the same time (8000 instead of 6100 instructions a tile).
-// Backward kernel, query-major form / this one, us: B2 H8 S32768 D64 R5 16300 / 13900, B1 H16 S1536 D32 R32 114 / 66, B1 H16
-// S743 D24 R8 21.0 / 18.6, B1 H50 S8192 D32 R2 causal 1277 / 1198.
+// Backward kernel, query-major form / this one, us: B2 H8 S32768 D64 R5 16300 / 13900, B1 H16 S1536 D32 R32 112 / 68, B1 H16
+// S743 D24 R8 20.5 / 18.5, B1 H50 S8192 D32 R2 causal 1277 / 1180.
 #pragma once
 
 #include "fb_bwd_sm100.cuh"

@@ -40,9 +40,10 @@ extern "C" {
 /* flags */
 #define FB_FLAG_FORCE_GENERAL 1 /* use the shape-generic CUDA-core kernels even where the tensor-core path applies */
 #define FB_FLAG_BWD_QUERY_MAJOR 2 /* backward without factor operands at head_dim 32: use the query-major tensor-core
-                                     kernel instead of the key-major one (cross-checks; same results up to rounding) */
+                                     kernel instead of the two-stream one, or with a mask the key-major one (cross-checks;
+                                     same results up to rounding) */
 #define FB_FLAG_BWD_ONE_ITEM 4   /* backward with factor operands at head_dim 32: one work item (128 keys of a (batch,
-                                     head)) per CTA, whatever the shape */
+                                     head)) per CTA, thread = query row, whatever the shape */
 #define FB_FLAG_BWD_PERSISTENT 8 /* ... one persistent CTA per SM walking the work items, whatever the shape (by
                                      default: chosen when a work item has few query tiles) */
 #define FB_FLAG_BWD_FUSED_DELTA 16 /* fb_bwd takes delta itself, in the launch that prepares its operands: no
