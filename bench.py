@@ -70,9 +70,9 @@ CPU_SAMPLE = {
 # number of (batch, head, row) units - the tiles a CTA re-streams (Q, dO per key tile) are served by L2 at both
 # sizes, so DRAM traffic grows with the rows, not with the tile pairs
 NCU_BWD_TRAFFIC_BYTES = {
-    "alibi": (47.78e6 + 0.379e6) * (50 * 8192) / (16 * 4096),
-    "swin": (826.6e6 + 370.3e6) * 4096 / 256,
-    "pde": 27.62e6 * (2 * 8 * 32768) / (4 * 8192),
+    "alibi": 47.99e6 * (50 * 8192) / (16 * 4096),
+    "swin": 1197.6e6 * 4096 / 256,
+    "pde": 27.61e6 * (2 * 8 * 32768) / (4 * 8192),
 }
 
 
