@@ -257,7 +257,10 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           float nl = -INFINITY;
           if (lse_raw[e] != -INFINITY) {
             nl = -lse_raw[e] * kLog2e;
-            if (MODE == BWD_ALIBI) nl -= slope2 * (float)(i_begin * 128 + x * HALF + lane + 32 * e);
+            // The term slope * (key - query) is counted from the half tile's first query on either side (the keys' share: ak).
+            // Counted from query 0, two large numbers would cancel near the diagonal, and P lose a bit for every doubling of
+            // the position (fp16, slope 0.9, S 65536: gradients 1.9e-3 from 64 bits instead of 3e-4).
+            if (MODE == BWD_ALIBI) nl -= slope2 * (float)(lane + 32 * e);
           }
           const uint32_t at = sStat + st * Cfg::STAT + (lane + 32 * e) * 4;
           st_shared_f32(at, nl);
@@ -439,12 +442,7 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    tP = tmem + Cfg::T_P + w * Cfg::P_STRIDE + lane_off, tDS = tmem + Cfg::T_DS + lane_off;
     const float sl2 = a.scale_log2;
     const int krow = wl * 32 + (lane >> 2), qcol = 2 * (lane & 3);  // first key and query of the thread's fragment
-    uint64_t ak[4];  // ALiBi: the keys' share of the term
-    if (MODE == BWD_ALIBI) {
-      const float slope2 = __ldg(a.alibi_slopes + h) * kLog2e;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ak[k] = f2(slope2 * (float)(k0 + krow + 8 * k), slope2 * (float)(k0 + krow + 8 * k));
-    }
+    const float slope2 = MODE == BWD_ALIBI ? __ldg(a.alibi_slopes + h) * kLog2e : 0.f;
     const uint64_t sl2p = f2(sl2, sl2);
     int stg = w;  // ring stage of the half tile
     // stmatrix addresses in the stream's [128 keys][64 queries] half of the dS^T tile (128-byte lines, swizzled): lane l
@@ -465,7 +463,14 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t st_n = sStat + stg * Cfg::STAT + qcol * 4;  // its statistics, from the thread's first query on
       stg = stg + 2 >= NST ? stg + 2 - NST : stg + 2;
       // s[k2][4j + 2i + e]: key krow + 16 k2 + 8 i, query qcol + 8 j + e
-      uint64_t nl[8];
+      uint64_t nl[8], ak[4];  // ALiBi: ak, the keys' share of the term
+      if (MODE == BWD_ALIBI) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float x = slope2 * (float)(k0 + krow + 8 * k - q0);
+          ak[k] = f2(x, x);
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) nl[j] = ld_shared_f2(st_n + j * 32);
       const bool dp_ok = mbar_test_wait(dp_full + 8 * w, n & 1);

@@ -67,6 +67,30 @@ def test_edges(case):
         check_close("streams/Sq%dSk%dD%dR%d/%s" % (Sq, Sk, D, R, name), got, ref, dtype)
 
 
+@pytest.mark.parametrize("D", [32, 64])
+def test_slopes_far_from_the_first_query(D):
+    """The slopes' term counted from query 0 is a difference of two numbers as large as the position: at 65500 and slope 0.9 their
+    fp32 rounding alone moves P by 1e-3 in the mean.  The last queries' dq, and dk and dv of the last keys, which no other query
+    sees, against 64 bits."""
+    S, H, n = 65500, 2, 96
+    g = torch.Generator().manual_seed(D)
+    q, k, v, do = (torch.randn(1, S, H, D, generator=g).to(HF) for _ in range(4))
+    m = torch.tensor([0.9, 0.5])
+    leaves = [t.cuda().requires_grad_(True) for t in (q, k, v)]
+    o = flash_bias_alibi_func(*leaves, m.cuda(), True)
+    grads = torch.autograd.grad(o, leaves, do.cuda())
+    torch.cuda.synchronize()
+    check_device_status()
+    i, j = torch.arange(S - n, S).double()[:, None], torch.arange(S).double()[None]
+    bias = torch.where(j > i, -math.inf, m.double()[:, None, None] * (j - i))[None]
+    last = [q[:, -n:], k, v]
+    o_ref, lse_ref = orc.attention_forward(*last, None, None, bias, False, dtype=torch.float64)
+    check_close("streams/far_D%d/o" % D, o[:, -n:], o_ref, HF)
+    want = orc.attention_backward(do[:, -n:], *last, o[:, -n:].detach().cpu(), lse_ref, None, None, bias, False, dtype=torch.float64)
+    for name, got, ref in zip(("dq", "dk", "dv"), grads, want):
+        check_close("streams/far_D%d/%s" % (D, name), got[:, -n:], ref[:, -n:], HF)
+
+
 # (both dS^T tiles; one dS^T tile; P^T in the place of S^T)
 @pytest.mark.parametrize("case", [(2, 8, 1000, 1000, 32, 8, True, None, BF, False), (2, 8, 777, 777, 64, 5, False, 0.1, BF, False),
                                   (1, 16, 900, 900, 32, 30, False, None, BF, False)], ids=lambda c: "D%dR%d" % (c[4], c[5]))
