@@ -67,7 +67,7 @@ def test_edges(case):
         check_close("streams/Sq%dSk%dD%dR%d/%s" % (Sq, Sk, D, R, name), got, ref, dtype)
 
 
-@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("D", [32, 64, 128])
 def test_slopes_far_from_the_first_query(D):
     """The slopes' term counted from query 0 is a difference of two numbers as large as the position: at 65500 and slope 0.9 their
     fp32 rounding alone moves P by 1e-3 in the mean.  The last queries' dq, and dk and dv of the last keys, which no other query
