@@ -28,7 +28,10 @@ struct FwdSCfg {
   static constexpr int TAIL = 256 + 2 * 2 * 128 * 8 + 2 * 128 * 4 + 1024;
   static constexpr int LIM = 227 * 1024;
   static constexpr int smem_for(int st) { return NQ * Q_BYTES + QB_BYTES + st * (2 * Q_BYTES + QB_BYTES) + TAIL; }
-  static constexpr int ST = smem_for(3) <= LIM ? 3 : 2;  // stages of K | Kb and of V
+  // Stages of K | Kb and of V.  Two, and not only because three do not fit: the wait for the other stream's last product ahead of a
+  // rescale relies on it.
+  static constexpr int ST = 2;
+  static_assert(smem_for(3) > LIM, "a third stage would fit");
   static constexpr int SMEM = smem_for(ST);
   static constexpr bool FITS = SMEM <= LIM;
   static constexpr int OFF_QB = NQ * Q_BYTES, OFF_K = OFF_QB + QB_BYTES, OFF_KB = OFF_K + ST * Q_BYTES,
@@ -52,12 +55,12 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t sQ = sbase, sQb = sbase + Cfg::OFF_QB, sK = sbase + Cfg::OFF_K, sKb = sbase + Cfg::OFF_KB,
                  sV = sbase + Cfg::OFF_V;
   const uint32_t bar0 = sbase + Cfg::OFF_BAR;
-  // (two slots: one per stream)
+  // (two slots: one per stream, or per stage)
   const uint32_t q_full = bar0, q_free = bar0 + 8, o_free = bar0 + 16, s_full = bar0 + 24, p_ready = bar0 + 40,
-                 pv_done = bar0 + 56, k_full = bar0 + 72 /*3*/, k_free = bar0 + 96 /*3*/, v_full = bar0 + 120 /*3*/,
-                 v_free = bar0 + 144 /*3*/, s_read = bar0 + 176, q_ready = bar0 + 192;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 168);
-  const uint32_t abort_flag = bar0 + 172;
+                 pv_done = bar0 + 56, k_full = bar0 + 72, k_free = bar0 + 88, v_full = bar0 + 104, v_free = bar0 + 120,
+                 s_read = bar0 + 136, q_ready = bar0 + 152;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::OFF_BAR + 160);
+  const uint32_t abort_flag = bar0 + 164;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BH = a.B * a.H;
@@ -297,7 +300,11 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           m_used = __uint_as_float(ld_shared_flag(m_other));
           const float m_new = fmaxf(m_used, mx);
           if (__any_sync(0xffffffffu, m_new - m_used > 8.f)) {
-            mbar_wait(pv_done + 8 * (x ^ 1), (co0 + ((j - 1) >> 1)) & 1, abort_flag);  // O is stable
+            // O is stable behind the product of tile j - 1.  The wait tests a parity, so the other stream's product before it, tile
+            // j - 3, must be known to have completed (or its phase would pass for this one): tile j's logits are here, K(j) was
+            // loaded behind V(j - 1), and V(j - 1), in a ring of two, where V(j - 3) had been, behind that product.
+            static_assert(ST == 2, "a deeper ring does not order the products of tiles j - 3 and j");
+            mbar_wait(pv_done + 8 * (x ^ 1), (co0 + ((j - 1) >> 1)) & 1, abort_flag);
             tc_fence_after_sync();
             const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m_used - m_new);
             m_used = m_new;
@@ -350,12 +357,13 @@ fwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_arrive_warp(p_ready + 8 * x);
       }
       if (NQ == 2 && item_index(w + 1) < a.total_items) split_q();
-      // ---- epilogue: O / l -> global, this warpgroup's half of the columns; lse.  (The last product's commit covers the ones
-      // before it, which the same thread issued.)
+      // ---- epilogue: O / l -> global, this warpgroup's half of the columns; lse.  The stream of the last tile knows its product
+      // to have completed (its commit covers the ones before it, which the same thread issued); the other learns it from the
+      // warpgroups' barrier.
       c = c0 + ((it.n_kv + 1 - x) >> 1);
       co = co0 + ((it.n_kv + x) >> 1);
       const int xl = (it.n_kv - 1) & 1;  // stream of the last tile
-      mbar_wait(pv_done + 8 * xl, ((xl == x ? c : co) - 1) & 1, abort_flag);
+      if (xl == x) mbar_wait(pv_done + 8 * x, (c - 1) & 1, abort_flag);
       float2* ml = reinterpret_cast<float2*>(smem + Cfg::OFF_ML) + (n & 1) * 256;
       ml[x * 128 + row] = make_float2(m_used, l);
       asm volatile("bar.sync 1, 256;" ::: "memory");  // both warpgroups

@@ -59,6 +59,28 @@ def test_edges(case):
         assert torch.equal(run()[0], o)
 
 
+@pytest.mark.parametrize("tiles", [(2,), (3,), (3, 4), (2, 6), (5, 6)], ids=str)
+def test_rescale_behind_tiles_without_one(tiles):
+    """One key of each named tile raises the running maximum of every row by 2^20 or more, behind tiles that leave it alone: the
+    accumulator is rescaled while the products of the tiles before may still be on their way into it."""
+    B, H, Sq, Sk, D = 2, 40, 256, 7 * 128, 128  # more items than SMs
+    g = torch.Generator().manual_seed(sum(tiles))
+    q, k, v = (torch.randn(B, S, H, D, generator=g).to(BF) for S in (Sq, Sk, Sk))
+    q[..., 0], k[..., 0] = 4.0, 0.0
+    for n, t in enumerate(tiles):
+        k[:, 128 * t + 77, :, 0] = 60.0 * (n + 1)  # a logit of 21 (n + 1); the others are N(0, 1)
+    scale = 1.0 / math.sqrt(D)
+    dev = [t.cuda() for t in (q, k, v)]
+    run = lambda: flash_bias_forward(*dev, None, None, None, False, scale)[0]
+    o = run()
+    torch.cuda.synchronize()
+    check_device_status()
+    o_ref, _ = orc.attention_forward(q[:1, :, :8], k[:1, :, :8], v[:1, :, :8], None, None, None, False, scale, dtype=torch.float64)
+    check_close("fwd_streams/rescale%s" % (tiles,), o[:1, :, :8], o_ref, BF)
+    for _ in range(20):
+        assert torch.equal(run(), o)
+
+
 @pytest.mark.parametrize("D", [32, 64])
 def test_causal_visits_keys_in_ascending_order_with_factors(D):
     """The last query sees every key with and without causal masking: the same tiles in the same order give the same bits.  (In
