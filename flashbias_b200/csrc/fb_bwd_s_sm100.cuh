@@ -248,7 +248,8 @@ bwd_s_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int x = 0; x < n_half; ++x) {
         const int st = x % NST;
         if (x >= NST) {
-          if (!mbar_wait(free_ + 8 * st, (x / NST - 1) & 1, abort_flag)) break;
+          // (the whole warp waits here, and leaves together: each lane polls for itself, and may see another end of an expired wait)
+          if (!__all_sync(0xffffffffu, mbar_wait(free_ + 8 * st, (x / NST - 1) & 1, abort_flag))) break;
           if (elect_one()) load_half(x);
           __syncwarp();
         }
