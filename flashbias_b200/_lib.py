@@ -19,7 +19,8 @@ FB_FLAG_BWD_QUERY_MAJOR = 2
 FB_FLAG_BWD_ONE_ITEM = 4
 FB_FLAG_BWD_PERSISTENT = 8
 FB_FLAG_BWD_FUSED_DELTA = 16
-KERNELS = ("general", "fwd_tiled", "fwd_one_query", "bwd_query_major", "bwd_persistent", "bwd_key_major")  # FB_KERNEL_*
+KERNELS = ("general", "fwd_tiled", "fwd_one_query", "bwd_query_major", "bwd_persistent", "bwd_key_major", "bwd_two_stream",
+           "fwd_two_stream")  # FB_KERNEL_*
 
 I64x3 = C.c_int64 * 3
 

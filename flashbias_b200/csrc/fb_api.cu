@@ -193,10 +193,10 @@ extern "C" int fb_read_status(const int32_t* status, int32_t* value, void* cuda_
 // The kernel a valid problem takes: the one place that decides it, for the launches, the workspace sizes and the queries.
 static int fwd_kernel_of(const fb_params* p, PackPlan* plan) {
   if (decode_supported(p)) return FB_KERNEL_FWD_ONE_QUERY;
-  return fwd_sm100_supported(p, plan) ? FB_KERNEL_FWD_TILED : FB_KERNEL_GENERAL;
+  return fwd_sm100_supported(p, plan) ? plan->kernel : FB_KERNEL_GENERAL;
 }
 static int bwd_kernel_of(const fb_params* p, PackPlan* plan) {
-  return bwd_sm100_supported(p, plan) ? bwd_sm100_form(p, *plan) : FB_KERNEL_GENERAL;
+  return bwd_sm100_supported(p, plan) ? plan->kernel : FB_KERNEL_GENERAL;
 }
 
 extern "C" int fb_fwd_kernel(const fb_params* p) {
@@ -231,7 +231,8 @@ extern "C" size_t fb_fwd_workspace_bytes(const fb_params* p) {
   PackPlan plan;
   switch (fwd_kernel_of(p, &plan)) {
     case FB_KERNEL_FWD_ONE_QUERY: return decode_workspace(p);
-    case FB_KERNEL_FWD_TILED: return plan.q_bytes + plan.k_bytes;
+    case FB_KERNEL_FWD_TILED:
+    case FB_KERNEL_FWD_TWO_STREAM: return plan.q_bytes + plan.k_bytes;
   }
   return 0;
 }
@@ -246,6 +247,7 @@ extern "C" int fb_fwd(const fb_params* p, void* cuda_stream) {
       if ((rc = check_workspace(p, decode_workspace(p)))) return rc;
       return launch_decode(p, st);
     case FB_KERNEL_FWD_TILED:
+    case FB_KERNEL_FWD_TWO_STREAM:
       if ((rc = check_workspace(p, plan.q_bytes + plan.k_bytes))) return rc;
       return launch_fwd_sm100(p, plan, st);
   }

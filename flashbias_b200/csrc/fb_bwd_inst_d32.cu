@@ -8,7 +8,7 @@ static int dispatch_rank(const fb_params* p, const PackPlan& plan, cudaStream_t 
   switch (plan.RP) {
     case 0:  // (without a mask: the two-stream kernel, unless the caller asks for the query-major form)
       if constexpr (MODE == BWD_MASK)
-        if (bwd_sm100_form(p, plan) == FB_KERNEL_BWD_KEY_MAJOR) return launch_bwd_t_t<T, 32, MODE>(p, plan, st);
+        if (plan.kernel == FB_KERNEL_BWD_KEY_MAJOR) return launch_bwd_t_t<T, 32, MODE>(p, plan, st);
       return launch_bwd_t<T, 32, 0, 1, MODE>(p, plan, st);
     case 16: return plan.nq == 2 ? launch_bwd_t<T, 32, 16, 2, MODE>(p, plan, st)
                                   : launch_bwd_t<T, 32, 16, 1, MODE>(p, plan, st);

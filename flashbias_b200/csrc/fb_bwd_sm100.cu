@@ -22,13 +22,38 @@ bool bwd_cfg_fits(int D, int RP, int nq) {
   return false;
 }
 
-// The two-stream kernel takes every problem without a mask at head_dim up to 64, except the short items of the persistent
-// form, calls that ask for another form by flag (head_dim 32), and ranks 9 to 16 above head_dim 32, whose accumulators leave
-// no room for dS^T in tensor memory.
-static bool takes_two_stream(const fb_params* p, const PackPlan& plan) {
-  if (plan.TD > 64 || p->mask_kind != FB_MASK_NONE || (plan.TD == 64 && plan.RP > 16)) return false;
-  if (plan.TD == 32 && (p->flags & (plan.RP ? FB_FLAG_BWD_ONE_ITEM : FB_FLAG_BWD_QUERY_MAJOR))) return false;
-  return bwd_sm100_form(p, plan) != FB_KERNEL_BWD_PERSISTENT;
+// Whether the persistent form of the query-major kernel is the better one for a problem with factors at head_dim 32.  What it
+// saves is the start and the drain of a CTA per work item, so: at least two items per SM, and few query tiles per item (mean):
+//  - up to rank 16, up to 20 (persistent / two-stream kernel, us: B256 H24 S256 R16 369 / 805, B1 H50 S1280 R2 80 / 88, S2304
+//    causal 119 / 134, S4096 causal 319 / 336; at 32 tiles, S8192 causal 1182 / 1179; B2 H8 S16384 R5 3058 / 2789);
+//  - above, where it has no staging tile to drain through, up to 4 (B16 H16 S512 R24 99 / 105, S2048 R32 107 / 86);
+//  - with a mask, where the other choice is the one-item form of the same kernel, up to 8.
+static bool bwd_prefers_persistent(const fb_params* p) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int sms = device_sm_count(dev);
+  const int nq = (p->Sq + 127) / 128, nk = (p->Sk + 127) / 128;
+  const int tiles_per_item = p->causal ? (nq + 1) / 2 : nq;  // mean, under causal masking
+  const int most = p->mask_kind != FB_MASK_NONE ? 8 : p->R <= 16 ? 20 : 4;
+  return sms > 0 && tiles_per_item <= most && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
+}
+
+// The kernel (FB_KERNEL_BWD_*) that takes a problem with this plan.
+static int bwd_kernel_for(const fb_params* p, const PackPlan& plan) {
+  const bool factors = plan.RP > 0, by_query = p->flags & (factors ? FB_FLAG_BWD_ONE_ITEM : FB_FLAG_BWD_QUERY_MAJOR);
+  // (the persistent form writes dK and dV with tile stores: their layout must be one a tensor map can describe)
+  if (plan.TD == 32 && factors && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
+      ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p)) &&
+      (!p->dk || tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B)) &&
+      (!p->dv || tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B)))
+    return FB_KERNEL_BWD_PERSISTENT;
+  // Every other problem without a mask at head_dim up to 64, except those that ask for another form by flag (head_dim 32), and ranks
+  // 9 to 16 above head_dim 32, whose accumulators leave no room for dS^T in tensor memory.
+  if (p->mask_kind == FB_MASK_NONE && plan.TD <= 64 && !(plan.TD == 32 && by_query) && !(plan.TD == 64 && plan.RP > 16))
+    return FB_KERNEL_BWD_TWO_STREAM;
+  // without factor operands: key-major where it is built
+  if (!factors && (plan.TD == 128 || (plan.TD == 32 && !by_query))) return FB_KERNEL_BWD_KEY_MAJOR;
+  return FB_KERNEL_BWD_QUERY_MAJOR;
 }
 
 bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
@@ -47,45 +72,18 @@ bool bwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (p->dk && !rows_16b_ok(p->dk, p->dk_stride)) return false;
   if (p->dv && !rows_16b_ok(p->dv, p->dv_stride)) return false;
   if ((int64_t)p->B * p->H * ((p->Sk + 127) / 128) > 0x7fffffffLL) return false;
-  if (takes_two_stream(p, *plan)) plan_two_stream(p, plan);
-  if (plan->two_stream || bwd_sm100_form(p, *plan) != FB_KERNEL_BWD_PERSISTENT) plan->qs_bytes = 0;  // k*scale is split on chip
+  plan->kernel = bwd_kernel_for(p, *plan);
+  if (plan->kernel == FB_KERNEL_BWD_TWO_STREAM) plan_two_stream(p, plan);
+  if (plan->kernel != FB_KERNEL_BWD_PERSISTENT) plan->qs_bytes = 0;  // k*scale is split on chip
   return true;
 }
 
 size_t bwd_sm100_workspace(const fb_params* p, const PackPlan& plan) { return bwd_layout(p, plan).total; }
 
-// Whether the persistent form of the query-major kernel is the better one for a problem with factors at head_dim 32.  What it
-// saves is the start and the drain of a CTA per work item, so: at least two items per SM, and few query tiles per item (mean):
-//  - up to rank 16, up to 20 (persistent / two-stream kernel, us: B256 H24 S256 R16 369 / 805, B1 H50 S1280 R2 80 / 88, S2304
-//    causal 119 / 134, S4096 causal 319 / 336; at 32 tiles, S8192 causal 1182 / 1179; B2 H8 S16384 R5 3058 / 2789);
-//  - above, where it has no staging tile to drain through, up to 4 (B16 H16 S512 R24 99 / 105, S2048 R32 107 / 86);
-//  - with a mask, where the other choice is the one-item form of the same kernel, up to 8.
-static bool bwd_prefers_persistent(const fb_params* p) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const int sms = device_sm_count(dev);
-  const int nq = (p->Sq + 127) / 128, nk = (p->Sk + 127) / 128;
-  const int tiles_per_item = p->causal ? (nq + 1) / 2 : nq;  // mean, under causal masking
-  const int most = p->mask_kind != FB_MASK_NONE ? 8 : p->R <= 16 ? 20 : 4;
-  return sms > 0 && tiles_per_item <= most && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
-}
-
-int bwd_sm100_form(const fb_params* p, const PackPlan& plan) {
-  // without factor operands: key-major where it is built, unless the caller asks for the other form
-  if (plan.RP == 0 && (plan.TD == 128 || (plan.TD == 32 && !(p->flags & FB_FLAG_BWD_QUERY_MAJOR))))
-    return FB_KERNEL_BWD_KEY_MAJOR;
-  // (the persistent form writes dK and dV with tile stores: their layout must be one a tensor map can describe)
-  if (plan.TD == 32 && plan.RP > 0 && !p->alibi_slopes && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
-      ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p)) &&
-      (!p->dk || tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B)) &&
-      (!p->dv || tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B)))
-    return FB_KERNEL_BWD_PERSISTENT;
-  return FB_KERNEL_BWD_QUERY_MAJOR;
-}
-
 int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
-  if (plan.two_stream) return plan.TD == 32 ? dispatch_bwd_s32(p, plan, st) : dispatch_bwd_s64(p, plan, st);
-  if (bwd_sm100_form(p, plan) == FB_KERNEL_BWD_PERSISTENT) return dispatch_bwd_d32p(p, plan, st);
+  if (plan.kernel == FB_KERNEL_BWD_TWO_STREAM)
+    return plan.TD == 32 ? dispatch_bwd_s32(p, plan, st) : dispatch_bwd_s64(p, plan, st);
+  if (plan.kernel == FB_KERNEL_BWD_PERSISTENT) return dispatch_bwd_d32p(p, plan, st);
   switch (plan.TD) {
     case 32: return dispatch_bwd_d32(p, plan, st);
     case 64: return dispatch_bwd_d64(p, plan, st);

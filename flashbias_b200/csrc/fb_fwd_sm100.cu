@@ -32,15 +32,16 @@ bool fwd_sm100_supported(const fb_params* p, PackPlan* plan) {
   if (!o_store_ok(p)) return false;
   if ((int64_t)p->B * p->H * ((p->Sq + 127) / 128) > 0x7fffffffLL) return false;
   if (!plan_pack(p, plan)) return false;
+  plan->kernel = plan->TD == 128 && p->mask_kind == FB_MASK_NONE && plan->RP <= 32 ? FB_KERNEL_FWD_TWO_STREAM : FB_KERNEL_FWD_TILED;
   return fwd_cfg_fits(plan->TD, plan->RP, plan->nq);  // shared or tensor memory of an SM exceeded: generic kernels
 }
 
 int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
+  if (plan.kernel == FB_KERNEL_FWD_TWO_STREAM) return dispatch_fwd_s(p, plan, st);
   switch (plan.TD) {
     case 32: return dispatch_fwd_d32(p, plan, st);
     case 64: return dispatch_fwd_d64(p, plan, st);
-    case 128:
-      return p->mask_kind == FB_MASK_NONE && plan.RP <= 32 ? dispatch_fwd_s(p, plan, st) : dispatch_fwd_d128(p, plan, st);
+    case 128: return dispatch_fwd_d128(p, plan, st);
   }
   return FB_ENOTBUILT;
 }

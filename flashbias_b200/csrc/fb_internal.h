@@ -55,7 +55,7 @@ struct PackPlan {
   int TD;          // head_dim padded to the tile width: 32, 64 or 128 (missing columns are read as zero)
   int RP;          // packed factor width: 0 (no bias), 16, 32 or 64
   int RC;          // width of the centred k-side copy of the backward (>= RP; 32 beside a head_dim-32 K tile)
-  bool two_stream; // backward: the two-stream kernel (its factor tiles are narrower)
+  int kernel;      // FB_KERNEL_* of the tensor-core kernel that takes the problem
   int Bq, Hq, Bk, Hk;
   size_t q_bytes, k_bytes, kc_bytes, qs_bytes;  // packed q factor, packed k factor, centred k factor, scaled-key
                                                // copy (each rounded to 256)
@@ -92,7 +92,6 @@ bool fwd_sm100_supported(const fb_params* p, PackPlan* plan);
 int launch_fwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 
 bool bwd_sm100_supported(const fb_params* p, PackPlan* plan);
-int bwd_sm100_form(const fb_params* p, const PackPlan& plan);  // FB_KERNEL_BWD_*
 size_t bwd_sm100_workspace(const fb_params* p, const PackPlan& plan);
 int launch_bwd_sm100(const fb_params* p, const PackPlan& plan, cudaStream_t st);
 

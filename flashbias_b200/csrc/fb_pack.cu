@@ -30,7 +30,7 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   plan->Bk = p->k_bias_stride[0] == 0 ? 1 : p->B;
   plan->Hk = p->k_bias_stride[1] == 0 ? 1 : p->H;
   plan->TD = p->D <= 32 ? 32 : p->D <= 64 ? 64 : 128;
-  plan->two_stream = false;
+  plan->kernel = FB_KERNEL_GENERAL;
   int e;
   bool pow2 = frexpf(p->softmax_scale, &e) == 0.5f;
   // fp16 factors divided by a scale below one could leave the range of the type: take the split form instead
@@ -67,7 +67,6 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
 }
 
 void plan_two_stream(const fb_params* p, PackPlan* plan) {
-  plan->two_stream = true;
   if (p->R <= 0) return;
   plan->RP = pad_pow2_16(p->R);
   plan->RC = plan->TD == 32 ? 2 * plan->RP : pad_pow2_16(2 * p->R);

@@ -135,12 +135,13 @@ const char *fb_strerror(int code);
  * pointers that are null count as aligned.)
  */
 #define FB_KERNEL_GENERAL 0         /* shape-generic CUDA-core kernels, either direction */
-#define FB_KERNEL_FWD_TILED 1       /* forward, tcgen05: tiles of 128 query rows */
+#define FB_KERNEL_FWD_TILED 1       /* forward, tcgen05: tiles of 128 query rows, one softmax stream */
 #define FB_KERNEL_FWD_ONE_QUERY 2   /* forward, CUDA cores: one query row per (batch, head), split over the keys */
-#define FB_KERNEL_BWD_QUERY_MAJOR 3 /* backward, tcgen05, one work item per CTA: head_dim 33..64, or factor operands.  (Thread
-                                       = query row with a mask or where flags ask for it; the two-stream kernel else.) */
-#define FB_KERNEL_BWD_PERSISTENT 4  /* ... thread = query row, one persistent CTA per SM walking the work items */
-#define FB_KERNEL_BWD_KEY_MAJOR 5   /* backward, tcgen05: key-major, no factor operands, head_dim up to 32 or above 64 */
+#define FB_KERNEL_BWD_QUERY_MAJOR 3 /* backward, tcgen05: thread = query row, one work item per CTA */
+#define FB_KERNEL_BWD_PERSISTENT 4  /* ... one persistent CTA per SM walking the work items */
+#define FB_KERNEL_BWD_KEY_MAJOR 5   /* backward, tcgen05: thread = key, no factor operands */
+#define FB_KERNEL_BWD_TWO_STREAM 6  /* backward, tcgen05: key-major, two streams of half query tiles; no mask */
+#define FB_KERNEL_FWD_TWO_STREAM 7  /* forward, tcgen05: tiles of 128 query rows, two softmax streams; head_dim above 64 */
 int fb_fwd_kernel(const fb_params *p);
 int fb_bwd_kernel(const fb_params *p);
 

@@ -80,15 +80,24 @@ def _problem(D=32, Sq=256, R=0, dtype=_lib.FB_DTYPE_BF16, scale=None, flags=0, s
 
 
 @pytest.mark.parametrize("problem,fwd,bwd", [
-    (dict(R=2), "fwd_tiled", "bwd_query_major"),
+    (dict(R=2), "fwd_tiled", "bwd_two_stream"),
     (dict(R=2, flags=_lib.FB_FLAG_BWD_PERSISTENT), "fwd_tiled", "bwd_persistent"),
     (dict(R=2, flags=_lib.FB_FLAG_BWD_PERSISTENT | _lib.FB_FLAG_BWD_ONE_ITEM), "fwd_tiled", "bwd_query_major"),
-    (dict(slopes=True), "fwd_tiled", "bwd_key_major"),
+    (dict(R=2, mask=True), "fwd_tiled", "bwd_query_major"),
+    (dict(slopes=True), "fwd_tiled", "bwd_two_stream"),
+    (dict(mask=True), "fwd_tiled", "bwd_key_major"),
+    (dict(slopes=True, flags=_lib.FB_FLAG_BWD_QUERY_MAJOR), "fwd_tiled", "bwd_query_major"),
     (dict(mask=True, flags=_lib.FB_FLAG_BWD_QUERY_MAJOR), "fwd_tiled", "bwd_query_major"),
-    (dict(D=64), "fwd_tiled", "bwd_query_major"),
-    (dict(D=72), "fwd_tiled", "bwd_key_major"),
-    (dict(D=128, slopes=True), "fwd_tiled", "bwd_key_major"),
-    (dict(D=128, R=2), "fwd_tiled", "general"),
+    (dict(D=64), "fwd_tiled", "bwd_two_stream"),
+    (dict(D=64, R=8), "fwd_tiled", "bwd_two_stream"),
+    (dict(D=64, R=9, scale=0.125), "fwd_tiled", "bwd_query_major"),
+    (dict(D=64, mask=True), "fwd_tiled", "bwd_query_major"),
+    (dict(D=72), "fwd_two_stream", "bwd_key_major"),
+    (dict(D=128, slopes=True), "fwd_two_stream", "bwd_key_major"),
+    (dict(D=128, mask=True), "fwd_tiled", "bwd_key_major"),
+    (dict(D=128, R=32), "fwd_two_stream", "general"),
+    (dict(D=128, R=33), "fwd_tiled", "general"),
+    (dict(D=128, R=2), "fwd_two_stream", "general"),
     (dict(D=64, R=12, dtype=_lib.FB_DTYPE_F16), "fwd_tiled", "general"),
     (dict(R=40), "fwd_tiled", "general"),
     (dict(R=130), "general", "general"),
@@ -96,9 +105,9 @@ def _problem(D=32, Sq=256, R=0, dtype=_lib.FB_DTYPE_BF16, scale=None, flags=0, s
     (dict(odd=True), "general", "general"),
     (dict(slopes=True, mask=True), "general", "general"),
     (dict(flags=_lib.FB_FLAG_FORCE_GENERAL), "general", "general"),
-    (dict(Sq=1), "fwd_one_query", "bwd_key_major"),
+    (dict(Sq=1), "fwd_one_query", "bwd_two_stream"),
     (dict(Sq=1, slopes=True, mask=True), "fwd_one_query", "general"),
-    (dict(Sq=1, R=17), "fwd_tiled", "bwd_query_major"),
+    (dict(Sq=1, R=17), "fwd_tiled", "bwd_two_stream"),
     (dict(Sq=1, scale=-1.0), "fwd_one_query", "general"),
     (dict(scale=-1.0), "general", "general"),
 ], ids=str)

@@ -8,7 +8,7 @@ import torch
 from flashbias_b200 import check_device_status, flash_bias_alibi_func, flash_bias_func
 from flashbias_b200.flash_bias import flash_bias_backward, flash_bias_forward
 from oracle import flashbias_oracle as orc
-from tests.helpers import check_close
+from tests.helpers import check_close, kernels_taken
 
 pytestmark = pytest.mark.gpu
 BF, HF = torch.bfloat16, torch.float16
@@ -49,6 +49,8 @@ def test_edges(case):
     scale = scale or 1.0 / math.sqrt(D)
     q, k, v, qb, kb, do = _inputs(case)
     leaves = [t.cuda().requires_grad_(True) for t in (q, k, v, qb, kb) if t is not None]
+    slopes = torch.ones(H, device="cuda") if R < 0 else None
+    assert kernels_taken(*(t.detach() for t in leaves), causal=causal, slopes=slopes)[1] == "bwd_two_stream"
     f = [t.float() if t is not None else None for t in (q, k, v, qb, kb)]
     if R < 0:
         m = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)])
@@ -96,6 +98,7 @@ def test_slopes_far_from_the_first_query(D):
                                   (1, 16, 900, 900, 32, 30, False, None, BF, False)], ids=lambda c: "D%dR%d" % (c[4], c[5]))
 def test_repeated_backward_is_bit_identical(case):
     q, k, v, qb, kb, do = (t.cuda() for t in _inputs(case))
+    assert kernels_taken(q, k, v, qb, kb, causal=case[6])[1] == "bwd_two_stream"
     o, lse, sc = flash_bias_forward(q, k, v, qb, kb, None, case[6], case[7])
     want = flash_bias_backward(do, q, k, v, o, qb, kb, lse, None, case[6], sc)
     for _ in range(60):

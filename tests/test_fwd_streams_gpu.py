@@ -8,7 +8,7 @@ import torch
 from flashbias_b200 import check_device_status, flash_bias_alibi_func
 from flashbias_b200.flash_bias import flash_bias_forward
 from oracle import flashbias_oracle as orc
-from tests.helpers import check_close
+from tests.helpers import check_close, kernels_taken
 
 pytestmark = pytest.mark.gpu
 BF, HF = torch.bfloat16, torch.float16
@@ -39,6 +39,7 @@ def test_edges(case):
     if R > 0:
         qb, kb = ((torch.randn(1, S, H, R, generator=g) * 0.5).to(dtype) for S in (Sq, Sk))
     dev = [t.cuda() if t is not None else None for t in (q, k, v, qb, kb)]
+    assert kernels_taken(*dev, causal=causal, slopes=torch.ones(H, device="cuda") if R < 0 else None)[0] == "fwd_two_stream"
     f = [t.float() if t is not None else None for t in (q, k, v, qb, kb)]
     if R < 0:
         m = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)])

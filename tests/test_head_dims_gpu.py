@@ -45,9 +45,9 @@ def test_head_dims(case):
     f = [t.float() for t in (q, k, v)] + [t.float() if t is not None else None for t in (qb, kb)]
     slopes_dev = torch.ones(H, device="cuda") if mode == "slopes" else None
     dev = [t.detach() for t in leaves] + [None] * (5 - len(leaves))
-    bwd = "bwd_key_major" if D > 64 else "bwd_persistent" if B == 40 else "bwd_query_major"
+    bwd = ("bwd_key_major" if D > 64 else "bwd_persistent" if B == 40 else "bwd_query_major" if mode == "mask" else "bwd_two_stream")
     assert kernels_taken(*dev, mask.cuda() if mask is not None else None, causal, 0, slopes_dev) == (
-        "fwd_one_query" if Sq == 1 else "fwd_tiled", bwd)
+        "fwd_one_query" if Sq == 1 else "fwd_two_stream" if D > 64 and mode != "mask" else "fwd_tiled", bwd)
     if mode == "slopes":
         slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / H) for h in range(H)])
         o = flash_bias_alibi_func(*leaves, slopes.cuda(), causal)
