@@ -57,6 +57,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   using Cfg = BwdPCfg<D, RP, NQ>;
   constexpr bool ASYNC = Cfg::ASYNC;
   constexpr int RPX = Cfg::RPX;
+  constexpr bool kPace = masked_pace(MODE, RP);
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   constexpr float kLog2e = 1.4426950408889634f;
 
@@ -163,7 +164,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   };
 
   if (warp == 12) {
-    if (elect_one()) {
+    if (kPace ? lane == 0 : elect_one()) {
       st_shared_flag(abort_flag, 0u);
       mbar_init(kva_full, 1);
       mbar_init(kvb_full, 1);
@@ -218,7 +219,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   setmaxnreg_dec<64>();
   if (warp == 12) {
     // ------------------------------------------------------------------ TMA producer, dQ | dQb chain
-    if (elect_one()) {
+    if (kPace ? lane == 0 : elect_one()) {
       // The same thread issues the dQ | dQb products: they become due when a query tile's P/dS are written,
       // the next load when the other chains have finished with that tile's stage -- in this order, every tile.
       constexpr uint32_t idQD = instr_desc(kBf16, false, true, 128, D);             // dQ: A K-major, B MN-major
@@ -285,7 +286,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     //   warp 13  also dKb when it is a separate accumulator      warp 14  dV
     //   warp 15  dK (or dK | dKb merged)
     // Every accumulator is only ever touched by one thread, which keeps its MMAs ordered.
-    if (elect_one()) {
+    if (kPace ? lane == 0 : elect_one()) {
       const int role = warp - 13;
       constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, 128);  // S, dP: both operands K-major
       constexpr uint32_t idTD = instr_desc(kBf16, true, true, 128, D);     // dV, dK: A^T (MN-major), B MN-major
@@ -425,12 +426,12 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int row = (warp & 3) * 32 + lane;
       const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
       float* s_kbc = reinterpret_cast<float*>(smem + Cfg::OFF_KBC);
-      // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32, laid out [column pair]
-      // [key group][2]: one entry per thread, fetched one item ahead so that the load is not waited for at the item's head
+      // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32: one entry per
+      // thread, fetched one item ahead so that the load is not waited for at the item's head
       float kbc_next = 0.f;
       auto fetch_kbc = [&](const BwdItem& y) {
         const int i = (int)threadIdx.x - 256;
-        const int c = (i >> 3) * 2 + (i & 1), g = (i >> 1) & 3;
+        const int c = kbc_column<!kPace>(i), g = kbc_group<!kPace>(i);
         kbc_next = 0.f;
         if (i < 2 * Cfg::RCX && c < a.R) {
           const T* kb_bh = a.k_bias_t<T>() + (a.bk_bcast ? 0 : y.b) * a.kb_stride[0] + (a.hk_bcast ? 0 : y.h) * a.kb_stride[1];
@@ -513,7 +514,7 @@ bwd_p_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           // accumulator laid out (Bq, Hq, query tiles, R, 128 rows): a tile is contiguous
           float* tileb = a.dqb_acc + (bh % a.dqb_slots) * a.dqb_slot_stride +
                          (((int64_t)bq * a.Hq + hq) * a.nq_tiles + (i_begin + it)) * (128 * a.R);
-          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (tn & 3) * 2048 + row * 4,
+          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED, !kPace>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (tn & 3) * 2048 + row * 4,
                                                    sbase + Cfg::OFF_KBC, sStgB + row * 4, tileb + row, grow < a.Sq, a.R);
         }
         tc_fence_before_sync();

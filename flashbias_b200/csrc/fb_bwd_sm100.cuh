@@ -169,24 +169,43 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+enum { BWD_PLAIN = 0, BWD_MASK = 1, BWD_ALIBI = 2 };
+
+// The query-major kernels with a mask, packed rank up to 32, keep the slower forms of two things: issuers behind `lane == 0`, and a
+// drain of dq_bias column by column.  Their compute threads are bound by the loads of the mask, and whatever the rest of the CTA gets
+// done sooner costs more there.  (Not shown why.  Spilled registers are not it: with fewer it was slower still.  28 KB of L1 are left
+// beside the tiles, and the lines that two warpgroups in step read a chunk of the mask from are 32 KB.)  Backward kernel, us, slow forms / elected issuers / paired drain / both: B1024 H24
+// S256 R16 2848 / 3090 / 2900 / 2962, B128 H24 S512 R8 1346 / 1440 / 1356 / 1413, B64 H2 S2048 R8 955 / 1027 / 964 / 1026, B128 H12
+// S512 D64 R8 944 / 976 / 970 / 1012; at packed rank 64, which drains without a staging tile, B512 H24 S256 R32 2221 / 2174 /
+// 2231 / 2153.
+constexpr __host__ __device__ bool masked_pace(int mode, int rp) { return mode == BWD_MASK && rp <= 32; }
+
+// Where entry i of the table of centre keys belongs: [column pair][key group][2], or for a drain by columns [column][key group].
+template <bool PAIRED>
+__device__ __forceinline__ int kbc_column(int i) { return PAIRED ? (i >> 3) * 2 + (i & 1) : i >> 2; }
+template <bool PAIRED>
+__device__ __forceinline__ int kbc_group(int i) { return PAIRED ? (i >> 1) & 3 : i & 3; }
+
 // dq_bias of one query tile, one thread per query row: dq_bias = dS . k_bias, evaluated per group of 32 keys as
 // dS16 . (k_bias - c) + c * rowsum_fp32(dS) with c the k_bias of the group's middle key (rows of dS sum to ~0, so
 // rounding dS to 16 bits against a large, slowly varying factor -- ALiBi positions -- would otherwise dominate the
 // result).  The accumulator holds dS16 . hi(k_bias - c) in columns [0, R) and dS16 . lo(k_bias - c) in columns
-// [HALF, HALF + R); s_kbc holds c as [column pair][key group][2], s_rowsum the row sums as [key group][128 rows].
+// [HALF, HALF + R); s_kbc holds c as kbc_column and kbc_group say, s_rowsum the row sums as [key group][128 rows].
 // The result goes rank-major ([R][128 rows]) into the staging tile (stg: this thread's row of it): consecutive threads then
 // write consecutive floats.  Eight columns are evaluated at a time, also those beyond the rank: a branch per column
-// serialised the loads of the centre keys and paced the whole kernel (B512 H24 S144 D32 R8: backward kernel 1094 -> 771 us).
+// serialised the loads of the centre keys and paced the whole kernel (B512 H24 S144 D32 R8: backward kernel 1094 -> 703 us).
+// PAIRED false: column by column all the same (masked_pace).
 // Without a staging tile it is added straight to the accumulator in global memory (STAGED false).
-template <int HALF, bool STAGED = true>
+template <int HALF, bool STAGED = true, bool PAIRED = true>
 __device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, uint32_t s_rowsum, uint32_t s_kbc, uint32_t stg,
                                               float* tileb = nullptr, bool row_ok = true, int R = HALF) {
-  constexpr int W = 8;
+  constexpr int W = !PAIRED && HALF >= 16 ? 16 : 8;
+  float rsum1[4];
   uint64_t rsum[4];
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    const float v = __uint_as_float(ld_shared_flag(s_rowsum + g * 512));
-    rsum[g] = f2(v, v);
+    rsum1[g] = __uint_as_float(ld_shared_flag(s_rowsum + g * 512));
+    rsum[g] = f2(rsum1[g], rsum1[g]);
   }
 #pragma unroll 1
   for (int c0 = 0; c0 < HALF && c0 < R; c0 += W) {
@@ -195,6 +214,22 @@ __device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, uint32_t s_rowsum
     tmem_ld(tq_dqb + HALF + c0, rl);
     tmem_wait_ld(rh);
     tmem_wait_ld(rl);
+    if constexpr (!PAIRED) {
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        if (c0 + i < R) {
+          const float4 kc = ld_shared_v4f(s_kbc + (c0 + i) * 16);
+          float v = __uint_as_float(rh[i]) + __uint_as_float(rl[i]);
+          v = fmaf(kc.x, rsum1[0], v);
+          v = fmaf(kc.y, rsum1[1], v);
+          v = fmaf(kc.z, rsum1[2], v);
+          v = fmaf(kc.w, rsum1[3], v);
+          if (STAGED) st_shared_f32(stg + (c0 + i) * 512, v);
+          else if (row_ok) atomicAdd(tileb + (c0 + i) * 128, v);
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < W; i += 2) {
       const float4 x = ld_shared_v4f(s_kbc + (c0 + i) * 16), y = ld_shared_v4f(s_kbc + (c0 + i) * 16 + 16);
@@ -217,7 +252,6 @@ __device__ __forceinline__ void drain_dq_bias(uint32_t tq_dqb, uint32_t s_rowsum
   }
 }
 
-enum { BWD_PLAIN = 0, BWD_MASK = 1, BWD_ALIBI = 2 };
 
 // MODE: how the logits are completed -- as computed (BWD_PLAIN), plus an additive mask tensor (BWD_MASK), plus the
 // fused ALiBi term (BWD_ALIBI).  A kernel parameter rather than a run-time branch: the mask path needs 32 more
@@ -230,6 +264,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmKc, const BwdArgs a) {
   using Cfg = BwdCfg<D, RP, NQ>;
   constexpr int RPX = Cfg::RPX;
+  constexpr bool kPace = masked_pace(MODE, RP);
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   constexpr float kLog2e = 1.4426950408889634f;
 
@@ -327,7 +362,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   setmaxnreg_dec<64>();
   if (warp == 12) {
     // ------------------------------------------------------------------ TMA producer, dQ | dQb chain
-    if (n_it > 0 && elect_one()) {
+    if (n_it > 0 && (kPace ? lane == 0 : elect_one())) {
       // The same thread issues the dQ | dQb products: they become due when a query tile's P/dS are written,
       // the next load when the other chains have finished with that tile's stage -- in this order, every tile.
       constexpr uint32_t idQD = instr_desc(kBf16, false, true, 128, D);             // dQ: A K-major, B MN-major
@@ -381,7 +416,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     //   warp 13  also dKb when it is a separate accumulator      warp 14  dV
     //   warp 15  dK (or dK | dKb merged)
     // Every accumulator is only ever touched by one thread, which keeps its MMAs ordered.
-    if (n_it > 0 && elect_one()) {
+    if (n_it > 0 && (kPace ? lane == 0 : elect_one())) {
       const int role = warp - 13;
       constexpr uint32_t idS = instr_desc(kBf16, false, false, 128, 128);  // S, dP: both operands K-major
       constexpr uint32_t idTD = instr_desc(kBf16, true, true, 128, D);     // dV, dK: A^T (MN-major), B MN-major
@@ -557,7 +592,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           // accumulator laid out (Bq, Hq, query tiles, R, 128 rows): a tile is contiguous
           float* tileb = a.dqb_acc + (bh % a.dqb_slots) * a.dqb_slot_stride +
                          (((int64_t)bq * a.Hq + hq) * a.nq_tiles + (i_begin + it)) * (128 * a.R);
-          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (it & 3) * 2048 + row * 4,
+          drain_dq_bias<Cfg::RCX / 2, Cfg::STAGED, !kPace>(tq + Cfg::T_DQB, sbase + Cfg::OFF_ROWSUM + (it & 3) * 2048 + row * 4,
                                                    sbase + Cfg::OFF_KBC, sStgB + row * 4, tileb + row, grow < a.Sq, a.R);
         }
         tc_fence_before_sync();
@@ -596,8 +631,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // k_bias of the four keys the centred copy refers to (one per 32-key group), as fp32; read by the drain
       // warpgroup, which is ordered after this through the first pds_ready -> dq_full chain
       const T* kb_bh = a.k_bias_t<T>() + (a.bk_bcast ? 0 : b) * a.kb_stride[0] + (a.hk_bcast ? 0 : h) * a.kb_stride[1];
-      for (int i = threadIdx.x; i < 2 * Cfg::RCX; i += 256) {  // [column pair][key group][2]
-        const int c = (i >> 3) * 2 + (i & 1), g = (i >> 1) & 3;
+      for (int i = threadIdx.x; i < 2 * Cfg::RCX; i += 256) {
+        const int c = kbc_column<!kPace>(i), g = kbc_group<!kPace>(i);
         s_kbc[i] = c < a.R ? to_f32(kb_bh[(int64_t)min(k0 + 32 * g + 16, a.Sk - 1) * a.kb_stride[2] + c]) : 0.f;
       }
     }
