@@ -26,15 +26,17 @@ bool bwd_cfg_fits(int D, int RP, int nq) {
 // saves is the start and the drain of a CTA per work item, so: at least two items per SM, and few query tiles per item (mean):
 //  - up to rank 16, up to 20 (persistent / two-stream kernel, us: B256 H24 S256 R16 369 / 805, B1 H50 S1280 R2 80 / 88, S2304
 //    causal 119 / 134, S4096 causal 319 / 336; at 32 tiles, S8192 causal 1182 / 1179; B2 H8 S16384 R5 3058 / 2789);
-//  - above, where it has no staging tile to drain through, up to 4 (B16 H16 S512 R24 99 / 105, S2048 R32 107 / 86);
+//  - above, where it has no staging tile to drain through, up to 4 with a split scale (B16 H16 R17 / R24 / R32, 5 tiles, 148 / 139,
+//    148 / 141, 158 / 154; 8 tiles 334 / 285, 335 / 294, 361 / 325), up to 7 without (5 tiles 128 / 137, 131 / 140, 139 / 154; 6 tiles
+//    178 / 184, 182 / 191, 191 / 208; 8 tiles 287 / 285, 291 / 293, 307 / 323, and causal R32 680 / 667);
 //  - with a mask, where the other choice is the one-item form of the same kernel, up to 8.
-static bool bwd_prefers_persistent(const fb_params* p) {
+static bool bwd_prefers_persistent(const fb_params* p, const PackPlan& plan) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = device_sm_count(dev);
   const int nq = (p->Sq + 127) / 128, nk = (p->Sk + 127) / 128;
   const int tiles_per_item = p->causal ? (nq + 1) / 2 : nq;  // mean, under causal masking
-  const int most = p->mask_kind != FB_MASK_NONE ? 8 : p->R <= 16 ? 20 : 4;
+  const int most = p->mask_kind != FB_MASK_NONE ? 8 : p->R <= 16 ? 20 : plan.nq == 2 ? 4 : 7;
   return sms > 0 && tiles_per_item <= most && (int64_t)nk * p->B * p->H >= 2 * (int64_t)sms;
 }
 
@@ -43,7 +45,7 @@ static int bwd_kernel_for(const fb_params* p, const PackPlan& plan) {
   const bool factors = plan.RP > 0, by_query = p->flags & (factors ? FB_FLAG_BWD_ONE_ITEM : FB_FLAG_BWD_QUERY_MAJOR);
   // (the persistent form writes dK and dV with tile stores: their layout must be one a tensor map can describe)
   if (plan.TD == 32 && factors && !(p->flags & FB_FLAG_BWD_ONE_ITEM) &&
-      ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p)) &&
+      ((p->flags & FB_FLAG_BWD_PERSISTENT) || bwd_prefers_persistent(p, plan)) &&
       (!p->dk || tma_compatible(p->dk, p->dk_stride[2], p->dk_stride[1], p->dk_stride[0], p->H, p->B)) &&
       (!p->dv || tma_compatible(p->dv, p->dv_stride[2], p->dv_stride[1], p->dv_stride[0], p->H, p->B)))
     return FB_KERNEL_BWD_PERSISTENT;
