@@ -1,4 +1,4 @@
-// Backward tensor-core kernels for head_dim 32 (every packed rank that fits, both 16-bit types).
+// Backward tensor-core kernels for head_dim 32 with a mask, or by flag (every packed rank that fits, both 16-bit types).
 #include "fb_bwd_t_sm100.cuh"
 
 namespace fb {
@@ -10,8 +10,6 @@ static int dispatch_rank(const fb_params* p, const PackPlan& plan, cudaStream_t 
       if constexpr (MODE == BWD_MASK)
         if (plan.kernel == FB_KERNEL_BWD_KEY_MAJOR) return launch_bwd_t_t<T, 32, MODE>(p, plan, st);
       return launch_bwd_t<T, 32, 0, 1, MODE>(p, plan, st);
-    case 16: return plan.nq == 2 ? launch_bwd_t<T, 32, 16, 2, MODE>(p, plan, st)
-                                  : launch_bwd_t<T, 32, 16, 1, MODE>(p, plan, st);
     case 32: return plan.nq == 2 ? launch_bwd_t<T, 32, 32, 2, MODE>(p, plan, st)
                                   : launch_bwd_t<T, 32, 32, 1, MODE>(p, plan, st);
     case 64: return plan.nq == 2 ? launch_bwd_t<T, 32, 64, 2, MODE>(p, plan, st)
@@ -22,7 +20,7 @@ static int dispatch_rank(const fb_params* p, const PackPlan& plan, cudaStream_t 
 
 template <typename T>
 static int dispatch_bwd_t(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
-  if (p->alibi_slopes) return dispatch_rank<T, BWD_ALIBI>(p, plan, st);
+  if (p->alibi_slopes) return launch_bwd_t<T, 32, 0, 1, BWD_ALIBI>(p, plan, st);
   if (p->mask_kind != FB_MASK_NONE) return dispatch_rank<T, BWD_MASK>(p, plan, st);
   return dispatch_rank<T, BWD_PLAIN>(p, plan, st);
 }

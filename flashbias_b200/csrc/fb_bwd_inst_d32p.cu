@@ -8,8 +8,6 @@ namespace fb {
 template <typename T, int MODE>
 static int dispatch_rank_p(const fb_params* p, const PackPlan& plan, cudaStream_t st) {
   switch (plan.RP) {
-    case 16: return plan.nq == 2 ? launch_bwd_p<T, 32, 16, 2, MODE>(p, plan, st)
-                                  : launch_bwd_p<T, 32, 16, 1, MODE>(p, plan, st);
     case 32: return plan.nq == 2 ? launch_bwd_p<T, 32, 32, 2, MODE>(p, plan, st)
                                   : launch_bwd_p<T, 32, 32, 1, MODE>(p, plan, st);
     case 64: return plan.nq == 2 ? launch_bwd_p<T, 32, 64, 2, MODE>(p, plan, st)

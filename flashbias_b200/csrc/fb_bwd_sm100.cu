@@ -15,7 +15,7 @@ static bool rows_16b_ok(const void* ptr, const int64_t* st) {
 bool bwd_cfg_fits(int D, int RP, int nq) {
 #define FB_FIT(DD, RR) \
   if (D == DD && RP == RR) return nq == 2 ? BwdCfg<DD, RR, 2>::FITS : BwdCfg<DD, RR, 1>::FITS;
-  FB_FIT(32, 0) FB_FIT(32, 16) FB_FIT(32, 32) FB_FIT(32, 64)
+  FB_FIT(32, 0) FB_FIT(32, 32) FB_FIT(32, 64)
   FB_FIT(64, 0) FB_FIT(64, 16) FB_FIT(64, 32)
 #undef FB_FIT
   if (D == 128 && RP == 0) return true;  // key-major kernel only
