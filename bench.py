@@ -51,7 +51,7 @@ FULL_SIZES = {
 # reduced cases for profiler captures (--profile-case): same kernels, inputs larger than L2, a few hundred MB at most
 PROFILE_SIZES = {
     "generic": dict(B=2, H=4, S=1024, D=32, R=8),
-    "alibi": dict(B=1, H=16, S=4096, D=32),
+    "alibi": dict(B=1, H=16, S=8192, D=32),
     "swin": dict(B=256, H=24, window=16, D=32, R=16),
     "pde": dict(B=1, H=4, S=8192, D=64),
     "pairformer": dict(B=1, H=16, S=1536, D=32, R=32),
@@ -238,6 +238,17 @@ class Timer:
         if kernel_class:
             self.lib.fb_prof_end(C.byref(kms), C.byref(kn))
         return ms, (kms.value / kn.value if kn.value else None), kn.value
+
+
+def bwd_kernel_name(lib, d, causal, scale):
+    """The __global__ function of the backward main kernel that these device tensors take."""
+    from flashbias_b200 import _lib
+    from flashbias_b200.flash_bias import _fill_common
+    p = _lib.FbParams()
+    _fill_common(p, d["q"], d["k"], d["v"], d["q_bias"], d["k_bias"], None, causal, scale, 0)
+    name = _lib.KERNELS[lib.fb_bwd_kernel(C.byref(p))]
+    return {"bwd_query_major": "bwd_sm100_kernel", "bwd_persistent": "bwd_p_sm100_kernel", "bwd_key_major": "bwd_t_sm100_kernel",
+            "bwd_two_stream": "bwd_s_sm100_kernel"}.get(name, name)
 
 
 def rooflines(peaks, fl_b, bytes_b, bwd_kernel_ms):
@@ -522,8 +533,8 @@ def main():
         frac_r0 = sum((s[1] - s[0]) * (s[3] - s[2]) for s in slabs) / (B * H)
         nfac = (w.q_bias.numel() + w.k_bias.numel()) if w.q_bias is not None else 0
         tensor, hbm, hbm_binds = rooflines(peaks, fl_b * frac_r0, bwd_bytes(sh, nfac) * frac_r0, bwd_kernel_ms)
-        # (bwd_sm100_kernel; its persistent form bwd_p_sm100_kernel where a work item has few query tiles)
-        roof = {"bound": "hbm" if hbm_binds else "tensor", "kernel": "bwd_sm100_kernel",
+        roof = {"bound": "hbm" if hbm_binds else "tensor",
+                "kernel": bwd_kernel_name(lib, dev_slabs[0], w.causal, w.softmax_scale),
                 **((hbm if hbm_binds else tensor) or {}), "peak_source": peaks["source"],
                 "ms_per_step_in_kernel": bwd_kernel_ms, "launches_timed": kn, "flop_per_step": fl_b * frac_r0,
                 "bytes_per_step": bwd_bytes(sh, nfac) * frac_r0, "other_roofline": tensor if hbm_binds else hbm,

@@ -10,8 +10,8 @@
 // more barrier (acc_free), and dV, dK and dk_bias leave as staged tiles through the copy engine (BwdPCfg: by which warps).
 //
 // Short sequences are what this form is for (windowed attention: two query tiles per item), where the set-up
-// and drain of a CTA cost more than its tiles; with many query tiles per item the one-item-per-CTA kernel, whose
-// item coordinates are launch constants, runs the tile loop faster and is the one used.
+// and drain of a CTA cost more than its tiles.  With more query tiles per item than bwd_prefers_persistent allows, the
+// two-stream kernel is the faster one, or with a mask the one-item form, whose item coordinates are launch constants.
 #pragma once
 
 #include "fb_bwd_sm100.cuh"

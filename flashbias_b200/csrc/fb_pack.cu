@@ -50,7 +50,8 @@ bool plan_pack(const fb_params* p, PackPlan* plan, bool for_bwd) {
   }
   // the centred k-side copy of the backward holds a (hi, lo) pair: twice the rank
   plan->RP = pad_pow2_16(for_bwd ? 2 * p->R : p->R);
-  // forward at head_dim 32: ranks up to 96 fit two CTAs per SM where 128 packed columns fit one
+  // forward at head_dim 32: 96 packed columns fit two CTAs per SM where 128 fit one, without a mask and with an unsplit scale
+  // (else one either way, with a quarter fewer columns to move and multiply)
   if (!for_bwd && plan->TD == 32 && p->R > 64 && p->R <= 96) plan->RP = 96;
   // backward at head_dim 32: factor tiles as wide as the Q/K tiles, so that [Q | Qb] and [K | Kc] are read as one
   // MMA operand each (one product instead of two per 16 query rows / keys)
