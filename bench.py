@@ -48,7 +48,7 @@ FULL_SIZES = {
     "pde": dict(B=2, H=8, S=32768, D=64),
     "pairformer": dict(B=1, H=16, S=1536, D=32, R=32),
 }
-# reduced cases for profiler captures (--profile-case): same kernels, inputs larger than L2, a few hundred MB at most
+# reduced cases for profiler captures (--profile-case): same kernels, a few hundred MB at most
 PROFILE_SIZES = {
     "generic": dict(B=2, H=4, S=1024, D=32, R=8),
     "alibi": dict(B=1, H=16, S=8192, D=32),
@@ -70,7 +70,7 @@ CPU_SAMPLE = {
 # number of (batch, head, row) units - the tiles a CTA re-streams (Q, dO per key tile) are served by L2 at both
 # sizes, so DRAM traffic grows with the rows, not with the tile pairs
 NCU_BWD_TRAFFIC_BYTES = {
-    "alibi": 47.99e6 * (50 * 8192) / (16 * 4096),
+    "alibi": 74.70e6 * (50 * 8192) / (16 * 8192),
     "swin": 1197.6e6 * 4096 / 256,
     "pde": 27.61e6 * (2 * 8 * 32768) / (4 * 8192),
 }

@@ -141,7 +141,7 @@ __device__ __forceinline__ void tma_tile_bwd(uint32_t dst, const CUtensorMap* m,
 
 // Row `row` of a [128][D] tile, times scale, as a (hi, lo) pair: hi in place, lo in the tile behind; ready for the tensor core.
 // (The persistent form reads k*scale split by a pass ahead of it: short items wait for the split between their tiles, B512 H24
-// S144 R8 996 instead of 701 us, which is more than the pass takes.)
+// S144 R8 996 instead of 703 us, which is more than the pass takes.)
 template <typename T, int D>
 __device__ __forceinline__ void split_scaled_row(uint32_t tile, int row, float scale) {
 #pragma unroll
