@@ -1,5 +1,5 @@
 """The two-stream backward kernel at the edges of its tiles (64-query halves, 128-key tiles), ranks and scale kinds, against the
-CPU checker; and repeated, since a race between its two streams would show as a different gradient."""
+CPU oracle; and repeated, since a race between its two streams would show as a different gradient."""
 import math
 
 import pytest
